@@ -68,3 +68,28 @@ def test_steps_match_the_sequential_sweep(case):
     np.testing.assert_allclose(np.array(res["nrm_m"]), ps[:, 3], rtol=1e-9)
     assert gpu.kernel_launches > 0
     gpu.close()
+
+
+def radial(n):
+    return [{"ne": 1, "Rmax": 0.6 + 0.5 * q if q < n - 1 else 5.0, "Zeff": 2.0 / (q + 1), "fixedW": q % 3 == 2}
+            for q in range(n)]
+
+
+# Interiors of one partial block, a block and one cell, two blocks and one, and whole blocks, of both
+# block edges (16: up to two shells; 8: more shells, and the coarse smoother)
+@pytest.mark.parametrize("mode", ["multigrid", "simultaneous"])
+@pytest.mark.parametrize("n_shells", [1, 2, 3, 8])
+@pytest.mark.parametrize("NN", [8, 10, 18, 34, 48])
+def test_block_edges_match_the_sequential_sweep(NN, n_shells, mode):
+    ref, gpu = pair(("", NN, 6.0, 2, radial(n_shells), 0.1, mode, 1))
+    E4, ps = ref.step()
+    res = gpu.step(1)
+    for m in range(n_shells):
+        g, r = gpu.fields(m), fields_of(ref, m)
+        for k in ("W", "P"):  # no sum enters these in the first step
+            assert np.array_equal(g[k].view(np.uint32), r[k].view(np.uint32)), (m, k)
+        np.testing.assert_allclose(g["U"], r["U"], rtol=2.4e-7, atol=0)  # the scale's last bit, then one rounding
+    for key, v in zip(("E", "E_T", "E_eK", "E_ee"), E4):
+        assert abs(res[key] - v) <= 1e-9 * max(1.0, abs(v)), (key, res[key], v)
+    np.testing.assert_allclose(np.array(res["nrm_m"]), ps[:, 3], rtol=1e-9)
+    gpu.close()
