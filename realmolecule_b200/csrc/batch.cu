@@ -186,14 +186,25 @@ __global__ void __launch_bounds__(256) kb_init(const BInst* __restrict__ ins, co
   nm_init_body<T>((T*)I.U[0], I.lab[0], I.seeds, I.nSeed, I.g, (float)I.h, it.bx, ss);
 }
 
+// force gathers: blocks of points (item: tile bx, by, bz), then one nucleus each (item: entry bx, part by)
 template <typename T>
-__global__ void __launch_bounds__(256) kb_force(const BInst* __restrict__ ins, const BItem* __restrict__ items, int cu,
-                                                double sigma_scale, double* __restrict__ F) {
-  __shared__ double sx[kNmForceTile], sy[kNmForceTile], sz[kNmForceTile], sr[kNmForceTile];
+__global__ void __launch_bounds__(256) kb_gather(const BInst* __restrict__ ins, const BItem* __restrict__ items, int cu,
+                                                 double sigma, double* __restrict__ F) {
+  __shared__ GatherSmem sm;
   const BItem it = items[blockIdx.x];
   const BInst& I = ins[it.inst];
-  nm_force_body<T>((const T*)I.U[cu], I.at, I.nAt, I.g, I.h, sigma_scale > 0 ? sigma_scale : I.h, F + 3 * I.at0, it.bx,
-                   it.by, it.bz, sx, sy, sz, sr);
+  const Geo g = I.g;
+  nm_gather_all_body<T>((const T*)I.U[cu], nullptr, I.at, I.nAt, g, I.h, sigma > 0 ? sigma : I.h, F + 3 * I.at0, it.bx,
+                        it.by, it.bz, sm);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) kb_gather_core(const BInst* __restrict__ ins, const BItem* __restrict__ items,
+                                                      int cu, double sigma, double* __restrict__ F) {
+  const BItem it = items[blockIdx.x];
+  const BInst& I = ins[it.inst];
+  const Geo g = I.g;
+  nm_gather_core_entry<T>((const T*)I.U[cu], nullptr, I.at, it.bx, g, I.h, sigma > 0 ? sigma : I.h, F + 3 * I.at0, it.by);
 }
 
 // Sum over the fine interior of the squared residual 2 pi psi^2 - A P (FP64), added into *out:
@@ -463,7 +474,7 @@ constexpr int kF32 = 0, kF64 = 1;
 struct InstItems {
   std::vector<BItem> march[kMaxLev], rbgs[kMaxLev], restr[kMaxLev], zero[kMaxLev], coarse[kMaxLev], rr[kMaxLev],
       pc[kMaxLev];
-  std::vector<BItem> flat16, flat1, force, one;  // one: a single item (per-instance domain work)
+  std::vector<BItem> flat16, flat1, gather, core, one;  // one: a single item (per-instance domain work)
 };
 
 struct rq_batch {
@@ -486,7 +497,7 @@ struct rq_batch {
   struct Plan { BItem* d = nullptr; int n = 0, cap = 0; };
   struct Plans {
     Plan march[kMaxLev], rbgs[kMaxLev], restr[kMaxLev], zero[kMaxLev], coarse[kMaxLev], rr[kMaxLev], pc[kMaxLev];
-    Plan flat16, flat1, force, one;
+    Plan flat16, flat1, gather, core, one;
   };
   Plans pl[2];
   size_t coarse_smem[kMaxLev] = {};
@@ -561,7 +572,8 @@ static void flat_items(std::vector<BItem>& v, int inst, long long npts, long lon
   for (long long x = 0; x < (npts + per_block - 1) / per_block; ++x) v.push_back({inst, (int)x, 0, 0});
 }
 
-static void make_items(const BInst& I, int q, InstItems& it, NmTile tile, const int* rr_pl, const int* pr_pl) {
+static void make_items(const BInst& I, const std::vector<rq_atom>& atoms, int q, InstItems& it, NmTile tile,
+                       const int* rr_pl, const int* pr_pl) {
   it = InstItems{};
   for (int l = 0; l < I.nlev; ++l) {
     march_items(it.march[l], q, I.lg[l], tile);
@@ -588,10 +600,13 @@ static void make_items(const BInst& I, int q, InstItems& it, NmTile tile, const 
   it.one.push_back({q, 0, 0, 0});
   flat_items(it.flat16, q, I.g.S3, 256 * kNmFlatChunk);
   flat_items(it.flat1, q, I.g.S3, 256);
-  const long long n1 = I.g.NN - 1, ntiles = (n1 * n1 * n1 + kNmForceTile - 1) / kNmForceTile;
-  const int groups = (int)std::min<long long>(ntiles, 32);
-  for (int ch = 0; ch < (I.nAt + 255) / 256; ++ch)
-    for (int t = 0; t < groups; ++t) it.force.push_back({q, t, groups, ch});
+  const dim3 gg = nm_gather_grid(I.g);
+  for (unsigned z = 0; z < gg.z; ++z)
+    for (unsigned y = 0; y < gg.y; ++y)
+      for (unsigned x = 0; x < gg.x; ++x) it.gather.push_back({q, (int)x, (int)y, (int)z});
+  for (int a = 0; a < (int)atoms.size(); ++a)
+    if (atoms[a].Z_nuc > 0)
+      for (int part = 0; part < kGaCoreParts; ++part) it.core.push_back({q, a, part, 0});
 }
 
 // Work lists of each precision set over the active instances (all of them at creation; solve
@@ -624,7 +639,8 @@ static int build_plans(rq_batch* b) {
     BRC(gather(P.flat16, [](const InstItems& it) -> const Items& { return it.flat16; }));
     BRC(gather(P.one, [](const InstItems& it) -> const Items& { return it.one; }));
     BRC(gather(P.flat1, [](const InstItems& it) -> const Items& { return it.flat1; }));
-    BRC(gather(P.force, [](const InstItems& it) -> const Items& { return it.force; }));
+    BRC(gather(P.gather, [](const InstItems& it) -> const Items& { return it.gather; }));
+    BRC(gather(P.core, [](const InstItems& it) -> const Items& { return it.core; }));
   }
   for (auto& g : b->graph)
     if (g) { cudaGraphExecDestroy(g); g = nullptr; }
@@ -738,7 +754,7 @@ static int build(rq_batch* b) {
   }
   b->items.resize(n);
   b_mg_planes(b);
-  for (int q = 0; q < n; ++q) make_items(b->hin[q], q, b->items[q], b->tile, b->rr_pl, b->pr_pl);
+  for (int q = 0; q < n; ++q) make_items(b->hin[q], b->atoms[q], q, b->items[q], b->tile, b->rr_pl, b->pr_pl);
   BRC(build_plans(b));
   size_t smax = 0;
   for (int l = 0; l < b->maxlev; ++l) smax = std::max(smax, b->coarse_smem[l]);
@@ -1392,10 +1408,14 @@ extern "C" int rq_batch_forces(rq_batch* b, double* F) {
   BCK(cudaMemsetAsync(b->dF, 0, sizeof(double) * 3 * b->A, b->st));
   BRC(each_set([&](auto tag, int p) -> int {
     using T = decltype(tag);
-    const rq_batch::Plan& f = b->pl[p].force;
+    const rq_batch::Plan &f = b->pl[p].gather, &core = b->pl[p].core;
     if (!f.n) return RQ_OK;
-    kb_force<T><<<f.n, 256, 0, b->st>>>(b->din, f.d, b->cu, b->cfg.sigma, b->dF);
-    BL("force");
+    kb_gather<T><<<f.n, 256, 0, b->st>>>(b->din, f.d, b->cu, b->cfg.sigma, b->dF);
+    BL("gather");
+    if (core.n) {
+      kb_gather_core<T><<<core.n, 256, 0, b->st>>>(b->din, core.d, b->cu, b->cfg.sigma, b->dF);
+      BL("gather_core");
+    }
     return RQ_OK;
   }));
   BCK(cudaMemcpyAsync(F, b->dF, sizeof(double) * 3 * b->A, cudaMemcpyDeviceToHost, b->st));
@@ -1539,7 +1559,7 @@ static void b_drop_graphs(rq_batch* b) {
 static int b_retile(rq_batch* b, NmTile t) {
   b->tile = t;
   b->cfg.batch_tile = t.lgk | (t.march << 8);
-  for (int q = 0; q < b->n; ++q) make_items(b->hin[q], q, b->items[q], t, b->rr_pl, b->pr_pl);
+  for (int q = 0; q < b->n; ++q) make_items(b->hin[q], b->atoms[q], q, b->items[q], t, b->rr_pl, b->pr_pl);
   return build_plans(b);
 }
 

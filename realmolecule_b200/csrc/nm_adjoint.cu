@@ -18,7 +18,7 @@
 //                lam += 4 pi psi dE/df.
 // The labels are integers and held fixed; the state the window starts from is held fixed (a
 // warm start).  F_a = -dE/dR_a is then the Hellmann-Feynman-shaped gather with the weight dE/dK
-// in place of -h^3 rho (nm_force_body); with no recorded step dE/dK = -h^3 rho and the force is
+// in place of -h^3 rho (nm_gather_points_body); with no recorded step dE/dK = -h^3 rho and the force is
 // the Hellmann-Feynman force, exact at a converged state.  dE/dv = dE/dK.
 //
 // The reference computes forces with the Hellmann-Feynman integral of its own softened nuclei

@@ -26,7 +26,6 @@ template <> struct Ar<double> {
 };
 
 constexpr int kNmFlatChunk = 16;     // points per thread of the flat (all S^3) bodies
-constexpr int kNmForceTile = 512;    // interior points staged per force tile
 constexpr int kNmRowPlanes = 4;      // planes i per block of the row-tiled multigrid bodies
 constexpr int kNmRowTJ = 8;           // rows j per block of the row-tiled bodies (block 32 x 8)
 // Thread coordinates of a body written for a block of W threads along x, from the linear thread
@@ -787,73 +786,190 @@ __device__ __forceinline__ void nm_evolve_body(const int* __restrict__ labIn, in
   }
 }
 
-// Gaussian-nucleus force: tiles t = t0, t0+stride, ... of interior points staged in smem as FP64
-// (x, y, z, weight) whatever the field type, thread = nucleus a of chunk `chunk`.  With gw ==
-// nullptr the Hellmann-Feynman gather F_a = -h^3 sum rho dK/dr (x-R)/r; with a weight field gw =
-// dE/dK (one value per grid point) the gradient gather F_a = -dE/dR_a = sum gw dK_a/dr (x-R)/r,
-// of which the first is the case gw = -h^3 rho.  The per-nucleus factor (weight scale x Z) is
-// applied once, after the sums.
+// Gaussian-nucleus force gathers.  F_a = f sum_x w(x) (dK_a/dr / Z) (x - R)/r over the interior points,
+// with w = rho and f = -h^3 Z (Hellmann-Feynman, gw == nullptr) or w = dE/dK and f = Z (gw given).  The
+// pairs split at the Gaussian range (nm_point_r2): beyond it the nucleus is a point charge, dK/dr = -Z/r^2,
+// and nm_gather_points_body sums them point by point; within it nm_gather_core_body sums the exact terms
+// around each nucleus.  Both form r^2 by the same rounded operations, so every pair is in exactly one.
+//
+// One thread per nucleus over staged points (the form before) let a warp take the erf/exp branch whenever
+// any of its 32 nuclei was close, and left most lanes idle when a grid has few nuclei: 60 ms for the 96
+// clusters (<= 36 nuclei on ~112^3 points each), 2 ms now.  Here a thread owns points and all lanes stay
+// busy; the point-charge pairs are 12 FP64 operations each, which is what bounds the kernel (64 per SM and
+// clock).
+__device__ __forceinline__ double nm_grid_coord(int i, double h) { return __dmul_rn((double)i, h); }
+__device__ __forceinline__ double nm_pair_r2(double dx, double dy, double dz) {
+  return __fma_rn(dx, dx, __fma_rn(dy, dy, __dmul_rn(dz, dz)));
+}
 template <typename T>
-__device__ __forceinline__ void nm_force_body(const T* __restrict__ U, const double* __restrict__ at, int nAt,
-                                              const Geo& g, double h, double sigma, double* __restrict__ F,
-                                              long long t0, long long tstride, int chunk, double* sx, double* sy,
-                                              double* sz, double* sr, const double* __restrict__ gw = nullptr) {
-  const int a = chunk * blockDim.x + threadIdx.x;
-  const bool valid = a < nAt && at[a * 4 + 3] > 0.0;
-  const double Z = valid ? at[a * 4 + 3] : 0.0;
-  const double ax = valid ? at[a * 4 + 0] : 0.0, ay = valid ? at[a * 4 + 1] : 0.0, az = valid ? at[a * 4 + 2] : 0.0;
-  const double inv = 1.0 / (1.4142135623730951 * sigma), gs = 0.7978845608028654 / sigma;
-  const double inv2 = inv * inv, rp2 = nm_point_r2(sigma);
-  const double h3 = h * h * h;
-  const long long n1 = g.NN - 1, nInt = n1 * n1 * n1;
-  const long long ntiles = (nInt + kNmForceTile - 1) / kNmForceTile;
-  double fx = 0, fy = 0, fz = 0;
-  for (long long t = t0; t < ntiles; t += tstride) {
+__device__ __forceinline__ double nm_gather_weight(const T* __restrict__ U, const double* __restrict__ gw, long long id) {
+  if (gw) return gw[id];
+  const double u = (double)U[id];
+  return u * u;
+}
+
+constexpr int kGaK = 32, kGaJ = 8, kGaI = 16;  // points of a block: a 32 x 8 tile of columns, 16 planes each
+constexpr int kGaChunk = 64;                   // nuclei staged at a time
+struct GatherSmem {
+  double pos[kGaChunk][3], fac[kGaChunk];
+  int out[kGaChunk];
+  double x[kGaI];
+  double sum[8][kGaChunk * 3];  // per warp
+  int wc[2];
+};
+
+// Point-charge pairs of the points [i0, i1) x [j0, j1) x [k0, k1) (at most 16 x 8 x 32; block of 256)
+// with the candidates 0 .. nCand - 1: fetch(m, x, y, z, f) gives a candidate's position and factor f and
+// returns its index in F, or -1 for none.  F[3 index + d] += f sum.
+template <typename T, class Fetch>
+__device__ __forceinline__ void nm_gather_points_body(const T* __restrict__ U, const double* __restrict__ gw,
+                                                      const Geo& g, double h, double rp2, int i0, int i1, int j0, int j1,
+                                                      int k0, int k1, int nCand, Fetch fetch, double* __restrict__ F,
+                                                      GatherSmem& sm) {
+  const int tid = (int)(threadIdx.x + blockDim.x * threadIdx.y), lane = tid & 31, warp = tid >> 5;
+  const int j = j0 + warp, k = k0 + lane;
+  const bool col = j < j1 && k < k1;
+  double w[kGaI];
+#pragma unroll
+  for (int p = 0; p < kGaI; ++p)
+    w[p] = (col && i0 + p < i1) ? nm_gather_weight<T>(U, gw, (long long)(i0 + p) * g.S2 + (long long)j * g.S + k) : 0.0;
+  const double y = nm_grid_coord(j, h), z = nm_grid_coord(k, h);
+  if (tid < kGaI) sm.x[tid] = nm_grid_coord(i0 + tid, h);
+  for (int base = 0; base < nCand; base += kGaChunk) {
+    double X = 0, Y = 0, Z = 0, f = 0;
+    int out = -1;
+    if (tid < kGaChunk && base + tid < nCand) out = fetch(base + tid, X, Y, Z, f);
+    const unsigned bal = __ballot_sync(0xffffffffu, out >= 0);
+    if (lane == 0 && warp < 2) sm.wc[warp] = __popc(bal);
     __syncthreads();
-    for (int q = threadIdx.x; q < kNmForceTile; q += blockDim.x) {
-      const long long v = t * kNmForceTile + q;
-      double wt = 0.0, x = 0.0, y = 0.0, z = 0.0;
-      if (v < nInt) {
-        const int i = 1 + (int)(v / (n1 * n1)), j = 1 + (int)((v / n1) % n1), k = 1 + (int)(v % n1);
-        const long long id = (long long)i * g.S2 + (long long)j * g.S + k;
-        if (gw) {
-          wt = gw[id];
-        } else {
-          const double u = (double)U[id];
-          wt = u * u;
-        }
-        x = i * h; y = j * h; z = k * h;
-      }
-      sx[q] = x; sy[q] = y; sz[q] = z; sr[q] = wt;
+    const int nf = sm.wc[0] + sm.wc[1];
+    if (out >= 0) {
+      const int o = (warp ? sm.wc[0] : 0) + __popc(bal & ((1u << lane) - 1u));
+      sm.pos[o][0] = X; sm.pos[o][1] = Y; sm.pos[o][2] = Z;
+      sm.fac[o] = f;
+      sm.out[o] = out;
     }
     __syncthreads();
-    if (valid) {
-      double lx = 0, ly = 0, lz = 0;  // sum weight x (dK/dr / Z) (x - R) / r
-      for (int q = 0; q < kNmForceTile; ++q) {
-        const double s = sr[q];
-        const double dx = sx[q] - ax, dy = sy[q] - ay, dz = sz[q] - az;
-        const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-        double w;
-        if (r2 >= rp2) {  // point charge: dK/dr / r = -Z / r^3
-          const double ir = rsqrt_refined(r2);
-          w = -s * (ir * ir * ir);
-        } else if (r2 < 1e-24) {
-          w = 0.0;
-        } else {
-          const double r = sqrt(r2);
-          w = s * (gs * exp(-r2 * inv2) / r - erf(r * inv) / r2) / r;
-        }
-        lx = fma(w, dx, lx); ly = fma(w, dy, ly); lz = fma(w, dz, lz);
+    for (int m = 0; m < nf; ++m) {
+      const double Xm = sm.pos[m][0], dy = __dsub_rn(y, sm.pos[m][1]), dz = __dsub_rn(z, sm.pos[m][2]);
+      const double c2 = __fma_rn(dy, dy, __dmul_rn(dz, dz));
+      double s = 0.0, sx = 0.0;
+#pragma unroll
+      for (int p = 0; p < kGaI; ++p) {
+        const double dx = __dsub_rn(sm.x[p], Xm);
+        const double r2 = __fma_rn(dx, dx, c2);
+        // r^-3 from the FP32 estimate y0 of r^-1: with e = 1 - r2 y0^2 (y0^2 is exact in FP64) it is
+        // y0^3 (1 - e)^(-3/2) = y0^3 (1 + 3e/2 + 15e^2/8 + O(e^3)), |e| < 2^-20
+        const double y0 = (double)rsqrtf((float)r2);
+        const double y2 = y0 * y0, e = fma(-r2, y2, 1.0), y3 = y2 * y0;
+        const double v = w[p] * fma(y3 * e, fma(1.875, e, 1.5), y3);
+        const double q = r2 >= rp2 ? v : 0.0;
+        s += q;
+        sx = fma(q, dx, sx);
       }
-      fx += lx; fy += ly; fz += lz;
+      double sy = s * dy, sz = s * dz;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        sx += __shfl_xor_sync(0xffffffffu, sx, o);
+        sy += __shfl_xor_sync(0xffffffffu, sy, o);
+        sz += __shfl_xor_sync(0xffffffffu, sz, o);
+      }
+      if (lane == 0) {
+        sm.sum[warp][3 * m] = -sx; sm.sum[warp][3 * m + 1] = -sy; sm.sum[warp][3 * m + 2] = -sz;
+      }
+    }
+    __syncthreads();
+    for (int q = tid; q < 3 * nf; q += 256) {
+      double v = 0.0;
+#pragma unroll
+      for (int x = 0; x < 8; ++x) v += sm.sum[x][q];
+      atomicAdd(&F[3 * sm.out[q / 3] + q % 3], sm.fac[q / 3] * v);
+    }
+    __syncthreads();
+  }
+}
+
+// The exact pairs of one nucleus: the interior points within the Gaussian range of (X, Y, Z), shared by
+// `parts` blocks of 256.  F[d] += f sum.
+template <typename T>
+__device__ __forceinline__ void nm_gather_core_body(const T* __restrict__ U, const double* __restrict__ gw, const Geo& g,
+                                                    double h, double sigma, double X, double Y, double Z, double f,
+                                                    double* __restrict__ F, int part, int parts) {
+  __shared__ double red[8][3];
+  const double rp2 = nm_point_r2(sigma), rp = sqrt(rp2);
+  const double inv = 1.0 / (1.4142135623730951 * sigma), gs = 0.7978845608028654 / sigma, inv2 = inv * inv;
+  int lo[3], n[3];
+  const double R[3] = {X, Y, Z};
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {  // one point of slack on either side; the test below decides
+    lo[d] = (int)fmin(fmax(floor((R[d] - rp) / h) - 1.0, 1.0), (double)g.NN);
+    n[d] = (int)fmin(fmax(ceil((R[d] + rp) / h) + 1.0, 0.0), (double)(g.NN - 1)) - lo[d] + 1;
+  }
+  double sx = 0, sy = 0, sz = 0;
+  if (part == 0 && threadIdx.x == 0) sx = (X - X) + (Y - Y) + (Z - Z);  // NaN for a position that is not finite
+  if (n[0] > 0 && n[1] > 0 && n[2] > 0) {
+    const int tot = n[0] * n[1] * n[2];
+    for (int q = part * 256 + (int)threadIdx.x; q < tot; q += 256 * parts) {
+      const int k = lo[2] + q % n[2], j = lo[1] + (q / n[2]) % n[1], i = lo[0] + q / (n[2] * n[1]);
+      const double dx = __dsub_rn(nm_grid_coord(i, h), X), dy = __dsub_rn(nm_grid_coord(j, h), Y),
+                   dz = __dsub_rn(nm_grid_coord(k, h), Z);
+      const double r2 = nm_pair_r2(dx, dy, dz);
+      if (r2 >= rp2 || r2 < 1e-24) continue;
+      const double r = sqrt(r2);
+      const double v = nm_gather_weight<T>(U, gw, (long long)i * g.S2 + (long long)j * g.S + k) *
+                       (gs * exp(-r2 * inv2) / r - erf(r * inv) / r2) / r;
+      sx = fma(v, dx, sx); sy = fma(v, dy, sy); sz = fma(v, dz, sz);
     }
   }
-  if (valid) {
-    const double f = (gw ? 1.0 : -h3) * Z;  // HF: the staged value is rho, its weight -h^3 rho
-    atomicAdd(&F[a * 3 + 0], f * fx);
-    atomicAdd(&F[a * 3 + 1], f * fy);
-    atomicAdd(&F[a * 3 + 2], f * fz);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sx += __shfl_xor_sync(0xffffffffu, sx, o);
+    sy += __shfl_xor_sync(0xffffffffu, sy, o);
+    sz += __shfl_xor_sync(0xffffffffu, sz, o);
   }
+  if (threadIdx.x % 32 == 0) {
+    red[threadIdx.x / 32][0] = sx; red[threadIdx.x / 32][1] = sy; red[threadIdx.x / 32][2] = sz;
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    double v = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) v += red[w][threadIdx.x];
+    atomicAdd(&F[threadIdx.x], f * v);
+  }
+}
+constexpr int kGaCoreParts = 4;  // blocks per nucleus of the core gather (19^3 points at sigma = h)
+
+// The two gathers over all entries of one grid (at: x, y, z, Z_nuc per entry; Z_nuc <= 0: no nucleus)
+template <typename T>
+__device__ __forceinline__ void nm_gather_all_body(const T* __restrict__ U, const double* __restrict__ gw,
+                                                   const double* __restrict__ at, int nAt, const Geo& g, double h,
+                                                   double sigma, double* __restrict__ F, int bx, int by, int bz,
+                                                   GatherSmem& sm) {
+  const double scale = gw ? 1.0 : -(h * h * h);
+  const int i0 = 1 + bz * kGaI, j0 = 1 + by * kGaJ, k0 = 1 + bx * kGaK;
+  nm_gather_points_body<T>(U, gw, g, h, nm_point_r2(sigma), i0, min(i0 + kGaI, g.NN), j0, min(j0 + kGaJ, g.NN), k0,
+                           min(k0 + kGaK, g.NN), nAt,
+                           [&](int m, double& X, double& Y, double& Z, double& f) -> int {
+                             const double q = at[m * 4 + 3];
+                             X = at[m * 4]; Y = at[m * 4 + 1]; Z = at[m * 4 + 2];
+                             f = scale * q;
+                             return q > 0.0 ? m : -1;
+                           },
+                           F, sm);
+}
+template <typename T>
+__device__ __forceinline__ void nm_gather_core_entry(const T* __restrict__ U, const double* __restrict__ gw,
+                                                     const double* __restrict__ at, int a, const Geo& g, double h,
+                                                     double sigma, double* __restrict__ F, int part) {
+  const double q = at[a * 4 + 3];
+  if (!(q > 0.0)) return;  // uniform per block
+  nm_gather_core_body<T>(U, gw, g, h, sigma, at[a * 4], at[a * 4 + 1], at[a * 4 + 2], (gw ? 1.0 : -(h * h * h)) * q,
+                         F + 3 * a, part, kGaCoreParts);
+}
+inline dim3 nm_gather_grid(const Geo& g) {
+  const unsigned n = (unsigned)(g.NN - 1);
+  return dim3((n + kGaK - 1) / kGaK, (n + kGaJ - 1) / kGaJ, (n + kGaI - 1) / kGaI);
 }
 
 }  // namespace rq

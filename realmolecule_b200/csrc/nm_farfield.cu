@@ -26,6 +26,7 @@ namespace rq {
 constexpr int kFfT = 32;                     // tile points per axis (at most)
 constexpr int kFfN = 16;                     // Chebyshev nodes per axis
 constexpr int kFfN3 = kFfN * kFfN * kFfN;
+static_assert(kFfT == 2 * kGaI && kFfT == kGaK, "the near gather's blocks cover a tile");
 constexpr double kFfFar = 3.0;               // near: distance to the tile box below 3 half-widths
 constexpr int kFfTabM = kFfT + 1;            // Lagrange tables for tile sizes m = 0..32
 // tabs layout: tau[16] (nodes on [-1, 1]), then L[m][p][q] = l_q(t_p), t_p = -1 + 2p/(m-1)
@@ -282,14 +283,6 @@ __global__ void __launch_bounds__(256) k_ff_near_potential(FfGeo f, const double
   }
 }
 
-// The weight of a grid point in a force gather: gw (dE/dK) when given, else the density u^2.
-template <typename T>
-__device__ __forceinline__ double ff_weight(const T* __restrict__ U, const double* __restrict__ gw, long long id) {
-  if (gw) return gw[id];
-  const double u = (double)U[id];
-  return u * u;
-}
-
 // Anterpolation: W[t][qa][qb][qc] = sum over the tile's points of w(x) Lx[p][qa] Ly[j][qb] Lz[k][qc],
 // plane by plane (z, then y, then x).  One block of 256 threads per tile; thread (qb, qc) keeps
 // the 16 sums over qa in registers.
@@ -316,7 +309,7 @@ __global__ void __launch_bounds__(256) k_ff_anterp(FfGeo f, const double* __rest
     __syncthreads();
     for (int q = threadIdx.x; q < kFfT * kFfT; q += blockDim.x) {
       const int j = q / kFfT, k = q % kFfT;
-      w[q] = (j < mj && k < mk) ? ff_weight<T>(U, gw, ip + (long long)(b.s[1] + j) * g.S + (b.s[2] + k)) : 0.0;
+      w[q] = (j < mj && k < mk) ? nm_gather_weight<T>(U, gw, ip + (long long)(b.s[1] + j) * g.S + (b.s[2] + k)) : 0.0;
     }
     __syncthreads();
     for (int q = threadIdx.x; q < kFfT * kFfN; q += blockDim.x) {
@@ -392,65 +385,42 @@ __global__ void __launch_bounds__(128) k_ff_force_far(FfGeo f, int nTiles, int t
   }
 }
 
-// Near force: thread = one of 64 near nuclei of a tile (chunk blockIdx.y of its near list); the
-// tile's points are staged 256 at a time as FP64 (x, y, z, weight).  Exact Gaussian-nucleus
-// terms, as the direct gather.
+// Near force, point-charge pairs: 8 blocks per tile, each 32 x 8 columns of 16 planes, over the tile's
+// near list (nm_gather_points_body).  One thread per nucleus over staged points (before) took 10.4 ms for 100
+// waters on 192^3, the erf/exp branch entered by almost every warp; the evaluation there went from 96.8
+// to 87.6 ms.
 template <typename T>
-__global__ void __launch_bounds__(64) k_ff_force_near(FfGeo f, const double* __restrict__ nuc, int nNuc,
-                                                      const int* __restrict__ near_idx,
-                                                      const int* __restrict__ near_cnt, const T* __restrict__ U,
-                                                      const double* __restrict__ gw, double sigma,
-                                                      double* __restrict__ Fraw, Geo g) {
-  __shared__ double sx[256], sy[256], sz[256], sw[256];
+__global__ void __launch_bounds__(256) k_ff_force_near(FfGeo f, const double* __restrict__ nuc, int nNuc,
+                                                       const int* __restrict__ near_idx,
+                                                       const int* __restrict__ near_cnt, const T* __restrict__ U,
+                                                       const double* __restrict__ gw, double sigma,
+                                                       double* __restrict__ Fraw, Geo g) {
+  __shared__ GatherSmem sm;
   const int t = blockIdx.x;
-  const int cnt = near_cnt[t];
-  if (blockIdx.y * 64 >= cnt) return;  // uniform per block
   const FfBox b = ff_box(f, t);
-  const int slot = blockIdx.y * 64 + threadIdx.x;
-  const bool valid = slot < cnt;
-  const int n = valid ? near_idx[(long long)t * nNuc + slot] : 0;
-  const double X = valid ? nuc[n * 4] : 0.0, Y = valid ? nuc[n * 4 + 1] : 0.0, Z = valid ? nuc[n * 4 + 2] : 0.0;
-  const double inv = 1.0 / (1.4142135623730951 * sigma), gs = 0.7978845608028654 / sigma;
-  const double inv2 = inv * inv, rp2 = nm_point_r2(sigma);
-  const int mj = b.m[1], mk = b.m[2];
-  const long long npts = (long long)b.m[0] * mj * mk;
-  double fx = 0.0, fy = 0.0, fz = 0.0;
-  for (long long base = 0; base < npts; base += 256) {
-    const int nb = (int)min(256LL, npts - base);
-    __syncthreads();
-    for (int q = threadIdx.x; q < nb; q += blockDim.x) {
-      const long long v = base + q;
-      const int p = (int)(v / (mj * mk)), j = (int)((v / mk) % mj), k = (int)(v % mk);
-      const int i = b.s[0] + p, jg = b.s[1] + j, kg = b.s[2] + k;
-      sx[q] = i * f.h; sy[q] = jg * f.h; sz[q] = kg * f.h;
-      sw[q] = ff_weight<T>(U, gw, (long long)i * g.S2 + (long long)jg * g.S + kg);
-    }
-    __syncthreads();
-    if (!valid) continue;
-    double lx = 0.0, ly = 0.0, lz = 0.0;
-    for (int q = 0; q < nb; ++q) {
-      const double s = sw[q];
-      const double dx = sx[q] - X, dy = sy[q] - Y, dz = sz[q] - Z;
-      const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-      double w;
-      if (r2 >= rp2) {
-        const double ir = rsqrt_refined(r2);
-        w = -s * (ir * ir * ir);
-      } else if (r2 < 1e-24) {
-        w = 0.0;
-      } else {
-        const double r = sqrt(r2);
-        w = s * (gs * exp(-r2 * inv2) / r - erf(r * inv) / r2) / r;
-      }
-      lx = fma(w, dx, lx); ly = fma(w, dy, ly); lz = fma(w, dz, lz);
-    }
-    fx += lx; fy += ly; fz += lz;
-  }
-  if (valid) {
-    atomicAdd(&Fraw[n * 3 + 0], fx);
-    atomicAdd(&Fraw[n * 3 + 1], fy);
-    atomicAdd(&Fraw[n * 3 + 2], fz);
-  }
+  const int i0 = b.s[0] + kGaI * (blockIdx.y & 1), j0 = b.s[1] + kGaJ * (blockIdx.y >> 1);
+  const int i1 = min(i0 + kGaI, b.s[0] + b.m[0]), j1 = min(j0 + kGaJ, b.s[1] + b.m[1]);
+  if (i0 >= i1 || j0 >= j1) return;  // uniform per block
+  const int* lst = near_idx + (long long)t * nNuc;
+  nm_gather_points_body<T>(U, gw, g, f.h, nm_point_r2(sigma), i0, i1, j0, j1, b.s[2], b.s[2] + b.m[2], near_cnt[t],
+                           [&](int m, double& X, double& Y, double& Z, double& fac) -> int {
+                             const int n = lst[m];
+                             X = nuc[n * 4]; Y = nuc[n * 4 + 1]; Z = nuc[n * 4 + 2];
+                             fac = 1.0;
+                             return n;
+                           },
+                           Fraw, sm);
+}
+
+// Near force, the pairs within the Gaussian range.  A nucleus' range reaches only tiles it is near
+// (ff_wanted), so these are pairs of the near lists, around each nucleus once.
+template <typename T>
+__global__ void __launch_bounds__(256) k_ff_force_core(const double* __restrict__ nuc, const T* __restrict__ U,
+                                                       const double* __restrict__ gw, double h, double sigma,
+                                                       double* __restrict__ Fraw, Geo g) {
+  const int n = blockIdx.x;
+  nm_gather_core_body<T>(U, gw, g, h, sigma, nuc[n * 4], nuc[n * 4 + 1], nuc[n * 4 + 2], 1.0, Fraw + 3 * n, blockIdx.y,
+                         kGaCoreParts);
 }
 
 // F[entry] += (weight scale x Z) Fraw[nucleus]: weight scale 1 for a dE/dK field, -h^3 for rho.
@@ -621,10 +591,12 @@ static int gather_t(rq_ctx* c, const T* U, const double* gw) {
   LAUNCH(RQ_KC_FORCES, 8.0 * kFfN3 * F.nTiles,
          (k_ff_force_far<<<gfar, 128, 0, c->st>>>(f, F.nTiles, tpb, F.tabs, F.nuc, F.nNuc, F.nodes, F.Fraw),
           cudaGetLastError()));
-  const dim3 gnear(F.nTiles, (F.nNuc + 63) / 64);
   LAUNCH(RQ_KC_FORCES, (gw ? 8.0 : sizeof(T)) * ni,
-         (k_ff_force_near<T><<<gnear, 64, 0, c->st>>>(f, F.nuc, F.nNuc, F.near_idx, F.near_cnt, U, gw, c->sigma,
-                                                      F.Fraw, g),
+         (k_ff_force_near<T><<<dim3(F.nTiles, 2 * kFfT / kGaJ), 256, 0, c->st>>>(f, F.nuc, F.nNuc, F.near_idx, F.near_cnt,
+                                                                                 U, gw, c->sigma, F.Fraw, g),
+          cudaGetLastError()));
+  LAUNCH(RQ_KC_FORCES, 32.0 * F.nNuc,
+         (k_ff_force_core<T><<<dim3(F.nNuc, kGaCoreParts), 256, 0, c->st>>>(F.nuc, U, gw, c->h, c->sigma, F.Fraw, g),
           cudaGetLastError()));
   LAUNCH(RQ_KC_FORCES, 48.0 * F.nNuc,
          (k_ff_force_finish<<<(F.nNuc + 127) / 128, 128, 0, c->st>>>(F.nuc, F.entry, F.nNuc, F.Fraw,

@@ -117,10 +117,16 @@ __global__ void __launch_bounds__(256) k_nm_evolve(const int* labIn, int* labOut
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_nm_force(const T* U, const double* at, int nAt, Geo g, double h, double sigma,
-                                                  double* F, const double* gw) {
-  __shared__ double sx[kNmForceTile], sy[kNmForceTile], sz[kNmForceTile], sr[kNmForceTile];
-  nm_force_body<T>(U, at, nAt, g, h, sigma, F, blockIdx.x, gridDim.x, blockIdx.y, sx, sy, sz, sr, gw);
+__global__ void __launch_bounds__(256) k_nm_gather(const T* U, const double* at, int nAt, Geo g, double h, double sigma,
+                                                   double* F, const double* gw) {
+  __shared__ GatherSmem sm;
+  nm_gather_all_body<T>(U, gw, at, nAt, g, h, sigma, F, blockIdx.x, blockIdx.y, blockIdx.z, sm);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_nm_gather_core(const T* U, const double* at, Geo g, double h, double sigma,
+                                                        double* F, const double* gw) {
+  nm_gather_core_entry<T>(U, gw, at, blockIdx.x, g, h, sigma, F, blockIdx.y);
 }
 
 template <typename T>
@@ -253,13 +259,8 @@ template <typename T>
 cudaError_t nm_force(const T* U, const double* at, int nAt, const Geo& g, double h, double sigma, double* F,
                      cudaStream_t st, const double* gw) {
   if (g.NN < 2 || nAt <= 0) return cudaSuccess;
-  const long long n1 = g.NN - 1, nInt = n1 * n1 * n1;
-  const long long ntiles = (nInt + kNmForceTile - 1) / kNmForceTile;
-  const int chunks = (nAt + 255) / 256;
-  long long bx = 148 * 8 / chunks;
-  if (bx < 1) bx = 1;
-  if (bx > ntiles) bx = ntiles;
-  k_nm_force<T><<<dim3((unsigned)bx, (unsigned)chunks), 256, 0, st>>>(U, at, nAt, g, h, sigma, F, gw);
+  k_nm_gather<T><<<nm_gather_grid(g), 256, 0, st>>>(U, at, nAt, g, h, sigma, F, gw);
+  k_nm_gather_core<T><<<dim3((unsigned)nAt, kGaCoreParts), 256, 0, st>>>(U, at, g, h, sigma, F, gw);
   return cudaGetLastError();
 }
 template <typename T>

@@ -128,3 +128,39 @@ def test_tiled_adjoint_matches_direct(precision):
     (F0, d0), (F1, d1) = out
     assert np.abs(F1 - F0).max() <= 1e-10 * np.abs(F0).max()
     assert np.abs(d1 - d0).max() <= 1e-12 * np.abs(d0).max()
+
+
+# Force gathers at the edges of their point tiles (32 x 8 columns of 16 planes), direct and tiled, with
+# nuclei on a grid point, between points, at a face and outside the box, sigma wider than the tile's
+# planes among them.  Bar: FP64 sums of n^3 terms, 1e-11 of the largest force.
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("nuclear_sum", [1, 2])
+@pytest.mark.parametrize("NN,sigma_h", [(16, 1.0), (18, 2.5), (32, 1.0), (36, 1.0), (64, 1.0), (68, 1.3)])
+def test_force_gather_edges(NN, sigma_h, nuclear_sum, precision):
+    from math import pi, sqrt
+    from scipy.special import erf
+    from realmolecule_b200 import Context
+    h = 0.25
+    c = NN / 2
+    nuc = [(c, c, c, 8.0), (c + 3.3, c - 2.7, c + 0.4, 1.0), (1.2, c, NN - 0.6, 6.0), (c - 4.0, 2.0, c, 1.0),
+           (-3.0, c + 1.5, c, 1.0)]
+    rows = [{"i": x, "j": y, "k": z, "Z": 0.0, "Z_nuc": q} for x, y, z, q in nuc]
+    rows += [{"i": c + d, "j": c - d, "k": c, "Z": 1.0, "Z_nuc": 0.0} for d in (-2.0, 2.0)]
+    ctx = Context(NN, NN * h, rows, flavor="new", precision=precision, sigma=sigma_h * h, nuclear_sum=nuclear_sum)
+    ctx.initialize()
+    F = ctx.forces()
+    rho = ctx.download(psi=True, label=False)["psi"].astype(np.float64).reshape((NN + 1,) * 3) ** 2
+    ctx.close()
+    x = np.arange(NN + 1) * h
+    s = sigma_h * h
+    ref = np.zeros_like(F)
+    for a, (X, Y, Z, q) in enumerate(nuc):
+        d = (x[:, None, None] - X * h, x[None, :, None] - Y * h, x[None, None, :] - Z * h)
+        r = np.sqrt(d[0] ** 2 + d[1] ** 2 + d[2] ** 2)
+        r[r < 1e-12] = np.inf  # no force from the nucleus' own point
+        w = -h ** 3 * q * rho * (sqrt(2 / pi) / s * np.exp(-r * r / (2 * s * s)) / r - erf(r / (sqrt(2) * s)) / r ** 2) / r
+        w[0] = w[-1] = 0
+        w[:, 0] = w[:, -1] = 0
+        w[:, :, 0] = w[:, :, -1] = 0
+        ref[a] = [(w * t).sum() for t in d]
+    assert np.abs(F - ref).max() <= 1e-11 * np.abs(ref).max()
