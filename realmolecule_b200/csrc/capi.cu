@@ -192,6 +192,7 @@ static int alloc_all(rq_ctx* c) {
   }
   DALLOC(c->atoms5, sizeof(float) * 5 * n);
   DALLOC(c->scratch_atoms5, sizeof(float) * 5 * n);
+  if (c->cfg.flavor == RQ_FLAVOR_SOLVER_PY) DALLOC(c->nbm, S3);
   if (c->cfg.flavor == RQ_FLAVOR_SOLVER_PY) {  // bins of ~1 atom each, at most 64 per axis
     const int S = c->g.S;
     int bin = (int)std::lround(std::cbrt((double)c->g.S3 / std::max(1, n)));
@@ -350,9 +351,9 @@ static int sp_step_one(rq_ctx* c, int s) {
   if (norm) CK(cudaMemsetAsync(c->dnorm, 0, sizeof(double) * c->n_atoms, c->st));
   double* nrm = norm ? c->dnorm : nullptr;
   auto fused = [&](bool first) -> int {
-    LAUNCH(RQ_KC_UPDATE, 24 * interior_points(c->g),
+    LAUNCH(RQ_KC_UPDATE, (nrm ? 25 : 21) * interior_points(c->g),
            launch_step_sp(first, (float*)c->U[c->cu], (float*)c->U[1 - c->cu], (float*)c->K, (float*)c->P[c->cp],
-                          (float*)c->P[1 - c->cp], c->lab[c->cl], c->g, (float)c->half_dv, (float)c->dt,
+                          (float*)c->P[1 - c->cp], c->nbm, c->lab[c->cl], c->g, (float)c->half_dv, (float)c->dt,
                           (float)c->h2, coeff, c->h3, c->n_atoms, nrm, c->st));
     c->cu ^= 1;
     return RQ_OK;
@@ -396,10 +397,12 @@ static int sp_step_one(rq_ctx* c, int s) {
                               (float)c->h2, c->st));
     else
       LAUNCH(RQ_KC_LABELS, 8 * interior_points(c->g),
-             launch_labels_binned_sp(c->lab[c->cl], c->lab[1 - c->cl], c->atoms5, c->n_atoms,
+             launch_labels_binned_sp(c->lab[c->cl], c->lab[1 - c->cl], c->nbm, (unsigned*)c->bestU,
+                                     (unsigned*)(c->err + 3), c->atoms5, c->n_atoms,
                                      AtomBins{c->bins_nb, c->bins_bin, c->bin_start, c->bin_idx, c->bin_far, c->bin_zmax},
                                      c->g, (float)c->h, (float)c->h2, c->st));
     c->cl ^= 1;
+    if ((rc = nm_label_mask(c)) != RQ_OK) return rc;
   }
   return RQ_OK;
 }
@@ -414,8 +417,9 @@ static int sp_initialize(rq_ctx* c) {
          launch_init_sp((float*)c->U[0], c->lab[0], (float*)c->K, c->bestU, c->atoms5, c->n_atoms, c->g, (float)c->h,
                         (float)c->h2, true, c->st));
   CK(cudaMemcpyAsync(c->lab[1], c->lab[0], sizeof(int) * c->g.S3, cudaMemcpyDeviceToDevice, c->st));
-  int rc = sp_normalize(c, true);
+  int rc = nm_label_mask(c);
   if (rc != RQ_OK) return rc;
+  if ((rc = sp_normalize(c, true)) != RQ_OK) return rc;
   for (int q = 0; q < 100; ++q)
     if ((rc = sp_poisson(c)) != RQ_OK) return rc;
   return RQ_OK;
@@ -631,8 +635,7 @@ static int upload_labels(rq_ctx* c, const int32_t* label) {
   }
   c->cl ^= 1;
   CK(cudaMemcpyAsync(c->lab[1 - c->cl], c->lab[c->cl], n * sizeof(int), cudaMemcpyDeviceToDevice, c->st));
-  if (c->cfg.flavor == RQ_FLAVOR_NEW) return nm_label_mask(c);
-  return RQ_OK;
+  return nm_label_mask(c);
 }
 
 extern "C" int rq_upload_state(rq_ctx* c, const float* psi, const int32_t* label, const float* W, const float* P) {

@@ -189,32 +189,7 @@ __device__ __forceinline__ float sr_round(double v, unsigned u24) {
 // scale[label] * update(psi), formed in FP64 and rounded once -- normalise-then-update up to
 // rounding, without a separate pass over psi.  With a non-null `seed` (fp32 fields) the stored
 // value is rounded without bias (sr_round) from its exact FP64 form.
-// Same-label neighbour mask of one interior point: bit q set when neighbour q (+i, -i, +j, -j,
-// +k, -k) carries the point's label.  The update reads it in place of the six neighbour labels
-// while the labels do not change (nm_mask_body writes it after every label change).
-constexpr int kNmIp = 1, kNmIm = 2, kNmJp = 4, kNmJm = 8, kNmKp = 16, kNmKm = 32;
-__device__ __forceinline__ unsigned char nm_same_label_mask(const int* __restrict__ label, long long id, long long S,
-                                                            long long S2) {
-  const int l = label[id];
-  return (unsigned char)((label[id + S2] == l ? kNmIp : 0) | (label[id - S2] == l ? kNmIm : 0) |
-                         (label[id + S] == l ? kNmJp : 0) | (label[id - S] == l ? kNmJm : 0) |
-                         (label[id + 1] == l ? kNmKp : 0) | (label[id - 1] == l ? kNmKm : 0));
-}
-
-// The mask of every point of S^3 (0 on the boundary planes), flat: 256 * kNmFlatChunk points from blk.
-__device__ __forceinline__ void nm_mask_body(const int* __restrict__ label, unsigned char* __restrict__ mask,
-                                             const Geo& g, long long blk) {
-  const long long base = blk * blockDim.x * kNmFlatChunk;
-  for (int q = 0; q < kNmFlatChunk; ++q) {
-    const long long id = base + (long long)q * blockDim.x + threadIdx.x;
-    if (id >= g.S3) break;
-    const int i = (int)(id / g.S2), j = (int)((id / g.S) % g.S), k = (int)(id % g.S);
-    const bool interior = i >= 1 && i < g.NN && j >= 1 && j < g.NN && k >= 1 && k < g.NN;
-    mask[id] = interior ? nm_same_label_mask(label, id, g.S, g.S2) : (unsigned char)0;
-  }
-}
-
-// MASK: neighbour-label equality from `mask` (nm_mask_body of the same labels) instead of six label
+// MASK: neighbour-label equality from `mask` (nm_mask of the same labels) instead of six label
 // loads; the centre label is then read only where it is used (norm accumulation, pending scale).
 // The arithmetic is the same, so both forms give the same bits.
 // SR: the unbiased rounding of fp32 fields (seed non-null), compiled only where it is asked for

@@ -34,7 +34,7 @@ size_t esize(const rq_ctx* c) { return c->fp64 ? sizeof(double) : sizeof(float);
 // the same-label neighbour mask of the current labels (read by the update)
 int nm_label_mask(rq_ctx* c) {
   if (!c->nbm) return RQ_OK;
-  LAUNCH(RQ_KC_LABELS, 25.0 * c->g.S3, nm_mask(c->lab[c->cl], c->nbm, c->g, c->st));
+  LAUNCH(RQ_KC_LABELS, 5.0 * c->g.S3, nm_mask(c->lab[c->cl], c->nbm, c->g, c->st));
   return RQ_OK;
 }
 
@@ -74,6 +74,7 @@ int nm_alloc_levels(rq_ctx* c) {
       cudaMalloc((void**)&c->nbm, (size_t)c->g.S3) != cudaSuccess)
     return rq_cuda(c, cudaErrorMemoryAllocation, "seed table");
   cudaMemsetAsync(c->rseed, 0, sizeof(unsigned) * 2, c->st);
+  cudaMemsetAsync(c->nbm, 0, (size_t)c->g.S3, c->st);  // the face points' masks stay 0
   if (!c->fp64 && cudaMalloc((void**)&c->K64, sizeof(double) * (size_t)c->g.S3) != cudaSuccess)
     return rq_cuda(c, cudaErrorMemoryAllocation, "FP64 potential of the readout");
   return RQ_OK;

@@ -7,6 +7,7 @@
 
 #include "nm_bodies.cuh"
 #include "rq_kernels.h"
+#include "vec_stencil.cuh"
 
 namespace rq {
 
@@ -23,13 +24,29 @@ __global__ void __launch_bounds__(256) k_nm_init(T* U, int* label, const float4*
   nm_init_body<T>(U, label, seeds, nSeed, g, h, blockIdx.x, ss);
 }
 
+// Same-label neighbour mask of the interior points (kNmIp ..): the updates read it in place of six
+// neighbour labels while the labels do not change.  The face bytes are 0 from the allocation.
+template <bool S1>
+__global__ void __launch_bounds__(256) k_nm_mask(const int* __restrict__ label, unsigned char* __restrict__ mask, Geo g) {
+  const int i = 1 + (int)blockIdx.y;
+  const VGroup r = vgroup<int>(g, i, (int)blockIdx.x);
+  const Star<int> l = vstar(VLoad<int, S1>(label, r, g));
+  if (!r.own) return;
+  const VRow row = vrow(g, r, i);
+  unsigned m4 = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int c = l.c.v[e];
+    const unsigned m = (l.ip.v[e] == c ? kNmIp : 0) | (l.im.v[e] == c ? kNmIm : 0) | (l.jp.v[e] == c ? kNmJp : 0) |
+                       (l.jm.v[e] == c ? kNmJm : 0) | (l.kp.v[e] == c ? kNmKp : 0) | (l.km.v[e] == c ? kNmKm : 0) | kNmIn;
+    if (vinterior(g, row, e)) m4 |= m << (8 * e);
+  }
+  *reinterpret_cast<unsigned*>(mask + r.a) = m4;
+}
+
 // seed[0]: the step seed of the unbiased fp32 rounding (null: round to nearest); the next step's
 // seed, seed[0] + 1, goes to seed_next (read and written in different words, so every block reads
 // the same value)
-__global__ void __launch_bounds__(256) k_nm_mask(const int* __restrict__ label, unsigned char* __restrict__ mask, Geo g) {
-  nm_mask_body(label, mask, g, blockIdx.x);
-}
-
 // mask: the same-label neighbour mask of `label` (null: the six neighbour labels are read)
 template <typename T, bool ACC, bool SR, bool MASK>
 __global__ void __launch_bounds__(256) k_nm_update(const T* U, T* Unew, const T* K, const T* P, const int* label, Geo g,
@@ -173,7 +190,10 @@ cudaError_t nm_update(const T* U, T* Unew, const T* K, const T* P, const int* la
   return cudaGetLastError();
 }
 cudaError_t nm_mask(const int* label, unsigned char* mask, const Geo& g, cudaStream_t st) {
-  k_nm_mask<<<nblk(g.S3, 256 * kNmFlatChunk), 256, 0, st>>>(label, mask, g);
+  if (g.S % 4 == 1)
+    k_nm_mask<true><<<vgrid<int>(g, 1), 256, 0, st>>>(label, mask, g);
+  else
+    k_nm_mask<false><<<vgrid<int>(g, 1), 256, 0, st>>>(label, mask, g);
   return cudaGetLastError();
 }
 template <typename T>

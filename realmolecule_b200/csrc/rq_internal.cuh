@@ -25,6 +25,10 @@ constexpr int kThreadsJ = 8;   // threads along j per block
 constexpr int kMarch = 16;     // planes along i marched by one thread
 constexpr int kNmPD = 5;       // new flavour: readout sums per domain (norm, T, V_eK, P rho, P A P)
 
+// bits of the same-label neighbour mask of a point: set when neighbour +i, -i, +j, -j, +k, -k carries the
+// point's label; kNmIn on every interior point (the mask of a face point is 0)
+constexpr int kNmIp = 1, kNmIm = 2, kNmJp = 4, kNmJm = 8, kNmKp = 16, kNmKm = 32, kNmIn = 64;
+
 struct Geo {
   int S;      // points per axis
   int NN;     // S - 1

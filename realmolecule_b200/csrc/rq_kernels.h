@@ -12,8 +12,8 @@ cudaError_t launch_update_sp(const float* U, float* Unew, const float* K, const 
 // update and Jacobi sweep in one pass (first: update then the sweep on the new psi; else the
 // sweep then the update with the new P)
 cudaError_t launch_step_sp(bool first, const float* U, float* Unew, const float* K, const float* P, float* Pnew,
-                           const int* label, const Geo& g, float half_dv, float dtv, float h2, float coeff, double h3,
-                           int nDom, double* norms, cudaStream_t st);
+                           const unsigned char* mask, const int* label, const Geo& g, float half_dv, float dtv, float h2,
+                           float coeff, double h3, int nDom, double* norms, cudaStream_t st);
 cudaError_t launch_jacobi_sp(const float* P, float* Pnew, const float* U, const Geo& g, float h2, float coeff,
                              cudaStream_t st);
 cudaError_t launch_labels_sp(const int* labIn, int* labOut, const float* atoms5, int nAtoms, const Geo& g, float h,
@@ -31,8 +31,9 @@ struct AtomBins {
 void build_atom_bins(const float* atoms5, int n, int nb, int bin, std::vector<int>& start, std::vector<int>& idx,
                      std::vector<int>& far, float& zmax);
 // the label step with the argmax over atoms found through the bins (same result as launch_labels_sp)
-cudaError_t launch_labels_binned_sp(const int* labIn, int* labOut, const float* atoms5, int nAtoms, AtomBins bins,
-                                    const Geo& g, float h, float h2, cudaStream_t st);
+cudaError_t launch_labels_binned_sp(const int* labIn, int* labOut, const unsigned char* mask, unsigned* list,
+                                    unsigned* count, const float* atoms5, int nAtoms, AtomBins bins, const Geo& g,
+                                    float h, float h2, cudaStream_t st);
 cudaError_t launch_init_sp(float* U, int* label, float* K, float* bestU, const float* atoms5, int nAtoms,
                            const Geo& g, float h, float h2, bool trial, cudaStream_t st);
 cudaError_t launch_norms_flat(const float* U, const int* label, const Geo& g, double h3, int nDom, double* norms,
