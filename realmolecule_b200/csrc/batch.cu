@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(256) kb_update(const BInst* __restrict__ ins, 
     __syncthreads();
   }
   const Geo g = I.g;
-  nm_update_body<T, ACC, false, SR>((const T*)I.U[cu], (T*)I.U[1 - cu], (const T*)I.K, (const T*)I.P[cp], I.lab[cl], g,
+  nm_update_body<T, ACC, SR>((const T*)I.U[cu], (T*)I.U[1 - cu], (const T*)I.K, (const T*)I.P[cp], I.lab[cl], g,
                                     half_dv, dt, I.h * I.h * I.h, I.nDom, nrm, tab, it.bx, it.by, it.bz,
                                     scale ? scale + I.dom0 : nullptr, seed, tile);
   if (ACC) {

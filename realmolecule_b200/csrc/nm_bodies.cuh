@@ -8,6 +8,7 @@
 // (oracle/rq_oracle.c, orc_nm_*).
 #pragma once
 #include "rq_internal.cuh"
+#include "vec_stencil.cuh"
 
 namespace rq {
 
@@ -181,6 +182,25 @@ __device__ __forceinline__ float sr_round(double v, unsigned u24) {
   return (double)u24 * 5.9604644775390625e-08 < frac ? b : a;   // u24 / 2^24
 }
 
+// One point of the update from its (already selected) neighbours.  With `scaled` the pending per-domain
+// scale multiplies the result, formed in FP64 and rounded once; with SR and `rnd` the exact FP64 value is
+// rounded without bias.
+template <typename T, bool SR>
+__device__ __forceinline__ T nm_update_point(T u_c, T a, T b, T c, T d, T e, T f, T kv, T pv, T half_dv, T dt, bool rnd,
+                                             unsigned sd, long long id, double scale, bool scaled) {
+  using A = Ar<T>;
+  const T lap = A::sub(A::add(A::add(A::add(A::add(A::add(a, b), c), d), e), f), A::mul(T(6), u_c));
+  if (SR && sizeof(T) == sizeof(float) && rnd) {
+    // the same f32 terms, summed exactly in FP64, scaled, then one unbiased rounding
+    double v = ((double)u_c + (double)A::mul(half_dv, lap)) + (double)A::mul(A::mul(dt, A::sub(kv, A::mul(T(2), pv))), u_c);
+    if (scaled) v *= scale;
+    return (T)sr_round(v, sr_uniform24((unsigned long long)id, sd));
+  }
+  T out = A::add(A::add(u_c, A::mul(half_dv, lap)), A::mul(A::mul(dt, A::sub(kv, A::mul(T(2), pv))), u_c));
+  if (scaled) out = (T)((double)out * scale);
+  return out;
+}
+
 // ITP update (same-label Neumann Laplacian) on the march tile (bx, by, bz); with ACC the FP64
 // norm of the new psi per label goes through the block table (caller inits and flushes it).
 // With a non-null `scale` the stored psi is one normalisation behind.  The update is linear in
@@ -189,19 +209,17 @@ __device__ __forceinline__ float sr_round(double v, unsigned u24) {
 // scale[label] * update(psi), formed in FP64 and rounded once -- normalise-then-update up to
 // rounding, without a separate pass over psi.  With a non-null `seed` (fp32 fields) the stored
 // value is rounded without bias (sr_round) from its exact FP64 form.
-// MASK: neighbour-label equality from `mask` (nm_mask of the same labels) instead of six label
-// loads; the centre label is then read only where it is used (norm accumulation, pending scale).
-// The arithmetic is the same, so both forms give the same bits.
-// SR: the unbiased rounding of fp32 fields (seed non-null), compiled only where it is asked for
-template <typename T, bool ACC, bool MASK = false, bool SR = false>
+// SR: the unbiased rounding of fp32 fields (seed non-null), compiled only where it is asked for.
+// This form walks a march tile over the labels; the persistent batch launch runs it (its blocks take march
+// tiles), every other launch the vector form below.
+template <typename T, bool ACC, bool SR = false>
 __device__ __forceinline__ void nm_update_body(const T* __restrict__ U, T* __restrict__ Unew, const T* __restrict__ K,
                                                const T* __restrict__ P, const int* __restrict__ label, const Geo& g,
                                                T half_dv, T dt, double h3, int nDom, double* __restrict__ norms,
                                                DomTable<1, 128>& tab, int bx, int by, int bz,
                                                const double* __restrict__ scale = nullptr,
                                                const unsigned* __restrict__ seed = nullptr,
-                                               const NmTile t = kNmTile,
-                                               const unsigned char* __restrict__ mask = nullptr) {
+                                               const NmTile t = kNmTile) {
   using A = Ar<T>;
   RunSum<1> rs;
   rs.reset();
@@ -212,46 +230,23 @@ __device__ __forceinline__ void nm_update_body(const T* __restrict__ U, T* __res
     const long long S = g.S, S2 = g.S2;
     long long id = (long long)i0 * S2 + j * S + k;
     const unsigned sd = (SR && seed) ? __ldg(seed) : 0u;
-    const bool need_l = !MASK || ACC || scale != nullptr;
     T u_m = __ldg(U + id - S2), u_c = __ldg(U + id);
-    int l_m = MASK ? 0 : __ldg(label + id - S2), l_c = need_l ? __ldg(label + id) : 0;
+    int l_m = __ldg(label + id - S2), l_c = __ldg(label + id);
     for (int i = i0; i < iend; ++i, id += S2) {
       const T u_p = __ldg(U + id + S2);
       const T ujp = __ldg(U + id + S), ujm = __ldg(U + id - S), ukp = __ldg(U + id + 1), ukm = __ldg(U + id - 1);
       const T kv = __ldg(K + id), pv = __ldg(P + id);
-      T a, b, c, d, e, f;
-      int l_p = 0;
-      if (MASK) {
-        const unsigned m = __ldg(mask + id);
-        if (need_l && i + 1 < iend) l_p = __ldg(label + id + S2);
-        a = (m & kNmIp) ? u_p : u_c;
-        b = (m & kNmIm) ? u_m : u_c;
-        c = (m & kNmJp) ? ujp : u_c;
-        d = (m & kNmJm) ? ujm : u_c;
-        e = (m & kNmKp) ? ukp : u_c;
-        f = (m & kNmKm) ? ukm : u_c;
-      } else {
-        l_p = __ldg(label + id + S2);
-        const int ljp = __ldg(label + id + S), ljm = __ldg(label + id - S), lkp = __ldg(label + id + 1),
-                  lkm = __ldg(label + id - 1);
-        a = (l_p == l_c) ? u_p : u_c;
-        b = (l_m == l_c) ? u_m : u_c;
-        c = (ljp == l_c) ? ujp : u_c;
-        d = (ljm == l_c) ? ujm : u_c;
-        e = (lkp == l_c) ? ukp : u_c;
-        f = (lkm == l_c) ? ukm : u_c;
-      }
-      const T lap = A::sub(A::add(A::add(A::add(A::add(A::add(a, b), c), d), e), f), A::mul(T(6), u_c));
-      T out;
-      if (SR && sizeof(T) == sizeof(float) && seed) {
-        // the same f32 terms, summed exactly in FP64, scaled, then one unbiased rounding
-        double v = ((double)u_c + (double)A::mul(half_dv, lap)) + (double)A::mul(A::mul(dt, A::sub(kv, A::mul(T(2), pv))), u_c);
-        if (scale) v *= __ldg(scale + min(max(l_c, 0), nDom - 1));
-        out = (T)sr_round(v, sr_uniform24((unsigned long long)id, sd));
-      } else {
-        out = A::add(A::add(u_c, A::mul(half_dv, lap)), A::mul(A::mul(dt, A::sub(kv, A::mul(T(2), pv))), u_c));
-        if (scale) out = (T)((double)out * __ldg(scale + min(max(l_c, 0), nDom - 1)));
-      }
+      const int l_p = __ldg(label + id + S2);
+      const int ljp = __ldg(label + id + S), ljm = __ldg(label + id - S), lkp = __ldg(label + id + 1),
+                lkm = __ldg(label + id - 1);
+      const T a = (l_p == l_c) ? u_p : u_c;
+      const T b = (l_m == l_c) ? u_m : u_c;
+      const T c = (ljp == l_c) ? ujp : u_c;
+      const T d = (ljm == l_c) ? ujm : u_c;
+      const T e = (lkp == l_c) ? ukp : u_c;
+      const T f = (lkm == l_c) ? ukm : u_c;
+      const T out = nm_update_point<T, SR>(u_c, a, b, c, d, e, f, kv, pv, half_dv, dt, seed != nullptr, sd, id,
+                                           scale ? __ldg(scale + min(max(l_c, 0), nDom - 1)) : 1.0, scale != nullptr);
       Unew[id] = out;
       if (ACC) {
         const double r = (double)out * (double)out * h3;
@@ -262,6 +257,74 @@ __device__ __forceinline__ void nm_update_body(const T* __restrict__ U, T* __res
   }
   if (ACC) rs.finish_warp(tab, norms);  // every lane of the block reaches this point
 }
+
+// The update on 16-byte groups (vec_stencil.cuh), planes [i0, iend) of block column bx, label equality from
+// the same-label mask (nm_mask of the same labels); the labels are read only where norms accumulate or a
+// pending scale applies.  Same values as nm_update_body.  Traffic 17 B per fp32 point; bound by HBM where
+// the field leaves L2.
+template <typename T, bool ACC, bool SR, bool S1>
+__device__ __forceinline__ void nm_vupdate_body(const T* __restrict__ U, T* __restrict__ Unew, const T* __restrict__ K,
+                                                const T* __restrict__ P, const int* __restrict__ label,
+                                                const unsigned char* __restrict__ mask, const Geo& g, T half_dv, T dt,
+                                                double h3, int nDom, double* __restrict__ norms, DomTable<1, 128>& tab,
+                                                int bx, int i0, int iend, const double* __restrict__ scale,
+                                                const unsigned* __restrict__ seed) {
+  constexpr int W = Vec<T>::W;
+  RunCols<1, W> rs;
+  if (ACC) rs.reset();
+  const unsigned sd = (SR && seed) ? __ldg(seed) : 0u;
+  for (int i = i0; i < iend; ++i) {
+    const VGroup r = vgroup<T>(g, i, bx);
+    const VLoad<T, S1> lu(U, r, g);
+    const Quad<T> kv = ldq<T>(K + r.a), pv = ldq<T>(P + r.a);
+    const unsigned mw = vbytes<T>(mask, r);
+    int l[W];
+    if (ACC || scale) vlabels<T>(label, r, l);
+    const Star<T> u = vstar(lu);
+    Quad<T> un;
+#pragma unroll
+    for (int e = 0; e < W; ++e) {
+      const unsigned m = mw >> (8 * e);
+      const T uc = u.c.v[e];
+      const T a = (m & kNmIp) ? u.ip.v[e] : uc, b = (m & kNmIm) ? u.im.v[e] : uc;
+      const T c = (m & kNmJp) ? u.jp.v[e] : uc, d = (m & kNmJm) ? u.jm.v[e] : uc;
+      const T f = (m & kNmKp) ? u.kp.v[e] : uc, q = (m & kNmKm) ? u.km.v[e] : uc;
+      const int lc = (ACC || scale) ? min(max(l[e], 0), nDom - 1) : 0;
+      const T out = nm_update_point<T, SR>(uc, a, b, c, d, f, q, kv.v[e], pv.v[e], half_dv, dt, seed != nullptr, sd,
+                                           r.a + e, scale ? __ldg(scale + lc) : 1.0, scale != nullptr);
+      const bool in = m & kNmIn;
+      un.v[e] = in ? out : T(0);
+      if (ACC && in && r.own) {
+        const double v = (double)out * (double)out * h3;
+        rs.add(e, lc, &v, tab, norms);
+      }
+    }
+    if (r.own) stq(Unew + r.a, un);
+  }
+  if (ACC) rs.finish_warp(tab, norms);
+}
+
+// Same-label neighbour mask of the interior points (kNmIp ..) of plane i, block column bx: the updates read
+// it in place of six neighbour labels while the labels do not change.  The face bytes are 0 from the
+// allocation.
+template <bool S1>
+__device__ __forceinline__ void nm_mask_body(const int* __restrict__ label, unsigned char* __restrict__ mask, const Geo& g,
+                                             int bx, int i) {
+  const VGroup r = vgroup<int>(g, i, bx);
+  const Star<int> l = vstar(VLoad<int, S1>(label, r, g));
+  if (!r.own) return;
+  const VRow row = vrow(g, r, i);
+  unsigned m4 = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int c = l.c.v[e];
+    const unsigned m = (l.ip.v[e] == c ? kNmIp : 0) | (l.im.v[e] == c ? kNmIm : 0) | (l.jp.v[e] == c ? kNmJp : 0) |
+                       (l.jm.v[e] == c ? kNmJm : 0) | (l.kp.v[e] == c ? kNmKp : 0) | (l.km.v[e] == c ? kNmKm : 0) | kNmIn;
+    if (vinterior(g, row, e)) m4 |= m << (8 * e);
+  }
+  *reinterpret_cast<unsigned*>(mask + r.a) = m4;
+}
+constexpr int kNmVPlanes = 4;  // planes per block of the vector update
 
 // U *= scale[label] (FP64 product, rounded once) for labels in [0, nDom) over kNmFlatChunk*256
 // points from blk.  With 16-byte aligned fields each thread moves 16-byte vectors of psi (and the
@@ -337,6 +400,37 @@ __device__ __forceinline__ T rhs_at(const T* __restrict__ f, long long id) {
     return Ar<T>::mul(Ar<T>::mul((T)6.283185307179586, u), u);
   }
   return f[id];
+}
+
+// One colour of a red-black sweep for A P = f, A P = (6P - sum_6 P)/h^2, on 16-byte groups: planes
+// [i0, iend) of block column bx.  S is odd, so i + j + k and the linear id have the same parity and a
+// group's elements alternate colours: the pass updates elements COLOR, COLOR + 2 and needs a shuffle only
+// for the one whose neighbour is in the next lane.  The pass is in place: it reads points of the other
+// colour only, which it does not write, and stores its own one by one.
+constexpr int kNmRbPlanes = 2;  // planes per block
+template <typename T, bool FINE, bool S1, int COLOR>
+__device__ __forceinline__ void nm_vrbgs_body(T* __restrict__ P, const T* __restrict__ f, const Geo& g, T h2, int bx,
+                                              int i0, int iend) {
+  using A = Ar<T>;
+  constexpr int W = Vec<T>::W;
+  for (int i = i0; i < iend; ++i) {
+    const VGroup r = vgroup<T>(g, i, bx);
+    const VLoad<T, S1, false> l(P, r, g);
+    const Quad<T> fq = ldq<T>(f + r.a);
+    const VRow row = vrow(g, r, i);
+    auto next = [&](const Quad<T>& q, int e) { return e + 1 < W ? q.v[(e + 1) % W] : __shfl_down_sync(0xffffffffu, q.v[0], 1); };
+    auto prev = [&](const Quad<T>& q, int e) { return e > 0 ? q.v[(e + W - 1) % W] : __shfl_up_sync(0xffffffffu, q.v[W - 1], 1); };
+#pragma unroll
+    for (int e = COLOR; e < W; e += 2) {
+      const T ip = next(l.ip, e), im = prev(l.im, e);
+      const T jp = S1 ? next(l.jp, e) : prev(l.jp, e), jm = S1 ? prev(l.jm, e) : next(l.jm, e);
+      const T kp = next(l.c, e), km = prev(l.c, e);
+      const T s = A::add(A::add(A::add(A::add(A::add(ip, im), jp), jm), kp), km);
+      T rhs = fq.v[e];
+      if (FINE) rhs = A::mul(A::mul((T)6.283185307179586, rhs), rhs);
+      if (r.own && vinterior(g, row, e)) P[r.a + e] = sixth(A::add(s, A::mul(h2, rhs)));
+    }
+  }
 }
 
 // one colour of a red-black sweep for A P = f, A P = (6P - sum_6 P)/h^2; block (32, 8): each

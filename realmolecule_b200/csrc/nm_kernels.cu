@@ -24,44 +24,28 @@ __global__ void __launch_bounds__(256) k_nm_init(T* U, int* label, const float4*
   nm_init_body<T>(U, label, seeds, nSeed, g, h, blockIdx.x, ss);
 }
 
-// Same-label neighbour mask of the interior points (kNmIp ..): the updates read it in place of six
-// neighbour labels while the labels do not change.  The face bytes are 0 from the allocation.
 template <bool S1>
 __global__ void __launch_bounds__(256) k_nm_mask(const int* __restrict__ label, unsigned char* __restrict__ mask, Geo g) {
-  const int i = 1 + (int)blockIdx.y;
-  const VGroup r = vgroup<int>(g, i, (int)blockIdx.x);
-  const Star<int> l = vstar(VLoad<int, S1>(label, r, g));
-  if (!r.own) return;
-  const VRow row = vrow(g, r, i);
-  unsigned m4 = 0;
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const int c = l.c.v[e];
-    const unsigned m = (l.ip.v[e] == c ? kNmIp : 0) | (l.im.v[e] == c ? kNmIm : 0) | (l.jp.v[e] == c ? kNmJp : 0) |
-                       (l.jm.v[e] == c ? kNmJm : 0) | (l.kp.v[e] == c ? kNmKp : 0) | (l.km.v[e] == c ? kNmKm : 0) | kNmIn;
-    if (vinterior(g, row, e)) m4 |= m << (8 * e);
-  }
-  *reinterpret_cast<unsigned*>(mask + r.a) = m4;
+  nm_mask_body<S1>(label, mask, g, blockIdx.x, 1 + (int)blockIdx.y);
 }
 
-// seed[0]: the step seed of the unbiased fp32 rounding (null: round to nearest); the next step's
-// seed, seed[0] + 1, goes to seed_next (read and written in different words, so every block reads
-// the same value)
-// mask: the same-label neighbour mask of `label` (null: the six neighbour labels are read)
-template <typename T, bool ACC, bool SR, bool MASK>
+// mask: the same-label neighbour mask of `label`.  seed[0]: the step seed of the unbiased fp32 rounding
+// (null: round to nearest); the next step's seed, seed[0] + 1, goes to seed_next (read and written in
+// different words, so every block reads the same value)
+template <typename T, bool ACC, bool SR, bool S1>
 __global__ void __launch_bounds__(256) k_nm_update(const T* U, T* Unew, const T* K, const T* P, const int* label, Geo g,
                                                    T half_dv, T dt, double h3, int nDom, double* norms, const double* scale,
                                                    const unsigned* seed, unsigned* seed_next,
-                                                   const unsigned char* __restrict__ mask) {
+                                                   const unsigned char* __restrict__ mask, int planes) {
   __shared__ DomTable<1, 128> tab;
-  if (SR && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0 && threadIdx.y == 0)
-    *seed_next = *seed + 1u;
+  if (SR && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *seed_next = *seed + 1u;
   if (ACC) {
     dom_table_init(tab);
     __syncthreads();
   }
-  nm_update_body<T, ACC, MASK, SR>(U, Unew, K, P, label, g, half_dv, dt, h3, nDom, norms, tab, blockIdx.x, blockIdx.y,
-                                   blockIdx.z, scale, seed, kNmTile, mask);
+  const int i0 = 1 + (int)blockIdx.y * planes;
+  nm_vupdate_body<T, ACC, SR, S1>(U, Unew, K, P, label, mask, g, half_dv, dt, h3, nDom, norms, tab, blockIdx.x, i0,
+                                  min(i0 + planes, g.NN), scale, seed);
   if (ACC) {
     __syncthreads();
     dom_table_flush(tab, norms);
@@ -93,9 +77,10 @@ __global__ void __launch_bounds__(256) k_nm_norms(const T* U, const int* label, 
   dom_table_flush(tab, norms);
 }
 
-template <typename T, bool FINE>
-__global__ void __launch_bounds__(256) k_nm_rbgs(T* P, const T* f, Geo g, T h2, int color) {
-  nm_rbgs_body<T, FINE>(P, f, g, h2, color, blockIdx.x, blockIdx.y, blockIdx.z);
+template <typename T, bool FINE, bool S1, int COLOR>
+__global__ void __launch_bounds__(256) k_nm_rbgs(T* P, const T* f, Geo g, T h2, int planes) {
+  const int i0 = 1 + (int)blockIdx.y * planes;
+  nm_vrbgs_body<T, FINE, S1, COLOR>(P, f, g, h2, blockIdx.x, i0, min(i0 + planes, g.NN));
 }
 
 template <typename T, bool FINE>
@@ -173,20 +158,16 @@ cudaError_t nm_update(const T* U, T* Unew, const T* K, const T* P, const int* la
                       double h3, int nDom, double* norms, cudaStream_t st, const double* scale, const unsigned* seed,
                       unsigned* seed_next, const unsigned char* mask) {
   if (g.NN < 2) return cudaSuccess;
-  const dim3 grd = nm_march_grid(g), blk = nm_march_block();
-  auto go = [&](auto acc, auto sr, auto msk) {
-    k_nm_update<T, decltype(acc)::value, decltype(sr)::value, decltype(msk)::value><<<grd, blk, 0, st>>>(
-        U, Unew, K, P, label, g, half_dv, dt, h3, nDom, norms, scale, seed, seed_next, mask);
+  auto go = [&](auto acc, auto sr, auto s1) {
+    const int planes = vplanes<T>(g, decltype(acc)::value);
+    k_nm_update<T, decltype(acc)::value, decltype(sr)::value, decltype(s1)::value><<<vgrid<T>(g, planes), 256, 0, st>>>(
+        U, Unew, K, P, label, g, half_dv, dt, h3, nDom, norms, scale, seed, seed_next, mask, planes);
   };
   using Y = std::true_type;
   using N = std::false_type;
-  if (mask) {
-    if (norms) { if (seed) go(Y{}, Y{}, Y{}); else go(Y{}, N{}, Y{}); }
-    else       { if (seed) go(N{}, Y{}, Y{}); else go(N{}, N{}, Y{}); }
-  } else {
-    if (norms) { if (seed) go(Y{}, Y{}, N{}); else go(Y{}, N{}, N{}); }
-    else       { if (seed) go(N{}, Y{}, N{}); else go(N{}, N{}, N{}); }
-  }
+  auto go2 = [&](auto acc, auto sr) { if (g.S % 4 == 1) go(acc, sr, Y{}); else go(acc, sr, N{}); };
+  if (norms) { if (seed) go2(Y{}, Y{}); else go2(Y{}, N{}); }
+  else       { if (seed) go2(N{}, Y{}); else go2(N{}, N{}); }
   return cudaGetLastError();
 }
 cudaError_t nm_mask(const int* label, unsigned char* mask, const Geo& g, cudaStream_t st) {
@@ -220,13 +201,18 @@ cudaError_t nm_norms(const T* U, const int* label, const Geo& g, double h3, int 
 }
 template <typename T>
 cudaError_t nm_rbgs(T* P, const T* f, bool fine, const Geo& g, double h2, int color, cudaStream_t st) {
-  const int n = g.NN - 1;
-  const dim3 blk(32, 8);
-  const dim3 grd((n + 63) / 64, (n + 7) / 8, (n + kNmRowPlanes - 1) / kNmRowPlanes);
-  if (fine)
-    k_nm_rbgs<T, true><<<grd, blk, 0, st>>>(P, f, g, (T)h2, color);
-  else
-    k_nm_rbgs<T, false><<<grd, blk, 0, st>>>(P, f, g, (T)h2, color);
+  const int planes = vplanes<T>(g, false);
+  const dim3 grd = vgrid<T>(g, planes);
+  auto go = [&](auto fn, auto s1) {
+    if (color)
+      k_nm_rbgs<T, decltype(fn)::value, decltype(s1)::value, 1><<<grd, 256, 0, st>>>(P, f, g, (T)h2, planes);
+    else
+      k_nm_rbgs<T, decltype(fn)::value, decltype(s1)::value, 0><<<grd, 256, 0, st>>>(P, f, g, (T)h2, planes);
+  };
+  using Y = std::true_type;
+  using N = std::false_type;
+  if (g.S % 4 == 1) { if (fine) go(Y{}, Y{}); else go(N{}, Y{}); }
+  else              { if (fine) go(Y{}, N{}); else go(N{}, N{}); }
   return cudaGetLastError();
 }
 template <typename T>

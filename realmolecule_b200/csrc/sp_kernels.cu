@@ -606,11 +606,8 @@ cudaError_t launch_step_sp(bool first, const float* U, float* Unew, const float*
                            const unsigned char* mask, const int* label, const Geo& g, float half_dv, float dtv, float h2,
                            float coeff, double h3, int nDom, double* norms, cudaStream_t st) {
   if (g.NN < 2) return cudaSuccess;
-  // planes per block: 4 where the grid still has 16 blocks per SM (the plane loads of neighbouring planes
-  // then hit L1: 300^3 16.6 ms a 100-step period against 17.3), else 1 (128^3: 1.07 against 1.09 ms);
-  // with norms always 4, for fewer block tables to flush
-  const dim3 g1 = vgrid<float>(g, 4);
-  const int planes = norms || (long long)g1.x * g1.y >= 16 * 148 ? 4 : 1;
+  // 300^3: 16.6 ms a 100-step period with 4 planes, 17.3 with 1; 128^3: 1.09 and 1.07 ms
+  const int planes = vplanes<float>(g, norms != nullptr);
   auto go = [&](auto f, auto acc, auto s1) {
     k_step_sp<decltype(f)::value, decltype(acc)::value, decltype(s1)::value><<<vgrid<float>(g, planes), 256, 0, st>>>(
         U, Unew, K, P, Pnew, mask, label, g, half_dv, dtv, h2, coeff, h3, nDom, norms, planes);

@@ -60,6 +60,14 @@ inline dim3 vgrid(const Geo& g, int planes) {
   return dim3((vgroups<T>(g) + kVOwn - 1) / kVOwn, (unsigned)((g.NN - 1 + planes - 1) / planes));
 }
 
+// Planes per block: 4 where the grid still has 16 blocks per SM (the loads of neighbouring planes then hit
+// L1), else 1; with per-domain sums always 4, for fewer block tables to flush.
+template <typename T>
+inline int vplanes(const Geo& g, bool sums) {
+  const dim3 q = vgrid<T>(g, 4);
+  return sums || (long long)q.x * q.y >= 16 * 148 ? 4 : 1;
+}
+
 // The thread's group of plane i.  The owned groups run from the one that holds (i, 1, 1) to the one that
 // holds (i, NN - 1, NN - 1); with one more on either side their +-S and +-S^2 shifts stay inside the
 // array (S >= 5).
@@ -153,6 +161,74 @@ __device__ __forceinline__ unsigned vbytes(const unsigned char* __restrict__ m, 
   if (Vec<T>::W == 4) return __ldg(reinterpret_cast<const unsigned*>(m + r.a));
   return __ldg(reinterpret_cast<const unsigned short*>(m + r.a));
 }
+
+// the W labels of the group
+template <typename T>
+__device__ __forceinline__ void vlabels(const int* __restrict__ label, const VGroup& r, int (&l)[Vec<T>::W]) {
+  if constexpr (Vec<T>::W == 4) {
+    const int4 x = __ldg(reinterpret_cast<const int4*>(label + r.a));
+    l[0] = x.x; l[1] = x.y; l[2] = x.z; l[3] = x.w;
+  } else {
+    const int2 x = __ldg(reinterpret_cast<const int2*>(label + r.a));
+    l[0] = x.x; l[1] = x.y;
+  }
+}
+
+// Running (label, NQ sums) of each of a thread's W columns while it walks planes: a column meets a new
+// label about once per domain it crosses, and only then touches the block table (RunSum, per column).
+template <int NQ, int W> struct RunCols {
+  int label[W];
+  double v[W][NQ];
+  __device__ __forceinline__ void reset() {
+#pragma unroll
+    for (int e = 0; e < W; ++e) {
+      label[e] = -1;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) v[e][q] = 0.0;
+    }
+  }
+  template <int NSLOT>
+  __device__ __forceinline__ void add(int e, int l, const double* x, DomTable<NQ, NSLOT>& t, double* global) {
+    if (l != label[e]) {
+      if (label[e] >= 0) dom_table_add(t, label[e], v[e], global);
+      label[e] = l;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) v[e][q] = x[q];
+    } else {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) v[e][q] += x[q];
+    }
+  }
+  // every lane of the warp together: a thread's columns of one label are merged, then runs of lanes with
+  // one label by a butterfly, so the table sees about one add per label and warp
+  template <int NSLOT>
+  __device__ __forceinline__ void finish_warp(DomTable<NQ, NSLOT>& t, double* global) {
+#pragma unroll
+    for (int e = W - 1; e > 0; --e) {
+      if (label[e] < 0) continue;
+      if (label[e] == label[e - 1] || label[e - 1] < 0) {
+        label[e - 1] = label[e];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) v[e - 1][q] += v[e][q];
+      } else {
+        dom_table_add(t, label[e], v[e], global);
+      }
+    }
+    const int lane = (int)threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int ol = __shfl_xor_sync(0xffffffffu, label[0], o);
+      const bool same = ol == label[0];
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        const double x = __shfl_xor_sync(0xffffffffu, v[0][q], o);
+        if (same && !(lane & o)) v[0][q] += x;
+      }
+      if (same && (lane & o)) label[0] = -1;
+    }
+    if (label[0] >= 0) dom_table_add(t, label[0], v[0], global);
+  }
+};
 
 // x / 6 correctly rounded, by the two-constant product of Brisebarre, Muller and Raina ("Accelerating
 // correctly rounded floating-point division when the divisor is known in advance", 2004): zh + zl is 1/6
