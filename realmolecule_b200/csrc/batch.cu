@@ -8,6 +8,7 @@
 // by level over the instances that still have a coarser level, solves each instance's coarsest
 // level (one block per instance, FP64) when it is reached, and ascends again.
 #include <algorithm>
+#include <type_traits>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -28,6 +29,7 @@ struct BInst {
   void* P[2];
   void* K;
   int* lab[2];
+  unsigned char* mask;  // same-label neighbour mask of the current labels (shared by both field sets)
   float* W;
   int nDom, dom0;  // domains of this instance and their offset in the batch-wide arrays
   int nlev;
@@ -48,33 +50,36 @@ struct BItem {
   int inst, bx, by, bz;
 };
 
+constexpr int kBVPlanes = 8;  // planes per block of the vector kernels: 4 / 8 / 16 give 42.8 / 38.4 / 38.7 ms for
+                              // 20 steps and the readouts of 96 clusters (fewer leave the block's table
+                              // look-ups uncovered)
+
 // ---------------------------------------------------------------------------------------
 // batched kernels: block b works on items[b].  Each copies its instance's geometry into
 // registers first: through a reference into the instance table the compiler would re-read it
 // after every store, as it cannot prove the field pointers do not alias the table.
 // ---------------------------------------------------------------------------------------
-template <typename T, bool ACC, bool SR>
-__global__ void __launch_bounds__(256) kb_update(const BInst* __restrict__ ins, const BItem* __restrict__ items, int cu,
-                                                 int cp, int cl, T half_dv, T dt, double* __restrict__ norms,
-                                                 const double* __restrict__ scale, const unsigned* __restrict__ seed,
-                                                 unsigned* __restrict__ seed_next, NmTile tile) {
-  __shared__ DomTable<1, 128> tab;
-  if (SR && blockIdx.x == 0 && threadIdx.x == 0 && threadIdx.y == 0) *seed_next = *seed + 1u;
+// (items of the vector kernels: block column bx of the planes from 1 + by * planes.)  Bound by memory
+// latency: 6 blocks per SM (40 registers) are faster than the compiler's 3, 8 spill.
+template <typename T, bool SR>
+__global__ void __launch_bounds__(256, 6) kb_update(const BInst* __restrict__ ins, const BItem* __restrict__ items, int cu,
+                                                    int cp, int cl, T half_dv, T dt, const double* __restrict__ scale,
+                                                    const unsigned* __restrict__ seed, unsigned* __restrict__ seed_next) {
+  if (SR && blockIdx.x == 0 && threadIdx.x == 0) *seed_next = *seed + 1u;
   const BItem it = items[blockIdx.x];
   const BInst& I = ins[it.inst];
-  double* nrm = norms ? norms + I.dom0 : nullptr;
-  if (ACC) {
-    dom_table_init(tab);
-    __syncthreads();
-  }
   const Geo g = I.g;
-  nm_update_body<T, ACC, SR>((const T*)I.U[cu], (T*)I.U[1 - cu], (const T*)I.K, (const T*)I.P[cp], I.lab[cl], g,
-                                    half_dv, dt, I.h * I.h * I.h, I.nDom, nrm, tab, it.bx, it.by, it.bz,
-                                    scale ? scale + I.dom0 : nullptr, seed, tile);
-  if (ACC) {
-    __syncthreads();
-    dom_table_flush(tab, nrm);
-  }
+  const int i0 = 1 + it.by * kBVPlanes, iend = min(i0 + kBVPlanes, g.NN);
+  nm_vupdate_body<T, SR, kRowAny>((const T*)I.U[cu], (T*)I.U[1 - cu], (const T*)I.K, (const T*)I.P[cp], I.lab[cl], I.mask, g,
+                                  half_dv, dt, I.nDom, it.bx, i0, iend, scale ? scale + I.dom0 : nullptr, seed);
+}
+
+__global__ void __launch_bounds__(256) kb_mask(const BInst* __restrict__ ins, const BItem* __restrict__ items, int cl) {
+  const BItem it = items[blockIdx.x];
+  const BInst& I = ins[it.inst];
+  const Geo g = I.g;
+  for (int i = 1 + it.by * kBVPlanes; i < min(1 + (it.by + 1) * kBVPlanes, g.NN); ++i)
+    nm_mask_body<kRowAny>(I.lab[cl], I.mask, g, it.bx, i);
 }
 
 template <typename T>
@@ -88,25 +93,30 @@ __global__ void __launch_bounds__(256) kb_apply_scale(const BInst* __restrict__ 
 template <typename T>
 __global__ void __launch_bounds__(256) kb_norms(const BInst* __restrict__ ins, const BItem* __restrict__ items, int cu,
                                                 int cl, double* __restrict__ norms) {
-  __shared__ DomTable<1, 128> tab;
+  __shared__ NormSmem sm;
   const BItem it = items[blockIdx.x];
   const BInst& I = ins[it.inst];
-  dom_table_init(tab);
+  dom_table_init(sm.tab);
   __syncthreads();
-  nm_norms_body<T>((const T*)I.U[cu], I.lab[cl], I.g.S3, I.h * I.h * I.h, I.nDom, norms + I.dom0, tab, it.bx);
+  const Geo g = I.g;
+  const int i0 = 1 + it.bz * kNmNormPlanes;
+  nm_norms_body<T>((const T*)I.U[cu], I.lab[cl], g, I.h * I.h * I.h, I.nDom, norms + I.dom0, sm, it.bx, it.by, i0,
+                   min(i0 + kNmNormPlanes, g.NN));
   __syncthreads();
-  dom_table_flush(tab, norms + I.dom0);
+  dom_table_flush(sm.tab, norms + I.dom0);
 }
 
-template <typename T, bool FINE>
+template <typename T, bool FINE, int COLOR>
 __global__ void __launch_bounds__(256) kb_rbgs(const BInst* __restrict__ ins, const BItem* __restrict__ items, int lev,
-                                               int cu, int cp, int color) {
+                                               int cu, int cp) {
   const BItem it = items[blockIdx.x];
   const BInst& I = ins[it.inst];
   T* P = FINE ? (T*)I.P[cp] : (T*)I.lP[lev];
   const T* f = FINE ? (const T*)I.U[cu] : (const T*)I.lf[lev];
   const Geo g = I.lg[lev];
-  nm_rbgs_body<T, FINE>(P, f, g, (T)(I.lh[lev] * I.lh[lev]), color, it.bx, it.by, it.bz);
+  const T h2 = (T)(I.lh[lev] * I.lh[lev]);
+  const int i0 = 1 + it.by * kBVPlanes, iend = min(i0 + kBVPlanes, g.NN);
+  nm_vrbgs_body<T, FINE, kRowAny, COLOR>(P, f, g, h2, it.bx, i0, iend);
 }
 
 // residual, full weighting and the zeroed coarse correction of level lev in one pass
@@ -145,16 +155,16 @@ __global__ void __launch_bounds__(1024) kb_coarsest(const BInst* __restrict__ in
 template <typename T>
 __global__ void __launch_bounds__(256) kb_energy(const BInst* __restrict__ ins, const BItem* __restrict__ items, int cu,
                                                  int cp, int cl, double* __restrict__ pd, NmTile tile) {
-  __shared__ DomTable<kNmPD, 128> tab;
+  __shared__ EnergySmem sm;
   const BItem it = items[blockIdx.x];
   const BInst& I = ins[it.inst];
-  dom_table_init(tab);
+  dom_table_init(sm.tab);
   __syncthreads();
   const Geo g = I.g;
   nm_energy_body<T>((const T*)I.U[cu], (const T*)I.K, (const T*)I.P[cp], I.lab[cl], g, I.h, I.nDom,
-                    pd + kNmPD * I.dom0, tab, it.bx, it.by, it.bz, sizeof(T) == sizeof(float) ? I.K64 : nullptr, tile);
+                    pd + kNmPD * I.dom0, sm, it.bx, it.by, it.bz, sizeof(T) == sizeof(float) ? I.K64 : nullptr, tile);
   __syncthreads();
-  dom_table_flush(tab, pd + kNmPD * I.dom0);
+  dom_table_flush(sm.tab, pd + kNmPD * I.dom0);
 }
 
 template <typename T>
@@ -474,7 +484,8 @@ constexpr int kF32 = 0, kF64 = 1;
 struct InstItems {
   std::vector<BItem> march[kMaxLev], rbgs[kMaxLev], restr[kMaxLev], zero[kMaxLev], coarse[kMaxLev], rr[kMaxLev],
       pc[kMaxLev];
-  std::vector<BItem> flat16, flat1, gather, core, one;  // one: a single item (per-instance domain work)
+  std::vector<BItem> vec[kMaxLev][2];  // vector kernels of each level, by precision set (16-byte groups)
+  std::vector<BItem> flat16, flat1, norms, gather, core, one;  // one: a single item (per-instance domain work)
 };
 
 struct rq_batch {
@@ -497,7 +508,8 @@ struct rq_batch {
   struct Plan { BItem* d = nullptr; int n = 0, cap = 0; };
   struct Plans {
     Plan march[kMaxLev], rbgs[kMaxLev], restr[kMaxLev], zero[kMaxLev], coarse[kMaxLev], rr[kMaxLev], pc[kMaxLev];
-    Plan flat16, flat1, gather, core, one;
+    Plan vec[kMaxLev], mask;  // mask: the level-0 groups of int labels (4 per group)
+    Plan flat16, flat1, norms, gather, core, one;
   };
   Plans pl[2];
   size_t coarse_smem[kMaxLev] = {};
@@ -524,7 +536,8 @@ struct rq_batch {
   int pgrid[4] = {};              // co-resident blocks of kb_persist<sets> (0: not yet queried)
   long long wait_ns = 2000000000LL;
   int extra_arrivals = 0;
-  NmTile tile = kNmTile;          // march tile of the update, readout and level-set work lists
+  bool mask_ok = false;           // the masks belong to the current labels
+  NmTile tile = kNmTile;          // march tile of the persistent update, the readout and the level-set work lists
   double* dtune = nullptr;        // the autotuner's residual sum
 };
 
@@ -577,6 +590,14 @@ static void make_items(const BInst& I, const std::vector<rq_atom>& atoms, int q,
   it = InstItems{};
   for (int l = 0; l < I.nlev; ++l) {
     march_items(it.march[l], q, I.lg[l], tile);
+    auto vec_items = [&](std::vector<BItem>& v, dim3 gr) {
+      for (unsigned y = 0; y < gr.y; ++y)
+        for (unsigned x = 0; x < gr.x; ++x) v.push_back({q, (int)x, (int)y, 0});
+    };
+    if (l == 0 || l < I.nlev - 1) {  // level 0 always has odd S; a coarsest level is solved in one block
+      vec_items(it.vec[l][0], vgrid<float>(I.lg[l], kBVPlanes));
+      vec_items(it.vec[l][1], vgrid<double>(I.lg[l], kBVPlanes));
+    }
     if (l == I.nlev - 1) {
       it.coarse[l].push_back({q, 0, 0, 0});
       continue;
@@ -600,10 +621,13 @@ static void make_items(const BInst& I, const std::vector<rq_atom>& atoms, int q,
   it.one.push_back({q, 0, 0, 0});
   flat_items(it.flat16, q, I.g.S3, 256 * kNmFlatChunk);
   flat_items(it.flat1, q, I.g.S3, 256);
-  const dim3 gg = nm_gather_grid(I.g);
-  for (unsigned z = 0; z < gg.z; ++z)
-    for (unsigned y = 0; y < gg.y; ++y)
-      for (unsigned x = 0; x < gg.x; ++x) it.gather.push_back({q, (int)x, (int)y, (int)z});
+  auto grid_items = [&](std::vector<BItem>& v, dim3 gr) {
+    for (unsigned z = 0; z < gr.z; ++z)
+      for (unsigned y = 0; y < gr.y; ++y)
+        for (unsigned x = 0; x < gr.x; ++x) v.push_back({q, (int)x, (int)y, (int)z});
+  };
+  grid_items(it.norms, nm_norms_grid(I.g));
+  grid_items(it.gather, nm_gather_grid(I.g));
   for (int a = 0; a < (int)atoms.size(); ++a)
     if (atoms[a].Z_nuc > 0)
       for (int part = 0; part < kGaCoreParts; ++part) it.core.push_back({q, a, part, 0});
@@ -630,15 +654,18 @@ static int build_plans(rq_batch* b) {
     for (int l = 0; l < b->maxlev; ++l) {
       BRC(gather(P.march[l], [l](const InstItems& it) -> const Items& { return it.march[l]; }));
       BRC(gather(P.rbgs[l], [l](const InstItems& it) -> const Items& { return it.rbgs[l]; }));
+      BRC(gather(P.vec[l], [l, p](const InstItems& it) -> const Items& { return it.vec[l][p]; }));
       BRC(gather(P.restr[l], [l](const InstItems& it) -> const Items& { return it.restr[l]; }));
       BRC(gather(P.zero[l], [l](const InstItems& it) -> const Items& { return it.zero[l]; }));
       BRC(gather(P.rr[l], [l](const InstItems& it) -> const Items& { return it.rr[l]; }));
       BRC(gather(P.pc[l], [l](const InstItems& it) -> const Items& { return it.pc[l]; }));
       BRC(gather(P.coarse[l], [l](const InstItems& it) -> const Items& { return it.coarse[l]; }));
     }
+    BRC(gather(P.mask, [](const InstItems& it) -> const Items& { return it.vec[0][kF32]; }));
     BRC(gather(P.flat16, [](const InstItems& it) -> const Items& { return it.flat16; }));
     BRC(gather(P.one, [](const InstItems& it) -> const Items& { return it.one; }));
     BRC(gather(P.flat1, [](const InstItems& it) -> const Items& { return it.flat1; }));
+    BRC(gather(P.norms, [](const InstItems& it) -> const Items& { return it.norms; }));
     BRC(gather(P.gather, [](const InstItems& it) -> const Items& { return it.gather; }));
     BRC(gather(P.core, [](const InstItems& it) -> const Items& { return it.core; }));
   }
@@ -696,6 +723,7 @@ static int build(rq_batch* b) {
     BInst& I = b->hin[q];
     BRC(alloc_fields(b, I, b->f64[q] ? sizeof(double) : sizeof(float)));
     for (int k = 0; k < 2; ++k) BALLOC(I.lab[k], (size_t)I.g.S3 * sizeof(int));
+    BALLOC(I.mask, (size_t)I.g.S3);  // face bytes stay 0
     BALLOC(I.W, (size_t)I.g.S3 * sizeof(float));
     const int lc = I.nlev - 1;
     b->coarse_smem[lc] = std::max(b->coarse_smem[lc], sizeof(double) * 2 * (size_t)I.lg[lc].S3);
@@ -811,10 +839,14 @@ static int b_vcycle(rq_batch* b, int p) {
         b_record(b, kPhRbgs, p, &P.rbgs[l], l, color);
         continue;
       }
-      if (l == 0)
-        kb_rbgs<T, true><<<P.rbgs[l].n, rb, 0, b->st>>>(b->din, P.rbgs[l].d, l, b->cu, b->cp, color);
-      else
-        kb_rbgs<T, false><<<P.rbgs[l].n, rb, 0, b->st>>>(b->din, P.rbgs[l].d, l, b->cu, b->cp, color);
+      auto go = [&](auto fn, auto col) {
+        kb_rbgs<T, decltype(fn)::value, decltype(col)::value><<<P.vec[l].n, 256, 0, b->st>>>(b->din, P.vec[l].d, l, b->cu,
+                                                                                           b->cp);
+      };
+      using C0 = std::integral_constant<int, 0>;
+      using C1 = std::integral_constant<int, 1>;
+      if (l == 0) { if (color) go(std::true_type{}, C1{}); else go(std::true_type{}, C0{}); }
+      else        { if (color) go(std::false_type{}, C1{}); else go(std::false_type{}, C0{}); }
       BL("rbgs");
     }
     return RQ_OK;
@@ -874,7 +906,7 @@ static int b_normalize(rq_batch* b) {
   BCK(cudaMemsetAsync(b->dnorm, 0, sizeof(double) * b->D, b->st));
   BRC(each_set([&](auto tag, int p) -> int {
     using T = decltype(tag);
-    const rq_batch::Plan& f = b->pl[p].flat16;
+    const rq_batch::Plan& f = b->pl[p].norms;
     if (!f.n) return RQ_OK;
     kb_norms<T><<<f.n, 256, 0, b->st>>>(b->din, f.d, b->cu, b->cl, b->dnorm);
     BL("norms");
@@ -901,6 +933,19 @@ static int b_flush(rq_batch* b) {
 static int b_ready(rq_batch* b) { return b->age == 0 ? b_flush(b) : b_normalize(b); }
 
 static bool any_active(const rq_batch* b) { return b->pl[kF32].march[0].n + b->pl[kF64].march[0].n > 0; }
+
+// The same-label masks of the current labels, which the updates of the per-kernel launches read: after every
+// label change (a persistent launch moves labels without them: its caller clears mask_ok instead).
+static int b_mask(rq_batch* b) {
+  for (int p = 0; p < 2; ++p) {
+    const rq_batch::Plan& m = b->pl[p].mask;
+    if (!m.n) continue;
+    kb_mask<<<m.n, 256, 0, b->st>>>(b->din, m.d, b->cl);
+    BL("mask");
+  }
+  b->mask_ok = true;
+  return RQ_OK;
+}
 
 static int b_step(rq_batch* b, int s) {
   const rq_config& f = b->cfg;
@@ -936,20 +981,16 @@ static int b_step(rq_batch* b, int s) {
       b->rec->back().seed_next = sn;
       return RQ_OK;
     }
-    double* nrm = norm ? b->dnorm : nullptr;
-    if (norm && sr)
-      kb_update<T, true, true><<<m.n, nm_march_block(), 0, b->st>>>(b->din, m.d, b->cu, b->cp, b->cl, (T)hd, (T)dt,
-                                                                   nrm, sc, sd, sn, b->tile);
-    else if (norm)
-      kb_update<T, true, false><<<m.n, nm_march_block(), 0, b->st>>>(b->din, m.d, b->cu, b->cp, b->cl, (T)hd, (T)dt,
-                                                                    nrm, sc, sd, sn, b->tile);
-    else if (sr)
-      kb_update<T, false, true><<<m.n, nm_march_block(), 0, b->st>>>(b->din, m.d, b->cu, b->cp, b->cl, (T)hd, (T)dt,
-                                                                    nrm, sc, sd, sn, b->tile);
+    const rq_batch::Plan& v = b->pl[p].vec[0];
+    if (sr)
+      kb_update<T, true><<<v.n, 256, 0, b->st>>>(b->din, v.d, b->cu, b->cp, b->cl, (T)hd, (T)dt, sc, sd, sn);
     else
-      kb_update<T, false, false><<<m.n, nm_march_block(), 0, b->st>>>(b->din, m.d, b->cu, b->cp, b->cl, (T)hd, (T)dt,
-                                                                     nrm, sc, sd, sn, b->tile);
+      kb_update<T, false><<<v.n, 256, 0, b->st>>>(b->din, v.d, b->cu, b->cp, b->cl, (T)hd, (T)dt, sc, sd, sn);
     BL("update");
+    if (norm) {
+      kb_norms<T><<<b->pl[p].norms.n, 256, 0, b->st>>>(b->din, b->pl[p].norms.d, 1 - b->cu, b->cl, b->dnorm);
+      BL("norms");
+    }
     return RQ_OK;
   }));
   b->cu ^= 1;
@@ -980,6 +1021,7 @@ static int b_step(rq_batch* b, int s) {
       return RQ_OK;
     }));
     b->cl ^= 1;
+    if (!b->rec) BRC(b_mask(b));
   }
   return RQ_OK;
 }
@@ -1004,6 +1046,7 @@ static int b_initialize(rq_batch* b) {
     for (int k = 0; k < 2; ++k) BCK(cudaMemsetAsync(I.P[k], 0, es * I.g.S3, b->st));
     BCK(launch_fill(I.W, 1.0f, I.g.S3, b->st));
   }
+  BRC(b_mask(b));
   BRC(b_normalize(b));
   for (int v = 0; v < 10; ++v) BRC(each_set([&](auto tag, int p) { return b_vcycle<decltype(tag)>(b, p); }));
   b->steps_done = 0;
@@ -1278,6 +1321,10 @@ extern "C" int rq_batch_step(rq_batch* b, int32_t n) {
     const int lu = b->cfg.label_until;
     const bool straddle = lu > 0 && b->steps_done < lu && b->steps_done + period > lu;
     const bool aligned = !straddle && period > 0 && period <= 4096 && b->steps_done % period == 0 && left >= period;
+    // the unbiased rounding's step seed advances on the device between steps, which needs the
+    // steps in order: that schedule keeps the per-kernel launches
+    const bool persist = aligned && b->cfg.batch_persistent == 1 && b->cfg.fp32_rounding != 1;
+    if (!persist && !b->mask_ok) BRC(b_mask(b));
     if (!aligned) {
       int todo = left;
       if (period > 0 && b->steps_done % period != 0) todo = std::min(left, period - b->steps_done % period);
@@ -1291,9 +1338,7 @@ extern "C" int rq_batch_step(rq_batch* b, int32_t n) {
     const int key = b->cu | (b->cp << 1) | (b->cl << 2) | (on << 3) | ((b->pending ? 1 : 0) << 4);
     if (!b->graph[key]) {
       const long long l0 = b->launches;
-      // the unbiased rounding's step seed advances on the device between steps, which needs the
-      // steps in order: that schedule keeps the per-kernel launches
-      if (b->cfg.batch_persistent == 1 && b->cfg.fp32_rounding != 1) {
+      if (persist) {
         BRC(b_persist_graph(b, key, period));
         b->launches++;
       } else {
@@ -1322,6 +1367,7 @@ extern "C" int rq_batch_step(rq_batch* b, int32_t n) {
       b->steps_done += period;
       b->launches += b->graph_launches[key];
     }
+    if (persist) b->mask_ok = false;
     left -= period;
   }
   return RQ_OK;
@@ -1468,6 +1514,7 @@ static int b_promote(rq_batch* b, int q) {
 
 int rq_batch_set_active_all(rq_batch* b) {
   b->active.assign(b->n, 1);
+  b->mask_ok = false;  // the label buffers of instances that had left the lists did not follow the parity
   return build_plans(b);
 }
 

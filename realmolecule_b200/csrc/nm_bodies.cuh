@@ -259,27 +259,25 @@ __device__ __forceinline__ void nm_update_body(const T* __restrict__ U, T* __res
 }
 
 // The update on 16-byte groups (vec_stencil.cuh), planes [i0, iend) of block column bx, label equality from
-// the same-label mask (nm_mask of the same labels); the labels are read only where norms accumulate or a
-// pending scale applies.  Same values as nm_update_body.  Traffic 17 B per fp32 point; bound by HBM where
-// the field leaves L2.
-template <typename T, bool ACC, bool SR, bool S1>
+// the same-label mask (nm_mask of the same labels); the labels are read only where a pending scale applies.
+// Same values as nm_update_body.  Traffic 17 B per fp32 point.  The norms of a normalising step are a pass
+// of their own (nm_norms_body): in this kernel their running sums cost more registers, and so more of the
+// loads in flight, than the second read of psi.
+template <typename T, bool SR, int ROW>
 __device__ __forceinline__ void nm_vupdate_body(const T* __restrict__ U, T* __restrict__ Unew, const T* __restrict__ K,
                                                 const T* __restrict__ P, const int* __restrict__ label,
                                                 const unsigned char* __restrict__ mask, const Geo& g, T half_dv, T dt,
-                                                double h3, int nDom, double* __restrict__ norms, DomTable<1, 128>& tab,
-                                                int bx, int i0, int iend, const double* __restrict__ scale,
+                                                int nDom, int bx, int i0, int iend, const double* __restrict__ scale,
                                                 const unsigned* __restrict__ seed) {
   constexpr int W = Vec<T>::W;
-  RunCols<1, W> rs;
-  if (ACC) rs.reset();
   const unsigned sd = (SR && seed) ? __ldg(seed) : 0u;
   for (int i = i0; i < iend; ++i) {
     const VGroup r = vgroup<T>(g, i, bx);
-    const VLoad<T, S1> lu(U, r, g);
+    const VLoad<T, ROW> lu(U, r, g);
     const Quad<T> kv = ldq<T>(K + r.a), pv = ldq<T>(P + r.a);
     const unsigned mw = vbytes<T>(mask, r);
     int l[W];
-    if (ACC || scale) vlabels<T>(label, r, l);
+    if (scale) vlabels<T>(label, r, l);
     const Star<T> u = vstar(lu);
     Quad<T> un;
 #pragma unroll
@@ -289,29 +287,23 @@ __device__ __forceinline__ void nm_vupdate_body(const T* __restrict__ U, T* __re
       const T a = (m & kNmIp) ? u.ip.v[e] : uc, b = (m & kNmIm) ? u.im.v[e] : uc;
       const T c = (m & kNmJp) ? u.jp.v[e] : uc, d = (m & kNmJm) ? u.jm.v[e] : uc;
       const T f = (m & kNmKp) ? u.kp.v[e] : uc, q = (m & kNmKm) ? u.km.v[e] : uc;
-      const int lc = (ACC || scale) ? min(max(l[e], 0), nDom - 1) : 0;
+      const int lc = scale ? min(max(l[e], 0), nDom - 1) : 0;
       const T out = nm_update_point<T, SR>(uc, a, b, c, d, f, q, kv.v[e], pv.v[e], half_dv, dt, seed != nullptr, sd,
                                            r.a + e, scale ? __ldg(scale + lc) : 1.0, scale != nullptr);
-      const bool in = m & kNmIn;
-      un.v[e] = in ? out : T(0);
-      if (ACC && in && r.own) {
-        const double v = (double)out * (double)out * h3;
-        rs.add(e, lc, &v, tab, norms);
-      }
+      un.v[e] = (m & kNmIn) ? out : T(0);
     }
     if (r.own) stq(Unew + r.a, un);
   }
-  if (ACC) rs.finish_warp(tab, norms);
 }
 
 // Same-label neighbour mask of the interior points (kNmIp ..) of plane i, block column bx: the updates read
 // it in place of six neighbour labels while the labels do not change.  The face bytes are 0 from the
 // allocation.
-template <bool S1>
+template <int ROW>
 __device__ __forceinline__ void nm_mask_body(const int* __restrict__ label, unsigned char* __restrict__ mask, const Geo& g,
                                              int bx, int i) {
   const VGroup r = vgroup<int>(g, i, bx);
-  const Star<int> l = vstar(VLoad<int, S1>(label, r, g));
+  const Star<int> l = vstar(VLoad<int, ROW>(label, r, g));
   if (!r.own) return;
   const VRow row = vrow(g, r, i);
   unsigned m4 = 0;
@@ -324,7 +316,6 @@ __device__ __forceinline__ void nm_mask_body(const int* __restrict__ label, unsi
   }
   *reinterpret_cast<unsigned*>(mask + r.a) = m4;
 }
-constexpr int kNmVPlanes = 4;  // planes per block of the vector update
 
 // U *= scale[label] (FP64 product, rounded once) for labels in [0, nDom) over kNmFlatChunk*256
 // points from blk.  With 16-byte aligned fields each thread moves 16-byte vectors of psi (and the
@@ -374,22 +365,47 @@ __device__ __forceinline__ void nm_apply_scale_body(T* __restrict__ U, const int
   }
 }
 
-// FP64 per-label psi^2 h^3 over kNmFlatChunk*256 points from blk (label clipped to [0, nDom))
+constexpr int kNmNormAhead = 8, kNmNormCap = 4;
+struct NormSmem {
+  DomTable<1, 128> tab;
+  RunList<1, kNmNormCap> list;
+};
+// FP64 per-label psi^2 h^3 over the interior (label clipped to [0, nDom); psi is 0 on the faces): a thread
+// walks the planes [i0, iend) of one column of the 32 x 8 tile (bx, by), so it touches the block table about
+// once per domain it crosses.  A flat walk, whose points are 256 apart, touched it at every point: 2.14 ms
+// against 0.40 ms for the 96 clusters.
 template <typename T>
-__device__ __forceinline__ void nm_norms_body(const T* __restrict__ U, const int* __restrict__ label, long long S3,
-                                              double h3, int nDom, double* __restrict__ norms, DomTable<1, 128>& tab,
-                                              long long blk) {
-  RunSum<1> rs;
+__device__ __forceinline__ void nm_norms_body(const T* __restrict__ U, const int* __restrict__ label, const Geo& g,
+                                              double h3, int nDom, double* __restrict__ norms, NormSmem& sm, int bx,
+                                              int by, int i0, int iend) {
+  RunSumL<1, kNmNormCap> rs;
   rs.reset();
-  const long long base = blk * blockDim.x * kNmFlatChunk;
-  for (int q = 0; q < kNmFlatChunk; ++q) {
-    const long long id = base + (long long)q * blockDim.x + threadIdx.x;
-    if (id >= S3) break;
-    const double u = (double)U[id];
-    const double r = u * u * h3;
-    rs.add(min(max(label[id], 0), nDom - 1), &r, tab, norms);
+  const int tid = (int)(threadIdx.x + blockDim.x * threadIdx.y);
+  const int k = 1 + bx * 32 + tile_x<32>(), j = 1 + by * 8 + tile_y<32>();
+  const bool in = k < g.NN && j < g.NN;
+  const long long col = in ? (long long)j * g.S + k : 0;
+  for (int i = i0; i < iend; i += kNmNormAhead) {  // the loads of some planes ahead of their sums, whose table
+    T u[kNmNormAhead];                             // atomics the compiler does not move loads across
+    int l[kNmNormAhead];
+#pragma unroll
+    for (int q = 0; q < kNmNormAhead; ++q) {
+      const long long id = (long long)min(i + q, g.NN) * g.S2 + col;
+      u[q] = __ldg(U + id);
+      l[q] = __ldg(label + id);
+    }
+#pragma unroll
+    for (int q = 0; q < kNmNormAhead; ++q) {
+      const bool on = in && i + q < iend;
+      const double r = on ? (double)u[q] * (double)u[q] * h3 : 0.0;
+      rs.add(on ? min(max(l[q], 0), nDom - 1) : -1, &r, sm.list, tid, sm.tab, norms);
+    }
   }
-  rs.finish(tab, norms);
+  rs.finish(sm.list, tid, sm.tab, norms);
+}
+constexpr int kNmNormPlanes = 16;
+inline dim3 nm_norms_grid(const Geo& g) {
+  const unsigned n = (unsigned)(g.NN - 1);
+  return dim3((n + 31) / 32, (n + 7) / 8, (n + kNmNormPlanes - 1) / kNmNormPlanes);
 }
 
 // fine-level right-hand side f = (2 pi psi) psi formed from psi on the fly
@@ -407,15 +423,14 @@ __device__ __forceinline__ T rhs_at(const T* __restrict__ f, long long id) {
 // group's elements alternate colours: the pass updates elements COLOR, COLOR + 2 and needs a shuffle only
 // for the one whose neighbour is in the next lane.  The pass is in place: it reads points of the other
 // colour only, which it does not write, and stores its own one by one.
-constexpr int kNmRbPlanes = 2;  // planes per block
-template <typename T, bool FINE, bool S1, int COLOR>
+template <typename T, bool FINE, int ROW, int COLOR>
 __device__ __forceinline__ void nm_vrbgs_body(T* __restrict__ P, const T* __restrict__ f, const Geo& g, T h2, int bx,
                                               int i0, int iend) {
   using A = Ar<T>;
   constexpr int W = Vec<T>::W;
   for (int i = i0; i < iend; ++i) {
     const VGroup r = vgroup<T>(g, i, bx);
-    const VLoad<T, S1, false> l(P, r, g);
+    const VLoad<T, ROW, false> l(P, r, g);
     const Quad<T> fq = ldq<T>(f + r.a);
     const VRow row = vrow(g, r, i);
     auto next = [&](const Quad<T>& q, int e) { return e + 1 < W ? q.v[(e + 1) % W] : __shfl_down_sync(0xffffffffu, q.v[0], 1); };
@@ -423,7 +438,8 @@ __device__ __forceinline__ void nm_vrbgs_body(T* __restrict__ P, const T* __rest
 #pragma unroll
     for (int e = COLOR; e < W; e += 2) {
       const T ip = next(l.ip, e), im = prev(l.im, e);
-      const T jp = S1 ? next(l.jp, e) : prev(l.jp, e), jm = S1 ? prev(l.jm, e) : next(l.jm, e);
+      const T n = next(l.jn, e), v = prev(l.jv, e);
+      const T jp = l.up ? n : v, jm = l.up ? v : n;
       const T kp = next(l.c, e), km = prev(l.c, e);
       const T s = A::add(A::add(A::add(A::add(A::add(ip, im), jp), jm), kp), km);
       T rhs = fq.v[e];
@@ -761,6 +777,11 @@ __device__ __forceinline__ void nm_coarsest_body(T* __restrict__ P, const T* __r
   for (long long q = threadIdx.x; q < g.S3; q += blockDim.x) P[q] = (T)sP[q];
 }
 
+constexpr int kNmEnergyCap = 2;
+struct EnergySmem {
+  DomTable<kNmPD, 128> tab;
+  RunList<kNmPD, kNmEnergyCap> list;
+};
 // Per-domain readout sums, kNmPD per domain: (norm, T, V_eK, h^3 sum P rho, h^3 sum P (A P)) on the
 // march tile, A = -lap_h with Dirichlet faces (the multigrid's operator).  T counts every
 // same-label edge with an interior end point once (forward edges + the edge to the Dirichlet face
@@ -773,38 +794,44 @@ __device__ __forceinline__ void nm_coarsest_body(T* __restrict__ P, const T* __r
 template <typename T>
 __device__ __forceinline__ void nm_energy_body(const T* __restrict__ U, const T* __restrict__ K, const T* __restrict__ P,
                                                const int* __restrict__ label, const Geo& g, double h, int nDom,
-                                               double* __restrict__ pd, DomTable<kNmPD, 128>& tab, int bx, int by,
-                                               int bz, const double* __restrict__ K64 = nullptr,
-                                               const NmTile t = kNmTile) {
-  RunSum<kNmPD> rs;
+                                               double* __restrict__ pd, EnergySmem& sm, int bx, int by, int bz,
+                                               const double* __restrict__ K64 = nullptr, const NmTile t = kNmTile) {
+  RunSumL<kNmPD, kNmEnergyCap> rs;
   rs.reset();
+  const int tid = (int)(threadIdx.x + blockDim.x * threadIdx.y);
   const double h3 = h * h * h;
   int k, j, i0;
   nm_tile_origin(t, bx, by, bz, k, j, i0);
-  if (k < g.NN && j < g.NN && i0 < g.NN) {
-    const int iend = min(i0 + t.march, g.NN);
-    const long long S = g.S, S2 = g.S2;
-    for (int i = i0; i < iend; ++i) {
+  const int iend = min(i0 + t.march, g.NN);  // uniform over the block
+  const bool col = k < g.NN && j < g.NN;
+  const long long S = g.S, S2 = g.S2;
+  for (int i = i0; i < iend; ++i) {
+    double v[kNmPD] = {};
+    int L = -1;
+    if (col) {
       const long long id = (long long)i * S2 + j * S + k;
-      const double u = U[id], rho = u * u;
-      const int L = label[id];
-      if (L < 0 || L >= nDom) continue;
-      const double a = (label[id + S2] == L) ? (double)U[id + S2] - u : 0.0;
-      const double b = (label[id + S] == L) ? (double)U[id + S] - u : 0.0;
-      const double c = (label[id + 1] == L) ? (double)U[id + 1] - u : 0.0;
-      double t = a * a + b * b + c * c;
-      if (i == 1 && label[id - S2] == L) t += u * u;
-      if (j == 1 && label[id - S] == L) t += u * u;
-      if (k == 1 && label[id - 1] == L) t += u * u;
-      const double pc = (double)P[id];
-      const double ap = (6.0 * pc - ((double)P[id + S2] + (double)P[id - S2] + (double)P[id + S] + (double)P[id - S] +
-                                     (double)P[id + 1] + (double)P[id - 1])) / (h * h);
-      const double kv = K64 ? K64[id] : (double)K[id];
-      double v[kNmPD] = {rho * h3, 0.5 * t * h, -kv * rho * h3, pc * rho * h3, pc * ap * h3};
-      rs.add(L, v, tab, pd);
+      L = label[id];
+      if (L < 0 || L >= nDom) {
+        L = -1;
+      } else {
+        const double u = U[id], rho = u * u;
+        const double a = (label[id + S2] == L) ? (double)U[id + S2] - u : 0.0;
+        const double b = (label[id + S] == L) ? (double)U[id + S] - u : 0.0;
+        const double c = (label[id + 1] == L) ? (double)U[id + 1] - u : 0.0;
+        double tt = a * a + b * b + c * c;
+        if (i == 1 && label[id - S2] == L) tt += u * u;
+        if (j == 1 && label[id - S] == L) tt += u * u;
+        if (k == 1 && label[id - 1] == L) tt += u * u;
+        const double pc = (double)P[id];
+        const double ap = (6.0 * pc - ((double)P[id + S2] + (double)P[id - S2] + (double)P[id + S] + (double)P[id - S] +
+                                       (double)P[id + 1] + (double)P[id - 1])) / (h * h);
+        const double kv = K64 ? K64[id] : (double)K[id];
+        v[0] = rho * h3; v[1] = 0.5 * tt * h; v[2] = -kv * rho * h3; v[3] = pc * rho * h3; v[4] = pc * ap * h3;
+      }
     }
+    rs.add(L, v, sm.list, tid, sm.tab, pd);
   }
-  rs.finish_warp(tab, pd);
+  rs.finish(sm.list, tid, sm.tab, pd);
 }
 
 // level-set label update (molecule.js:426-540 rule) on psi of type T, march tile

@@ -175,8 +175,9 @@ static int nm_step_t(rq_ctx* c, int s) {
   if (c->adj.cap > 0 && (rc = nm_adj_record_step(c, s % f.poisson_interval == 0, norm)) != RQ_OK) return rc;
   if (norm) CK(cudaMemsetAsync(c->dnorm, 0, sizeof(double) * c->n_atoms, c->st));
   const bool sr = !c->fp64 && f.fp32_rounding == 1;
-  // bytes: psi, K, P read, psi' written, the neighbour mask; the centre label where it is needed
-  LAUNCH(RQ_KC_UPDATE, (4.0 * sizeof(T) + 1.0 + ((norm || c->nm_pending) ? 4.0 : 0.0)) * interior(c->g),
+  // bytes: psi, K, P read, psi' written, the neighbour mask; the centre label under a pending scale; the norms'
+  // second read of psi and the labels
+  LAUNCH(RQ_KC_UPDATE, (4.0 * sizeof(T) + 1.0 + (c->nm_pending ? 4.0 : 0.0) + (norm ? sizeof(T) + 4.0 : 0.0)) * interior(c->g),
          nm_update<T>((const T*)c->U[c->cu], (T*)c->U[1 - c->cu], (const T*)c->K, (const T*)c->P[c->cp], c->lab[c->cl],
                       c->g, (T)c->half_dv, (T)c->dt, c->h3, c->n_atoms, norm ? c->dnorm : nullptr, c->st,
                       c->nm_pending ? (const double*)c->scale64 : nullptr, sr ? c->rseed + c->cu : nullptr,

@@ -24,32 +24,22 @@ __global__ void __launch_bounds__(256) k_nm_init(T* U, int* label, const float4*
   nm_init_body<T>(U, label, seeds, nSeed, g, h, blockIdx.x, ss);
 }
 
-template <bool S1>
+template <int ROW>
 __global__ void __launch_bounds__(256) k_nm_mask(const int* __restrict__ label, unsigned char* __restrict__ mask, Geo g) {
-  nm_mask_body<S1>(label, mask, g, blockIdx.x, 1 + (int)blockIdx.y);
+  nm_mask_body<ROW>(label, mask, g, blockIdx.x, 1 + (int)blockIdx.y);
 }
 
 // mask: the same-label neighbour mask of `label`.  seed[0]: the step seed of the unbiased fp32 rounding
 // (null: round to nearest); the next step's seed, seed[0] + 1, goes to seed_next (read and written in
 // different words, so every block reads the same value)
-template <typename T, bool ACC, bool SR, bool S1>
+template <typename T, bool SR, int ROW>
 __global__ void __launch_bounds__(256) k_nm_update(const T* U, T* Unew, const T* K, const T* P, const int* label, Geo g,
-                                                   T half_dv, T dt, double h3, int nDom, double* norms, const double* scale,
-                                                   const unsigned* seed, unsigned* seed_next,
-                                                   const unsigned char* __restrict__ mask, int planes) {
-  __shared__ DomTable<1, 128> tab;
+                                                   T half_dv, T dt, int nDom, const double* scale, const unsigned* seed,
+                                                   unsigned* seed_next, const unsigned char* __restrict__ mask, int planes) {
   if (SR && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *seed_next = *seed + 1u;
-  if (ACC) {
-    dom_table_init(tab);
-    __syncthreads();
-  }
   const int i0 = 1 + (int)blockIdx.y * planes;
-  nm_vupdate_body<T, ACC, SR, S1>(U, Unew, K, P, label, mask, g, half_dv, dt, h3, nDom, norms, tab, blockIdx.x, i0,
-                                  min(i0 + planes, g.NN), scale, seed);
-  if (ACC) {
-    __syncthreads();
-    dom_table_flush(tab, norms);
-  }
+  nm_vupdate_body<T, SR, ROW>(U, Unew, K, P, label, mask, g, half_dv, dt, nDom, blockIdx.x, i0, min(i0 + planes, g.NN),
+                              scale, seed);
 }
 
 // scale[l] = sqrt(Zdom_l / n_l) (FP64) for every domain of the (concatenated) arrays; a norm
@@ -67,20 +57,20 @@ __global__ void __launch_bounds__(256) k_nm_apply_scale(T* U, const int* label, 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_nm_norms(const T* U, const int* label, long long S3, double h3, int nDom,
-                                                  double* norms) {
-  __shared__ DomTable<1, 128> tab;
-  dom_table_init(tab);
+__global__ void __launch_bounds__(256) k_nm_norms(const T* U, const int* label, Geo g, double h3, int nDom, double* norms) {
+  __shared__ NormSmem sm;
+  dom_table_init(sm.tab);
   __syncthreads();
-  nm_norms_body<T>(U, label, S3, h3, nDom, norms, tab, blockIdx.x);
+  const int i0 = 1 + (int)blockIdx.z * kNmNormPlanes;
+  nm_norms_body<T>(U, label, g, h3, nDom, norms, sm, blockIdx.x, blockIdx.y, i0, min(i0 + kNmNormPlanes, g.NN));
   __syncthreads();
-  dom_table_flush(tab, norms);
+  dom_table_flush(sm.tab, norms);
 }
 
-template <typename T, bool FINE, bool S1, int COLOR>
+template <typename T, bool FINE, int ROW, int COLOR>
 __global__ void __launch_bounds__(256) k_nm_rbgs(T* P, const T* f, Geo g, T h2, int planes) {
   const int i0 = 1 + (int)blockIdx.y * planes;
-  nm_vrbgs_body<T, FINE, S1, COLOR>(P, f, g, h2, blockIdx.x, i0, min(i0 + planes, g.NN));
+  nm_vrbgs_body<T, FINE, ROW, COLOR>(P, f, g, h2, blockIdx.x, i0, min(i0 + planes, g.NN));
 }
 
 template <typename T, bool FINE>
@@ -104,12 +94,12 @@ __global__ void __launch_bounds__(1024) k_nm_coarsest(T* P, const T* f, Geo g, d
 template <typename T>
 __global__ void __launch_bounds__(256) k_nm_energy(const T* U, const T* K, const T* P, const int* label, Geo g, double h,
                                                    int nDom, double* pd, const double* K64) {
-  __shared__ DomTable<kNmPD, 128> tab;
-  dom_table_init(tab);
+  __shared__ EnergySmem sm;
+  dom_table_init(sm.tab);
   __syncthreads();
-  nm_energy_body<T>(U, K, P, label, g, h, nDom, pd, tab, blockIdx.x, blockIdx.y, blockIdx.z, K64);
+  nm_energy_body<T>(U, K, P, label, g, h, nDom, pd, sm, blockIdx.x, blockIdx.y, blockIdx.z, K64);
   __syncthreads();
-  dom_table_flush(tab, pd);
+  dom_table_flush(sm.tab, pd);
 }
 
 template <typename T>
@@ -140,6 +130,8 @@ __global__ void k_nm_add(T* __restrict__ K, const T* __restrict__ v, long long n
 // ======================================================================================
 // host launchers (T = float or double)
 // ======================================================================================
+using RowP = std::integral_constant<int, kRowP>;
+using RowM = std::integral_constant<int, kRowM>;
 static unsigned nblk(long long n, long long b = 256) { return (unsigned)((n + b - 1) / b); }
 
 template <typename T>
@@ -158,23 +150,23 @@ cudaError_t nm_update(const T* U, T* Unew, const T* K, const T* P, const int* la
                       double h3, int nDom, double* norms, cudaStream_t st, const double* scale, const unsigned* seed,
                       unsigned* seed_next, const unsigned char* mask) {
   if (g.NN < 2) return cudaSuccess;
-  auto go = [&](auto acc, auto sr, auto s1) {
-    const int planes = vplanes<T>(g, decltype(acc)::value);
-    k_nm_update<T, decltype(acc)::value, decltype(sr)::value, decltype(s1)::value><<<vgrid<T>(g, planes), 256, 0, st>>>(
-        U, Unew, K, P, label, g, half_dv, dt, h3, nDom, norms, scale, seed, seed_next, mask, planes);
+  const int planes = vplanes<T>(g, false);
+  auto go = [&](auto sr, auto row) {
+    k_nm_update<T, decltype(sr)::value, decltype(row)::value><<<vgrid<T>(g, planes), 256, 0, st>>>(
+        U, Unew, K, P, label, g, half_dv, dt, nDom, scale, seed, seed_next, mask, planes);
   };
   using Y = std::true_type;
   using N = std::false_type;
-  auto go2 = [&](auto acc, auto sr) { if (g.S % 4 == 1) go(acc, sr, Y{}); else go(acc, sr, N{}); };
-  if (norms) { if (seed) go2(Y{}, Y{}); else go2(Y{}, N{}); }
-  else       { if (seed) go2(N{}, Y{}); else go2(N{}, N{}); }
+  if (g.S % 4 == 1) { if (seed) go(Y{}, RowP{}); else go(N{}, RowP{}); }
+  else              { if (seed) go(Y{}, RowM{}); else go(N{}, RowM{}); }
+  if (norms) k_nm_norms<T><<<nm_norms_grid(g), 256, 0, st>>>(Unew, label, g, h3, nDom, norms);
   return cudaGetLastError();
 }
 cudaError_t nm_mask(const int* label, unsigned char* mask, const Geo& g, cudaStream_t st) {
   if (g.S % 4 == 1)
-    k_nm_mask<true><<<vgrid<int>(g, 1), 256, 0, st>>>(label, mask, g);
+    k_nm_mask<kRowP><<<vgrid<int>(g, 1), 256, 0, st>>>(label, mask, g);
   else
-    k_nm_mask<false><<<vgrid<int>(g, 1), 256, 0, st>>>(label, mask, g);
+    k_nm_mask<kRowM><<<vgrid<int>(g, 1), 256, 0, st>>>(label, mask, g);
   return cudaGetLastError();
 }
 template <typename T>
@@ -196,23 +188,23 @@ cudaError_t nm_norm_scale(const double* norms, const double* Zdom, int nDom, dou
 }
 template <typename T>
 cudaError_t nm_norms(const T* U, const int* label, const Geo& g, double h3, int nDom, double* norms, cudaStream_t st) {
-  k_nm_norms<T><<<nblk(g.S3, 256 * kNmFlatChunk), 256, 0, st>>>(U, label, g.S3, h3, nDom, norms);
+  k_nm_norms<T><<<nm_norms_grid(g), 256, 0, st>>>(U, label, g, h3, nDom, norms);
   return cudaGetLastError();
 }
 template <typename T>
 cudaError_t nm_rbgs(T* P, const T* f, bool fine, const Geo& g, double h2, int color, cudaStream_t st) {
   const int planes = vplanes<T>(g, false);
   const dim3 grd = vgrid<T>(g, planes);
-  auto go = [&](auto fn, auto s1) {
+  auto go = [&](auto fn, auto row) {
     if (color)
-      k_nm_rbgs<T, decltype(fn)::value, decltype(s1)::value, 1><<<grd, 256, 0, st>>>(P, f, g, (T)h2, planes);
+      k_nm_rbgs<T, decltype(fn)::value, decltype(row)::value, 1><<<grd, 256, 0, st>>>(P, f, g, (T)h2, planes);
     else
-      k_nm_rbgs<T, decltype(fn)::value, decltype(s1)::value, 0><<<grd, 256, 0, st>>>(P, f, g, (T)h2, planes);
+      k_nm_rbgs<T, decltype(fn)::value, decltype(row)::value, 0><<<grd, 256, 0, st>>>(P, f, g, (T)h2, planes);
   };
   using Y = std::true_type;
   using N = std::false_type;
-  if (g.S % 4 == 1) { if (fine) go(Y{}, Y{}); else go(N{}, Y{}); }
-  else              { if (fine) go(Y{}, N{}); else go(N{}, N{}); }
+  if (g.S % 4 == 1) { if (fine) go(Y{}, RowP{}); else go(N{}, RowP{}); }
+  else              { if (fine) go(Y{}, RowM{}); else go(N{}, RowM{}); }
   return cudaGetLastError();
 }
 template <typename T>

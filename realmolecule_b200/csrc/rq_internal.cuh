@@ -170,6 +170,79 @@ struct RunSum {
   }
 };
 
+// Running sums of threads that walk columns across many domains.  A thread that meets a new label parks the
+// finished (label, sums) in its own list in shared memory; at the end of the walk the warp goes through the
+// lists together, one entry per lane at a time: a butterfly merges lanes of one label, and the leaders add
+// to the block table.  Adding to the table on the spot cost a compare-and-swap loop per lane (the table's
+// FP64 adds are such loops, and a warp's lanes cross a domain face together), and a butterfly on every
+// plane 130 instructions a point.  A thread that meets more than CAP labels adds the rest on the spot.
+template <int NQ, int CAP>
+struct RunList {
+  int label[CAP][256];
+  double v[CAP][NQ][256];
+};
+
+template <int NQ, int CAP>
+struct RunSumL {
+  int label, n;
+  double v[NQ];
+  __device__ __forceinline__ void reset() {
+    label = -1;
+    n = 0;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) v[q] = 0.0;
+  }
+  // l = -1: nothing to add
+  template <int NSLOT>
+  __device__ __forceinline__ void add(int l, const double* x, RunList<NQ, CAP>& list, int tid, DomTable<NQ, NSLOT>& t,
+                                      double* global) {
+    if (l != label) {
+      if (label >= 0) {
+        if (n < CAP) {
+          list.label[n][tid] = label;
+#pragma unroll
+          for (int q = 0; q < NQ; ++q) list.v[n][q][tid] = v[q];
+          ++n;
+        } else {
+          dom_table_add(t, label, v, global);
+        }
+      }
+      label = l;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) v[q] = x[q];
+    } else {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) v[q] += x[q];
+    }
+  }
+  // every lane of the warp together
+  template <int NSLOT>
+  __device__ __forceinline__ void finish(RunList<NQ, CAP>& list, int tid, DomTable<NQ, NSLOT>& t, double* global) {
+    const int lane = lane_id();
+    for (int s = -1; s < CAP; ++s) {  // the running entry, then the parked ones
+      int fl = label;
+      if (s >= 0) {
+        fl = s < n ? list.label[s][tid] : -1;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) v[q] = fl >= 0 ? list.v[s][q][tid] : 0.0;
+        if (!__any_sync(0xffffffffu, fl >= 0)) break;
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int ol = __shfl_xor_sync(0xffffffffu, fl, o);
+        const bool same = ol == fl;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+          const double y = __shfl_xor_sync(0xffffffffu, v[q], o);
+          if (same && !(lane & o)) v[q] += y;
+        }
+        if (same && (lane & o)) fl = -1;
+      }
+      if (fl >= 0) dom_table_add(t, fl, v, global);
+    }
+  }
+};
+
 // Weight Z/N that turns a domain's energy partials (each linear in its density for a fixed P)
 // into those of the exactly normalised domain; 1 when Z or the measured norm N is not positive.
 inline double domain_norm_weight(double Z, double N) { return (Z > 0.0 && N > 0.0) ? Z / N : 1.0; }

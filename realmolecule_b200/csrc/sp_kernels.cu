@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(256) k_jacobi_sp(const float* __restrict__ P, 
 // mask byte; write psi', P' = 21 B per point.  Bound: HBM at 300^3 (95 us, 5.9 TB/s, where the scalar
 // march over labels took 165 us), L2 and latency at 128^3 (10.2 us against 14.4 us in the replayed period).
 // ---------------------------------------------------------------------------------------
-template <bool FIRST, bool ACC, bool S1>
+template <bool FIRST, bool ACC, int ROW>
 __global__ void __launch_bounds__(256) k_step_sp(const float* __restrict__ U, float* __restrict__ Unew,
                                                  const float* __restrict__ K, const float* __restrict__ P,
                                                  float* __restrict__ Pnew, const unsigned char* __restrict__ mask,
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(256) k_step_sp(const float* __restrict__ U, fl
   const int i0 = 1 + (int)blockIdx.y * planes, iend = min(i0 + planes, g.NN);
   for (int i = i0; i < iend; ++i) {
     const VGroup r = vgroup<float>(g, i, (int)blockIdx.x);
-    const VLoad<float, S1> lu(U, r, g), lp(P, r, g);
+    const VLoad<float, ROW> lu(U, r, g), lp(P, r, g);
     const Quad<float> kv = ldq<float>(K + r.a);
     const unsigned m4 = vbytes<float>(mask, r);
     const Star<float> u = vstar(lu), p = vstar(lp);
@@ -608,13 +608,15 @@ cudaError_t launch_step_sp(bool first, const float* U, float* Unew, const float*
   if (g.NN < 2) return cudaSuccess;
   // 300^3: 16.6 ms a 100-step period with 4 planes, 17.3 with 1; 128^3: 1.09 and 1.07 ms
   const int planes = vplanes<float>(g, norms != nullptr);
-  auto go = [&](auto f, auto acc, auto s1) {
-    k_step_sp<decltype(f)::value, decltype(acc)::value, decltype(s1)::value><<<vgrid<float>(g, planes), 256, 0, st>>>(
+  auto go = [&](auto f, auto acc, auto row) {
+    k_step_sp<decltype(f)::value, decltype(acc)::value, decltype(row)::value><<<vgrid<float>(g, planes), 256, 0, st>>>(
         U, Unew, K, P, Pnew, mask, label, g, half_dv, dtv, h2, coeff, h3, nDom, norms, planes);
   };
   using Y = std::true_type;
   using N = std::false_type;
-  auto go2 = [&](auto f, auto acc) { if (g.S % 4 == 1) go(f, acc, Y{}); else go(f, acc, N{}); };
+  using RowP = std::integral_constant<int, kRowP>;
+  using RowM = std::integral_constant<int, kRowM>;
+  auto go2 = [&](auto f, auto acc) { if (g.S % 4 == 1) go(f, acc, RowP{}); else go(f, acc, RowM{}); };
   if (first) { if (norms) go2(Y{}, Y{}); else go2(Y{}, N{}); }
   else       { if (norms) go2(N{}, Y{}); else go2(N{}, N{}); }
   return cudaGetLastError();

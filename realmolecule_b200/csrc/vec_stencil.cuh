@@ -104,21 +104,26 @@ __device__ __forceinline__ bool vinterior(const Geo& g, const VRow& r, int e) {
 // the next lane's first element; d = -1 mod W the aligned group at a + d + 1 and the previous lane's last.
 // Every load is issued by the constructor of VLoad (the shuffles of vstar would otherwise order them), so
 // a thread has all its vectors in flight at once.  LDG: through the read-only path (not for a field the
-// pass writes).  S1: S = 1 mod 4, else 3 mod 4 (for W = 2 both forms are the same shift).
-template <typename T, bool S1, bool LDG = true> struct VLoad {
-  Quad<T> ip, im, jp, jm, c;
+// pass writes).  ROW: the form of the +-S shifts, kRowP for S = 1 mod 4 (+S is the one taken from the next
+// lane), kRowM for 3 mod 4, kRowAny decided at run time by a swap (batches, whose grids differ; the two
+// forms side by side cost registers).  For W = 2 both forms are the same shift.
+constexpr int kRowP = 1, kRowM = 0, kRowAny = 2;
+template <typename T, int ROW, bool LDG = true> struct VLoad {
+  Quad<T> ip, im, jn, jv, c;  // jn: the row shift taken from the next lane, jv: from the previous
+  bool up;                    // jn is +S
   static __device__ __forceinline__ Quad<T> q(const T* p) {
     if (LDG) return ldq<T>(p);
     return *reinterpret_cast<const Quad<T>*>(p);
   }
   __device__ __forceinline__ VLoad(const T* p, const VGroup& r, const Geo& g) {
     const T* x = p + r.a;
-    const long long S = g.S, S2 = g.S2;
+    up = ROW == kRowAny ? (g.S & 3) == 1 : ROW == kRowP;
+    const long long S = up ? (long long)g.S : -(long long)g.S, S2 = g.S2;
     c = q(x);
     ip = q(x + S2 - 1);
     im = q(x - S2 + 1);
-    jp = q(S1 ? x + S - 1 : x + S + 1);
-    jm = q(S1 ? x - S + 1 : x - S - 1);
+    jn = q(x + S - 1);
+    jv = q(x - S + 1);
   }
 };
 template <typename T> struct Star {
@@ -142,14 +147,18 @@ __device__ __forceinline__ Quad<T> vprev(const Quad<T>& q) {  // the run shifted
   o.v[0] = __shfl_up_sync(0xffffffffu, q.v[W - 1], 1);
   return o;
 }
-template <typename T, bool S1, bool LDG>
-__device__ __forceinline__ Star<T> vstar(const VLoad<T, S1, LDG>& l) {
+template <typename T, int ROW, bool LDG>
+__device__ __forceinline__ Star<T> vstar(const VLoad<T, ROW, LDG>& l) {
   Star<T> s;
   s.c = l.c;
   s.ip = vnext(l.ip);
   s.im = vprev(l.im);
-  s.jp = S1 ? vnext(l.jp) : vprev(l.jp);
-  s.jm = S1 ? vprev(l.jm) : vnext(l.jm);
+  const Quad<T> n = vnext(l.jn), v = vprev(l.jv);
+#pragma unroll
+  for (int e = 0; e < Vec<T>::W; ++e) {
+    s.jp.v[e] = l.up ? n.v[e] : v.v[e];
+    s.jm.v[e] = l.up ? v.v[e] : n.v[e];
+  }
   s.kp = vnext(l.c);
   s.km = vprev(l.c);
   return s;
@@ -173,62 +182,6 @@ __device__ __forceinline__ void vlabels(const int* __restrict__ label, const VGr
     l[0] = x.x; l[1] = x.y;
   }
 }
-
-// Running (label, NQ sums) of each of a thread's W columns while it walks planes: a column meets a new
-// label about once per domain it crosses, and only then touches the block table (RunSum, per column).
-template <int NQ, int W> struct RunCols {
-  int label[W];
-  double v[W][NQ];
-  __device__ __forceinline__ void reset() {
-#pragma unroll
-    for (int e = 0; e < W; ++e) {
-      label[e] = -1;
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) v[e][q] = 0.0;
-    }
-  }
-  template <int NSLOT>
-  __device__ __forceinline__ void add(int e, int l, const double* x, DomTable<NQ, NSLOT>& t, double* global) {
-    if (l != label[e]) {
-      if (label[e] >= 0) dom_table_add(t, label[e], v[e], global);
-      label[e] = l;
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) v[e][q] = x[q];
-    } else {
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) v[e][q] += x[q];
-    }
-  }
-  // every lane of the warp together: a thread's columns of one label are merged, then runs of lanes with
-  // one label by a butterfly, so the table sees about one add per label and warp
-  template <int NSLOT>
-  __device__ __forceinline__ void finish_warp(DomTable<NQ, NSLOT>& t, double* global) {
-#pragma unroll
-    for (int e = W - 1; e > 0; --e) {
-      if (label[e] < 0) continue;
-      if (label[e] == label[e - 1] || label[e - 1] < 0) {
-        label[e - 1] = label[e];
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) v[e - 1][q] += v[e][q];
-      } else {
-        dom_table_add(t, label[e], v[e], global);
-      }
-    }
-    const int lane = (int)threadIdx.x & 31;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int ol = __shfl_xor_sync(0xffffffffu, label[0], o);
-      const bool same = ol == label[0];
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        const double x = __shfl_xor_sync(0xffffffffu, v[0][q], o);
-        if (same && !(lane & o)) v[0][q] += x;
-      }
-      if (same && (lane & o)) label[0] = -1;
-    }
-    if (label[0] >= 0) dom_table_add(t, label[0], v[0], global);
-  }
-};
 
 // x / 6 correctly rounded, by the two-constant product of Brisebarre, Muller and Raina ("Accelerating
 // correctly rounded floating-point division when the divisor is known in advance", 2004): zh + zl is 1/6
