@@ -27,10 +27,12 @@
 // actually reaches after a finite number of warm-started iterations.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <cstring>
 
 #include "nm_bodies.cuh"
 #include "rq_flavors.h"
+#include "vec_stencil.cuh"
 
 using namespace rq;
 
@@ -101,28 +103,41 @@ __global__ void __launch_bounds__(256) k_adj_seed(const T* __restrict__ U, const
   gK[id] = -w * h3 * u * u;
 }
 
-// per-domain <psi, lam> in FP64 over all S^3 points
+// per-domain <psi, lam> in FP64 over the interior (both are 0 on the faces), by columns as nm_norms_body
 template <typename T>
 __global__ void __launch_bounds__(256) k_adj_dot(const T* __restrict__ psi, const T* __restrict__ lam,
-                                                 const int* __restrict__ label, long long S3, int nDom,
+                                                 const int* __restrict__ label, Geo g, int nDom,
                                                  double* __restrict__ dots) {
-  __shared__ DomTable<1, 128> tab;
-  dom_table_init(tab);
+  __shared__ NormSmem sm;
+  dom_table_init(sm.tab);
   __syncthreads();
-  RunSum<1> rs;
+  RunSumL<1, kNmNormCap> rs;
   rs.reset();
-  const long long base = (long long)blockIdx.x * blockDim.x * kNmFlatChunk;
-  for (int t = 0; t < kNmFlatChunk; ++t) {
-    const long long id = base + (long long)t * blockDim.x + threadIdx.x;
-    if (id >= S3) break;
-    const int l = label[id];
-    if (l < 0 || l >= nDom) continue;
-    const double v = (double)psi[id] * (double)lam[id];
-    rs.add(l, &v, tab, dots);
+  const int tid = (int)threadIdx.x, k = 1 + (int)blockIdx.x * 32 + (tid & 31), j = 1 + (int)blockIdx.y * 8 + (tid >> 5);
+  const int i0 = 1 + (int)blockIdx.z * kNmNormPlanes, iend = min(i0 + kNmNormPlanes, g.NN);
+  const bool in = k < g.NN && j < g.NN;
+  const long long col = in ? (long long)j * g.S + k : 0;
+  constexpr int AH = 4;  // planes loaded ahead of their sums
+  for (int i = i0; i < iend; i += AH) {
+    T p[AH], q[AH];
+    int l[AH];
+#pragma unroll
+    for (int t = 0; t < AH; ++t) {
+      const long long id = (long long)min(i + t, g.NN) * g.S2 + col;
+      p[t] = __ldg(psi + id);
+      q[t] = __ldg(lam + id);
+      l[t] = __ldg(label + id);
+    }
+#pragma unroll
+    for (int t = 0; t < AH; ++t) {
+      const bool on = in && i + t < iend && l[t] >= 0 && l[t] < nDom;
+      const double v = on ? (double)p[t] * (double)q[t] : 0.0;
+      rs.add(on ? l[t] : -1, &v, sm.list, tid, sm.tab, dots);
+    }
   }
-  rs.finish(tab, dots);
+  rs.finish(sm.list, tid, sm.tab, dots);
   __syncthreads();
-  dom_table_flush(tab, dots);
+  dom_table_flush(sm.tab, dots);
 }
 
 // per-domain (c, beta) of a transposed normalisation: c = the forward scale, beta = c h^3 <psi, lam> / Z
@@ -135,43 +150,220 @@ __global__ void k_adj_norm_coef(const double* __restrict__ scale, const double* 
   coef[2 * d + 1] = Z > 0.0 ? c * h3 * dots[d] / Z : 0.0;
 }
 
-// lam <- c lam - beta psi per domain (boundary points hold 0 in both and stay 0)
-template <typename T>
-__global__ void __launch_bounds__(256) k_adj_norm_apply(T* __restrict__ lam, const T* __restrict__ psi,
-                                                        const int* __restrict__ label, const double* __restrict__ coef,
-                                                        long long S3, int nDom) {
-  const long long base = (long long)blockIdx.x * blockDim.x * kNmFlatChunk;
-  for (int t = 0; t < kNmFlatChunk; ++t) {
-    const long long id = base + (long long)t * blockDim.x + threadIdx.x;
-    if (id >= S3) break;
-    const int l = label[id];
-    if (l < 0 || l >= nDom) continue;
-    lam[id] = (T)(coef[2 * l] * (double)lam[id] - coef[2 * l + 1] * (double)psi[id]);
+// update^T on 16-byte groups: out = A(K, P) in.  With NORM the input is first normalised (transposed):
+// in <- c in - beta psi_s with the domain's (c, beta), rounded to T; the same-label neighbours share the
+// centre's, so the pass needs psi_s where it needs `in`, and the normalised input goes to `inn` for the
+// accumulation below.
+template <typename T, bool NORM, int ROW>
+__global__ void __launch_bounds__(256) k_adj_update(const T* __restrict__ in, T* __restrict__ inn, T* __restrict__ out,
+                                                    const T* __restrict__ K, const T* __restrict__ P,
+                                                    const unsigned char* __restrict__ mask, const int* __restrict__ label,
+                                                    const T* __restrict__ psi_s, const double* __restrict__ coef, Geo g,
+                                                    double half_dv, double dt, int nDom, int planes) {
+  constexpr int W = Vec<T>::W;
+  const int i0 = 1 + (int)blockIdx.y * planes, iend = min(i0 + planes, g.NN);
+  for (int i = i0; i < iend; ++i) {
+    const VGroup r = vgroup<T>(g, i, blockIdx.x);
+    const VLoad<T, ROW> l(in, r, g);
+    const Quad<T> kq = ldq<T>(K + r.a), pq = ldq<T>(P + r.a);
+    const unsigned mw = vbytes<T>(mask, r);
+    Quad<T> o, n;
+    auto point = [&](int e, const Star<T>& u, auto val) {  // val(neighbour element) -> its (normalised) value
+      const unsigned m = mw >> (8 * e);
+      const double lc = val(u.c.v[e], 0);
+      double lap = 0.0;
+      if (m & kNmIp) lap += val(u.ip.v[e], 1) - lc;
+      if (m & kNmIm) lap += val(u.im.v[e], 2) - lc;
+      if (m & kNmJp) lap += val(u.jp.v[e], 3) - lc;
+      if (m & kNmJm) lap += val(u.jm.v[e], 4) - lc;
+      if (m & kNmKp) lap += val(u.kp.v[e], 5) - lc;
+      if (m & kNmKm) lap += val(u.km.v[e], 6) - lc;
+      o.v[e] = (m & kNmIn) ? (T)(lc + half_dv * lap + dt * ((double)kq.v[e] - 2.0 * (double)pq.v[e]) * lc) : T(0);
+      n.v[e] = (T)lc;
+    };
+    if constexpr (NORM) {
+      const VLoad<T, ROW> lp(psi_s, r, g);
+      int lab[W];
+      vlabels<T>(label, r, lab);
+      const Star<T> u = vstar(l), s = vstar(lp);
+#pragma unroll
+      for (int e = 0; e < W; ++e) {
+        const bool ok = lab[e] >= 0 && lab[e] < nDom;
+        const double c = ok ? coef[2 * lab[e]] : 1.0, b = ok ? coef[2 * lab[e] + 1] : 0.0;
+        const T sv[7] = {s.c.v[e], s.ip.v[e], s.im.v[e], s.jp.v[e], s.jm.v[e], s.kp.v[e], s.km.v[e]};
+        point(e, u, [&](T x, int q) { return ok ? (double)(T)(c * (double)x - b * (double)sv[q]) : (double)x; });
+      }
+      if (r.own) stq(inn + r.a, n);
+    } else {
+      const Star<T> u = vstar(l);
+#pragma unroll
+      for (int e = 0; e < W; ++e) point(e, u, [](T x, int) { return (double)x; });
+    }
+    if (r.own) stq(out + r.a, o);
   }
 }
 
-// update^T: out = A(K, P) in (the update's operator applied to lam), gK += dt psi in,
-// muP += -2 dt psi in, where psi is the state the forward update started from
+// dE/dK += dt psi lam and dE/dP += -2 dt psi lam of up to kAdjPend reverse steps in one pass, in the order of
+// the steps (newest first), each muP step rounded to T: lam is the input of the step's transposed update, psi
+// the state the forward update started from.  Once per step these sums were 24 of its 45 B per point (and
+// in the kernel above a third of its loads); per group of steps dE/dK and dE/dP move once.
+constexpr int kAdjPend = 4;
+struct AdjPend {
+  const void *lam[kAdjPend], *psi[kAdjPend];
+  int n;
+};
 template <typename T>
-__global__ void __launch_bounds__(256) k_adj_update(const T* __restrict__ in, T* __restrict__ out,
-                                                    const T* __restrict__ K, const T* __restrict__ P,
-                                                    const int* __restrict__ label, const T* __restrict__ psi, Geo g,
-                                                    double half_dv, double dt, double* __restrict__ gK,
-                                                    T* __restrict__ muP) {
-  Pt p;
-  if (!interior_pt3(g, p)) return;
-  const long long id = p.id, S = g.S, S2 = g.S2;
-  const int L = label[id];
-  const double lc = (double)in[id];
-  const long long nb[6] = {id + S2, id - S2, id + S, id - S, id + 1, id - 1};
-  double lap = 0.0;
+__global__ void __launch_bounds__(256) k_adj_accum(const AdjPend p, double* __restrict__ gK, T* __restrict__ muP, double dt,
+                                                   long long S3) {
+  constexpr int W = Vec<T>::W;
+  const long long a = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * W;
+  auto sums = [&](int n, double* k, T* m, const T (*l)[W], const T (*s)[W], int w) {
+    for (int e = 0; e < w; ++e)
 #pragma unroll
-  for (int t = 0; t < 6; ++t)
-    if (label[nb[t]] == L) lap += (double)in[nb[t]] - lc;
-  out[id] = (T)(lc + half_dv * lap + dt * ((double)K[id] - 2.0 * (double)P[id]) * lc);
-  const double pv = (double)psi[id];
-  gK[id] += dt * pv * lc;
-  muP[id] = (T)((double)muP[id] - 2.0 * dt * pv * lc);
+      for (int q = 0; q < kAdjPend; ++q)
+        if (q < n) {
+          const double pv = (double)s[q][e], lc = (double)l[q][e];
+          k[e] += dt * pv * lc;
+          m[e] = (T)((double)m[e] - 2.0 * dt * pv * lc);
+        }
+  };
+  T l[kAdjPend][W], s[kAdjPend][W], m[W];
+  double k[W];
+  if (a + W <= S3) {
+#pragma unroll
+    for (int q = 0; q < kAdjPend; ++q)
+      if (q < p.n) {
+        const Quad<T> x = ldq<T>((const T*)p.lam[q] + a), y = ldq<T>((const T*)p.psi[q] + a);
+#pragma unroll
+        for (int e = 0; e < W; ++e) { l[q][e] = x.v[e]; s[q][e] = y.v[e]; }
+      }
+    Quad<T> mq = *reinterpret_cast<const Quad<T>*>(muP + a);
+    Quad<double> kq[W / 2];
+#pragma unroll
+    for (int h = 0; h < W / 2; ++h) kq[h] = *reinterpret_cast<const Quad<double>*>(gK + a + 2 * h);
+#pragma unroll
+    for (int e = 0; e < W; ++e) { m[e] = mq.v[e]; k[e] = kq[e / 2].v[e % 2]; }
+    sums(p.n, k, m, l, s, W);
+#pragma unroll
+    for (int e = 0; e < W; ++e) { mq.v[e] = m[e]; kq[e / 2].v[e % 2] = k[e]; }
+    stq(muP + a, mq);
+#pragma unroll
+    for (int h = 0; h < W / 2; ++h) stq(gK + a + 2 * h, kq[h]);
+  } else if (a < S3) {
+    const int w = (int)(S3 - a);
+    for (int e = 0; e < w; ++e) {
+      for (int q = 0; q < p.n; ++q) { l[q][e] = ((const T*)p.lam[q])[a + e]; s[q][e] = ((const T*)p.psi[q])[a + e]; }
+      m[e] = muP[a + e];
+      k[e] = gK[a + e];
+    }
+    sums(p.n, k, m, l, s, w);
+    for (int e = 0; e < w; ++e) { muP[a + e] = m[e]; gK[a + e] = k[e]; }
+  }
+}
+
+// A red-black sweep (colour 0, then 1) transposed is two half passes, colour 1 first.  With m the adjoint
+// of P after the sweep:
+//   k_adj_half   (colour 1 transposed)  m0 += (1/6) sum_6 m1, in place: the points of colour 1 are kept
+//   k_adj_other  (colour 0 transposed)  m1' = (1/6) sum_6 m0, m0' = 0, into another buffer
+// and the sweep's share of dE/df is (h^2 / 6) m between the two passes, at every point: the buffer of the
+// half pass holds it, so nothing is accumulated on the way.  The kernels before (out of place, a running
+// dE/df per colour) moved 3.5 fields per colour; values and roundings are the same.
+template <typename T, int ROW>
+__global__ void __launch_bounds__(256) k_adj_half(T* __restrict__ m, Geo g, int planes) {
+  constexpr int W = Vec<T>::W;
+  const int i0 = 1 + (int)blockIdx.y * planes, iend = min(i0 + planes, g.NN);
+  for (int i = i0; i < iend; ++i) {
+    const VGroup r = vgroup<T>(g, i, blockIdx.x);
+    const VLoad<T, ROW, false> l(m, r, g);
+    const VRow row = vrow(g, r, i);
+    const Star<T> u = vstar(l);
+#pragma unroll
+    for (int e = 0; e < W; e += 2) {  // colour 0: even ids (S is odd)
+      const double s = (double)u.ip.v[e] + (double)u.im.v[e] + (double)u.jp.v[e] + (double)u.jm.v[e] +
+                       (double)u.kp.v[e] + (double)u.km.v[e];
+      if (r.own && vinterior(g, row, e)) m[r.a + e] = (T)((double)u.c.v[e] + sixth(s));
+    }
+  }
+}
+
+// the second half pass; PRE on the finest level also takes the whole dE/df of the V-cycle -- the two
+// sweeps' shares and the residual's, muf = (h^2/6) mA + mur + (h^2/6) m, each sum rounded to T as it forms --
+// into lam += 4 pi psi muf (the right-hand side is f = 2 pi psi^2).  out may be mA's buffer.
+template <typename T, bool PRE, int ROW>
+__global__ void __launch_bounds__(256) k_adj_other(const T* __restrict__ m, T* out, const T* mA, const T* __restrict__ mur,
+                                                   const T* __restrict__ psi, T* __restrict__ lam, Geo g, double c6,
+                                                   int planes) {
+  constexpr int W = Vec<T>::W;
+  const int i0 = 1 + (int)blockIdx.y * planes, iend = min(i0 + planes, g.NN);
+  for (int i = i0; i < iend; ++i) {
+    const VGroup r = vgroup<T>(g, i, blockIdx.x);
+    const VLoad<T, ROW> l(m, r, g);
+    Quad<T> qa, qr, qs, ql;
+    if (PRE) {
+      qa = *reinterpret_cast<const Quad<T>*>(mA + r.a);
+      qr = ldq<T>(mur + r.a);
+      qs = ldq<T>(psi + r.a);
+      ql = *reinterpret_cast<const Quad<T>*>(lam + r.a);
+    }
+    const VRow row = vrow(g, r, i);
+    const Star<T> u = vstar(l);
+    Quad<T> o;
+#pragma unroll
+    for (int e = 0; e < W; ++e) {
+      const bool in = vinterior(g, row, e);
+      o.v[e] = T(0);
+      if (e & 1) {
+        const double s = (double)u.ip.v[e] + (double)u.im.v[e] + (double)u.jp.v[e] + (double)u.jm.v[e] +
+                         (double)u.kp.v[e] + (double)u.km.v[e];
+        if (in) o.v[e] = (T)(0.0 + sixth(s));
+      }
+      if (PRE && in) {
+        T f = (T)(c6 * (double)qa.v[e]);
+        f = (T)((double)f + (double)qr.v[e]);
+        f = (T)fma(c6, (double)u.c.v[e], (double)f);
+        ql.v[e] = (T)((double)ql.v[e] + 12.566370614359172 * (double)qs.v[e] * (double)f);
+      }
+    }
+    if (r.own) {
+      stq(out + r.a, o);
+      if (PRE) stq(lam + r.a, ql);
+    }
+  }
+}
+
+// the same dE/df on a coarser level (whose cycle starts from P = 0, so nothing else is needed there)
+template <typename T>
+__global__ void __launch_bounds__(256) k_adj_muf(const T* __restrict__ mA, const T* __restrict__ mur, const T* __restrict__ mB,
+                                                 T* __restrict__ muf, long long S3, double c6) {
+  const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= S3) return;
+  T f = (T)(c6 * (double)mA[q]);
+  f = (T)((double)f + (double)mur[q]);
+  muf[q] = (T)fma(c6, (double)mB[q], (double)f);
+}
+
+// residual transposed (forward r = f + (sum_6 P - 6 P) / h^2) on the adjoint of P: m += (sum_6 mur - 6 mur) / h^2
+// (its share of dE/df, mur itself, is added where dE/df is used)
+template <typename T, int ROW>
+__global__ void __launch_bounds__(256) k_adj_res(const T* __restrict__ mur, T* __restrict__ m, Geo g, double inv_h2,
+                                                 int planes) {
+  constexpr int W = Vec<T>::W;
+  const int i0 = 1 + (int)blockIdx.y * planes, iend = min(i0 + planes, g.NN);
+  for (int i = i0; i < iend; ++i) {
+    const VGroup r = vgroup<T>(g, i, blockIdx.x);
+    const VLoad<T, ROW> l(mur, r, g);
+    Quad<T> q = *reinterpret_cast<const Quad<T>*>(m + r.a);
+    const VRow row = vrow(g, r, i);
+    const Star<T> u = vstar(l);
+#pragma unroll
+    for (int e = 0; e < W; ++e) {
+      const double c = (double)u.c.v[e];
+      const double s = (double)u.ip.v[e] + (double)u.im.v[e] + (double)u.jp.v[e] + (double)u.jm.v[e] +
+                       (double)u.kp.v[e] + (double)u.km.v[e];
+      if (vinterior(g, row, e)) q.v[e] = (T)((double)q.v[e] + (s - 6.0 * c) * inv_h2);
+    }
+    if (r.own) stq(m + r.a, q);
+  }
 }
 
 // one colour of a red-black sweep, transposed.  Forward: P <- (sum_6 P + h^2 f) / 6 at the points
@@ -209,18 +401,56 @@ __global__ void __launch_bounds__(256) k_adj_residual(const T* __restrict__ mur,
   muP[id] = (T)((double)muP[id] + (s - 6.0 * r) * inv_h2);
 }
 
-// full weighting transposed: mur = (1/8) trilinear(mufc) at the fine interior points
+// full weighting transposed: mur = (1/8) trilinear(mufc) at the fine interior points, by coarse cells (the
+// walk of nm_prolong_cells_body: every load unconditional, a coarse plane loaded once)
 template <typename T>
-__global__ void __launch_bounds__(256) k_adj_restrict(const T* __restrict__ mufc, T* __restrict__ mur, Geo g, Geo gc) {
-  Pt p;
-  if (!interior_pt3(g, p)) return;
-  const int oi = p.i & 1, oj = p.j & 1, ok = p.k & 1;
-  double v = 0.0;
-  for (int a = 0; a <= oi; ++a)
-    for (int b = 0; b <= oj; ++b)
-      for (int cc = 0; cc <= ok; ++cc)
-        v += (double)mufc[(long long)((p.i >> 1) + a) * gc.S2 + (long long)((p.j >> 1) + b) * gc.S + (p.k >> 1) + cc];
-  mur[p.id] = (T)(v / (8.0 * (1 + oi) * (1 + oj) * (1 + ok)));
+__global__ void __launch_bounds__(256) k_adj_restrict(const T* __restrict__ mufc, T* __restrict__ mur, Geo g, Geo gc,
+                                                      int planes) {
+  const int nc = gc.NN;
+  const int K = blockIdx.x * kNmPrTK + tile_x<32>(), J = blockIdx.y * kNmPrTJ + tile_y<32>();
+  if (K >= nc || J >= nc) return;
+  const int I0 = blockIdx.z * planes, Iend = min(I0 + planes, nc);
+  const long long S = g.S, S2 = g.S2, Sc = gc.S, Sc2 = gc.S2;
+  double c0[2][2], c1[2][2];
+#pragma unroll
+  for (int b = 0; b < 2; ++b)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) c0[b][c] = (double)mufc[(long long)I0 * Sc2 + (long long)(J + b) * Sc + K + c];
+  for (int I = I0; I < Iend; ++I) {
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) c1[b][c] = (double)mufc[(long long)(I + 1) * Sc2 + (long long)(J + b) * Sc + K + c];
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int i = 2 * I + a, j = 2 * J + b, k = 2 * K + c;
+          if (i < 1 || j < 1 || k < 1) continue;
+          double v = 0.0;
+          v += c0[0][0];
+          if (c) v += c0[0][1];
+          if (b) {
+            v += c0[1][0];
+            if (c) v += c0[1][1];
+          }
+          if (a) {
+            v += c1[0][0];
+            if (c) v += c1[0][1];
+            if (b) {
+              v += c1[1][0];
+              if (c) v += c1[1][1];
+            }
+          }
+          mur[(long long)i * S2 + (long long)j * S + k] = (T)(v * (1.0 / (8.0 * (1 + a) * (1 + b) * (1 + c))));
+        }
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) c0[b][c] = c1[b][c];
+  }
 }
 
 // trilinear prolongation transposed: muPc = (1/8) sum (8,4,2,1 weights) muP at the coarse interior points
@@ -304,9 +534,11 @@ __global__ void __launch_bounds__(256) k_adj_ckpt(const T* __restrict__ U, const
 
 size_t esize(const rq_ctx* c) { return c->fp64 ? sizeof(double) : sizeof(float); }
 
+// a recorded field: the slots are padded to 16 bytes, as the vector kernels read them
+long long slot_stride(long long S3) { return (S3 + 3) & ~3LL; }
 template <typename T>
 T* slot(void* base, long long k, long long S3) {
-  return (T*)base + k * S3;
+  return (T*)base + k * slot_stride(S3);
 }
 
 // a new P snapshot slot holding the P in effect now.  A window reaches back at most cap steps,
@@ -317,7 +549,8 @@ int snapshot_p(rq_ctx* c) {
   const size_t bytes = (size_t)c->g.S3 * esize(c);
   const int s = A.next_p % A.np;
   A.next_p++;
-  CK(cudaMemcpyAsync((char*)A.psum + (size_t)s * bytes, c->P[c->cp], bytes, cudaMemcpyDeviceToDevice, c->st));
+  CK(cudaMemcpyAsync((char*)A.psum + (size_t)s * slot_stride(c->g.S3) * esize(c), c->P[c->cp], bytes,
+                     cudaMemcpyDeviceToDevice, c->st));
   A.cur_p = s;
   return RQ_OK;
 }
@@ -329,7 +562,9 @@ int snapshot_p(rq_ctx* c) {
 // ----------------------------------------------------------------------------------------
 void nm_adj_free(rq_ctx* c) {
   rq_adj& A = c->adj;
-  void* p[] = {A.psi, A.psum, A.scales, A.lam[0], A.lam[1], A.muP[0], A.muP[1], A.muf, A.gK, A.dots, A.coef, A.wq};
+  for (void* q : A.lam)
+    if (q) cudaFree(q);
+  void* p[] = {A.psi, A.psum, A.scales, A.muP[0], A.muP[1], A.muf, A.gK, A.dots, A.coef, A.wq};
   for (void* q : p)
     if (q) cudaFree(q);
   for (auto& L : A.lv)
@@ -356,14 +591,16 @@ int nm_adj_set_window(rq_ctx* c, int steps) {
     if (cudaMalloc(p, bytes) != cudaSuccess) return false;
     return cudaMemsetAsync(*p, 0, bytes, c->st) == cudaSuccess;
   };
-  bool ok = alloc(&A.psi, (size_t)steps * S3 * es) && alloc(&A.psum, (size_t)np * S3 * es) &&
-            alloc((void**)&A.scales, sizeof(double) * (size_t)steps * n) && alloc(&A.lam[0], S3 * es) &&
-            alloc(&A.lam[1], S3 * es) && alloc(&A.muP[0], S3 * es) && alloc(&A.muP[1], S3 * es) &&
+  const size_t slot_bytes = (size_t)slot_stride((long long)S3) * es;
+  bool ok = alloc(&A.psi, steps * slot_bytes) && alloc(&A.psum, np * slot_bytes) &&
+            alloc((void**)&A.scales, sizeof(double) * (size_t)steps * n) && alloc(&A.muP[0], S3 * es) &&
+            alloc(&A.muP[1], S3 * es) &&
             alloc(&A.muf, S3 * es) && alloc((void**)&A.gK, S3 * sizeof(double)) &&
             alloc((void**)&A.dots, sizeof(double) * n) && alloc((void**)&A.coef, sizeof(double) * 2 * n) &&
             alloc((void**)&A.wq, sizeof(double) * 2 * n);
   const int levels = (int)c->mg.size();
   A.lv.assign(levels, rq_adj::Level());
+  for (void*& p : A.lam) ok = ok && alloc(&p, S3 * es);
   for (int l = 0; ok && l < levels; ++l) {
     const size_t s3 = (size_t)c->mg[l].g.S3;
     if (l > 0) ok = alloc(&A.lv[l].mu[0], s3 * es) && alloc(&A.lv[l].mu[1], s3 * es) && alloc(&A.lv[l].muf, s3 * es);
@@ -427,27 +664,111 @@ void nm_adj_record_label(rq_ctx* c) {
 // ----------------------------------------------------------------------------------------
 namespace {
 
-// transposed normalisation of lam with the forward scales `scale` at the normalised state psi
+// the per-domain coefficients of a transposed normalisation of lam, with the forward scales `scale` at the
+// normalised state psi (applied by the next k_adj_update)
 template <typename T>
-int adj_norm(rq_ctx* c, const T* psi, T* lam, const double* scale) {
+int adj_norm(rq_ctx* c, const T* psi, const T* lam, const double* scale) {
   rq_adj& A = c->adj;
   const int n = c->n_atoms;
-  const long long S3 = c->g.S3;
   CK(cudaMemsetAsync(A.dots, 0, sizeof(double) * n, c->st));
-  LAUNCH(RQ_KC_FORCES, 2.0 * sizeof(T) * S3 + 4.0 * S3,
-         (k_adj_dot<T><<<nblk(S3, 256 * kNmFlatChunk), 256, 0, c->st>>>(psi, lam, c->lab[c->cl], S3, n, A.dots),
-          cudaGetLastError()));
+  LAUNCH(RQ_KC_FORCES, (2.0 * sizeof(T) + 4.0) * c->g.S3,
+         (k_adj_dot<T><<<nm_norms_grid(c->g), 256, 0, c->st>>>(psi, lam, c->lab[c->cl], c->g, n, A.dots), cudaGetLastError()));
   LAUNCH(RQ_KC_FORCES, 32.0 * n,
          (k_adj_norm_coef<<<nblk(n, 128), 128, 0, c->st>>>(scale, c->Zdom64, A.dots, n, c->h3, A.coef),
-          cudaGetLastError()));
-  LAUNCH(RQ_KC_FORCES, 3.0 * sizeof(T) * S3 + 4.0 * S3,
-         (k_adj_norm_apply<T><<<nblk(S3, 256 * kNmFlatChunk), 256, 0, c->st>>>(lam, psi, c->lab[c->cl], A.coef, S3, n),
           cudaGetLastError()));
   return RQ_OK;
 }
 
-// transposed V-cycle on level l: mu[*cur] holds dE/dP of the level after the cycle and becomes
-// dE/dP before it; dE/df of the level is accumulated into its muf
+// f(row form of the grid) for the vector kernels
+template <class F>
+void with_row(const Geo& g, F&& f) {
+  if (g.S % 4 == 1) f(std::integral_constant<int, kRowP>{});
+  else f(std::integral_constant<int, kRowM>{});
+}
+
+template <typename T>
+cudaError_t adj_half(const Geo& g, T* m, cudaStream_t st) {
+  const int planes = vplanes<T>(g, false);
+  with_row(g, [&](auto row) { k_adj_half<T, decltype(row)::value><<<vgrid<T>(g, planes), 256, 0, st>>>(m, g, planes); });
+  return cudaGetLastError();
+}
+
+// restriction^T of the coarse dE/df onto level l's mur
+template <typename T>
+int adj_restrict(rq_ctx* c, int l) {
+  rq_adj& A = c->adj;
+  const Geo &g = c->mg[l].g, &gc = c->mg[l + 1].g;
+  const int nc = gc.NN;
+  const dim3 t((nc + kNmPrTK - 1) / kNmPrTK, (nc + kNmPrTJ - 1) / kNmPrTJ);
+  const int planes = nm_mg_planes((long long)t.x * t.y, nc);
+  LAUNCH(RQ_KC_MG, sizeof(T) * 1.125 * g.S3,
+         (k_adj_restrict<T><<<dim3(t.x, t.y, (nc + planes - 1) / planes), 256, 0, c->st>>>(
+              (const T*)A.lv[l + 1].muf, (T*)A.lv[l].mur, g, gc, planes),
+          cudaGetLastError()));
+  return RQ_OK;
+}
+
+template <typename T>
+int adj_coarsest(rq_ctx* c, int l) {
+  rq_adj& A = c->adj;
+  const rq_mg_level& L = c->mg[l];
+  const size_t smem = sizeof(double) * 2 * (size_t)L.g.S3;
+  CK(cudaFuncSetAttribute(k_adj_coarsest<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LAUNCH(RQ_KC_MG, 2.0 * sizeof(T) * L.g.S3,
+         (k_adj_coarsest<T><<<1, kCoarsestThreads, smem, c->st>>>((const T*)A.lv[l].mu[0], (T*)A.lv[l].muf, L.g, L.h * L.h,
+                                                                 c->cfg.mg_coarse_sweeps),
+          cudaGetLastError()));
+  return RQ_OK;
+}
+
+// Transposed V(1,1) cycle on level l.  mA holds dE/dP of the level after the cycle.  On level 0 it holds
+// dE/dP before it on return, and lam has taken the right-hand side's share; on coarser levels (whose
+// cycle starts from P = 0) dE/df of the level is left in its muf.
+template <typename T>
+int adj_vcycle11(rq_ctx* c, int l, T* mA, T* m2, const T* psi, T* lam) {
+  rq_adj& A = c->adj;
+  const rq_mg_level &L = c->mg[l], &C = c->mg[l + 1];
+  const Geo& g = L.g;
+  const double h2 = L.h * L.h, c6 = h2 / 6.0;
+  const long long ni = (long long)(g.NN - 1) * (g.NN - 1) * (g.NN - 1);
+  const int planes = vplanes<T>(g, false);
+  const dim3 grd = vgrid<T>(g, planes);
+  T* mur = (T*)A.lv[l].mur;
+  LAUNCH(RQ_KC_MG, 1.5 * sizeof(T) * ni, adj_half<T>(g, mA, c->st));
+  LAUNCH(RQ_KC_MG, 2.0 * sizeof(T) * ni,
+         (with_row(g, [&](auto row) {
+    k_adj_other<T, false, decltype(row)::value><<<grd, 256, 0, c->st>>>(mA, m2, nullptr, nullptr, nullptr, nullptr, g, c6,
+                                                                      planes);
+          }),
+          cudaGetLastError()));
+  LAUNCH(RQ_KC_MG, sizeof(T) * 1.125 * ni,
+         (k_adj_prolong<T><<<grid3(C.g), kBlk3, 0, c->st>>>(m2, (T*)A.lv[l + 1].mu[0], g, C.g), cudaGetLastError()));
+  int rc = l + 1 == (int)c->mg.size() - 1
+               ? adj_coarsest<T>(c, l + 1)
+               : adj_vcycle11<T>(c, l + 1, (T*)A.lv[l + 1].mu[0], (T*)A.lv[l + 1].mu[1], nullptr, nullptr);
+  if (rc != RQ_OK || (rc = adj_restrict<T>(c, l)) != RQ_OK) return rc;
+  LAUNCH(RQ_KC_MG, 3.0 * sizeof(T) * ni,
+         (with_row(g, [&](auto row) {
+    k_adj_res<T, decltype(row)::value><<<grd, 256, 0, c->st>>>(mur, m2, g, 1.0 / h2, planes);
+          }),
+          cudaGetLastError()));
+  LAUNCH(RQ_KC_MG, 1.5 * sizeof(T) * ni, adj_half<T>(g, m2, c->st));
+  if (l > 0) {
+    LAUNCH(RQ_KC_MG, 4.0 * sizeof(T) * g.S3,
+           (k_adj_muf<T><<<nblk(g.S3), 256, 0, c->st>>>(mA, mur, m2, (T*)A.lv[l].muf, g.S3, c6), cudaGetLastError()));
+    return RQ_OK;
+  }
+  LAUNCH(RQ_KC_MG, 7.0 * sizeof(T) * ni,
+         (with_row(g, [&](auto row) {
+    k_adj_other<T, true, decltype(row)::value><<<grd, 256, 0, c->st>>>(m2, mA, mA, mur, psi, lam, g, c6, planes);
+          }),
+          cudaGetLastError()));
+  return RQ_OK;
+}
+
+// The same for any number of sweeps (mg_pre, mg_post), colour by colour out of place with a running dE/df:
+// mu[*cur] holds dE/dP of level l after the cycle and becomes dE/dP before it; dE/df of the level is
+// accumulated into its muf
 template <typename T>
 int adj_vcycle(rq_ctx* c, int l, int* cur) {
   rq_adj& A = c->adj;
@@ -457,14 +778,7 @@ int adj_vcycle(rq_ctx* c, int l, int* cur) {
   const double h2 = L.h * L.h;
   const long long ni = (long long)(L.g.NN - 1) * (L.g.NN - 1) * (L.g.NN - 1);
   const int last = (int)c->mg.size() - 1;
-  if (l == last) {
-    const size_t smem = sizeof(double) * 2 * (size_t)L.g.S3;
-    CK(cudaFuncSetAttribute(k_adj_coarsest<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    LAUNCH(RQ_KC_MG, 2.0 * sizeof(T) * L.g.S3,
-           (k_adj_coarsest<T><<<1, kCoarsestThreads, smem, c->st>>>(mu[*cur], muf, L.g, h2, c->cfg.mg_coarse_sweeps),
-            cudaGetLastError()));
-    return RQ_OK;
-  }
+  if (l == last) return adj_coarsest<T>(c, l);
   auto smooth = [&](int sweeps) -> int {
     for (int s = 0; s < sweeps; ++s)
       for (int color = 1; color >= 0; --color) {
@@ -484,9 +798,7 @@ int adj_vcycle(rq_ctx* c, int l, int* cur) {
          (k_adj_prolong<T><<<grid3(C.g), kBlk3, 0, c->st>>>(mu[*cur], (T*)A.lv[l + 1].mu[0], L.g, C.g), cudaGetLastError()));
   CK(cudaMemsetAsync(A.lv[l + 1].muf, 0, sizeof(T) * C.g.S3, c->st));
   if ((rc = adj_vcycle<T>(c, l + 1, &ccur)) != RQ_OK) return rc;
-  LAUNCH(RQ_KC_MG, sizeof(T) * (ni + nc),
-         (k_adj_restrict<T><<<grid3(L.g), kBlk3, 0, c->st>>>((const T*)A.lv[l + 1].muf, (T*)A.lv[l].mur, L.g, C.g),
-          cudaGetLastError()));
+  if ((rc = adj_restrict<T>(c, l)) != RQ_OK) return rc;
   LAUNCH(RQ_KC_MG, 5.0 * sizeof(T) * ni,
          (k_adj_residual<T><<<grid3(L.g), kBlk3, 0, c->st>>>((const T*)A.lv[l].mur, mu[*cur], muf, L.g, 1.0 / h2),
           cudaGetLastError()));
@@ -521,33 +833,69 @@ int adjoint_t(rq_ctx* c, double* F, double* dEdv) {
     wq[2 * d + 1] = x[0] > 0.0 ? (x[1] + x[2] + 2.0 * x[3]) / x[0] : 0.0;
   }
   CK(cudaMemcpyAsync(A.wq, wq.data(), sizeof(double) * wq.size(), cudaMemcpyHostToDevice, c->st));
-  int li = 0, mi = 0;
-  T* lam[2] = {(T*)A.lam[0], (T*)A.lam[1]};
+  int mi = 0;
   T* muP[2] = {(T*)A.muP[0], (T*)A.muP[1]};
+  T* lam = (T*)A.lam[0];
+  AdjPend pend{};
+  // a lambda buffer that neither the sweep nor a pending sum holds, other than `also`
+  auto spare = [&](const T* also) -> T* {
+    for (void* p : A.lam) {
+      bool held = p == lam || p == also;
+      for (int q = 0; q < pend.n; ++q) held = held || p == pend.lam[q];
+      if (!held) return (T*)p;
+    }
+    return nullptr;  // not reached: kAdjPend pending, the input and two outputs are A.lam's size
+  };
+  auto accumulate = [&]() -> int {
+    if (!pend.n) return RQ_OK;
+    LAUNCH(RQ_KC_FORCES, (2.0 * sizeof(T) * pend.n + 16.0 + 2.0 * sizeof(T)) * S3,
+           (k_adj_accum<T><<<nblk(S3, 256 * Vec<T>::W), 256, 0, c->st>>>(pend, A.gK, muP[mi], c->dt, S3), cudaGetLastError()));
+    pend.n = 0;
+    return RQ_OK;
+  };
   LAUNCH(RQ_KC_FORCES, (4.0 * sizeof(T) + 4.0 + 2.0 * sizeof(T) + 8.0) * ni,
-         (k_adj_seed<T><<<grid3(g), kBlk3, 0, c->st>>>(psi, K, (const T*)c->P[c->cp], lab, g, c->h, n, A.wq, lam[li],
-                                                     muP[mi], A.gK, c->K64),
+         (k_adj_seed<T><<<grid3(g), kBlk3, 0, c->st>>>(psi, K, (const T*)c->P[c->cp], lab, g, c->h, n, A.wq, lam, muP[mi],
+                                                     A.gK, c->K64),
           cudaGetLastError()));
+  const int planes = vplanes<T>(g, false);
   for (int r = (int)A.rec.size() - 1; r >= 0; --r) {
     const rq_adj::Rec& R = A.rec[r];
     const T* psi_prev = slot<T>(A.psi, R.psi_slot, S3);
     const T* P_s = slot<T>(A.psum, R.p_slot, S3);
+    T* out = spare(nullptr);
     if (R.norm) {
       const T* psi_s = r + 1 < (int)A.rec.size() ? slot<T>(A.psi, A.rec[r + 1].psi_slot, S3) : psi;
-      if ((rc = adj_norm<T>(c, psi_s, lam[li], A.scales + (size_t)R.psi_slot * n)) != RQ_OK) return rc;
+      if ((rc = adj_norm<T>(c, psi_s, lam, A.scales + (size_t)R.psi_slot * n)) != RQ_OK) return rc;
+      T* inn = spare(out);
+      LAUNCH(RQ_KC_FORCES, (6.0 * sizeof(T) + 5.0) * ni,
+             (with_row(g, [&](auto row) {
+        k_adj_update<T, true, decltype(row)::value><<<vgrid<T>(g, planes), 256, 0, c->st>>>(
+            lam, inn, out, K, P_s, c->nbm, lab, psi_s, A.coef, g, c->half_dv, c->dt, n, planes);
+              }),
+              cudaGetLastError()));
+      lam = inn;
+    } else {
+      LAUNCH(RQ_KC_FORCES, (4.0 * sizeof(T) + 1.0) * ni,
+             (with_row(g, [&](auto row) {
+        k_adj_update<T, false, decltype(row)::value><<<vgrid<T>(g, planes), 256, 0, c->st>>>(
+            lam, nullptr, out, K, P_s, c->nbm, lab, nullptr, nullptr, g, c->half_dv, c->dt, n, planes);
+              }),
+              cudaGetLastError()));
     }
-    LAUNCH(RQ_KC_FORCES, (6.0 * sizeof(T) + 4.0 + 16.0) * ni,
-           (k_adj_update<T><<<grid3(g), kBlk3, 0, c->st>>>(lam[li], lam[1 - li], K, P_s, lab, psi_prev, g, c->half_dv,
-                                                         c->dt, A.gK, muP[mi]),
-            cudaGetLastError()));
-    li ^= 1;
-    if (R.vcycle) {
+    pend.lam[pend.n] = lam;
+    pend.psi[pend.n++] = psi_prev;
+    lam = out;
+    if ((R.vcycle || pend.n == kAdjPend) && (rc = accumulate()) != RQ_OK) return rc;
+    if (R.vcycle && c->cfg.mg_pre == 1 && c->cfg.mg_post == 1) {
+      if ((rc = adj_vcycle11<T>(c, 0, muP[mi], muP[1 - mi], psi_prev, lam)) != RQ_OK) return rc;
+    } else if (R.vcycle) {
       CK(cudaMemsetAsync(A.muf, 0, sizeof(T) * S3, c->st));
       if ((rc = adj_vcycle<T>(c, 0, &mi)) != RQ_OK) return rc;
       LAUNCH(RQ_KC_FORCES, 4.0 * sizeof(T) * ni,
-             (k_adj_rhs<T><<<grid3(g), kBlk3, 0, c->st>>>(lam[li], psi_prev, (const T*)A.muf, g), cudaGetLastError()));
+             (k_adj_rhs<T><<<grid3(g), kBlk3, 0, c->st>>>(lam, psi_prev, (const T*)A.muf, g), cudaGetLastError()));
     }
   }
+  if ((rc = accumulate()) != RQ_OK) return rc;
   if (F) {
     CK(cudaMemsetAsync(c->dF, 0, sizeof(double) * 3 * n, c->st));
     if ((rc = nm_gather(c, psi, A.gK)) != RQ_OK) return rc;
