@@ -30,8 +30,9 @@
 #include <type_traits>
 #include <cstring>
 
-#include "nm_bodies.cuh"
+#include "nm_tail.cuh"
 #include "rq_flavors.h"
+#include "rq_kernels.h"
 #include "vec_stencil.cuh"
 
 using namespace rq;
@@ -743,9 +744,17 @@ int adj_vcycle11(rq_ctx* c, int l, T* mA, T* m2, const T* psi, T* lam) {
           cudaGetLastError()));
   LAUNCH(RQ_KC_MG, sizeof(T) * 1.125 * ni,
          (k_adj_prolong<T><<<grid3(C.g), kBlk3, 0, c->st>>>(m2, (T*)A.lv[l + 1].mu[0], g, C.g), cudaGetLastError()));
-  int rc = l + 1 == (int)c->mg.size() - 1
-               ? adj_coarsest<T>(c, l + 1)
-               : adj_vcycle11<T>(c, l + 1, (T*)A.lv[l + 1].mu[0], (T*)A.lv[l + 1].mu[1], nullptr, nullptr);
+  T* mc = (T*)A.lv[l + 1].mu[0];
+  NmTail t;
+  size_t smem = 0;
+  int rc = RQ_OK;
+  if (l + 1 == nm_tail_plan<T>((int)c->mg.size(), [&](int q) { return c->mg[q].g; }, [&](int q) { return c->mg[q].h; },
+                               c->cfg.mg_coarse_sweeps, t, smem))
+    LAUNCH(RQ_KC_MG, 2.0 * sizeof(T) * C.g.S3, nm_adj_tail<T>(t, smem, mc, (T*)A.lv[l + 1].muf, c->st));
+  else if (l + 1 == (int)c->mg.size() - 1)
+    rc = adj_coarsest<T>(c, l + 1);
+  else
+    rc = adj_vcycle11<T>(c, l + 1, mc, (T*)A.lv[l + 1].mu[1], nullptr, nullptr);
   if (rc != RQ_OK || (rc = adj_restrict<T>(c, l)) != RQ_OK) return rc;
   LAUNCH(RQ_KC_MG, 3.0 * sizeof(T) * ni,
          (with_row(g, [&](auto row) {

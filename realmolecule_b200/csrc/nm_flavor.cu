@@ -12,6 +12,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "nm_tail.cuh"
 #include "rq_flavors.h"
 #include "rq_kernels.h"
 
@@ -80,6 +81,15 @@ int nm_alloc_levels(rq_ctx* c) {
   return RQ_OK;
 }
 
+// the first level of the one-block tail of the V-cycle, the level count if there is none
+template <typename T>
+static int tail_of(const rq_ctx* c, NmTail& t, size_t& smem) {
+  const int levels = (int)c->mg.size();
+  if (c->cfg.mg_pre != 1 || c->cfg.mg_post != 1) return levels;
+  return nm_tail_plan<T>(levels, [&](int l) { return c->mg[l].g; }, [&](int l) { return c->mg[l].h; },
+                         c->cfg.mg_coarse_sweeps, t, smem);
+}
+
 template <typename T>
 static int vcycle_level(rq_ctx* c, int l) {
   rq_mg_level& L = c->mg[l];
@@ -102,8 +112,14 @@ static int vcycle_level(rq_ctx* c, int l) {
   rq_mg_level& C = c->mg[l + 1];
   LAUNCH(kc, sizeof(T) * (2.0 * ip + 2.0 * interior(C.g)),
          nm_resrestrict<T>(P, f, fine, (T*)C.f, (T*)C.P, L.g, C.g, 1.0 / h2, c->st));
-  int rc = vcycle_level<T>(c, l + 1);
-  if (rc != RQ_OK) return rc;
+  NmTail t;
+  size_t smem = 0;
+  if (l + 1 == tail_of<T>(c, t, smem)) {
+    LAUNCH(RQ_KC_MG, 2.0 * sizeof(T) * interior(C.g), nm_tail<T>(t, smem, (const T*)C.f, (T*)C.P, c->st));
+  } else {
+    const int rc = vcycle_level<T>(c, l + 1);
+    if (rc != RQ_OK) return rc;
+  }
   LAUNCH(RQ_KC_MG, sizeof(T) * (2.0 * ip + interior(C.g)), nm_prolong<T>((const T*)C.P, P, L.g, C.g, c->st));
   for (int s = 0; s < c->cfg.mg_post; ++s)
     for (int color = 0; color < 2; ++color)

@@ -6,6 +6,7 @@
 #include <type_traits>
 
 #include "nm_bodies.cuh"
+#include "nm_tail.cuh"
 #include "rq_kernels.h"
 #include "vec_stencil.cuh"
 
@@ -240,6 +241,20 @@ cudaError_t nm_coarsest(T* P, const T* f, const Geo& g, double h2, int sweeps, c
   return cudaGetLastError();
 }
 template <typename T>
+cudaError_t nm_tail(const NmTail& t, size_t smem, const T* f, T* P, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(k_nm_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k_nm_tail<T><<<1, kTailThreads, smem, st>>>(t, f, P);
+  return cudaGetLastError();
+}
+template <typename T>
+cudaError_t nm_adj_tail(const NmTail& t, size_t smem, const T* mA, T* muf, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(k_adj_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k_adj_tail<T><<<1, kTailThreads, smem, st>>>(t, mA, muf);
+  return cudaGetLastError();
+}
+template <typename T>
 cudaError_t nm_energy(const T* U, const T* K, const T* P, const int* label, const Geo& g, double h, int nDom, double* pd,
                       cudaStream_t st, const double* K64) {
   if (g.NN < 2) return cudaSuccess;
@@ -284,6 +299,8 @@ cudaError_t nm_add(T* K, const T* v, long long n, cudaStream_t st) {
                                          cudaStream_t);                                                            \
   template cudaError_t nm_prolong<T>(const T*, T*, const Geo&, const Geo&, cudaStream_t);                           \
   template cudaError_t nm_coarsest<T>(T*, const T*, const Geo&, double, int, cudaStream_t);                         \
+  template cudaError_t nm_tail<T>(const NmTail&, size_t, const T*, T*, cudaStream_t);                                \
+  template cudaError_t nm_adj_tail<T>(const NmTail&, size_t, const T*, T*, cudaStream_t);                            \
   template cudaError_t nm_energy<T>(const T*, const T*, const T*, const int*, const Geo&, double, int, double*,     \
                                     cudaStream_t, const double*);                                                    \
   template cudaError_t nm_evolve<T>(const int*, int*, const T*, float*, const Geo&, double, double, cudaStream_t);  \

@@ -154,6 +154,12 @@ template <typename T>
 cudaError_t nm_prolong(const T* Ec, T* P, const Geo& g, const Geo& gc, cudaStream_t st);
 template <typename T>
 cudaError_t nm_coarsest(T* P, const T* f, const Geo& g, double h2, int sweeps, cudaStream_t st);
+// the small levels of a V(1,1) cycle in one launch (nm_tail.cuh), and their transpose
+struct NmTail;
+template <typename T>
+cudaError_t nm_tail(const NmTail& t, size_t smem, const T* f, T* P, cudaStream_t st);
+template <typename T>
+cudaError_t nm_adj_tail(const NmTail& t, size_t smem, const T* mA, T* muf, cudaStream_t st);
 template <typename T>
 cudaError_t nm_energy(const T* U, const T* K, const T* P, const int* label, const Geo& g, double h, int nDom, double* pd,
                       cudaStream_t st, const double* K64 = nullptr);

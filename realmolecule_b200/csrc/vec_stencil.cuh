@@ -195,8 +195,9 @@ __device__ __forceinline__ float sixth(float x) {
 }
 __device__ __forceinline__ double sixth(double x) {
   constexpr double zh = 0x1.5555555555555p-3, zl = 0x1.5555555555555p-57;
-  const double a = fabs(x);
-  if (a >= 0x1p-900 && a <= 0x1p1000) return __fma_rn(x, zh, __dmul_rn(x, zl));
+  // |x| in [2^-900, 2^1000), by the exponent field: FP64 comparisons are as long a wait as the product
+  const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+  if (ex - (1023u - 900u) < 1900u) return __fma_rn(x, zh, __dmul_rn(x, zl));
   return __ddiv_rn(x, 6.0);
 }
 

@@ -190,3 +190,36 @@ def test_glycine_all_30_coordinates_against_finite_differences():
     errs = np.array([abs(fd[c] - F[c]) for c in coords])
     assert errs.max() < 1e-4, errs.max()
     ctx.close()
+
+
+# The vector reverse sweep at its edges: both row alignments (S = 1 and 3 mod 4), a normalisation on every
+# step, V-cycles further apart than the steps whose sums run together, one and several sweeps per side.
+# The same FP64 sweep restated: 1e-9 of the largest value, as above.
+@pytest.mark.parametrize("NN,opts,steps", [(16, {}, 9), (22, {}, 8), (16, dict(norm_interval=1), 7),
+                                           (22, dict(poisson_interval=7, norm_interval=3), 16),
+                                           (20, dict(mg_pre=2, mg_post=1), 8), (16, dict(mg_pre=1, mg_post=2), 5)])
+def test_reverse_sweep_edges_match_the_oracle_adjoint(NN, opts, steps):
+    import oracle as orc
+    import nm_adjoint as adj
+    from realmolecule_b200 import Context, _lib as L
+    h = 7.2 / NN
+    N2, d = NN / 2, 1.4 / 2 / h
+    rows = [{"i": N2 - d, "j": N2, "k": N2 + 0.2, "Z": 0.0, "Z_nuc": 1.0},
+            {"i": N2 + d, "j": N2 + 0.3, "k": N2, "Z": 0.0, "Z_nuc": 1.0},
+            {"i": N2 - d + 0.05, "j": N2, "k": N2, "Z": 1.0, "Z_nuc": 0.0},
+            {"i": N2 + d - 0.05, "j": N2, "k": N2, "Z": 1.0, "Z_nuc": 0.0}]
+    kw = {"poisson_interval": 4, **opts}
+    okw = {{"mg_pre": "pre", "mg_post": "post"}.get(k, k): v for k, v in kw.items()}
+    drv = orc.NewMethodDriver(NN, NN * h, rows, label_until=1, **okw)
+    drv.initialize()
+    ctx = Context(NN, NN * h, rows, flavor="new", precision="fp64", label_until=1, **kw)
+    ctx.initialize()
+    ctx.upload(psi=drv.U, label=drv.label, P=drv.P)
+    ctx.set_adjoint_window(steps)
+    ctx.step(steps)
+    F, g = ctx.adjoint(forces=True, potential=True)
+    out = adj.gradient(drv, steps)
+    Fo, go = np.asarray(out[1]), np.asarray(out[2])
+    assert np.abs(F - Fo).max() <= 1e-9 * np.abs(Fo).max()
+    assert np.abs(g - go.ravel()).max() <= 1e-9 * np.abs(go).max()
+    ctx.close()
