@@ -119,18 +119,27 @@ __global__ void __launch_bounds__(256) kb_rbgs(const BInst* __restrict__ ins, co
   nm_vrbgs_body<T, FINE, kRowAny, COLOR>(P, f, g, h2, it.bx, i0, iend);
 }
 
-// residual, full weighting and the zeroed coarse correction of level lev in one pass
 template <typename T, bool FINE>
-__global__ void __launch_bounds__(256, 4) kb_resrestrict(const BInst* __restrict__ ins, const BItem* __restrict__ items,
-                                                      int lev, int cu, int cp, int planes) {
-  __shared__ T patch[kNmRrBuf][kNmRrPatch];
+__global__ void __launch_bounds__(256) kb_residual(const BInst* __restrict__ ins, const BItem* __restrict__ items, int lev,
+                                                   int cu, int cp) {
   const BItem it = items[blockIdx.x];
   const BInst& I = ins[it.inst];
-  const T* P = FINE ? (const T*)I.P[cp] : (const T*)I.lP[lev];
-  const T* f = FINE ? (const T*)I.U[cu] : (const T*)I.lf[lev];
+  const Geo g = I.lg[lev];
+  const int i0 = 1 + it.by * kBVPlanes, iend = min(i0 + kBVPlanes, g.NN);
+  nm_vresidual_body<T, FINE, kRowAny>(FINE ? (const T*)I.P[cp] : (const T*)I.lP[lev],
+                                      FINE ? (const T*)I.U[cu] : (const T*)I.lf[lev], (T*)I.lr[lev], g,
+                                      (T)(1.0 / (I.lh[lev] * I.lh[lev])), it.bx, i0, iend);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) kb_restrict(const BInst* __restrict__ ins, const BItem* __restrict__ items, int lev,
+                                                   int planes) {
+  const BItem it = items[blockIdx.x];
+  const BInst& I = ins[it.inst];
   const Geo g = I.lg[lev], gc = I.lg[lev + 1];
-  nm_resrestrict_body<T, FINE>(P, f, (T*)I.lf[lev + 1], (T*)I.lP[lev + 1], g, gc, (T)(1.0 / (I.lh[lev] * I.lh[lev])),
-                               it.bx, it.by, it.bz, planes, patch);
+  const int I0 = 1 + it.bz * planes;
+  nm_restrict_tile_body<T>((const T*)I.lr[lev], (T*)I.lf[lev + 1], (T*)I.lP[lev + 1], g, gc, it.bx, it.by, I0,
+                           min(I0 + planes, gc.NN));
 }
 
 template <typename T>
@@ -503,7 +512,7 @@ struct rq_batch {
   unsigned* rseed = nullptr;      // the step seed of the fp32 set's unbiased rounding (2 words by parity)
   float4* seeds_all = nullptr;
   int maxlev = 0;
-  int rr_pl[kMaxLev] = {}, pr_pl[kMaxLev] = {};  // coarse planes per block of the level's residual-restriction / prolongation
+  int rr_pl[kMaxLev] = {}, pr_pl[kMaxLev] = {};  // coarse planes per block of the level's restriction / prolongation
   // work lists, one set per precision
   struct Plan { BItem* d = nullptr; int n = 0, cap = 0; };
   struct Plans {
@@ -609,7 +618,7 @@ static void make_items(const BInst& I, const std::vector<rq_atom>& atoms, int q,
     const long long nc = (long long)(I.lg[l + 1].NN - 1) * (I.lg[l + 1].NN - 1) * (I.lg[l + 1].NN - 1);
     flat_items(it.restr[l], q, nc, 256);
     flat_items(it.zero[l], q, I.lg[l + 1].S3, 256 * kNmFlatChunk);
-    const int cn = I.lg[l + 1].NN - 1;  // coarse interior of the fused residual + restriction
+    const int cn = I.lg[l + 1].NN - 1;  // coarse interior of the restriction
     for (int zz = 0; zz < (cn + rr_pl[l] - 1) / rr_pl[l]; ++zz)
       for (int y = 0; y < (cn + kNmRrTJ - 1) / kNmRrTJ; ++y)
         for (int x = 0; x < (cn + kNmRrTK - 1) / kNmRrTK; ++x) it.rr[l].push_back({q, x, y, zz});
@@ -695,7 +704,7 @@ static int alloc_fields(rq_batch* b, BInst& I, size_t es) {
   return RQ_OK;
 }
 
-// Coarse planes per block of each level's residual-restriction and prolongation over all
+// Coarse planes per block of each level's restriction and prolongation over all
 // instances: 8, halved while the level's launch would have fewer than 8 blocks per SM.
 static void b_mg_planes(rq_batch* b) {
   for (int l = 0; l + 1 < b->maxlev; ++l) {
@@ -871,10 +880,12 @@ static int b_vcycle(rq_batch* b, int p) {
     }
     // the coarse correction's boundary stays zero from the allocation: only its interior is cleared
     if (l == 0)
-      kb_resrestrict<T, true><<<P.rr[l].n, rb, 0, b->st>>>(b->din, P.rr[l].d, l, b->cu, b->cp, b->rr_pl[l]);
+      kb_residual<T, true><<<P.vec[l].n, 256, 0, b->st>>>(b->din, P.vec[l].d, l, b->cu, b->cp);
     else
-      kb_resrestrict<T, false><<<P.rr[l].n, rb, 0, b->st>>>(b->din, P.rr[l].d, l, b->cu, b->cp, b->rr_pl[l]);
-    BL("resrestrict");
+      kb_residual<T, false><<<P.vec[l].n, 256, 0, b->st>>>(b->din, P.vec[l].d, l, b->cu, b->cp);
+    BL("residual");
+    kb_restrict<T><<<P.rr[l].n, 256, 0, b->st>>>(b->din, P.rr[l].d, l, b->rr_pl[l]);
+    BL("restrict");
   }
   for (int l = b->maxlev - 2; l >= 0; --l) {
     if (!P.rbgs[l].n) continue;

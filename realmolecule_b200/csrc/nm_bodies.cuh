@@ -659,97 +659,63 @@ __device__ __forceinline__ void nm_restrict_body(const T* __restrict__ fine, T* 
   coarse[(long long)I * gc.S2 + (long long)J * gc.S + K2] = A::div(v, T(64));
 }
 
-// Residual and full weighting in one pass: fc = R (f - A P) on the coarse interior without storing
-// the fine residual, and the coarse correction Pc (when given) zeroed on the same points.  The
-// block (256 threads, read as 32 x 8) owns the coarse points (K, J) = (K0 + x, J0 + y) of a 32 x 8
-// tile on `planes` coarse planes from I0, and walks the fine planes 2 I0 - 1 .. 2 Ilast + 1.
-// On each fine plane it forms the residual on the 65 x 17 fine patch under the tile into shared
-// memory (every thread keeps the P values of its patch points on the planes below and above in
-// registers).  One step per coarse plane I forms the fine planes 2I and 2I + 1 and, after one
-// barrier, adds the 3 x 3 patch values of the fine planes 2I - 1, 2I and 2I + 1 around each coarse
-// point with their weights.  The sums run in the (a, b, c) order of nm_restrict_body and the
-// residual is nm_residual_value, so the result is the one of the residual pass and the
-// restriction.  A ring of kNmRrBuf (5) patch planes lets the next step's planes be written while
-// slower threads still read this step's three: one barrier per coarse plane.
-constexpr int kNmRrTK = 32, kNmRrTJ = 8;
-
-// Coarse planes per block of the residual-restriction and prolongation kernels for a launch of
-// `blocks_per_plane` blocks on each of n coarse planes: 8, halved while the launch would have
-// fewer than 8 blocks per SM (small levels and single grids favour more blocks over the extra
-// fine plane a block forms at its chunk's ends).
-inline int nm_mg_planes(long long blocks_per_plane, int n) {
-  int planes = 8;
-  while (planes > 1 && blocks_per_plane * ((n + planes - 1) / planes) < 8LL * 148) planes /= 2;
-  return planes;
-}
-constexpr int kNmRrPK = 2 * kNmRrTK + 1;                      // fine patch row (65 points)
-constexpr int kNmRrPatch = kNmRrPK * (2 * kNmRrTJ + 1);       // 65 x 17 fine points
-constexpr int kNmRrPer = (kNmRrPatch + 255) / 256;            // patch points per thread
-constexpr int kNmRrBuf = 5;                                   // patch planes in the ring
-
-template <typename T, bool FINE>
-__device__ __forceinline__ void nm_resrestrict_body(const T* __restrict__ P, const T* __restrict__ f, T* __restrict__ fc,
-                                                    T* __restrict__ Pc, const Geo& g, const Geo& gc, T inv_h2, int bx,
-                                                    int by, int bz, int planes, T (*patch)[kNmRrPatch]) {
+// residual r = f - A P on 16-byte groups: planes [i0, iend) of block column bx
+template <typename T, bool FINE, int ROW>
+__device__ __forceinline__ void nm_vresidual_body(const T* __restrict__ P, const T* __restrict__ f, T* __restrict__ r,
+                                                  const Geo& g, T inv_h2, int bx, int i0, int iend) {
   using A = Ar<T>;
-  const int n = gc.NN - 1;  // coarse interior 1..n
-  const int I0 = 1 + bz * planes;
-  if (I0 > n) return;  // the whole block
-  const int Ilast = min(I0 + planes - 1, n);
-  const int tx = tile_x<32>(), ty = tile_y<32>(), tid = tx + 32 * ty;
-  const int K0 = 1 + bx * kNmRrTK, J0 = 1 + by * kNmRrTJ;
-  const int K = K0 + tx, J = J0 + ty;
-  const bool own = K <= n && J <= n;
-  const long long S = g.S, S2 = g.S2;
-  const int fi0 = 2 * I0 - 1;
-  // fine (j, k) offset of each patch point of this thread; points outside the grid use the
-  // offset of (1, 1) (in bounds, their residuals are not stored)
-  int col[kNmRrPer];
-  bool in[kNmRrPer];
-  T pm[kNmRrPer], pc[kNmRrPer];  // P of each patch point on the planes below and at the next residual plane
+  for (int i = i0; i < iend; ++i) {
+    const VGroup q = vgroup<T>(g, i, bx);
+    const VLoad<T, ROW> l(P, q, g);
+    const Quad<T> fq = ldq<T>(f + q.a);
+    const Star<T> u = vstar(l);
+    const VRow row = vrow(g, q, i);
+    Quad<T> o;
 #pragma unroll
-  for (int m = 0; m < kNmRrPer; ++m) {
-    const int p = tid + 256 * m;
-    const int fj = 2 * J0 - 1 + p / kNmRrPK, fk = 2 * K0 - 1 + p % kNmRrPK;
-    in[m] = p < kNmRrPatch && fj < g.NN && fk < g.NN;
-    col[m] = in[m] ? fj * g.S + fk : g.S + 1;
-    pm[m] = P[(long long)(fi0 - 1) * S2 + col[m]];
-    pc[m] = P[(long long)fi0 * S2 + col[m]];
-  }
-  auto residual_plane = [&](int i) {  // the residuals of fine plane i into its ring slot
-    T* buf = patch[i % kNmRrBuf];
-    const long long base = (long long)i * S2;
-#pragma unroll
-    for (int m = 0; m < kNmRrPer; ++m) {
-      const long long id = base + col[m];
-      const T pp = P[id + S2];
-      const T r = nm_residual_value<T>(pp, pm[m], P[id + S], P[id - S], P[id + 1], P[id - 1], pc[m],
-                                       rhs_at<T, FINE>(f, id), inv_h2);
-      if (in[m]) buf[tid + 256 * m] = r;
-      pm[m] = pc[m];
-      pc[m] = pp;
+    for (int e = 0; e < Vec<T>::W; ++e) {
+      T rhs = fq.v[e];
+      if (FINE) rhs = A::mul(A::mul((T)6.283185307179586, rhs), rhs);
+      const T v = nm_residual_value<T>(u.ip.v[e], u.im.v[e], u.jp.v[e], u.jm.v[e], u.kp.v[e], u.km.v[e], u.c.v[e], rhs, inv_h2);
+      o.v[e] = vinterior(g, row, e) ? v : T(0);
     }
-  };
-  residual_plane(fi0);
-  for (int I = I0; I <= Ilast; ++I) {
-    residual_plane(2 * I);
-    residual_plane(2 * I + 1);
-    __syncthreads();
-    if (!own) continue;
+    if (q.own) stq(r + q.a, o);
+  }
+}
+
+// full weighting (1/64)(8,4,2,1) of r at the coarse point (K, J) of a 32 x 8 tile on planes I0 .. Iend - 1, in
+// the (a, b, c) order of nm_restrict_body; the coarse correction Pc is cleared on the same points
+template <typename T>
+__device__ __forceinline__ void nm_restrict_tile_body(const T* __restrict__ r, T* __restrict__ fc, T* __restrict__ Pc,
+                                                      const Geo& g, const Geo& gc, int bx, int by, int I0, int Iend) {
+  using A = Ar<T>;
+  const int K = 1 + bx * 32 + tile_x<32>(), J = 1 + by * 8 + tile_y<32>();
+  if (K >= gc.NN || J >= gc.NN) return;
+  for (int I = I0; I < Iend; ++I) {
+    const T* q = r + (long long)(2 * I - 1) * g.S2 + (long long)(2 * J - 1) * g.S + 2 * K - 1;
     T v = T(0);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const T* q = patch[(2 * I - 1 + a) % kNmRrBuf] + (2 * ty) * kNmRrPK + 2 * tx;  // fine (2J - 1, 2K - 1)
+    for (int a = 0; a < 3; ++a)
 #pragma unroll
       for (int b = 0; b < 3; ++b)
 #pragma unroll
         for (int c = 0; c < 3; ++c)
-          v = A::add(v, A::mul((T)((a == 1 ? 2 : 1) * (b == 1 ? 2 : 1) * (c == 1 ? 2 : 1)), q[b * kNmRrPK + c]));
-    }
-    const long long cid = (long long)I * gc.S2 + (long long)J * gc.S + K;
-    fc[cid] = A::div(v, T(64));
-    if (Pc) Pc[cid] = T(0);
+          v = A::add(v, A::mul((T)((a == 1 ? 2 : 1) * (b == 1 ? 2 : 1) * (c == 1 ? 2 : 1)),
+                               __ldg(q + a * g.S2 + b * g.S + c)));
+    const long long id = (long long)I * gc.S2 + (long long)J * gc.S + K;
+    fc[id] = A::mul(v, T(1.0 / 64));
+    Pc[id] = T(0);
   }
+}
+
+constexpr int kNmRrTK = 32, kNmRrTJ = 8;
+
+// Coarse planes per block of the restriction and prolongation kernels for a launch of
+// `blocks_per_plane` blocks on each of n coarse planes: 8, halved while the launch would have
+// fewer than 8 blocks per SM (small levels and single grids favour more blocks).
+inline int nm_mg_planes(long long blocks_per_plane, int n) {
+  int planes = 8;
+  while (planes > 1 && blocks_per_plane * ((n + planes - 1) / planes) < 8LL * 148) planes /= 2;
+  return planes;
 }
 
 // coarsest level: `sweeps` red-black sweeps in FP64 by one block; sm: 2*S^3 doubles of smem

@@ -72,7 +72,8 @@ int nm_alloc_levels(rq_ctx* c) {
   if (cudaMalloc(&c->seeds, sizeof(float4) * c->n_atoms) != cudaSuccess ||
       cudaMalloc(&c->scale64, sizeof(double) * c->n_atoms) != cudaSuccess ||
       cudaMalloc((void**)&c->rseed, sizeof(unsigned) * 2) != cudaSuccess ||
-      cudaMalloc((void**)&c->nbm, (size_t)c->g.S3) != cudaSuccess)
+      cudaMalloc((void**)&c->nbm, (size_t)c->g.S3) != cudaSuccess ||
+      cudaMalloc(&c->mg_res, (size_t)c->g.S3 * es) != cudaSuccess)
     return rq_cuda(c, cudaErrorMemoryAllocation, "seed table");
   cudaMemsetAsync(c->rseed, 0, sizeof(unsigned) * 2, c->st);
   cudaMemsetAsync(c->nbm, 0, (size_t)c->g.S3, c->st);  // the face points' masks stay 0
@@ -107,11 +108,11 @@ static int vcycle_level(rq_ctx* c, int l) {
   for (int s = 0; s < c->cfg.mg_pre; ++s)
     for (int color = 0; color < 2; ++color)
       LAUNCH(kc, sizeof(T) * 2.5 * ip, nm_rbgs<T>(P, f, fine, L.g, h2, color, c->st));
-  // the residual, its full weighting and the cleared coarse correction in one pass (the coarse
-  // boundary stays zero from the allocation)
+  // the residual, then its full weighting with the coarse correction cleared (its boundary stays zero from
+  // the allocation)
   rq_mg_level& C = c->mg[l + 1];
-  LAUNCH(kc, sizeof(T) * (2.0 * ip + 2.0 * interior(C.g)),
-         nm_resrestrict<T>(P, f, fine, (T*)C.f, (T*)C.P, L.g, C.g, 1.0 / h2, c->st));
+  LAUNCH(kc, sizeof(T) * 3.0 * ip, nm_residual<T>(P, f, fine, (T*)c->mg_res, L.g, 1.0 / h2, c->st));
+  LAUNCH(kc, sizeof(T) * (ip + 2.0 * interior(C.g)), nm_restrict<T>((const T*)c->mg_res, (T*)C.f, (T*)C.P, L.g, C.g, c->st));
   NmTail t;
   size_t smem = 0;
   if (l + 1 == tail_of<T>(c, t, smem)) {
@@ -335,8 +336,8 @@ int nm_promote(rq_ctx* c) {
   // Every FP64 buffer (fields and multigrid levels) is allocated before anything is freed or
   // swapped: if one allocation fails the context is left exactly as it was (fp32, its captured
   // graphs still valid).
-  void* nb[6] = {};  // U0, U1, P0, P1, K, Kext
-  void* old[6] = {c->U[0], c->U[1], c->P[0], c->P[1], c->K, c->Kext};
+  void* nb[7] = {};  // U0, U1, P0, P1, K, Kext, the multigrid residual
+  void* old[7] = {c->U[0], c->U[1], c->P[0], c->P[1], c->K, c->Kext, c->mg_res};
   std::vector<void*> lv;  // new multigrid buffers, in the order of the (L.P, L.f) walk below
   auto undo = [&]() {
     for (void* p : nb)
@@ -344,7 +345,7 @@ int nm_promote(rq_ctx* c) {
     for (void* p : lv)
       if (p) cudaFree(p);
   };
-  for (int q = 0; q < 6; ++q)
+  for (int q = 0; q < 7; ++q)
     if (old[q] && cudaMalloc(&nb[q], bytes) != cudaSuccess) {
       undo();
       return rq_cuda(c, cudaErrorMemoryAllocation, "promotion to FP64");
@@ -360,7 +361,7 @@ int nm_promote(rq_ctx* c) {
       lv.push_back(q);
     }
   for (int q = 0; q < 6; ++q)
-    if (old[q] && q != 4) {  // K is recomputed below
+    if (old[q] && q != 4) {  // K is recomputed below (and the residual holds nothing between cycles)
       k_nm_widen<<<148 * 4, 256, 0, c->st>>>((const float*)old[q], (double*)nb[q], n);
       const cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) {
@@ -383,6 +384,7 @@ int nm_promote(rq_ctx* c) {
   for (void* p : old)
     if (p) cudaFree(p);
   c->U[0] = nb[0]; c->U[1] = nb[1]; c->P[0] = nb[2]; c->P[1] = nb[3]; c->K = nb[4]; c->Kext = nb[5];
+  c->mg_res = nb[6];
   li = 0;
   for (rq_mg_level& L : c->mg)
     for (void** p : {&L.P, &L.f})

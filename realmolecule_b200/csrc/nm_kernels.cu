@@ -74,11 +74,15 @@ __global__ void __launch_bounds__(256) k_nm_rbgs(T* P, const T* f, Geo g, T h2, 
   nm_vrbgs_body<T, FINE, ROW, COLOR>(P, f, g, h2, blockIdx.x, i0, min(i0 + planes, g.NN));
 }
 
-template <typename T, bool FINE>
-__global__ void __launch_bounds__(256, 4) k_nm_resrestrict(const T* P, const T* f, T* fc, T* Pc, Geo g, Geo gc, T inv_h2,
-                                                        int planes) {
-  __shared__ T patch[kNmRrBuf][kNmRrPatch];
-  nm_resrestrict_body<T, FINE>(P, f, fc, Pc, g, gc, inv_h2, blockIdx.x, blockIdx.y, blockIdx.z, planes, patch);
+template <typename T, bool FINE, int ROW>
+__global__ void __launch_bounds__(256) k_nm_residual(const T* P, const T* f, T* r, Geo g, T inv_h2, int planes) {
+  const int i0 = 1 + (int)blockIdx.y * planes;
+  nm_vresidual_body<T, FINE, ROW>(P, f, r, g, inv_h2, blockIdx.x, i0, min(i0 + planes, g.NN));
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_nm_restrict(const T* r, T* fc, T* Pc, Geo g, Geo gc) {
+  nm_restrict_tile_body<T>(r, fc, Pc, g, gc, blockIdx.x, blockIdx.y, 1 + (int)blockIdx.z, 2 + (int)blockIdx.z);
 }
 
 template <typename T>
@@ -209,17 +213,23 @@ cudaError_t nm_rbgs(T* P, const T* f, bool fine, const Geo& g, double h2, int co
   return cudaGetLastError();
 }
 template <typename T>
-cudaError_t nm_resrestrict(const T* P, const T* f, bool fine, T* fc, T* Pc, const Geo& g, const Geo& gc, double inv_h2,
-                           cudaStream_t st) {
-  const int n = gc.NN - 1;
+cudaError_t nm_residual(const T* P, const T* f, bool fine, T* r, const Geo& g, double inv_h2, cudaStream_t st) {
+  const int planes = vplanes<T>(g, false);
+  const dim3 grd = vgrid<T>(g, planes);
+  auto go = [&](auto fn, auto row) {
+    k_nm_residual<T, decltype(fn)::value, decltype(row)::value><<<grd, 256, 0, st>>>(P, f, r, g, (T)inv_h2, planes);
+  };
+  using Y = std::true_type;
+  using N = std::false_type;
+  if (g.S % 4 == 1) { if (fine) go(Y{}, RowP{}); else go(N{}, RowP{}); }
+  else              { if (fine) go(Y{}, RowM{}); else go(N{}, RowM{}); }
+  return cudaGetLastError();
+}
+template <typename T>
+cudaError_t nm_restrict(const T* r, T* fc, T* Pc, const Geo& g, const Geo& gc, cudaStream_t st) {
+  const unsigned n = (unsigned)(gc.NN - 1);
   if (n < 1) return cudaSuccess;
-  const long long tiles = (long long)((n + kNmRrTK - 1) / kNmRrTK) * ((n + kNmRrTJ - 1) / kNmRrTJ);
-  const int planes = nm_mg_planes(tiles, n);
-  const dim3 blk(32, 8), grd((n + kNmRrTK - 1) / kNmRrTK, (n + kNmRrTJ - 1) / kNmRrTJ, (n + planes - 1) / planes);
-  if (fine)
-    k_nm_resrestrict<T, true><<<grd, blk, 0, st>>>(P, f, fc, Pc, g, gc, (T)inv_h2, planes);
-  else
-    k_nm_resrestrict<T, false><<<grd, blk, 0, st>>>(P, f, fc, Pc, g, gc, (T)inv_h2, planes);
+  k_nm_restrict<T><<<dim3((n + 31) / 32, (n + 7) / 8, n), 256, 0, st>>>(r, fc, Pc, g, gc);
   return cudaGetLastError();
 }
 template <typename T>
@@ -295,8 +305,8 @@ cudaError_t nm_add(T* K, const T* v, long long n, cudaStream_t st) {
   template cudaError_t nm_norm_scale<T>(const double*, const double*, int, double*, int*, cudaStream_t);            \
   template cudaError_t nm_norms<T>(const T*, const int*, const Geo&, double, int, double*, cudaStream_t);           \
   template cudaError_t nm_rbgs<T>(T*, const T*, bool, const Geo&, double, int, cudaStream_t);                       \
-  template cudaError_t nm_resrestrict<T>(const T*, const T*, bool, T*, T*, const Geo&, const Geo&, double,          \
-                                         cudaStream_t);                                                            \
+  template cudaError_t nm_residual<T>(const T*, const T*, bool, T*, const Geo&, double, cudaStream_t);               \
+  template cudaError_t nm_restrict<T>(const T*, T*, T*, const Geo&, const Geo&, cudaStream_t);                       \
   template cudaError_t nm_prolong<T>(const T*, T*, const Geo&, const Geo&, cudaStream_t);                           \
   template cudaError_t nm_coarsest<T>(T*, const T*, const Geo&, double, int, cudaStream_t);                         \
   template cudaError_t nm_tail<T>(const NmTail&, size_t, const T*, T*, cudaStream_t);                                \

@@ -4,7 +4,7 @@
 // 2-5 us whose work is a fraction of that, and the coarsest solve waits for all of them.  One block of 1024
 // threads runs every level from the first that fits through the coarsest and back in shared memory, a
 // barrier where a launch was.  Half a warp takes a row.  Arithmetic and roundings are those of the kernels
-// it stands for (nm_vrbgs_body, nm_resrestrict_body, nm_prolong_cells_body, nm_coarsest_body; k_adj_half,
+// it stands for (nm_vrbgs_body, nm_vresidual_body, nm_restrict_tile_body, nm_prolong_cells_body, nm_coarsest_body; k_adj_half,
 // k_adj_other, k_adj_prolong, k_adj_restrict, k_adj_res, k_adj_muf, k_adj_coarsest), bit for bit.
 // Bound by the barriers and the dependent FP64 chain of the coarsest sweeps.
 #pragma once

@@ -93,6 +93,7 @@ struct rq_ctx {
 
   // new flavour multigrid hierarchy (level 0 = fine)
   std::vector<rq_mg_level> mg;
+  void* mg_res = nullptr;  // new flavour: the residual of the level being restricted (T, S^3)
 
   // atoms on the device
   float* atoms5 = nullptr;    // [i,j,k,Z,rc] f32 (cloud/solver.py:378-382)

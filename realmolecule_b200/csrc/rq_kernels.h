@@ -148,8 +148,9 @@ template <typename T>
 cudaError_t nm_rbgs(T* P, const T* f, bool fine, const Geo& g, double h2, int color, cudaStream_t st);
 // fc = R (f - A P) (the residual and its full weighting in one pass) and Pc = 0 on the coarse interior
 template <typename T>
-cudaError_t nm_resrestrict(const T* P, const T* f, bool fine, T* fc, T* Pc, const Geo& g, const Geo& gc, double inv_h2,
-                           cudaStream_t st);
+cudaError_t nm_residual(const T* P, const T* f, bool fine, T* r, const Geo& g, double inv_h2, cudaStream_t st);
+template <typename T>
+cudaError_t nm_restrict(const T* r, T* fc, T* Pc, const Geo& g, const Geo& gc, cudaStream_t st);
 template <typename T>
 cudaError_t nm_prolong(const T* Ec, T* P, const Geo& g, const Geo& gc, cudaStream_t st);
 template <typename T>
