@@ -17,8 +17,8 @@
 // What bounds it: the dependent chain, ~3 N planes per sweep, not bandwidth.  One launch per cell
 // plane (the form before) cost 3.7 us a plane for a sweep and 32 us for the cell update, whose
 // energy sums were FP64 atomics on one shared word per quantity; a plane inside a block costs a
-// barrier and the f64 chain, ~0.4 us (B200).  A physicsStep of two half-space shells at N = 100 with the
-// multigrid solve: 12.0 ms in 1880 launches before, 3.0 ms in 131.
+// barrier and the f64 chain, ~0.2 us (B200).  A physicsStep of two half-space shells at N = 100 with the
+// multigrid solve: 12.0 ms in 1880 launches before, 1.56 ms in 131.
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -81,18 +81,47 @@ __device__ __forceinline__ bool at_block(const AtGeo& g, int d, AtBlock& b) {
   return true;
 }
 
-// the block's cells and its six face layers of `src` into the tile (edges and corners of the halo are
-// not read: those cells may be written by another block of the same launch)
+// The block's cells and its six face layers of `src` into the tile, a B x B layer per round and thread
+// (edges and corners of the halo are not read: those cells may be written by another block of the same
+// launch).  All loads are issued before a value is stored.  Taken cell by cell with divisions, one load at a
+// time, the tiles' loads and stores were most of a launch: 31 us for a smoothing launch of blocks of 16,
+// 14 us now (83 and 34 us for the cell update).
 template <int B, typename T>
 __device__ __forceinline__ void at_load(T* __restrict__ tile, const float* __restrict__ src, const AtGeo& g,
                                         const AtBlock& b) {
   using L = AtTile<B, T>;
-  for (int q = threadIdx.x; q < (B + 2) * (B + 2) * (B + 2); q += B * B) {
-    const int k = q % (B + 2), j = (q / (B + 2)) % (B + 2), i = q / ((B + 2) * (B + 2));
-    const int out = (i == 0 || i == b.ni + 1) + (j == 0 || j == b.nj + 1) + (k == 0 || k == b.nk + 1);
-    if (i <= b.ni + 1 && j <= b.nj + 1 && k <= b.nk + 1 && out <= 1)
-      tile[i * L::PS + j * L::R + k] =
-          (T)src[(long long)(b.i0 - 1 + i) * g.S2 + (long long)(b.j0 - 1 + j) * g.S + (b.k0 - 1 + k)];
+  const int x = (int)threadIdx.x % B, y = (int)threadIdx.x / B;
+  const float* base = src + (long long)b.i0 * g.S2 + (long long)b.j0 * g.S + b.k0;
+  float v[B + 6];
+  const bool jk = y < b.nj && x < b.nk, ik = y < b.ni && x < b.nk, ij = y < b.ni && x < b.nj;
+  const float* c = base + (long long)y * g.S + x;                // (i, y, x)
+#pragma unroll
+  for (int i = 0; i < B; ++i) v[i] = (jk && i < b.ni) ? c[i * g.S2] : 0.0f;
+  v[B] = jk ? c[-g.S2] : 0.0f;
+  v[B + 1] = jk ? c[b.ni * g.S2] : 0.0f;
+  const float* ci = base + (long long)y * g.S2 + x;              // (y, j, x)
+  v[B + 2] = ik ? ci[-g.S] : 0.0f;
+  v[B + 3] = ik ? ci[(long long)b.nj * g.S] : 0.0f;
+  const float* cj = base + (long long)y * g.S2 + (long long)x * g.S;  // (y, x, k)
+  v[B + 4] = ij ? cj[-1] : 0.0f;
+  v[B + 5] = ij ? cj[b.nk] : 0.0f;
+  T* t = tile + (y + 1) * L::R + x + 1;
+#pragma unroll
+  for (int i = 0; i < B; ++i)
+    if (jk && i < b.ni) t[(i + 1) * L::PS] = (T)v[i];
+  if (jk) {
+    t[0] = (T)v[B];
+    t[(b.ni + 1) * L::PS] = (T)v[B + 1];
+  }
+  if (ik) {
+    T* ti = tile + (y + 1) * L::PS + x + 1;
+    ti[0] = (T)v[B + 2];
+    ti[(b.nj + 1) * L::R] = (T)v[B + 3];
+  }
+  if (ij) {
+    T* tj = tile + (y + 1) * L::PS + (x + 1) * L::R;
+    tj[0] = (T)v[B + 4];
+    tj[b.nk + 1] = (T)v[B + 5];
   }
 }
 
@@ -100,23 +129,27 @@ __device__ __forceinline__ void at_load(T* __restrict__ tile, const float* __res
 template <int B>
 __device__ __forceinline__ void at_load_centre(float* __restrict__ tile, const float* __restrict__ src, const AtGeo& g,
                                                const AtBlock& b) {
-  for (int q = threadIdx.x; q < B * B * B; q += B * B) {
-    const int k = q % B, j = (q / B) % B, i = q / (B * B);
-    if (i < b.ni && j < b.nj && k < b.nk)
-      tile[q] = src[(long long)(b.i0 + i) * g.S2 + (long long)(b.j0 + j) * g.S + (b.k0 + k)];
-  }
+  const float* base = src + (long long)b.i0 * g.S2 + (long long)b.j0 * g.S + b.k0;
+  const int k = (int)threadIdx.x % B, j = (int)threadIdx.x / B;
+  const float* c = base + (long long)j * g.S + k;
+  float v[B];
+#pragma unroll
+  for (int i = 0; i < B; ++i) v[i] = (i < b.ni && j < b.nj && k < b.nk) ? c[i * g.S2] : 0.0f;
+#pragma unroll
+  for (int i = 0; i < B; ++i) tile[(i * B + j) * B + k] = v[i];
 }
 
 template <int B, typename T>
 __device__ __forceinline__ void at_store(const T* __restrict__ tile, float* __restrict__ dst, const AtGeo& g,
                                          const AtBlock& b) {
   using L = AtTile<B, T>;
-  for (int q = threadIdx.x; q < B * B * B; q += B * B) {
-    const int k = q % B, j = (q / B) % B, i = q / (B * B);
-    if (i < b.ni && j < b.nj && k < b.nk)
-      dst[(long long)(b.i0 + i) * g.S2 + (long long)(b.j0 + j) * g.S + (b.k0 + k)] =
-          (float)tile[(i + 1) * L::PS + (j + 1) * L::R + k + 1];
-  }
+  const int k = (int)threadIdx.x % B, j = (int)threadIdx.x / B;
+  if (j >= b.nj || k >= b.nk) return;
+  float* c = dst + (long long)b.i0 * g.S2 + (long long)(b.j0 + j) * g.S + (b.k0 + k);
+  const T* t = tile + L::PS + (j + 1) * L::R + k + 1;
+#pragma unroll
+  for (int i = 0; i < B; ++i)
+    if (i < b.ni) c[i * g.S2] = (float)t[i * L::PS];
 }
 
 struct AtFixed {
@@ -138,7 +171,7 @@ constexpr size_t at_cells_smem(int nS, bool simultaneous) {
 
 // physicsStep's cell body (atom.js:217-315) for every shell on the block diagonal d.
 // acc: E_T, E_ee, E_eK (3) then per shell (ET, Eee, EeK, nrm): f64 sums per thread, one atomic per
-// block and quantity.  Two half-space shells at N = 100: 297 launches, 9.6 ms, before; 19 launches, 1.1 ms.
+// block and quantity.  Two half-space shells at N = 100: 297 launches, 9.6 ms, before; 19 launches, 0.65 ms.
 template <int B, int NS, bool SIM>
 __global__ void __launch_bounds__(B * B) k_at_cells(float* __restrict__ U, float* __restrict__ W, float* __restrict__ P,
                                                     const float* __restrict__ K, AtFixed fixed, AtGeo g, double h,
@@ -310,7 +343,7 @@ __global__ void k_at_rhs(const float* __restrict__ U, const float* __restrict__ 
 // launch tau of pipelined in-place Gauss-Seidel sweeps (atom.js:127-138): sweep blockIdx.y works on
 // the block diagonal tau - 2 blockIdx.y, shell blockIdx.z on its own P and rhs.  The tile holds the
 // f32 values widened, so a cell converts once; a thread owns a column (i, j) and walks k.
-// Two shells at N = 100, four sweeps: 301 launches of 3.7 us per shell before, 25 of 22 us for both now.
+// Two shells at N = 100, four sweeps: 301 launches of 3.7 us per shell before, 25 of 14 us for both now.
 template <int B>
 __global__ void __launch_bounds__(B * B) k_at_gs(float* __restrict__ P, const float* __restrict__ rhs, AtGeo g, double h2,
                                                  int tau) {
