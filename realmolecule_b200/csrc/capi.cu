@@ -132,7 +132,7 @@ static void free_ctx(rq_ctx* c) {
   for (auto& gx : c->graph)
     if (gx) cudaGraphExecDestroy(gx);
   void* ptrs[] = {c->U[0], c->U[1], c->P[0], c->P[1], c->K, c->W, c->bestU, c->rho, c->Pother, c->resid, c->lab[0], c->lab[1],
-                  c->Ec[0], c->Ec[1], c->fc, c->atoms5, c->scratch_atoms5, c->sic, c->sic2, c->pdirect, c->lob, c->lob_part, c->lob_scal, c->lock, c->splits, c->bin_start, c->bin_idx, c->bin_far, c->bin_zmax, c->atoms_mj, c->atoms_nm, c->Zdom, c->Zdom64, c->dnorm,
+                  c->Ec[0], c->Ec[1], c->fc, c->atoms5, c->scratch_atoms5, c->sic, c->sic2, c->pdirect, c->lob, c->lob_part, c->lob_scal, c->lob_done, c->lock, c->splits, c->bin_start, c->bin_idx, c->bin_far, c->bin_zmax, c->atoms_mj, c->atoms_nm, c->Zdom, c->Zdom64, c->dnorm,
                   c->dpd, c->dF, c->dsum, c->unorm, c->scale, c->err, c->seeds, c->scale64, c->Kext, c->rseed, c->K64, c->nbm, c->mg_res};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -174,14 +174,15 @@ static int alloc_all(rq_ctx* c) {
     if (c->cfg.sic) {
       DALLOC(c->sic, S3 * sizeof(float));
       DALLOC(c->sic2, S3 * sizeof(float));
-      if (mj_direct(c)) DALLOC(c->pdirect, S3 * sizeof(float) * n);
+      if (mj_direct(c)) DALLOC(c->pdirect, c->slot() * sizeof(float) * 2 * n);
     }
     DALLOC(c->lock, sizeof(unsigned long long) * n);
     DALLOC(c->splits, sizeof(MjSplit) * n);
     if (c->cfg.lobpcg) {
-      DALLOC(c->lob, S3 * sizeof(float) * 5);
-      DALLOC(c->lob_part, sizeof(float) * kLobMaxWG * kLobNR);
-      DALLOC(c->lob_scal, sizeof(float) * kLobScal);
+      DALLOC(c->lob, c->slot() * sizeof(float) * 5);
+      DALLOC(c->lob_part, sizeof(float) * kLobMaxWG * kLobNR * n);
+      DALLOC(c->lob_scal, sizeof(float) * kLobScal * n);
+      DALLOC(c->lob_done, sizeof(unsigned) * n);
     }
     const int SC = c->g.NN / 2 + 1;
     c->gc = make_geo(SC);

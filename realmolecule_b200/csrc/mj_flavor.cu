@@ -130,7 +130,7 @@ int mj_initialize(rq_ctx* c) {
     for (int m = 0; m < c->n_atoms; ++m)
       if (c->atoms[m].Z != 0)
         LAUNCH(RQ_KC_OTHER, 8.0 * c->g.S3,
-               launch_mj_direct_init(atoms_dev(c), c->n_atoms, m, c->pdirect + (size_t)m * n, c->Pother, c->g, p.h,
+               launch_mj_direct_init(atoms_dev(c), c->n_atoms, m, c->pdirect + (size_t)m * c->slot(), c->Pother, c->g, p.h,
                                      p.h2, c->st));
   }
   return RQ_OK;
@@ -198,14 +198,43 @@ static float mj_cheb_omega(rq_ctx* c) {
   return (float)std::min(1.95, std::max(1.0, omega));
 }
 
+// The direct per-electron Poisson solve of every domain with electrons, in shared launches.
+static int mj_direct_solve(rq_ctx* c, const MjParams& p) {
+  std::vector<int> m;
+  for (int q = 0; q < c->n_atoms; ++q)
+    if ((float)c->atoms[q].Z != 0.f) m.push_back(q);
+  const size_t slot = c->slot();
+  LAUNCH(RQ_KC_POISSON, 120 * interior(c->g) * (double)m.size(),
+         launch_mj_direct((float*)c->U[c->cu], c->lab[c->cl], c->Pother, m.data(), (int)m.size(), c->pdirect,
+                          c->pdirect + (size_t)c->n_atoms * slot, (long long)slot, c->g, p.h2, p.two_pi, c->st));
+  return RQ_OK;
+}
+
+// The level-set passes of a frame.  A pass writes interior cells only, and the spare buffer takes the new labels'
+// faces (those of the page's label2Buf); from then on both buffers have the same faces, so one copy serves
+// all passes.
+static int mj_level_set(rq_ctx* c, const MjParams& p) {
+  const int spf = c->cfg.steps_per_frame;
+  const int wsteps = c->freeze ? 0 : spf > 1 ? spf : 1;  // W_STEPS_PER_FRAME (:107); FREEZE_BOUNDARY (:3095, :3643)
+  for (int q = 0; q < wsteps; ++q) {
+    LAUNCH(RQ_KC_LABELS, 20 * interior(c->g),
+           launch_mj_evolve(c->lab[c->cl], c->lab[1 - c->cl], (float*)c->U[c->cu], c->W, atoms_dev(c), c->n_atoms, c->g,
+                            p.dt_w, p.curvReg, p.h, p.hasBare, c->lock, c->splits, c->st));
+    c->cl ^= 1;
+    if (q == 0)
+      LAUNCH(RQ_KC_LABELS, 8.0 * 6 * c->g.S2, launch_copy_faces(c->lab[c->cl], c->lab[1 - c->cl], c->g, c->st));
+  }
+  return RQ_OK;
+}
+
 // One LOBPCG frame (doLOBPCGStep, molecule.js:3323-3740).  Phase 1: the Poisson solve on the current
 // psi -- the direct per-electron path, or 4 Jacobi sweeps and the V-cycle (vcycleEnabled, :1815) --
 // and Pother: P, minus every domain's own potential when the correction is on (:3405-3451; no
-// SIC_INTERVAL here).  Phase 2: per domain 10 iterations (:3460-3588) of H applied to X, the
-// Rayleigh quotient, the preconditioned residual W, H applied to W and P, the Ritz problem over
-// span{X, W[, P]} and the update of X and P on the domain; the page reads the sums back and solves
-// the small problem on the host, here one device thread does it (k_lob_finalize), so no step waits
-// for the host.  Phase 3 (:3591-3660): the fixed-point normalisation, one ITP update, the level-set
+// SIC_INTERVAL here).  Phase 2: 10 iterations (:3460-3588) of H applied to X, the Rayleigh quotient,
+// the preconditioned residual W, H applied to W and P, the Ritz problem over span{X, W[, P]} and the
+// update of X and P, all domains together (the page takes them one after the other; they share
+// nothing); the page reads the sums back and solves the small problem on the host, here one device
+// thread per domain does it (k_lob_inner), so no step waits for the host.  Phase 3 (:3591-3660): the fixed-point normalisation, one ITP update, the level-set
 // passes.  The search direction P persists across frames; frame 0 starts without one.
 static int mj_lobpcg_frame(rq_ctx* c) {
   const MjParams p = mj_params(c);
@@ -215,12 +244,8 @@ static int mj_lobpcg_frame(rq_ctx* c) {
   const bool direct = mj_direct(c);
   const size_t S3 = (size_t)c->g.S3;
   if (poisson && direct) {
-    for (int m = 0; m < c->n_atoms; ++m) {
-      if ((float)c->atoms[m].Z == 0.f) continue;
-      LAUNCH(RQ_KC_POISSON, 128 * ip,
-             launch_mj_direct_domain((float*)c->U[c->cu], c->lab[c->cl], c->Pother, m, c->pdirect + (size_t)m * S3,
-                                     c->sic, c->rho, c->g, p.h2, p.two_pi, c->st));
-    }
+    int rc = mj_direct_solve(c, p);
+    if (rc != RQ_OK) return rc;
   } else if (poisson) {
     for (int js = 0; js < 4; ++js) {
       LAUNCH(RQ_KC_POISSON, 12 * ip,
@@ -247,57 +272,39 @@ static int mj_lobpcg_frame(rq_ctx* c) {
                                     c->st));
       }
   }
-  float *HX = c->lob, *LW = HX + S3, *HW = LW + S3, *LP = HW + S3, *HP = LP + S3;
-  if (c->frame == 0) CK(cudaMemsetAsync(LP, 0, 2 * S3 * sizeof(float), c->st));  // P and HP
-  const int nwg = lob_workgroups(c->g);
+  const size_t slot = c->slot();
+  float *HX = c->lob, *LW = HX + slot, *HW = LW + slot, *LP = HW + slot, *HP = LP + slot;
+  if (c->frame == 0) CK(cudaMemsetAsync(LW, 0, 4 * slot * sizeof(float), c->st));  // W, HW, P and HP
   float* X = (float*)c->U[c->cu];
   const MjAtom* at = atoms_dev(c);
-  for (int m = 0; m < c->n_atoms; ++m) {
-    if ((float)c->atoms[m].Z == 0.f) continue;
-    for (int it = 0; it < 10; ++it) {
-      const bool hasP = c->frame > 0 || it > 0;
-      LAUNCH(RQ_KC_UPDATE, 20 * ip,
-             launch_lob_apply_h(X, HX, (float*)c->K, c->lab[c->cl], c->Pother, at, c->g, p.h, p.inv_h2, p.hasBare,
-                                c->st));
-      if (it == 0 && !hasP) CK(cudaMemsetAsync(LW, 0, 2 * S3 * sizeof(float), c->st));  // W and HW
-      LAUNCH(RQ_KC_NORMALIZE, 28 * ip,
-             launch_lob_inner(X, HX, LW, HW, LP, HP, c->lab[c->cl], m, c->g, p.h3, c->lob_part, c->st));
-      LAUNCH(RQ_KC_NORMALIZE, 48.0 * nwg, launch_lob_finalize(c->lob_part, nwg, true, hasP, c->lob_scal, c->st));
-      LAUNCH(RQ_KC_UPDATE, 24 * ip,
-             launch_lob_residual(X, HX, LW, c->lab[c->cl], (float*)c->K, c->Pother, c->lob_scal, m, c->g, p.inv_h2,
-                                 c->st));
-      LAUNCH(RQ_KC_UPDATE, 20 * ip,
-             launch_lob_apply_h(LW, HW, (float*)c->K, c->lab[c->cl], c->Pother, at, c->g, p.h, p.inv_h2, p.hasBare,
-                                c->st));
-      if (hasP)
-        LAUNCH(RQ_KC_UPDATE, 20 * ip,
-               launch_lob_apply_h(LP, HP, (float*)c->K, c->lab[c->cl], c->Pother, at, c->g, p.h, p.inv_h2, p.hasBare,
-                                  c->st));
-      LAUNCH(RQ_KC_NORMALIZE, 28 * ip,
-             launch_lob_inner(X, HX, LW, HW, LP, HP, c->lab[c->cl], m, c->g, p.h3, c->lob_part, c->st));
-      LAUNCH(RQ_KC_NORMALIZE, 48.0 * nwg, launch_lob_finalize(c->lob_part, nwg, false, hasP, c->lob_scal, c->st));
-      LAUNCH(RQ_KC_UPDATE, 24 * ip, launch_lob_update(X, LW, LP, c->lab[c->cl], c->lob_scal + 1, m, c->g, c->st));
-    }
+  for (int it = 0; it < 10; ++it) {
+    const bool hasP = c->frame > 0 || it > 0;
+    LAUNCH(RQ_KC_UPDATE, 20 * ip,
+           launch_lob_apply_h(X, HX, nullptr, nullptr, (float*)c->K, c->lab[c->cl], c->Pother, at, c->g, p.h, p.inv_h2,
+                              p.hasBare, c->st));
+    LAUNCH(RQ_KC_NORMALIZE, 12 * ip,
+           launch_lob_inner(X, HX, LW, HW, LP, HP, c->lab[c->cl], at, c->n_atoms, c->g, p.h3, true, hasP, c->lob_part,
+                            c->lob_done, c->lob_scal, c->st));
+    LAUNCH(RQ_KC_UPDATE, 24 * ip,
+           launch_lob_residual(X, HX, LW, c->lab[c->cl], (float*)c->K, c->Pother, c->lob_scal, at, c->g, p.inv_h2,
+                               c->st));
+    LAUNCH(RQ_KC_UPDATE, (hasP ? 40 : 20) * ip,
+           launch_lob_apply_h(LW, HW, hasP ? LP : nullptr, HP, (float*)c->K, c->lab[c->cl], c->Pother, at, c->g, p.h,
+                              p.inv_h2, p.hasBare, c->st));
+    LAUNCH(RQ_KC_NORMALIZE, 28 * ip,
+           launch_lob_inner(X, HX, LW, HW, LP, HP, c->lab[c->cl], at, c->n_atoms, c->g, p.h3, false, hasP, c->lob_part,
+                            c->lob_done, c->lob_scal, c->st));
+    LAUNCH(RQ_KC_UPDATE, 24 * ip, launch_lob_update(X, LW, LP, c->lab[c->cl], c->lob_scal, at, c->g, c->st));
   }
   CK(cudaMemsetAsync(c->unorm, 0, sizeof(unsigned) * c->n_atoms, c->st));
   LAUNCH(RQ_KC_NORMALIZE, 8 * ip, launch_mj_accum_norms(X, c->lab[c->cl], c->g, p.h3, c->unorm, c->st));
-  LAUNCH(RQ_KC_NORMALIZE, 8.0 * c->n_atoms, launch_mj_norm_scale(c->unorm, at, c->n_atoms, c->scale, c->st));
-  LAUNCH(RQ_KC_NORMALIZE, 12 * ip, launch_mj_apply_scale(X, c->lab[c->cl], c->scale, c->g, c->st));
+  LAUNCH(RQ_KC_NORMALIZE, 12 * ip, launch_mj_apply_scale(X, c->lab[c->cl], c->unorm, at, c->g, c->st));
   LAUNCH(RQ_KC_UPDATE, 20 * ip,
          launch_mj_update(X, (float*)c->U[1 - c->cu], (float*)c->K, c->lab[c->cl], c->Pother, c->g, p.half_d, p.dt,
-                          p.h3, c->n_atoms, nullptr, c->st));
+                          p.h3, nullptr, c->st));
   c->cu ^= 1;
   c->frame++;
-  const int wsteps = c->freeze ? 0 : f.steps_per_frame > 1 ? f.steps_per_frame : 1;  // :107; FREEZE_BOUNDARY :3643
-  for (int q = 0; q < wsteps; ++q) {
-    LAUNCH(RQ_KC_LABELS, 20 * ip,
-           launch_mj_evolve(c->lab[c->cl], c->lab[1 - c->cl], (float*)c->U[c->cu], c->W, at, c->n_atoms, c->g, p.dt_w,
-                            p.curvReg, p.h, p.hasBare, c->lock, c->splits, c->st));
-    c->cl ^= 1;
-    // the spare buffer takes the new labels' faces: those of the page's label2Buf
-    LAUNCH(RQ_KC_LABELS, 8.0 * 6 * c->g.S2, launch_copy_faces(c->lab[c->cl], c->lab[1 - c->cl], c->g, c->st));
-  }
-  return RQ_OK;
+  return mj_level_set(c, p);
 }
 
 int mj_step_one(rq_ctx* c, int s) {
@@ -310,12 +317,8 @@ int mj_step_one(rq_ctx* c, int s) {
   const double ip = interior(c->g);
   const bool direct = mj_direct(c);
   if (poisson && direct) {
-    for (int m = 0; m < c->n_atoms; ++m) {
-      if ((float)c->atoms[m].Z == 0.f) continue;
-      LAUNCH(RQ_KC_POISSON, 128 * ip,
-             launch_mj_direct_domain((float*)c->U[c->cu], c->lab[c->cl], c->Pother, m,
-                                     c->pdirect + (size_t)m * c->g.S3, c->sic, c->rho, c->g, p.h2, p.two_pi, c->st));
-    }
+    int rc = mj_direct_solve(c, p);
+    if (rc != RQ_OK) return rc;
   } else if (poisson) {
     for (int js = 0; js < f.jacobi_per_step; ++js) {
       LAUNCH(RQ_KC_POISSON, 12 * ip,
@@ -334,18 +337,16 @@ int mj_step_one(rq_ctx* c, int s) {
     const float omega = mj_cheb_omega(c);
     LAUNCH(RQ_KC_UPDATE, 24 * ip,
            launch_mj_update_cheb((float*)c->U[c->cu], (float*)c->U[1 - c->cu], (float*)c->K, c->lab[c->cl], c->Pother,
-                                 c->g, p.half_d, p.dt, p.h3, c->n_atoms, norm ? c->unorm : nullptr, omega, c->st));
+                                 c->g, p.half_d, p.dt, p.h3, norm ? c->unorm : nullptr, omega, c->st));
   } else {
     LAUNCH(RQ_KC_UPDATE, 20 * ip,
            launch_mj_update((float*)c->U[c->cu], (float*)c->U[1 - c->cu], (float*)c->K, c->lab[c->cl], c->Pother, c->g,
-                            p.half_d, p.dt, p.h3, c->n_atoms, norm ? c->unorm : nullptr, c->st));
+                            p.half_d, p.dt, p.h3, norm ? c->unorm : nullptr, c->st));
   }
   c->cu ^= 1;
-  if (norm) {
-    LAUNCH(RQ_KC_NORMALIZE, 8.0 * c->n_atoms,
-           launch_mj_norm_scale(c->unorm, atoms_dev(c), c->n_atoms, c->scale, c->st));
-    LAUNCH(RQ_KC_NORMALIZE, 12 * ip, launch_mj_apply_scale((float*)c->U[c->cu], c->lab[c->cl], c->scale, c->g, c->st));
-  }
+  if (norm)
+    LAUNCH(RQ_KC_NORMALIZE, 12 * ip,
+           launch_mj_apply_scale((float*)c->U[c->cu], c->lab[c->cl], c->unorm, atoms_dev(c), c->g, c->st));
   if (sf == spf - 1) {
     // frame tail: Pother <- P_buf[0], the self-interaction correction on its frames (the frame
     // counter is the reference's frameCount, incremented before the level-set passes), then the
@@ -367,17 +368,11 @@ int mj_step_one(rq_ctx* c, int s) {
       }
     }
     c->frame++;
-    const int wsteps = c->freeze ? 0 : spf > 1 ? spf : 1;  // W_STEPS_PER_FRAME (:107); FREEZE_BOUNDARY (:3095)
-    for (int q = 0; q < wsteps; ++q) {
-      LAUNCH(RQ_KC_LABELS, 20 * ip,
-             launch_mj_evolve(c->lab[c->cl], c->lab[1 - c->cl], (float*)c->U[c->cu], c->W, atoms_dev(c), c->n_atoms,
-                              c->g, p.dt_w, p.curvReg, p.h, p.hasBare, c->lock, c->splits, c->st));
-      c->cl ^= 1;
-      LAUNCH(RQ_KC_LABELS, 8.0 * 6 * c->g.S2, launch_copy_faces(c->lab[c->cl], c->lab[1 - c->cl], c->g, c->st));
-    }
+    int rc = mj_level_set(c, p);
+    if (rc != RQ_OK) return rc;
     if (c->cfg.chebyshev) {  // the page's E at the frame's end feeds the next frame's omega (:3186)
       double e[RQ_ENERGY_LEN], ekk = 0;
-      int rc = mj_energy(c, e, nullptr);
+      rc = mj_energy(c, e, nullptr);
       if (rc != RQ_OK) return rc;
       mj_nuclear_terms(c, &ekk, nullptr);
       c->cheb_E = e[RQ_E_T] + e[RQ_E_EK] + e[RQ_E_EE] + ekk;

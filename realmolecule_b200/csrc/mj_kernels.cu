@@ -13,6 +13,7 @@
 
 #include "rq_flavors.h"
 #include "rq_kernels.h"
+#include "vec_stencil.cuh"
 
 namespace rq {
 
@@ -161,156 +162,201 @@ __global__ void __launch_bounds__(256) k_mj_flags(int* __restrict__ label, const
 }
 
 // ---------------------------------------------------------------------------------------
-// updateU (molecule.js:263-343, W_CUTOFF = 0): 20 B per interior point.  With ACC the new
-// psi's u32 fixed-point norm per label (molecule.js:912-933) is accumulated as well.
+// The passes of a step own 16-byte vectors of a plane (vec_stencil.cuh).  A page's grid is small (64^3 and
+// its fields stay in L2), so what bounds them is how many loads are in flight: the scalar form marched 16
+// planes per thread on 64 blocks, one dependent load after another, 11.9 us for a sweep at 64^3 and 15.6 us for
+// the update.  Elements outside the interior keep what the output buffer holds (psi's faces are not 0).
 // ---------------------------------------------------------------------------------------
+__device__ __forceinline__ unsigned mj_inside(const Geo& g, const VGroup& r, int i) {
+  if (!r.own) return 0u;
+  const VRow w = vrow(g, r, i);
+  unsigned m = 0u;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) m |= vinterior(g, w, e) ? 1u << e : 0u;
+  return m;
+}
+__device__ __forceinline__ void mj_store(float* p, const VGroup& r, unsigned in, const Quad<float>& q) {
+  if (in == 15u) {
+    stq(p + r.a, q);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (in >> e & 1u) p[r.a + e] = q.v[e];
+  }
+}
+
+// x / 9 correctly rounded by the two-constant product of sixth() (checked for every mantissa at |x| >= 2^-119)
+__device__ __forceinline__ float ninth(float x) {
+  constexpr float zh = 0x1.c71c72p-4f, zl = -0x1.c71c72p-31f;
+  const float a = fabsf(x);
+  if (a >= 0x1p-100f && a <= 0x1p126f) return __fmaf_rn(x, zh, __fmul_rn(x, zl));
+  return F_DIV(x, 9.0f);
+}
+
+// ---------------------------------------------------------------------------------------
+// updateU (molecule.js:263-343, W_CUTOFF = 0): 20 B per interior point.  With ACC the new
+// psi's u32 fixed-point norm per label (molecule.js:912-933) is accumulated as well: sums of
+// integers modulo 2^32, so their order is free.
 // With CHEB the Chebyshev step (molecule.js:345-421): out = omega * (the ITP step) + (1 - omega) *
 // psi_{n-1}, where psi_{n-1} is what Uo holds (the input of the previous step), read at the cell
 // before it is overwritten.
-template <bool ACC, bool CHEB = false>
+// ---------------------------------------------------------------------------------------
+template <bool ACC, bool CHEB>
 __global__ void __launch_bounds__(256) k_mj_update(const float* __restrict__ U, float* __restrict__ Uo,
                                                    const float* __restrict__ K, const int* __restrict__ label,
-                                                   const float* __restrict__ Pother, Geo g, float half_d, float dt,
-                                                   float h3, int nDom, unsigned* __restrict__ unorm,
-                                                   float omega = 1.0f) {
+                                                   const float* __restrict__ Pother, Geo g, int planes, float half_d,
+                                                   float dt, float h3, unsigned* __restrict__ unorm, float omega) {
   constexpr int NSLOT = 128;
   __shared__ int keys[NSLOT];
   __shared__ unsigned vals[NSLOT];
-  const int tid = threadIdx.x + blockDim.x * threadIdx.y;
+  const int tid = threadIdx.x;
   if (ACC) {
-    for (int s = tid; s < NSLOT; s += blockDim.x * blockDim.y) { keys[s] = -1; vals[s] = 0u; }
+    for (int s = tid; s < NSLOT; s += blockDim.x) { keys[s] = -1; vals[s] = 0u; }
     __syncthreads();
   }
-  const int k = 1 + blockIdx.x * kThreadsK + threadIdx.x;
-  const int j = 1 + blockIdx.y * kThreadsJ + threadIdx.y;
-  const int i0 = 1 + blockIdx.z * kMarch;
   int runL = -1;
   unsigned runV = 0u;
-  auto flush_run = [&]() {
-    if (runL < 0) return;
-    unsigned slot = ((unsigned)runL * 2654435761u) & (NSLOT - 1);
+  auto add_label = [&](int L, unsigned v) {
+    unsigned slot = ((unsigned)L * 2654435761u) & (NSLOT - 1);
     for (int p = 0; p < NSLOT; ++p) {
-      const int old = atomicCAS(&keys[slot], -1, runL);
-      if (old == -1 || old == runL) { atomicAdd(&vals[slot], runV); return; }
+      const int old = atomicCAS(&keys[slot], -1, L);
+      if (old == -1 || old == L) { atomicAdd(&vals[slot], v); return; }
       slot = (slot + 1) & (NSLOT - 1);
     }
-    atomicAdd(&unorm[runL], runV);
+    atomicAdd(&unorm[L], v);
   };
-  if (k < g.NN && j < g.NN && i0 < g.NN) {
-    const int iend = min(i0 + kMarch, g.NN);
-    const long long S = g.S, S2 = g.S2;
-    long long id = (long long)i0 * S2 + j * S + k;
-    float u_m = __ldg(U + id - S2), u_c = __ldg(U + id);
-    int l_m = __ldg(label + id - S2), l_c = __ldg(label + id);
-    for (int i = i0; i < iend; ++i, id += S2) {
-      const float u_p = __ldg(U + id + S2);
-      const int l_p = __ldg(label + id + S2);
-      float out;
-      if (l_c & kMjExcl) {
-        out = 0.0f;  // Dirichlet inside the own r_c sphere
-      } else {
-        const float ujp = __ldg(U + id + S), ujm = __ldg(U + id - S), ukp = __ldg(U + id + 1), ukm = __ldg(U + id - 1);
-        const int ljp = __ldg(label + id + S), ljm = __ldg(label + id - S), lkp = __ldg(label + id + 1),
-                  lkm = __ldg(label + id - 1);
+  const int i0 = 1 + blockIdx.y * planes, iend = min(i0 + planes, g.NN);
+  for (int i = i0; i < iend; ++i) {
+    const VGroup r = vgroup<float>(g, i, blockIdx.x);
+    const VLoad<int, kRowAny> ll(label, r, g);
+    const VLoad<float, kRowAny> lu(U, r, g);
+    const Quad<float> k4 = ldq(K + r.a), p4 = ldq(Pother + r.a);
+    Quad<float> w4;
+    if (CHEB) w4 = *reinterpret_cast<const Quad<float>*>(Uo + r.a);
+    const unsigned in = mj_inside(g, r, i);
+    const Star<int> l = vstar(ll);
+    const Star<float> u = vstar(lu);
+    Quad<float> o;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int lc = l.c.v[e];
+      const float uc = u.c.v[e];
+      float out = 0.0f;  // Dirichlet inside the own r_c sphere
+      if (!(lc & kMjExcl)) {
         // a neighbour is used iff same label and not inside its r_c sphere: packed words equal
-        const float a = (l_p == l_c) ? u_p : u_c;
-        const float b = (l_m == l_c) ? u_m : u_c;
-        const float c = (ljp == l_c) ? ujp : u_c;
-        const float d = (ljm == l_c) ? ujm : u_c;
-        const float e = (lkp == l_c) ? ukp : u_c;
-        const float f = (lkm == l_c) ? ukm : u_c;
-        const float lap = F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(a, b), c), d), e), f), F_MUL(6.0f, u_c));
-        out = F_ADD(F_ADD(u_c, F_MUL(half_d, lap)),
-                    F_MUL(F_MUL(dt, F_SUB(__ldg(K + id), F_MUL(2.0f, __ldg(Pother + id)))), u_c));
-        if (CHEB) out = F_ADD(F_MUL(omega, out), F_MUL(F_SUB(1.0f, omega), Uo[id]));
+        const float a = l.ip.v[e] == lc ? u.ip.v[e] : uc, b = l.im.v[e] == lc ? u.im.v[e] : uc;
+        const float c = l.jp.v[e] == lc ? u.jp.v[e] : uc, d = l.jm.v[e] == lc ? u.jm.v[e] : uc;
+        const float q = l.kp.v[e] == lc ? u.kp.v[e] : uc, f = l.km.v[e] == lc ? u.km.v[e] : uc;
+        const float lap = F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(a, b), c), d), q), f), F_MUL(6.0f, uc));
+        out = F_ADD(F_ADD(uc, F_MUL(half_d, lap)), F_MUL(F_MUL(dt, F_SUB(k4.v[e], F_MUL(2.0f, p4.v[e]))), uc));
+        if (CHEB) out = F_ADD(F_MUL(omega, out), F_MUL(F_SUB(1.0f, omega), w4.v[e]));
       }
-      Uo[id] = out;
-      if (ACC) {
+      o.v[e] = out;
+      if (ACC && (in >> e & 1u)) {
         const unsigned contrib = __float2uint_rz(F_MUL(F_MUL(F_MUL(out, out), h3), 16777216.0f));
-        const int L = l_c & kMjMask;
-        if (L != runL) { flush_run(); runL = L; runV = contrib; } else { runV += contrib; }
+        const int L = lc & kMjMask;
+        if (L != runL) {
+          if (runL >= 0) add_label(runL, runV);
+          runL = L;
+          runV = contrib;
+        } else {
+          runV += contrib;
+        }
       }
-      u_m = u_c; u_c = u_p; l_m = l_c; l_c = l_p;
     }
+    mj_store(Uo, r, in, o);
   }
   if (ACC) {
-    flush_run();
+    int same;
+    __match_all_sync(0xffffffffu, runL, &same);
+    if (same) {  // the usual warp: one label
+      runV = __reduce_add_sync(0xffffffffu, runV);
+      if ((tid & 31) != 0) runL = -1;
+    }
+    if (runL >= 0) add_label(runL, runV);
     __syncthreads();
-    for (int s = tid; s < NSLOT; s += blockDim.x * blockDim.y)
+    for (int s = tid; s < NSLOT; s += blockDim.x)
       if (keys[s] >= 0) atomicAdd(&unorm[keys[s]], vals[s]);
   }
 }
 
-// decodeNorms + the scale of normalize (molecule.js:938-946, :1098-1104): n = f32(acc)*2^-24,
-// scale = sqrt(Z/n) if n > 0 and Z > 0 else 1.
-__global__ void k_mj_norm_scale(const unsigned* __restrict__ unorm, const MjAtom* __restrict__ atoms, int nDom,
-                                float* __restrict__ scale) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= nDom) return;
-  const float n = F_MUL((float)unorm[l], 5.9604644775390625e-08f);
-  const float Z = atoms[l].Z;
-  scale[l] = (n > 0.f && Z > 0.f) ? F_SQRT(F_DIV(Z, n)) : 1.0f;
-}
-
+// decodeNorms + normalize (molecule.js:938-946, :1079-1104): n = f32(acc) * 2^-24, psi *= sqrt(Z/n) if n > 0 and
+// Z > 0 else 1.  The factor is made where it is used, again for each run of a label in a thread: a launch less.
 __global__ void __launch_bounds__(256) k_mj_apply_scale(float* __restrict__ U, const int* __restrict__ label,
-                                                        const float* __restrict__ scale, Geo g) {
-  const int k = 1 + blockIdx.x * kThreadsK + threadIdx.x;
-  const int j = 1 + blockIdx.y * kThreadsJ + threadIdx.y;
-  const int i0 = 1 + blockIdx.z * kMarch;
-  if (k >= g.NN || j >= g.NN || i0 >= g.NN) return;
-  const int iend = min(i0 + kMarch, g.NN);
+                                                        const unsigned* __restrict__ unorm,
+                                                        const MjAtom* __restrict__ atoms, Geo g, int planes) {
+  const int i0 = 1 + blockIdx.y * planes, iend = min(i0 + planes, g.NN);
+  int last = -1;
+  float scale = 1.0f;
   for (int i = i0; i < iend; ++i) {
-    const long long id = (long long)i * g.S2 + (long long)j * g.S + k;
-    U[id] = F_MUL(U[id], scale[label[id] & kMjMask]);
+    const VGroup r = vgroup<float>(g, i, blockIdx.x);
+    const unsigned in = mj_inside(g, r, i);
+    const Quad<int> l = ldq(label + r.a);
+    Quad<float> u = *reinterpret_cast<const Quad<float>*>(U + r.a);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (!(in >> e & 1u)) continue;
+      const int L = l.v[e] & kMjMask;
+      if (L != last) {
+        const float n = F_MUL((float)__ldg(unorm + L), 5.9604644775390625e-08f);
+        const float Z = atoms[L].Z;
+        scale = (n > 0.f && Z > 0.f) ? F_SQRT(F_DIV(Z, n)) : 1.0f;
+        last = L;
+      }
+      u.v[e] = F_MUL(u.v[e], scale);
+    }
+    mj_store(U, r, in, u);
   }
 }
 
-// Weighted Jacobi with rho = psi^2 inline (molecule.js:723-749, :754-774).  12 B per point.
+// Weighted Jacobi (molecule.js:723-749, :754-774).  RHS: the density from psi, from a buffer (the
+// self-potential solve of the self-interaction correction, :3024-3030), or psi^2 outside the
+// domain (computeRhoOther, :593-612) for the direct path, where one launch sweeps all its domains' P_m
+// (they do not depend on one another): slot d % nd of Pin / Pout holds domain doms.m[d].  Blocks of the same
+// cells are neighbours in the grid, so psi and the labels come from memory once for all domains.  LAST:
+// copyPotherForLabel (:651-671) on the way out.  10 sweeps of water's 3 domains at 64^3, with the density and
+// the copy: 387 us as 36 launches of 64 to 1073 blocks, 41 us as 10.
+constexpr int kMjRhoPsi = 0, kMjRhoBuf = 1, kMjRhoOther = 2;
+constexpr int kMjDoms = 8;  // domains of a launch
+struct MjDoms {
+  int n;
+  int m[kMjDoms];
+  long long slot;  // elements between two domains' P
+};
+template <int RHS, bool LAST>
 __global__ void __launch_bounds__(256) k_mj_jacobi(const float* __restrict__ Pin, float* __restrict__ Pout,
-                                                   const float* __restrict__ U, Geo g, float h2, float two_pi) {
-  const int k = 1 + blockIdx.x * kThreadsK + threadIdx.x;
-  const int j = 1 + blockIdx.y * kThreadsJ + threadIdx.y;
-  const int i0 = 1 + blockIdx.z * kMarch;
-  if (k >= g.NN || j >= g.NN || i0 >= g.NN) return;
-  const int iend = min(i0 + kMarch, g.NN);
-  const long long S = g.S, S2 = g.S2;
-  long long id = (long long)i0 * S2 + j * S + k;
-  float p_m = __ldg(Pin + id - S2), p_c = __ldg(Pin + id);
-  const float c0 = F_MUL(h2, two_pi);
-  for (int i = i0; i < iend; ++i, id += S2) {
-    const float p_p = __ldg(Pin + id + S2);
-    const float u = __ldg(U + id);
-    const float sn = F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(p_p, p_m), __ldg(Pin + id + S)), __ldg(Pin + id - S)),
-                                 __ldg(Pin + id + 1)),
-                           __ldg(Pin + id - 1));
-    const float rhs = F_MUL(c0, F_MUL(u, u));
-    Pout[id] = F_ADD(F_MUL(0.3333f, p_c), F_DIV(F_ADD(sn, rhs), 9.0f));
-    p_m = p_c; p_c = p_p;
+                                                   const float* __restrict__ R, const int* __restrict__ label,
+                                                   float* __restrict__ Pother, MjDoms doms, Geo g, int planes, float h2,
+                                                   float two_pi) {
+  int blk = blockIdx.x, m = 0;
+  if (RHS == kMjRhoOther) {
+    blk = (int)blockIdx.x / doms.n;
+    m = doms.m[(int)blockIdx.x - blk * doms.n];
+    Pin += m * doms.slot;
+    Pout += m * doms.slot;
   }
-}
-
-// The same weighted Jacobi sweep with the right-hand side read from a density buffer: the
-// self-potential solve of the self-interaction correction (jacobiSmooth with rhoTotal bound to
-// the single-domain density, molecule.js:723-749, :3024-3030).
-__global__ void __launch_bounds__(256) k_mj_jacobi_rho(const float* __restrict__ Pin, float* __restrict__ Pout,
-                                                       const float* __restrict__ rho, Geo g, float h2, float two_pi) {
-  const int k = 1 + blockIdx.x * kThreadsK + threadIdx.x;
-  const int j = 1 + blockIdx.y * kThreadsJ + threadIdx.y;
-  const int i0 = 1 + blockIdx.z * kMarch;
-  if (k >= g.NN || j >= g.NN || i0 >= g.NN) return;
-  const int iend = min(i0 + kMarch, g.NN);
-  const long long S = g.S, S2 = g.S2;
-  long long id = (long long)i0 * S2 + j * S + k;
-  float p_m = __ldg(Pin + id - S2), p_c = __ldg(Pin + id);
   const float c0 = F_MUL(h2, two_pi);
-  for (int i = i0; i < iend; ++i, id += S2) {
-    const float p_p = __ldg(Pin + id + S2);
-    const float sn = F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(p_p, p_m), __ldg(Pin + id + S)), __ldg(Pin + id - S)),
-                                 __ldg(Pin + id + 1)),
-                           __ldg(Pin + id - 1));
-    const float rhs = F_MUL(c0, __ldg(rho + id));
-    Pout[id] = F_ADD(F_MUL(0.3333f, p_c), F_DIV(F_ADD(sn, rhs), 9.0f));
-    p_m = p_c; p_c = p_p;
+  const int i0 = 1 + blockIdx.y * planes, iend = min(i0 + planes, g.NN);
+  for (int i = i0; i < iend; ++i) {
+    const VGroup r = vgroup<float>(g, i, blk);
+    const VLoad<float, kRowAny> lp(Pin, r, g);
+    const Quad<float> q = ldq(R + r.a);
+    Quad<int> l;
+    if (RHS == kMjRhoOther) l = ldq(label + r.a);
+    const unsigned in = mj_inside(g, r, i);
+    const Star<float> p = vstar(lp);
+    Quad<float> o;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float rho = q.v[e];
+      if (RHS != kMjRhoBuf) rho = F_MUL(rho, rho);
+      if (RHS == kMjRhoOther && (l.v[e] & kMjMask) == m) rho = 0.0f;
+      const float sn = F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(p.ip.v[e], p.im.v[e]), p.jp.v[e]), p.jm.v[e]), p.kp.v[e]),
+                             p.km.v[e]);
+      o.v[e] = F_ADD(F_MUL(0.3333f, p.c.v[e]), ninth(F_ADD(sn, F_MUL(c0, rho))));
+      if (LAST && (in >> e & 1u) && (l.v[e] & kMjMask) == m) Pother[r.a + e] = o.v[e];
+    }
+    mj_store(Pout, r, in, o);
   }
 }
 
@@ -348,25 +394,6 @@ __global__ void k_mj_sub_self(const float* __restrict__ Pm, float* __restrict__ 
   int i, j, k;
   if (id >= g.S3 || !interior_of(id, g, i, j, k)) return;
   if ((label[id] & kMjMask) == m) Pother[id] = F_SUB(Pother[id], F_MUL(Pm[id], frac));
-}
-
-// computeRhoOther (molecule.js:593-612): psi^2 except where the label is m (interior points)
-__global__ void k_mj_rho_other(const float* __restrict__ U, const int* __restrict__ label, int m,
-                               float* __restrict__ rho, Geo g) {
-  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, k;
-  if (id >= g.S3 || !interior_of(id, g, i, j, k)) return;
-  const float u = U[id];
-  rho[id] = ((label[id] & kMjMask) == m) ? 0.0f : F_MUL(u, u);
-}
-
-// copyPotherForLabel (molecule.js:651-671): Pother = Psrc where the label is m
-__global__ void k_mj_copy_for_label(const float* __restrict__ Psrc, float* __restrict__ Pother,
-                                    const int* __restrict__ label, int m, Geo g) {
-  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, k;
-  if (id >= g.S3 || !interior_of(id, g, i, j, k)) return;
-  if ((label[id] & kMjMask) == m) Pother[id] = Psrc[id];
 }
 
 // initPdirect (molecule.js:614-649): P_m = sum over charged n != m of 0.5 / sqrt(r^2 + h^2) (f32,
@@ -684,42 +711,46 @@ cudaError_t launch_mj_flags(int* label, const MjAtom* atoms, int nAt, const Geo&
   k_mj_flags<<<flat_blocks(g.S3), 256, 0, st>>>(label, atoms, nAt, g, h, hasBare);
   return cudaGetLastError();
 }
+template <bool ACC, bool CHEB>
+static void mj_update(const float* U, float* Uo, const float* K, const int* label, const float* Pother, const Geo& g,
+                      float half_d, float dt, float h3, unsigned* unorm, float omega, cudaStream_t st) {
+  const int planes = vplanes<float>(g, false);
+  k_mj_update<ACC, CHEB><<<vgrid<float>(g, planes), 256, 0, st>>>(U, Uo, K, label, Pother, g, planes, half_d, dt, h3,
+                                                                  unorm, omega);
+}
 cudaError_t launch_mj_update(const float* U, float* Uo, const float* K, const int* label, const float* Pother,
-                             const Geo& g, float half_d, float dt, float h3, int nDom, unsigned* unorm,
-                             cudaStream_t st) {
-  if (g.NN < 2) return cudaSuccess;
+                             const Geo& g, float half_d, float dt, float h3, unsigned* unorm, cudaStream_t st) {
   if (unorm)
-    k_mj_update<true><<<march_grid(g), march_block(), 0, st>>>(U, Uo, K, label, Pother, g, half_d, dt, h3, nDom, unorm);
+    mj_update<true, false>(U, Uo, K, label, Pother, g, half_d, dt, h3, unorm, 1.0f, st);
   else
-    k_mj_update<false><<<march_grid(g), march_block(), 0, st>>>(U, Uo, K, label, Pother, g, half_d, dt, h3, nDom,
-                                                                 nullptr);
+    mj_update<false, false>(U, Uo, K, label, Pother, g, half_d, dt, h3, nullptr, 1.0f, st);
   return cudaGetLastError();
 }
 cudaError_t launch_mj_update_cheb(const float* U, float* Uo, const float* K, const int* label, const float* Pother,
-                                  const Geo& g, float half_d, float dt, float h3, int nDom, unsigned* unorm,
-                                  float omega, cudaStream_t st) {
-  if (g.NN < 2) return cudaSuccess;
+                                  const Geo& g, float half_d, float dt, float h3, unsigned* unorm, float omega,
+                                  cudaStream_t st) {
   if (unorm)
-    k_mj_update<true, true><<<march_grid(g), march_block(), 0, st>>>(U, Uo, K, label, Pother, g, half_d, dt, h3, nDom,
-                                                                      unorm, omega);
+    mj_update<true, true>(U, Uo, K, label, Pother, g, half_d, dt, h3, unorm, omega, st);
   else
-    k_mj_update<false, true><<<march_grid(g), march_block(), 0, st>>>(U, Uo, K, label, Pother, g, half_d, dt, h3, nDom,
-                                                                       nullptr, omega);
+    mj_update<false, true>(U, Uo, K, label, Pother, g, half_d, dt, h3, nullptr, omega, st);
   return cudaGetLastError();
 }
-cudaError_t launch_mj_norm_scale(const unsigned* unorm, const MjAtom* atoms, int nDom, float* scale, cudaStream_t st) {
-  k_mj_norm_scale<<<(nDom + 127) / 128, 128, 0, st>>>(unorm, atoms, nDom, scale);
+cudaError_t launch_mj_apply_scale(float* U, const int* label, const unsigned* unorm, const MjAtom* atoms, const Geo& g,
+                                  cudaStream_t st) {
+  const int planes = vplanes<float>(g, false);
+  k_mj_apply_scale<<<vgrid<float>(g, planes), 256, 0, st>>>(U, label, unorm, atoms, g, planes);
   return cudaGetLastError();
 }
-cudaError_t launch_mj_apply_scale(float* U, const int* label, const float* scale, const Geo& g, cudaStream_t st) {
-  if (g.NN < 2) return cudaSuccess;
-  k_mj_apply_scale<<<march_grid(g), march_block(), 0, st>>>(U, label, scale, g);
-  return cudaGetLastError();
+template <int RHS>
+static void mj_jacobi(const float* Pin, float* Pout, const float* R, const Geo& g, float h2, float two_pi,
+                      cudaStream_t st) {
+  const int planes = vplanes<float>(g, false);
+  k_mj_jacobi<RHS, false><<<vgrid<float>(g, planes), 256, 0, st>>>(Pin, Pout, R, nullptr, nullptr, MjDoms{}, g, planes,
+                                                                   h2, two_pi);
 }
 cudaError_t launch_mj_jacobi(const float* Pin, float* Pout, const float* U, const Geo& g, float h2, float two_pi,
                              cudaStream_t st) {
-  if (g.NN < 2) return cudaSuccess;
-  k_mj_jacobi<<<march_grid(g), march_block(), 0, st>>>(Pin, Pout, U, g, h2, two_pi);
+  mj_jacobi<kMjRhoPsi>(Pin, Pout, U, g, h2, two_pi, st);
   return cudaGetLastError();
 }
 // molecule.js:2879-2907 (and :3031-3061 for the self-potential): residual of P for the density
@@ -751,16 +782,23 @@ cudaError_t launch_mj_direct_init(const MjAtom* atoms, int nAt, int m, float* Pm
   return cudaGetLastError();
 }
 
-cudaError_t launch_mj_direct_domain(const float* U, const int* label, float* Pother, int m, float* Pm, float* scratch,
-                                    float* rho, const Geo& g, float h2, float two_pi, cudaStream_t st) {
-  // molecule.js:2835-2857 for one domain: the density of every other domain, 10 Jacobi sweeps of
-  // the persistent P_m (P_m <-> scratch, ending in P_m), then Pother = P_m on the domain
-  if (g.NN < 2) return cudaSuccess;
-  k_mj_rho_other<<<flat_blocks(g.S3), 256, 0, st>>>(U, label, m, rho, g);
-  for (int js = 0; js < 10; ++js)
-    k_mj_jacobi_rho<<<march_grid(g), march_block(), 0, st>>>(js % 2 ? scratch : Pm, js % 2 ? Pm : scratch, rho, g, h2,
-                                                             two_pi);
-  k_mj_copy_for_label<<<flat_blocks(g.S3), 256, 0, st>>>(Pm, Pother, label, m, g);
+cudaError_t launch_mj_direct(const float* U, const int* label, float* Pother, const int* m, int n, float* P, float* P2,
+                             long long slot, const Geo& g, float h2, float two_pi, cudaStream_t st) {
+  // molecule.js:2835-2857 for n domains: 10 Jacobi sweeps of each persistent P_m (P <-> P2, ending
+  // in P) on the density of every other domain, then Pother = P_m on the domain
+  const int planes = vplanes<float>(g, false);
+  const dim3 grid = vgrid<float>(g, planes);
+  for (int d0 = 0; d0 < n; d0 += kMjDoms) {
+    MjDoms doms;
+    doms.n = std::min(n - d0, kMjDoms);
+    doms.slot = slot;
+    for (int d = 0; d < doms.n; ++d) doms.m[d] = m[d0 + d];
+    const dim3 gd(grid.x * doms.n, grid.y);
+    for (int js = 0; js < 9; ++js)
+      k_mj_jacobi<kMjRhoOther, false><<<gd, 256, 0, st>>>(js % 2 ? P2 : P, js % 2 ? P : P2, U, label, Pother, doms, g,
+                                                          planes, h2, two_pi);
+    k_mj_jacobi<kMjRhoOther, true><<<gd, 256, 0, st>>>(P2, P, U, label, Pother, doms, g, planes, h2, two_pi);
+  }
   return cudaGetLastError();
 }
 
@@ -769,17 +807,14 @@ cudaError_t launch_mj_sic_domain(const float* U, const int* label, float* Pother
                                  const Geo& gc, float h2, float inv_h2, float two_pi, cudaStream_t st) {
   // molecule.js:3018-3075 for one domain: its density, 4 Jacobi sweeps from 0 (sic <-> sic2),
   // the coarse correction, 4 more sweeps, then Pother -= P_m / Z_m on the domain
-  if (g.NN < 2) return cudaSuccess;
   k_mj_rho_self<<<flat_blocks(g.S3), 256, 0, st>>>(U, label, m, rho, g);
   cudaError_t e = cudaMemsetAsync(sic, 0, sizeof(float) * g.S3, st);
   if (e != cudaSuccess) return e;
   for (int js = 0; js < 4; ++js)
-    k_mj_jacobi_rho<<<march_grid(g), march_block(), 0, st>>>(js % 2 ? sic2 : sic, js % 2 ? sic : sic2, rho, g, h2,
-                                                             two_pi);
+    mj_jacobi<kMjRhoBuf>(js % 2 ? sic2 : sic, js % 2 ? sic : sic2, rho, g, h2, two_pi, st);
   if ((e = mj_vcycle_core(sic, rho, resid, Ec0, Ec1, fc, g, gc, h2, inv_h2, two_pi, st)) != cudaSuccess) return e;
   for (int js = 0; js < 4; ++js)
-    k_mj_jacobi_rho<<<march_grid(g), march_block(), 0, st>>>(js % 2 ? sic2 : sic, js % 2 ? sic : sic2, rho, g, h2,
-                                                             two_pi);
+    mj_jacobi<kMjRhoBuf>(js % 2 ? sic2 : sic, js % 2 ? sic : sic2, rho, g, h2, two_pi, st);
   k_mj_sub_self<<<flat_blocks(g.S3), 256, 0, st>>>(sic, Pother, label, m, frac, g);
   return cudaGetLastError();
 }
@@ -901,99 +936,94 @@ __device__ __forceinline__ bool lob_inside_rc(int ci, int cj, int ck, int lbl, c
   return a.rc > 0.f && mj_dist(ci, cj, ck, a, h) < a.rc;
 }
 
+// The domains of a frame do not depend on one another: a domain's X, W and P are read and written on its own
+// cells only (a neighbour of another label counts as the centre), so the page's loop over domains, 10
+// iterations each, runs here as 10 iterations of all domains, each pass one launch, every sum as the page
+// forms it.  Water at 64^3: 89 launches of 4 to 13 us per domain and frame before, 60 for all domains now.
+
 // applyH (molecule.js:1483-1525): HU = -0.5*lap/h^2 + (-K + 2*Pother)*u, 0 inside the own r_c
 // sphere, a neighbour of another label or inside its label's sphere replaced by the centre.
 // Without bare nuclei the stored exclusion bit is exactly this test (packed words compare equal
 // iff same label and the neighbour is not excluded); with them (BARE) the bit also marks the
 // bare nuclei's spheres, which this shader ignores, so the spheres are tested directly.
+// blockIdx.z = 1 is the second field (P beside W).
 template <bool BARE>
-__global__ void __launch_bounds__(256) k_lob_apply_h(const float* __restrict__ U, float* __restrict__ HU,
+__global__ void __launch_bounds__(256) k_lob_apply_h(const float* __restrict__ U0, float* __restrict__ H0,
+                                                     const float* __restrict__ U1, float* __restrict__ H1,
                                                      const float* __restrict__ K, const int* __restrict__ label,
                                                      const float* __restrict__ Pother, const MjAtom* __restrict__ atoms,
-                                                     Geo g, float h, float inv_h2) {
-  // one interior cell per thread: the LOBPCG grids are small, and a march along i would leave
-  // most SMs idle (64 blocks at 64^3)
-  const int k = 1 + blockIdx.x * 32 + threadIdx.x, j = 1 + blockIdx.y * 8 + threadIdx.y, i = 1 + blockIdx.z;
-  if (k >= g.NN || j >= g.NN) return;
-  const long long S = g.S, S2 = g.S2;
-  const long long id = (long long)i * S2 + j * S + k;
-  const int l_c = __ldg(label + id), l_p = __ldg(label + id + S2), l_m = __ldg(label + id - S2);
-  const int ljp = __ldg(label + id + S), ljm = __ldg(label + id - S), lkp = __ldg(label + id + 1),
-            lkm = __ldg(label + id - 1);
-  bool excl, up, um, ujp, ujm, ukp, ukm;  // excl: centre excluded; uX: neighbour X is used
-  if (BARE) {
-    const int L = l_c & kMjMask;
-    excl = lob_inside_rc(i, j, k, L, atoms, h);
-    up = (l_p & kMjMask) == L && !lob_inside_rc(i + 1, j, k, l_p & kMjMask, atoms, h);
-    um = (l_m & kMjMask) == L && !lob_inside_rc(i - 1, j, k, l_m & kMjMask, atoms, h);
-    ujp = (ljp & kMjMask) == L && !lob_inside_rc(i, j + 1, k, ljp & kMjMask, atoms, h);
-    ujm = (ljm & kMjMask) == L && !lob_inside_rc(i, j - 1, k, ljm & kMjMask, atoms, h);
-    ukp = (lkp & kMjMask) == L && !lob_inside_rc(i, j, k + 1, lkp & kMjMask, atoms, h);
-    ukm = (lkm & kMjMask) == L && !lob_inside_rc(i, j, k - 1, lkm & kMjMask, atoms, h);
-  } else {
-    excl = (l_c & kMjExcl) != 0;
-    up = l_p == l_c; um = l_m == l_c; ujp = ljp == l_c; ujm = ljm == l_c; ukp = lkp == l_c; ukm = lkm == l_c;
+                                                     Geo g, int planes, float h, float inv_h2) {
+  const float* __restrict__ U = blockIdx.z ? U1 : U0;
+  float* __restrict__ HU = blockIdx.z ? H1 : H0;
+  const int i0 = 1 + blockIdx.y * planes, iend = min(i0 + planes, g.NN);
+  for (int i = i0; i < iend; ++i) {
+    const VGroup r = vgroup<float>(g, i, blockIdx.x);
+    const VLoad<int, kRowAny> ll(label, r, g);
+    const VLoad<float, kRowAny> lu(U, r, g);
+    const Quad<float> k4 = ldq(K + r.a), p4 = ldq(Pother + r.a);
+    const unsigned in = mj_inside(g, r, i);
+    const Star<int> l = vstar(ll);
+    const Star<float> u = vstar(lu);
+    Quad<float> o;
+    const VRow vr = vrow(g, r, i);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int lc = l.c.v[e];
+      bool excl, up, um, ujp, ujm, ukp, ukm;  // excl: centre excluded; uX: neighbour X is used
+      if (BARE) {
+        if (!(in >> e & 1u)) continue;
+        int j = vr.j, k = vr.k + e;
+        if (k >= g.S) { k -= g.S; ++j; }
+        const int L = lc & kMjMask;
+        excl = lob_inside_rc(i, j, k, L, atoms, h);
+        up = (l.ip.v[e] & kMjMask) == L && !lob_inside_rc(i + 1, j, k, L, atoms, h);
+        um = (l.im.v[e] & kMjMask) == L && !lob_inside_rc(i - 1, j, k, L, atoms, h);
+        ujp = (l.jp.v[e] & kMjMask) == L && !lob_inside_rc(i, j + 1, k, L, atoms, h);
+        ujm = (l.jm.v[e] & kMjMask) == L && !lob_inside_rc(i, j - 1, k, L, atoms, h);
+        ukp = (l.kp.v[e] & kMjMask) == L && !lob_inside_rc(i, j, k + 1, L, atoms, h);
+        ukm = (l.km.v[e] & kMjMask) == L && !lob_inside_rc(i, j, k - 1, L, atoms, h);
+      } else {
+        excl = (lc & kMjExcl) != 0;
+        up = l.ip.v[e] == lc; um = l.im.v[e] == lc; ujp = l.jp.v[e] == lc; ujm = l.jm.v[e] == lc;
+        ukp = l.kp.v[e] == lc; ukm = l.km.v[e] == lc;
+      }
+      const float uc = u.c.v[e];
+      const float a = up ? u.ip.v[e] : uc, b = um ? u.im.v[e] : uc, c = ujp ? u.jp.v[e] : uc;
+      const float d = ujm ? u.jm.v[e] : uc, q = ukp ? u.kp.v[e] : uc, f = ukm ? u.km.v[e] : uc;
+      const float lap = F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(a, b), c), d), q), f), F_MUL(6.0f, uc));
+      const float out =
+          F_ADD(F_MUL(F_MUL(-0.5f, lap), inv_h2), F_MUL(F_ADD(-k4.v[e], F_MUL(2.0f, p4.v[e])), uc));
+      o.v[e] = excl ? 0.0f : out;
+    }
+    mj_store(HU, r, in, o);
   }
-  float out = 0.0f;
-  if (!excl) {
-    const float u_c = __ldg(U + id);
-    const float a = up ? __ldg(U + id + S2) : u_c;
-    const float b = um ? __ldg(U + id - S2) : u_c;
-    const float c = ujp ? __ldg(U + id + S) : u_c;
-    const float d = ujm ? __ldg(U + id - S) : u_c;
-    const float e = ukp ? __ldg(U + id + 1) : u_c;
-    const float f = ukm ? __ldg(U + id - 1) : u_c;
-    const float lap = F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(a, b), c), d), e), f), F_MUL(6.0f, u_c));
-    out = F_ADD(F_MUL(F_MUL(-0.5f, lap), inv_h2), F_MUL(F_ADD(-__ldg(K + id), F_MUL(2.0f, __ldg(Pother + id))), u_c));
-  }
-  HU[id] = out;
 }
 
-// lobpcgInner (molecule.js:1535-1610): interior cells numbered with k fastest; block w thread l
-// takes cells w*128+l, then every gridDim*128-th, summing a*b*h^3 for the 12 products over the
-// cells of domain m; the block's 128 sums fold pairwise (l += l+s, s = 64 .. 1).
-__global__ void __launch_bounds__(kLobWG) k_lob_inner(const float* __restrict__ X, const float* __restrict__ HX,
-                                                      const float* __restrict__ W, const float* __restrict__ HW,
-                                                      const float* __restrict__ Pv, const float* __restrict__ HP,
-                                                      const int* __restrict__ label, int m, Geo g, float h3,
-                                                      float* __restrict__ partials) {
-  __shared__ float sn[kLobWG][kLobNR + 1];
+// The pairwise fold of 128 threads' sums (l += l+s, s = 64 .. 1): the last five levels by shuffles.
+// Afterwards thread 0 holds the totals in acc.
+template <int NS>
+__device__ __forceinline__ void lob_fold(float (&acc)[NS], float (&sn)[64][NS + 1]) {
   const int l = threadIdx.x;
-  float acc[kLobNR];
-#pragma unroll
-  for (int q = 0; q < kLobNR; ++q) acc[q] = 0.0f;
-  const unsigned NM = (unsigned)(g.NN - 1), tot = NM * NM * NM, stride = gridDim.x * kLobWG;
-  for (unsigned cell = blockIdx.x * kLobWG + l; cell < tot; cell += stride) {
-    const unsigned k = cell % NM + 1, j = (cell / NM) % NM + 1, i = cell / (NM * NM) + 1;
-    const long long id = (long long)i * g.S2 + (long long)j * g.S + k;
-    if ((__ldg(label + id) & kMjMask) != m) continue;
-    const float x = __ldg(X + id), hx = __ldg(HX + id), w = __ldg(W + id), hw = __ldg(HW + id), pv = __ldg(Pv + id),
-                hp = __ldg(HP + id);
-    acc[0] = F_ADD(acc[0], F_MUL(F_MUL(x, x), h3));
-    acc[1] = F_ADD(acc[1], F_MUL(F_MUL(x, hx), h3));
-    acc[2] = F_ADD(acc[2], F_MUL(F_MUL(w, w), h3));
-    acc[3] = F_ADD(acc[3], F_MUL(F_MUL(w, hw), h3));
-    acc[4] = F_ADD(acc[4], F_MUL(F_MUL(x, w), h3));
-    acc[5] = F_ADD(acc[5], F_MUL(F_MUL(x, hw), h3));
-    acc[6] = F_ADD(acc[6], F_MUL(F_MUL(pv, pv), h3));
-    acc[7] = F_ADD(acc[7], F_MUL(F_MUL(pv, hp), h3));
-    acc[8] = F_ADD(acc[8], F_MUL(F_MUL(x, pv), h3));
-    acc[9] = F_ADD(acc[9], F_MUL(F_MUL(x, hp), h3));
-    acc[10] = F_ADD(acc[10], F_MUL(F_MUL(w, pv), h3));
-    acc[11] = F_ADD(acc[11], F_MUL(F_MUL(w, hp), h3));
-  }
-#pragma unroll
-  for (int q = 0; q < kLobNR; ++q) sn[l][q] = acc[q];
   __syncthreads();
-  for (int s = kLobWG / 2; s > 0; s >>= 1) {
-    if (l < s)
+  if (l >= 64)
 #pragma unroll
-      for (int q = 0; q < kLobNR; ++q) sn[l][q] = F_ADD(sn[l][q], sn[l + s][q]);
-    __syncthreads();
+    for (int q = 0; q < NS; ++q) sn[l - 64][q] = acc[q];
+  __syncthreads();
+  if (l < 64)
+#pragma unroll
+    for (int q = 0; q < NS; ++q) acc[q] = F_ADD(acc[q], sn[l][q]);
+  __syncthreads();
+  if (l >= 32 && l < 64)
+#pragma unroll
+    for (int q = 0; q < NS; ++q) sn[l][q] = acc[q];
+  __syncthreads();
+  if (l < 32) {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) acc[q] = F_ADD(acc[q], sn[l + 32][q]);
+    for (int s = 16; s > 0; s >>= 1)
+#pragma unroll
+      for (int q = 0; q < NS; ++q) acc[q] = F_ADD(acc[q], __shfl_down_sync(0xffffffffu, acc[q], s));
   }
-  if (l == 0)
-#pragma unroll
-    for (int q = 0; q < kLobNR; ++q) partials[blockIdx.x * kLobNR + q] = sn[0][q];
 }
 
 // JavaScript Math.min / Math.max: NaN if either argument is NaN, -0 below +0.
@@ -1076,11 +1106,14 @@ __device__ void lob_ritz3(const double* ip, double* out) {
       A[i][j] = s;
     }
   double V[3][3] = {{1.0, 0.0, 0.0}, {0.0, 1.0, 0.0}, {0.0, 0.0, 1.0}};
-  for (int sweep = 0; sweep < 20; ++sweep)
+  bool turned = true;  // a sweep without a rotation leaves nothing to the later ones
+  for (int sweep = 0; sweep < 20 && turned; ++sweep) {
+    turned = false;
     for (int e = 0; e < 3; ++e) {
       const int p = e == 2 ? 1 : 0, q = e == 0 ? 1 : 2;  // (0,1), (0,2), (1,2)
       const double apq = A[p][q];
       if (fabs(apq) < 1e-15) continue;
+      turned = true;
       const double tau = D_DIV(D_SUB(A[q][q], A[p][p]), D_MUL(2.0, apq));
       const double t = D_DIV(tau >= 0 ? 1.0 : -1.0, D_ADD(fabs(tau), D_SQRT(D_ADD(1.0, D_MUL(tau, tau)))));
       const double c = D_DIV(1.0, D_SQRT(D_ADD(1.0, D_MUL(t, t))));
@@ -1104,6 +1137,7 @@ __device__ void lob_ritz3(const double* ip, double* out) {
         V[r][q] = D_ADD(D_MUL(s, vrp), D_MUL(c, vrq));
       }
     }
+  }
   int mi = 0;
   if (A[1][1] < A[mi][mi]) mi = 1;
   if (A[2][2] < A[mi][mi]) mi = 2;
@@ -1114,85 +1148,167 @@ __device__ void lob_ritz3(const double* ip, double* out) {
   out[3] = D_MUL(Li[2][2], y2);
 }
 
-// lobpcgFinalize (molecule.js:1612-1648) -- thread l adds block results l, l+128, .. in order, the
-// same pairwise fold -- and then, in thread 0, the page's host step on the 12 sums:
-//   FIRST pass: lambda = <X|HX> / <X|X> in double, stored as f32 (0 when <X|X> <= 0, :3486);
-//   second pass: the Ritz problem (3x3 when hasP and <P|P> > 1e-20, else 2x2, :3570-3576), its
+// lobpcgInner (molecule.js:1535-1610), lobpcgFinalize (:1612-1648) and the page's host step, per domain m =
+// blockIdx.x.  Interior cells are numbered with k fastest; block w (of gridDim.y) thread l takes cells w*128+l,
+// then every gridDim.y*128-th, summing a*b*h^3 over the cells of the domain in that order; the block's
+// 128 sums fold pairwise.  The domain's last block to finish adds the block results (thread l: l, l+128,
+// .. in order, the same fold) and its thread 0 does the host's arithmetic:
+//   FIRST pass, 2 sums: lambda = <X|HX> / <X|X> in double, stored as f32 (0 when <X|X> <= 0, :3486);
+//   second pass, 12 sums: the Ritz problem (3x3 when hasP and <P|P> > 1e-20, else 2x2, :3570-3576), its
 //   coefficients stored as f32 (:3581).
-// scal: [0] lambda, [1..3] coefficients, [4..15] second-pass sums, [16..27] first-pass sums,
-// [28] the Ritz value (f32).
+// scal, kLobScal floats per domain: [0] lambda, [1..3] coefficients.  The cells per thread are few (8 at 64^3) and
+// each is a chain label -> fields -> sums, so four cells' labels, then their fields, are loaded together.
 template <bool FIRST>
-__global__ void __launch_bounds__(kLobWG) k_lob_finalize(const float* __restrict__ partials, int nwg, int hasP,
-                                                         float* __restrict__ scal) {
-  __shared__ float wg[kLobWG][kLobNR + 1];
-  const int l = threadIdx.x;
-  float acc[kLobNR];
+__global__ void __launch_bounds__(kLobWG) k_lob_inner(const float* __restrict__ X, const float* __restrict__ HX,
+                                                      const float* __restrict__ W, const float* __restrict__ HW,
+                                                      const float* __restrict__ Pv, const float* __restrict__ HP,
+                                                      const int* __restrict__ label, const MjAtom* __restrict__ atoms,
+                                                      Geo g, float h3, int hasP, float* __restrict__ partials,
+                                                      unsigned* __restrict__ done, float* __restrict__ scal) {
+  constexpr int NS = FIRST ? 2 : kLobNR, B = 4;
+  __shared__ float sn[64][NS + 1];
+  __shared__ bool last;
+  const int l = threadIdx.x, m = blockIdx.x, nwg = gridDim.y;
+  if (atoms[m].Z == 0.0f) return;
+  float acc[NS];
 #pragma unroll
-  for (int q = 0; q < kLobNR; ++q) acc[q] = 0.0f;
+  for (int q = 0; q < NS; ++q) acc[q] = 0.0f;
+  const unsigned NM = (unsigned)(g.NN - 1), tot = NM * NM * NM, stride = (unsigned)nwg * kLobWG;
+  for (unsigned c0 = blockIdx.y * kLobWG + l; c0 < tot; c0 += B * stride) {
+    long long id[B];
+    bool on[B];
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      const unsigned cell = c0 + b * stride, y = cell / NM, k = cell - y * NM + 1, i = y / NM, j = y - i * NM + 1;
+      id[b] = (long long)(i + 1) * g.S2 + (long long)j * g.S + k;
+      on[b] = cell < tot && (__ldg(label + id[b]) & kMjMask) == m;
+    }
+    float x[B], hx[B], w[B], hw[B], pv[B], hp[B];
+#pragma unroll
+    for (int b = 0; b < B; ++b)
+      if (on[b]) {
+        x[b] = __ldg(X + id[b]);
+        hx[b] = __ldg(HX + id[b]);
+        if (!FIRST) {
+          w[b] = __ldg(W + id[b]);
+          hw[b] = __ldg(HW + id[b]);
+          pv[b] = __ldg(Pv + id[b]);
+          hp[b] = __ldg(HP + id[b]);
+        }
+      }
+#pragma unroll
+    for (int b = 0; b < B; ++b)
+      if (on[b]) {
+        acc[0] = F_ADD(acc[0], F_MUL(F_MUL(x[b], x[b]), h3));
+        acc[1] = F_ADD(acc[1], F_MUL(F_MUL(x[b], hx[b]), h3));
+        if constexpr (!FIRST) {
+          acc[2] = F_ADD(acc[2], F_MUL(F_MUL(w[b], w[b]), h3));
+          acc[3] = F_ADD(acc[3], F_MUL(F_MUL(w[b], hw[b]), h3));
+          acc[4] = F_ADD(acc[4], F_MUL(F_MUL(x[b], w[b]), h3));
+          acc[5] = F_ADD(acc[5], F_MUL(F_MUL(x[b], hw[b]), h3));
+          acc[6] = F_ADD(acc[6], F_MUL(F_MUL(pv[b], pv[b]), h3));
+          acc[7] = F_ADD(acc[7], F_MUL(F_MUL(pv[b], hp[b]), h3));
+          acc[8] = F_ADD(acc[8], F_MUL(F_MUL(x[b], pv[b]), h3));
+          acc[9] = F_ADD(acc[9], F_MUL(F_MUL(x[b], hp[b]), h3));
+          acc[10] = F_ADD(acc[10], F_MUL(F_MUL(w[b], pv[b]), h3));
+          acc[11] = F_ADD(acc[11], F_MUL(F_MUL(w[b], hp[b]), h3));
+        }
+      }
+  }
+  lob_fold<NS>(acc, sn);
+  float* part = partials + (size_t)m * kLobMaxWG * kLobNR;
+  if (l == 0) {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) __stcg(part + blockIdx.y * kLobNR + q, acc[q]);
+    __threadfence();
+    last = atomicAdd(done + m, 1u) == (unsigned)nwg - 1u;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+#pragma unroll
+  for (int q = 0; q < NS; ++q) acc[q] = 0.0f;
   for (int w = l; w < nwg; w += kLobWG)
 #pragma unroll
-    for (int q = 0; q < kLobNR; ++q) acc[q] = F_ADD(acc[q], partials[w * kLobNR + q]);
-#pragma unroll
-  for (int q = 0; q < kLobNR; ++q) wg[l][q] = acc[q];
-  __syncthreads();
-  for (int s = kLobWG / 2; s > 0; s >>= 1) {
-    if (l < s)
-#pragma unroll
-      for (int q = 0; q < kLobNR; ++q) wg[l][q] = F_ADD(wg[l][q], wg[l + s][q]);
-    __syncthreads();
-  }
+    for (int q = 0; q < NS; ++q) acc[q] = F_ADD(acc[q], __ldcg(part + w * kLobNR + q));
+  lob_fold<NS>(acc, sn);
   if (l != 0) return;
-  double ip[kLobNR];
-  for (int q = 0; q < kLobNR; ++q) {
-    ip[q] = (double)wg[0][q];
-    scal[(FIRST ? 16 : 4) + q] = wg[0][q];
-  }
-  if (FIRST) {
-    scal[0] = ip[0] > 0.0 ? __double2float_rn(D_DIV(ip[1], ip[0])) : 0.0f;
+  done[m] = 0u;
+  float* out = scal + (size_t)m * kLobScal;
+  double ip[NS];
+#pragma unroll
+  for (int q = 0; q < NS; ++q) ip[q] = (double)acc[q];
+  if constexpr (FIRST) {
+    out[0] = ip[0] > 0.0 ? __double2float_rn(D_DIV(ip[1], ip[0])) : 0.0f;
   } else {
     double r[4];
     if (hasP && ip[6] > 1e-20)
       lob_ritz3(ip, r);
     else
       lob_ritz2(ip, r);
-    scal[1] = __double2float_rn(r[1]);
-    scal[2] = __double2float_rn(r[2]);
-    scal[3] = __double2float_rn(r[3]);
-    scal[28] = __double2float_rn(r[0]);
+    out[1] = __double2float_rn(r[1]);
+    out[2] = __double2float_rn(r[2]);
+    out[3] = __double2float_rn(r[3]);
   }
 }
 
-// lobpcgResidual (molecule.js:1652-1689): on domain m W = (HX - lambda*X) / (3/h^2 + |-K + 2*Pother|
-// + 0.1), 0 on every other interior cell; lambda read from the device.
+// lobpcgResidual (molecule.js:1652-1689): W = (HX - lambda*X) / (3/h^2 + |-K + 2*Pother| + 0.1) with the domain's
+// lambda, 0 on the cells of domains without electrons.
 __global__ void __launch_bounds__(256) k_lob_residual(const float* __restrict__ X, const float* __restrict__ HX,
                                                       float* __restrict__ W, const int* __restrict__ label,
                                                       const float* __restrict__ K, const float* __restrict__ Pot,
-                                                      const float* __restrict__ lam, int m, Geo g, float inv_h2) {
-  const int k = 1 + blockIdx.x * 32 + threadIdx.x, j = 1 + blockIdx.y * 8 + threadIdx.y, i = 1 + blockIdx.z;
-  if (k >= g.NN || j >= g.NN) return;
-  const long long id = (long long)i * g.S2 + (long long)j * g.S + k;
-  if ((__ldg(label + id) & kMjMask) != m) {
-    W[id] = 0.0f;
-    return;
+                                                      const float* __restrict__ scal, const MjAtom* __restrict__ atoms,
+                                                      Geo g, int planes, float inv_h2) {
+  const int i0 = 1 + blockIdx.y * planes, iend = min(i0 + planes, g.NN);
+  for (int i = i0; i < iend; ++i) {
+    const VGroup r = vgroup<float>(g, i, blockIdx.x);
+    const Quad<int> l = ldq(label + r.a);
+    const Quad<float> hx = ldq(HX + r.a), x = ldq(X + r.a), k4 = ldq(K + r.a), p4 = ldq(Pot + r.a);
+    const unsigned in = mj_inside(g, r, i);
+    Quad<float> o;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      o.v[e] = 0.0f;
+      if (!(in >> e & 1u)) continue;
+      const int L = l.v[e] & kMjMask;
+      if (atoms[L].Z == 0.0f) continue;
+      const float res = F_SUB(hx.v[e], F_MUL(__ldg(scal + (size_t)L * kLobScal), x.v[e]));
+      const float vEff = fabsf(F_ADD(-k4.v[e], F_MUL(2.0f, p4.v[e])));
+      const float diagH = F_ADD(F_ADD(F_MUL(3.0f, inv_h2), vEff), 0.1f);
+      o.v[e] = F_DIV(res, diagH);
+    }
+    mj_store(W, r, in, o);
   }
-  const float r = F_SUB(__ldg(HX + id), F_MUL(*lam, __ldg(X + id)));
-  const float vEff = fabsf(F_ADD(-__ldg(K + id), F_MUL(2.0f, __ldg(Pot + id))));
-  const float diagH = F_ADD(F_ADD(F_MUL(3.0f, inv_h2), vEff), 0.1f);
-  W[id] = F_DIV(r, diagH);
 }
 
-// lobpcgUpdate (molecule.js:1693-1724): on domain m X = c0*X + c1*W + c2*P, P = c1*W + c2*P.
+// lobpcgUpdate (molecule.js:1693-1724): X = c0*X + c1*W + c2*P, P = c1*W + c2*P with the domain's coefficients.
 __global__ void __launch_bounds__(256) k_lob_update(float* __restrict__ X, const float* __restrict__ W,
                                                     float* __restrict__ Pv, const int* __restrict__ label,
-                                                    const float* __restrict__ coef, int m, Geo g) {
-  const int k = 1 + blockIdx.x * 32 + threadIdx.x, j = 1 + blockIdx.y * 8 + threadIdx.y, i = 1 + blockIdx.z;
-  if (k >= g.NN || j >= g.NN) return;
-  const long long id = (long long)i * g.S2 + (long long)j * g.S + k;
-  if ((__ldg(label + id) & kMjMask) != m) return;
-  const float c0 = coef[0], c1 = coef[1], c2 = coef[2];
-  const float x = X[id], w = __ldg(W + id), pv = Pv[id];
-  X[id] = F_ADD(F_ADD(F_MUL(c0, x), F_MUL(c1, w)), F_MUL(c2, pv));
-  Pv[id] = F_ADD(F_MUL(c1, w), F_MUL(c2, pv));
+                                                    const float* __restrict__ scal, const MjAtom* __restrict__ atoms,
+                                                    Geo g, int planes) {
+  const int i0 = 1 + blockIdx.y * planes, iend = min(i0 + planes, g.NN);
+  for (int i = i0; i < iend; ++i) {
+    const VGroup r = vgroup<float>(g, i, blockIdx.x);
+    const Quad<int> l = ldq(label + r.a);
+    const Quad<float> w = ldq(W + r.a);
+    Quad<float> x = *reinterpret_cast<const Quad<float>*>(X + r.a), p = *reinterpret_cast<const Quad<float>*>(Pv + r.a);
+    unsigned in = mj_inside(g, r, i);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (!(in >> e & 1u)) continue;
+      const int L = l.v[e] & kMjMask;
+      if (atoms[L].Z == 0.0f) {
+        in &= ~(1u << e);
+        continue;
+      }
+      const float4 c = __ldg(reinterpret_cast<const float4*>(scal + (size_t)L * kLobScal));
+      const float c0 = c.y, c1 = c.z, c2 = c.w, pv = p.v[e];
+      x.v[e] = F_ADD(F_ADD(F_MUL(c0, x.v[e]), F_MUL(c1, w.v[e])), F_MUL(c2, pv));
+      p.v[e] = F_ADD(F_MUL(c1, w.v[e]), F_MUL(c2, pv));
+    }
+    mj_store(X, r, in, x);
+    mj_store(Pv, r, in, p);
+  }
 }
 
 // accumNorms (molecule.js:911-930) as its own pass: norm[label] += u32(u*u*h3*2^24) over the
@@ -1253,39 +1369,43 @@ int lob_workgroups(const Geo& g) {
   return (int)std::min<long long>(kLobMaxWG, (tot + kLobWG - 1) / kLobWG);
 }
 
-cudaError_t launch_lob_apply_h(const float* U, float* HU, const float* K, const int* label, const float* Pother,
-                               const MjAtom* atoms, const Geo& g, float h, float inv_h2, bool bare, cudaStream_t st) {
+cudaError_t launch_lob_apply_h(const float* U0, float* H0, const float* U1, float* H1, const float* K, const int* label,
+                               const float* Pother, const MjAtom* atoms, const Geo& g, float h, float inv_h2, bool bare,
+                               cudaStream_t st) {
+  const int planes = vplanes<float>(g, false);
+  dim3 grid = vgrid<float>(g, planes);
+  grid.z = U1 ? 2 : 1;
   if (bare)
-    k_lob_apply_h<true><<<lob_cells_grid(g), dim3(32, 8), 0, st>>>(U, HU, K, label, Pother, atoms, g, h, inv_h2);
+    k_lob_apply_h<true><<<grid, 256, 0, st>>>(U0, H0, U1, H1, K, label, Pother, atoms, g, planes, h, inv_h2);
   else
-    k_lob_apply_h<false><<<lob_cells_grid(g), dim3(32, 8), 0, st>>>(U, HU, K, label, Pother, atoms, g, h, inv_h2);
+    k_lob_apply_h<false><<<grid, 256, 0, st>>>(U0, H0, U1, H1, K, label, Pother, atoms, g, planes, h, inv_h2);
   return cudaGetLastError();
 }
 
 cudaError_t launch_lob_inner(const float* X, const float* HX, const float* W, const float* HW, const float* Pv,
-                             const float* HP, const int* label, int m, const Geo& g, float h3, float* partials,
-                             cudaStream_t st) {
-  k_lob_inner<<<lob_workgroups(g), kLobWG, 0, st>>>(X, HX, W, HW, Pv, HP, label, m, g, h3, partials);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_lob_finalize(const float* partials, int nwg, bool first, bool hasP, float* scal, cudaStream_t st) {
+                             const float* HP, const int* label, const MjAtom* atoms, int nAt, const Geo& g, float h3,
+                             bool first, bool hasP, float* partials, unsigned* done, float* scal, cudaStream_t st) {
+  const dim3 grid((unsigned)nAt, (unsigned)lob_workgroups(g));
   if (first)
-    k_lob_finalize<true><<<1, kLobWG, 0, st>>>(partials, nwg, hasP ? 1 : 0, scal);
+    k_lob_inner<true><<<grid, kLobWG, 0, st>>>(X, HX, W, HW, Pv, HP, label, atoms, g, h3, 0, partials, done, scal);
   else
-    k_lob_finalize<false><<<1, kLobWG, 0, st>>>(partials, nwg, hasP ? 1 : 0, scal);
+    k_lob_inner<false><<<grid, kLobWG, 0, st>>>(X, HX, W, HW, Pv, HP, label, atoms, g, h3, hasP ? 1 : 0, partials, done,
+                                                scal);
   return cudaGetLastError();
 }
 
 cudaError_t launch_lob_residual(const float* X, const float* HX, float* W, const int* label, const float* K,
-                                const float* Pot, const float* lam, int m, const Geo& g, float inv_h2, cudaStream_t st) {
-  k_lob_residual<<<lob_cells_grid(g), dim3(32, 8), 0, st>>>(X, HX, W, label, K, Pot, lam, m, g, inv_h2);
+                                const float* Pot, const float* scal, const MjAtom* atoms, const Geo& g, float inv_h2,
+                                cudaStream_t st) {
+  const int planes = vplanes<float>(g, false);
+  k_lob_residual<<<vgrid<float>(g, planes), 256, 0, st>>>(X, HX, W, label, K, Pot, scal, atoms, g, planes, inv_h2);
   return cudaGetLastError();
 }
 
-cudaError_t launch_lob_update(float* X, const float* W, float* Pv, const int* label, const float* coef, int m,
-                              const Geo& g, cudaStream_t st) {
-  k_lob_update<<<lob_cells_grid(g), dim3(32, 8), 0, st>>>(X, W, Pv, label, coef, m, g);
+cudaError_t launch_lob_update(float* X, const float* W, float* Pv, const int* label, const float* scal,
+                              const MjAtom* atoms, const Geo& g, cudaStream_t st) {
+  const int planes = vplanes<float>(g, false);
+  k_lob_update<<<vgrid<float>(g, planes), 256, 0, st>>>(X, W, Pv, label, scal, atoms, g, planes);
   return cudaGetLastError();
 }
 

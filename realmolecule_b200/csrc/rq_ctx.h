@@ -99,9 +99,11 @@ struct rq_ctx {
   float* atoms5 = nullptr;    // [i,j,k,Z,rc] f32 (cloud/solver.py:378-382)
   float* scratch_atoms5 = nullptr;  // per-call atom table for force variants
   float *sic = nullptr, *sic2 = nullptr;  // molecule.js flavour with SIC: self-potential ping-pong
-  float* pdirect = nullptr;   // molecule.js direct path: persistent P_m of every domain (n_atoms x S^3)
-  // molecule.js LOBPCG frames: HX, W, HW, P, HP (5 x S^3), the inner-product partial sums of
-  // each workgroup (256 x 12) and the scalars (lambda, Ritz coefficients, the 12 sums of each pass)
+  // molecule.js direct path: the persistent P_m of every domain, then as many fields for the sweeps to alternate with
+  // (2 n_atoms x slot())
+  float* pdirect = nullptr;
+  // molecule.js LOBPCG frames: HX, W, HW, P, HP (5 x slot()) and, per domain, the inner-product partial
+  // sums of each workgroup (256 x 12), the count of finished workgroups and the scalars (lambda, Ritz coefficients)
   float* lob = nullptr;
   // molecule.js locked groups: per label the bit set of its groups (n_atoms, zero = none)
   unsigned long long* lock = nullptr;
@@ -114,6 +116,9 @@ struct rq_ctx {
   MjSplit* splits = nullptr;
   float* lob_part = nullptr;
   float* lob_scal = nullptr;
+  unsigned* lob_done = nullptr;
+  // elements between the fields of one allocation: S^3 rounded up to 16-byte vectors
+  size_t slot() const { return ((size_t)g.S3 + 3) & ~(size_t)3; }
   // solver.py flavour: atom bins of the label step's argmax (rebuilt whenever atoms change)
   int bins_nb = 0, bins_bin = 0;
   int *bin_start = nullptr, *bin_idx = nullptr, *bin_far = nullptr;

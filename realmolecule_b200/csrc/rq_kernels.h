@@ -64,24 +64,24 @@ cudaError_t launch_mj_recompute_k(float* K, const MjAtom* atoms, int nAt, const 
 cudaError_t launch_mj_flags(int* label, const MjAtom* atoms, int nAt, const Geo& g, float h, bool hasBare,
                             cudaStream_t st);
 cudaError_t launch_mj_update(const float* U, float* Uo, const float* K, const int* label, const float* Pother,
-                             const Geo& g, float half_d, float dt, float h3, int nDom, unsigned* unorm, cudaStream_t st);
-cudaError_t launch_mj_norm_scale(const unsigned* unorm, const MjAtom* atoms, int nDom, float* scale, cudaStream_t st);
+                             const Geo& g, float half_d, float dt, float h3, unsigned* unorm, cudaStream_t st);
 cudaError_t launch_mj_update_cheb(const float* U, float* Uo, const float* K, const int* label, const float* Pother,
-                                  const Geo& g, float half_d, float dt, float h3, int nDom, unsigned* unorm,
-                                  float omega, cudaStream_t st);
+                                  const Geo& g, float half_d, float dt, float h3, unsigned* unorm, float omega,
+                                  cudaStream_t st);
 cudaError_t launch_mj_extract(const float* U, const int* label, const float* K, const MjAtom* atoms, int nAt,
                               const Geo& g, int sk, float* out, cudaStream_t st);
-cudaError_t launch_mj_apply_scale(float* U, const int* label, const float* scale, const Geo& g, cudaStream_t st);
+cudaError_t launch_mj_apply_scale(float* U, const int* label, const unsigned* unorm, const MjAtom* atoms, const Geo& g,
+                                  cudaStream_t st);
 cudaError_t launch_mj_jacobi(const float* Pin, float* Pout, const float* U, const Geo& g, float h2, float two_pi,
                              cudaStream_t st);
 cudaError_t launch_mj_vcycle(float* P, const float* U, float* rho, float* resid, float* Ec0, float* Ec1, float* fc,
                              const Geo& g, const Geo& gc, float h2, float inv_h2, float two_pi, cudaStream_t st);
-// the direct per-electron Poisson of small systems (molecule.js:2833-2858, :614-671): P_m init and
-// one step's solve for domain m (Pm persistent; rho, scratch are scratch)
+// the direct per-electron Poisson of small systems (molecule.js:2833-2858, :614-671): P_m init and one step's
+// solve for the n domains m (slot m of P persistent, of P2 scratch)
 cudaError_t launch_mj_direct_init(const MjAtom* atoms, int nAt, int m, float* Pm, float* Pother, const Geo& g, float h,
                                   float h2, cudaStream_t st);
-cudaError_t launch_mj_direct_domain(const float* U, const int* label, float* Pother, int m, float* Pm, float* scratch,
-                                    float* rho, const Geo& g, float h2, float two_pi, cudaStream_t st);
+cudaError_t launch_mj_direct(const float* U, const int* label, float* Pother, const int* m, int n, float* P, float* P2,
+                             long long slot, const Geo& g, float h2, float two_pi, cudaStream_t st);
 // the self-interaction correction of one domain m (molecule.js:3018-3075); rho, sic, sic2, resid,
 // Ec0, Ec1 and fc are scratch
 cudaError_t launch_mj_sic_domain(const float* U, const int* label, float* Pother, int m, float frac, float* rho,
@@ -99,20 +99,22 @@ cudaError_t launch_mj_gradp(const float* P, const MjAtom* atoms, int nAt, const 
 cudaError_t launch_fill(float* f, float v, long long n, cudaStream_t st);
 // the six faces of label buffer src copied into dst
 cudaError_t launch_copy_faces(const int* src, int* dst, const Geo& g, cudaStream_t st);
-// LOBPCG frames (molecule.js:1455-1724): inner products in workgroups of kLobWG threads, at most
-// kLobMaxWG of them (molecule.js:1533-1534); kLobScal floats of per-iteration scalars
-constexpr int kLobNR = 12, kLobWG = 128, kLobMaxWG = 256, kLobScal = 32;
+// LOBPCG frames (molecule.js:1455-1724), every domain with electrons in each launch: inner products in workgroups
+// of kLobWG threads, at most kLobMaxWG of them per domain (molecule.js:1533-1534); kLobScal floats per
+// domain, lambda and the three Ritz coefficients
+constexpr int kLobNR = 12, kLobWG = 128, kLobMaxWG = 256, kLobScal = 4;
 int lob_workgroups(const Geo& g);
-cudaError_t launch_lob_apply_h(const float* U, float* HU, const float* K, const int* label, const float* Pother,
-                               const MjAtom* atoms, const Geo& g, float h, float inv_h2, bool bare, cudaStream_t st);
+cudaError_t launch_lob_apply_h(const float* U0, float* H0, const float* U1, float* H1, const float* K, const int* label,
+                               const float* Pother, const MjAtom* atoms, const Geo& g, float h, float inv_h2, bool bare,
+                               cudaStream_t st);  // U1 null: one field
 cudaError_t launch_lob_inner(const float* X, const float* HX, const float* W, const float* HW, const float* Pv,
-                             const float* HP, const int* label, int m, const Geo& g, float h3, float* partials,
-                             cudaStream_t st);
-cudaError_t launch_lob_finalize(const float* partials, int nwg, bool first, bool hasP, float* scal, cudaStream_t st);
+                             const float* HP, const int* label, const MjAtom* atoms, int nAt, const Geo& g, float h3,
+                             bool first, bool hasP, float* partials, unsigned* done, float* scal, cudaStream_t st);
 cudaError_t launch_lob_residual(const float* X, const float* HX, float* W, const int* label, const float* K,
-                                const float* Pot, const float* lam, int m, const Geo& g, float inv_h2, cudaStream_t st);
-cudaError_t launch_lob_update(float* X, const float* W, float* Pv, const int* label, const float* coef, int m,
-                              const Geo& g, cudaStream_t st);
+                                const float* Pot, const float* scal, const MjAtom* atoms, const Geo& g, float inv_h2,
+                                cudaStream_t st);
+cudaError_t launch_lob_update(float* X, const float* W, float* Pv, const int* label, const float* scal,
+                              const MjAtom* atoms, const Geo& g, cudaStream_t st);
 cudaError_t launch_mj_accum_norms(const float* U, const int* label, const Geo& g, float h3, unsigned* unorm,
                                   cudaStream_t st);
 

@@ -441,3 +441,37 @@ def test_init_positions(kind):
     st = ctx.download(psi=True, label=True)
     assert np.array_equal(st["psi"].view(np.uint32), ref.U.view(np.uint32))
     assert np.array_equal(st["label"], ref.label.astype(np.int32))
+
+
+# Edges of the 16-byte vectors: both pitches modulo 4, grids of less than a warp's groups, several planes per
+# block (from 16 blocks per SM on) with a remainder; domains without electrons among the others.
+def edge_rows(NN):
+    c = NN // 2
+    return [{"i": c, "j": c, "k": c, "Z": 2, "Z_nuc": 2, "rc": 0.3},
+            {"i": c, "j": c - 1, "k": c, "Z": 0, "Z_nuc": 0, "rc": 0.0},
+            {"i": c + 1, "j": c + 1, "k": c, "Z": 1, "Z_nuc": 1, "rc": 0.0},
+            {"i": c - 1, "j": c, "k": c - 1, "Z": 1, "Z_nuc": 1, "rc": 0.0}]
+
+
+@pytest.mark.parametrize("NN,opts,steps", [
+    (4, dict(steps_per_frame=3, sic=True), 4), (6, dict(steps_per_frame=3, sic=True), 4),
+    (6, dict(steps_per_frame=3, chebyshev=True), 7), (34, dict(steps_per_frame=4, sic=True), 5),
+    (34, dict(steps_per_frame=2, sic=True, lobpcg=True), 3), (6, dict(steps_per_frame=2, lobpcg=True), 3),
+    (214, dict(steps_per_frame=2, sic=True), 2), (214, dict(steps_per_frame=2, lobpcg=True), 1)],
+    ids=lambda v: str(v) if isinstance(v, int) else "-".join(k for k in v if k != "steps_per_frame"))
+def test_vector_edges_bit_exact(NN, opts, steps):
+    from realmolecule_b200 import Context
+    rows = edge_rows(NN)
+    ref = orc.MoleculeJsDriver(NN, NN * 0.25, rows, **opts)
+    ref.initialize()
+    ctx = Context(NN, NN * 0.25, rows, flavor="molecule.js", **{k: int(v) for k, v in opts.items()})
+    ctx.initialize()
+    ctx.upload(psi=ref.U, label=ref.label.astype(np.int32))
+    for _ in range(steps):
+        ref.step()
+    ctx.step(steps)
+    st = ctx.download(psi=True, label=True, W=True, P=True)
+    assert np.array_equal(st["psi"].view(np.uint32), ref.U.view(np.uint32))
+    assert np.array_equal(st["label"] & 0x3FFFFFFF, ref.label.astype(np.int32))
+    assert np.array_equal(st["W"].view(np.uint32), ref.W.view(np.uint32))
+    assert np.array_equal(st["P"].view(np.uint32), ref.P.view(np.uint32))
