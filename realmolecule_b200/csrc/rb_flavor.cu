@@ -4,11 +4,12 @@
 //
 // The reference launches one pass per electron for every stage of a step (uNearest, red W+U,
 // red P, black W+U, black P).  The electrons of a colour touch disjoint data -- W+U of m writes
-// u_m, w_m; P of m reads u_m at the cell itself, the precomputed rho_total and P_m of the other
-// colour -- so one thread here owns a cell of the colour and runs W+U then P for every electron.
-// The per-step rho_total and competitor max come from one pass (the competitor of electron m is
-// the cell's largest u unless m holds it, then the second largest: exact selections, equal to the
-// reference's max chain).  A step is three launches; a frame is one CUDA graph.  The f32
+// u_m, w_m; P of m reads u_m at the cell itself, rho_total and P_m of the other colour -- so one
+// thread here owns an electron on a cell of the colour and runs W+U then P; the threads of a cell
+// exchange their u for rho_total and the competitor (of electron m the cell's largest u unless m
+// holds it, then the second largest: exact selections, equal to the reference's max chain).  Both
+// colours see the u of the step's start, since a pass changes only its own cells.  A step is two
+// launches; a frame is one CUDA graph.  The f32
 // arithmetic is the shaders' in their order (explicit round-to-nearest operations); the norm
 // reduction keeps the reference's grid-stride partial sums and workgroup trees, so the scales are
 // the reference's; the energies are the host formula in FP64.
@@ -25,7 +26,11 @@
 namespace rq {
 
 constexpr int kRbMax = 16;
-constexpr int kRbTK = 32, kRbTJ = 8;  // a block: 32 cells of one colour along k (64 k) x 8 j
+constexpr int kRbTK = 32;  // cells of one colour along k in a block: 64 k
+constexpr int kRbNormWG = 256;  // workgroups of the norm reduction at most
+
+// rows of a block of k_rb_color, which holds n electrons' threads of each of its cells
+__host__ __device__ inline int rb_rows(int n) { return n >= 8 ? 1 : 8 / n; }
 
 struct RbParams {
   int NN, S, N2, n;
@@ -34,106 +39,98 @@ struct RbParams {
   int masked[kRbMax];       // the electron's nucleus has an r_c exclusion mask
 };
 
-struct RbCell {
-  long long id;
-  int i, j, k;
-};
-
-// the thread's cell of colour `color` in plane blockIdx.z + 1; false when outside the interior
-__device__ __forceinline__ bool rb_cell(const RbParams& p, int color, RbCell& c) {
-  c.i = blockIdx.z + 1;
-  c.j = blockIdx.y * kRbTJ + threadIdx.y + 1;
-  const int k0 = 1 + ((c.i + c.j + 1 + color) & 1);  // (i + j + k0) % 2 == color
-  c.k = k0 + 2 * (blockIdx.x * kRbTK + threadIdx.x);
-  if (c.j >= p.NN || c.k >= p.NN) return false;
-  c.id = (long long)c.i * p.S * p.S + (long long)c.j * p.S + c.k;
-  return true;
-}
-
-// rhoTotal (realqm_rb.js:190-215) and the inputs of uNearest (:225-251): per interior cell
-// (rho_total, largest u, second largest u, index of the largest)
-__global__ void __launch_bounds__(256) k_rb_rho_top2(const RbParams p, const float* __restrict__ U,
-                                                     float4* __restrict__ top) {
-  const int k = blockIdx.x * 32 + threadIdx.x + 1, j = blockIdx.y * 8 + threadIdx.y + 1, i = blockIdx.z + 1;
-  if (k >= p.NN || j >= p.NN) return;
-  const long long S3 = (long long)p.S * p.S * p.S;
-  const long long id = (long long)i * p.S * p.S + (long long)j * p.S + k;
-  float rho = 0.0f, m1 = -INFINITY, m2 = -INFINITY;
-  int a1 = -1;
-  for (int q = 0; q < p.n; ++q) {
-    const float u = __ldg(U + q * S3 + id);
-    rho = q == 0 ? F_MUL(u, u) : F_ADD(rho, F_MUL(u, u));
-    if (u > m1) { m2 = m1; m1 = u; a1 = q; }
-    else if (u > m2) m2 = u;
-  }
-  top[id] = make_float4(rho, m1, m2, __int_as_float(a1));
-}
-
-// fusedWU_RB_WGSL (:256-311) then updateP_RB_WGSL (:318-353) of every electron on one cell of
-// the colour, in place
-__global__ void __launch_bounds__(256) k_rb_color(const RbParams p, int color, float* __restrict__ U,
+// One colour of a step: rhoTotal (:190-215), uNearest (:225-251), fusedWU_RB_WGSL (:256-311), then
+// updateP_RB_WGSL (:318-353), in place.  Block (32, rows, n): thread z is electron z of the cell.  All loads
+// are issued before the first store, and no thread waits for another electron's arithmetic; what bounds the pass
+// is load latency.  H2 at 100^3 per step: 81 us with a pass for rho_total and the competitor, a thread per cell
+// and a loop over electrons whose stores fenced the next one's loads; 35 us now.
+__global__ void __launch_bounds__(512) k_rb_color(const RbParams p, int color, float* __restrict__ U,
                                                   float* __restrict__ W, float* __restrict__ P,
-                                                  const float* __restrict__ K, const float4* __restrict__ top,
-                                                  const unsigned char* __restrict__ mask) {
-  RbCell c;
-  if (!rb_cell(p, color, c)) return;
-  const long long S = p.S, S2 = S * S, S3 = S2 * S;
-  const float4 t = top[c.id];
-  const int a1 = __float_as_int(t.w);
-  const float Kc = __ldg(K + c.id);
+                                                  const float* __restrict__ K, const unsigned char* __restrict__ mask) {
+  __shared__ float su[512];
+  const int m = threadIdx.z;
+  const int i = blockIdx.z + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  const int k0 = 1 + ((i + j + 1 + color) & 1);  // (i + j + k0) % 2 == color
+  const int k = k0 + 2 * (blockIdx.x * kRbTK + threadIdx.x);
+  const bool in = j < p.NN && k < p.NN;
+  const int S = p.S, S2 = S * S;
+  const int id = in ? i * S2 + j * S + k : S2 + S + 1;  // an interior cell whatever the thread
+  const long long S3 = (long long)S2 * S;
+  float* u = U + m * S3 + id;
+  float* w = W + m * S3 + id;
+  float* Pm = P + m * S3 + id;
+  const float uc = *u;
+  const int cell = threadIdx.y * kRbTK + threadIdx.x, cells = blockDim.y * kRbTK;
+  su[m * cells + cell] = uc;
+  const float wc = *w, wxp = w[S2], wxm = w[-S2], wyp = w[S], wym = w[-S], wzp = w[1], wzm = w[-1];
+  const float uxp = u[S2], uxm = u[-S2], uyp = u[S], uym = u[-S], uzp = u[1], uzm = u[-1];
+  const float Pc = *Pm, pxp = Pm[S2], pxm = Pm[-S2], pyp = Pm[S], pym = Pm[-S], pzp = Pm[1], pzm = Pm[-1];
+  const float Kc = __ldg(K + id);
+  const bool masked = p.masked[m];
+  const unsigned char mk8 = masked ? mask[m * S3 + id] : 1;
+  __syncthreads();
+  if (!in) return;
+  float rho = 0.0f, un = -INFINITY;
+  for (int q = 0; q < p.n; ++q) {
+    const float v = su[q * cells + cell];
+    rho = q == 0 ? F_MUL(v, v) : F_ADD(rho, F_MUL(v, v));
+    if (q != m && v > un) un = v;
+  }
   const float dt = p.dt, inv_h = p.inv_h, inv_h2 = p.inv_h2;
   const float dt05 = F_MUL(0.5f, dt), dt10 = F_MUL(10.0f, dt);
-  for (int m = 0; m < p.n; ++m) {
-    float* u = U + m * S3 + c.id;
-    float* w = W + m * S3 + c.id;
-    float* Pm = P + m * S3 + c.id;
-    const float un = m == a1 ? t.z : t.y;
-    const float uc = *u;
-    const float cc = F_MUL(0.1f, F_SUB(uc, un));
-    const float wc = *w;
-    const float wxp = w[S2], wxm = w[-S2], wyp = w[S], wym = w[-S], wzp = w[1], wzm = w[-1];
-    const float lap_w = F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(wxp, wxm), wyp), wym), wzp), wzm), F_MUL(6.0f, wc));
-    const float gwx = F_MUL(F_SUB(wxp, wxm), inv_h), gwy = F_MUL(F_SUB(wyp, wym), inv_h),
-                gwz = F_MUL(F_SUB(wzp, wzm), inv_h);
-    const float grad_w = F_SQRT(F_ADD(F_ADD(F_MUL(gwx, gwx), F_MUL(gwy, gwy)), F_MUL(gwz, gwz)));
-    const float wc2 = F_ADD(F_ADD(wc, F_MUL(F_MUL(F_MUL(dt05, fabsf(cc)), lap_w), inv_h2)), F_MUL(F_MUL(dt10, cc), grad_w));
-    const float fxp = F_MUL(F_MUL(F_SUB(u[S2], uc), F_ADD(wxp, wc2)), 0.5f);
-    const float fxm = F_MUL(F_MUL(F_SUB(uc, u[-S2]), F_ADD(wc2, wxm)), 0.5f);
-    const float fyp = F_MUL(F_MUL(F_SUB(u[S], uc), F_ADD(wyp, wc2)), 0.5f);
-    const float fym = F_MUL(F_MUL(F_SUB(uc, u[-S]), F_ADD(wc2, wym)), 0.5f);
-    const float fzp = F_MUL(F_MUL(F_SUB(u[1], uc), F_ADD(wzp, wc2)), 0.5f);
-    const float fzm = F_MUL(F_MUL(F_SUB(uc, u[-1]), F_ADD(wc2, wzm)), 0.5f);
-    const float wlap = F_ADD(F_ADD(F_SUB(fxp, fxm), F_SUB(fyp, fym)), F_SUB(fzp, fzm));
-    const float Pc = *Pm;
-    float un_new = F_ADD(F_ADD(uc, F_MUL(p.half_d, wlap)), F_MUL(F_MUL(F_MUL(dt, F_SUB(Kc, F_MUL(2.0f, Pc))), uc), wc2));
-    float wn_new = wc2;
-    if (p.masked[m]) {
-      const float mk = mask[m * S3 + c.id] ? 1.0f : 0.0f;
-      un_new = F_MUL(un_new, mk);
-      wn_new = F_MUL(wn_new, mk);
-    }
-    *u = un_new;
-    *w = wn_new;
-    const float lap = F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(Pm[S2], Pm[-S2]), Pm[S]), Pm[-S]), Pm[1]), Pm[-1]), F_MUL(6.0f, Pc));
-    const float ro = fmaxf(F_SUB(t.x, F_MUL(F_MUL(p.self_frac[m], un_new), un_new)), 0.0f);
-    *Pm = F_ADD(Pc, F_MUL(dt, F_ADD(F_MUL(lap, inv_h2), F_MUL(p.two_pi, ro))));
+  const float cc = F_MUL(0.1f, F_SUB(uc, un));
+  const float lap_w = F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(wxp, wxm), wyp), wym), wzp), wzm), F_MUL(6.0f, wc));
+  const float gwx = F_MUL(F_SUB(wxp, wxm), inv_h), gwy = F_MUL(F_SUB(wyp, wym), inv_h),
+              gwz = F_MUL(F_SUB(wzp, wzm), inv_h);
+  const float grad_w = F_SQRT(F_ADD(F_ADD(F_MUL(gwx, gwx), F_MUL(gwy, gwy)), F_MUL(gwz, gwz)));
+  const float wc2 =
+      F_ADD(F_ADD(wc, F_MUL(F_MUL(F_MUL(dt05, fabsf(cc)), lap_w), inv_h2)), F_MUL(F_MUL(dt10, cc), grad_w));
+  const float fxp = F_MUL(F_MUL(F_SUB(uxp, uc), F_ADD(wxp, wc2)), 0.5f);
+  const float fxm = F_MUL(F_MUL(F_SUB(uc, uxm), F_ADD(wc2, wxm)), 0.5f);
+  const float fyp = F_MUL(F_MUL(F_SUB(uyp, uc), F_ADD(wyp, wc2)), 0.5f);
+  const float fym = F_MUL(F_MUL(F_SUB(uc, uym), F_ADD(wc2, wym)), 0.5f);
+  const float fzp = F_MUL(F_MUL(F_SUB(uzp, uc), F_ADD(wzp, wc2)), 0.5f);
+  const float fzm = F_MUL(F_MUL(F_SUB(uc, uzm), F_ADD(wc2, wzm)), 0.5f);
+  const float wlap = F_ADD(F_ADD(F_SUB(fxp, fxm), F_SUB(fyp, fym)), F_SUB(fzp, fzm));
+  float un_new = F_ADD(F_ADD(uc, F_MUL(p.half_d, wlap)), F_MUL(F_MUL(F_MUL(dt, F_SUB(Kc, F_MUL(2.0f, Pc))), uc), wc2));
+  float wn_new = wc2;
+  if (masked) {
+    const float mk = mk8 ? 1.0f : 0.0f;
+    un_new = F_MUL(un_new, mk);
+    wn_new = F_MUL(wn_new, mk);
   }
+  *u = un_new;
+  *w = wn_new;
+  const float lap = F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(pxp, pxm), pyp), pym), pzp), pzm), F_MUL(6.0f, Pc));
+  const float ro = fmaxf(F_SUB(rho, F_MUL(F_MUL(p.self_frac[m], un_new), un_new)), 0.0f);
+  *Pm = F_ADD(Pc, F_MUL(dt, F_ADD(F_MUL(lap, inv_h2), F_MUL(p.two_pi, ro))));
 }
 
-// reduceNormWGSL (:356-394): blockIdx.y = electron; nwg blocks of 128 threads, each thread a
-// grid-stride f32 sum over the interior cells in linear order, then the workgroup tree
-__global__ void __launch_bounds__(128) k_rb_norm_partial(const RbParams p, const float* __restrict__ U,
-                                                         float* __restrict__ part) {
-  __shared__ float sd[128];
-  const int m = blockIdx.y, lid = threadIdx.x;
-  const long long NM = p.NN - 1, tot = NM * NM * NM, stride = (long long)gridDim.x * 128;
-  const long long S = p.S, S2 = S * S, S3 = S2 * S;
-  const float* u = U + m * S3;
+// reduceNormWGSL (:356-394): blockIdx.y = electron; gridDim.x workgroups of 128 threads, each thread a
+// grid-stride f32 sum over the interior cells in linear order, then the workgroup tree; and normalizeWGSL's sum of
+// the workgroups in order (:398-422) by the electron's last one: norm and scale.  Eight cells are loaded
+// ahead of the chain of additions.  H2 at 100^3: 35 us as two kernels, 13 us.
+__global__ void __launch_bounds__(128) k_rb_norm(const RbParams p, const float* __restrict__ U,
+                                                 float* __restrict__ part, const float* __restrict__ tgt,
+                                                 unsigned* __restrict__ done, float2* __restrict__ scale) {
+  __shared__ float sd[kRbNormWG];
+  __shared__ bool last;
+  constexpr int B = 8;
+  const int m = blockIdx.y, lid = threadIdx.x, nwg = gridDim.x;
+  const unsigned NM = (unsigned)(p.NN - 1), tot = NM * NM * NM, stride = (unsigned)nwg * 128u;
+  const int S = p.S, S2 = S * S;
+  const float* u = U + m * ((long long)S2 * S);
   float acc = 0.0f;
-  for (long long cell = (long long)blockIdx.x * 128 + lid; cell < tot; cell += stride) {
-    const int k = (int)(cell % NM) + 1, j = (int)((cell / NM) % NM) + 1, i = (int)(cell / (NM * NM)) + 1;
-    const float v = __ldg(u + (long long)i * S2 + (long long)j * S + k);
-    acc = F_ADD(acc, F_MUL(F_MUL(v, v), p.h3));
+  for (unsigned c0 = blockIdx.x * 128u + lid; c0 < tot; c0 += B * stride) {
+    float v[B];
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      const unsigned cell = c0 + b * stride, y = cell / NM, k = cell - y * NM + 1, i = y / NM, j = y - i * NM + 1;
+      if (cell < tot) v[b] = __ldg(u + (int)((i + 1) * (unsigned)S2 + j * (unsigned)S + k));
+    }
+#pragma unroll
+    for (int b = 0; b < B; ++b)
+      if (c0 + b * stride < tot) acc = F_ADD(acc, F_MUL(F_MUL(v[b], v[b]), p.h3));
   }
   sd[lid] = acc;
   __syncthreads();
@@ -141,16 +138,21 @@ __global__ void __launch_bounds__(128) k_rb_norm_partial(const RbParams p, const
     if (lid < s) sd[lid] = F_ADD(sd[lid], sd[lid + s]);
     __syncthreads();
   }
-  if (lid == 0) part[m * gridDim.x + blockIdx.x] = sd[0];
-}
-
-// normalizeWGSL's sum of the partials (:398-422), once per electron: norm and scale
-__global__ void k_rb_norm_scale(const RbParams p, const float* __restrict__ part, int nwg,
-                                const float* __restrict__ tgt, float2* __restrict__ scale) {
-  const int m = threadIdx.x;
-  if (m >= p.n) return;
+  if (lid == 0) {
+    __stcg(part + m * nwg + blockIdx.x, sd[0]);
+    __threadfence();
+    last = atomicAdd(done + m, 1u) == (unsigned)nwg - 1u;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int q = lid; q < nwg; q += 128) sd[q] = __ldcg(part + m * nwg + q);
+  __syncthreads();
+  if (lid != 0) return;
+  done[m] = 0u;
   float norm = 0.0f;
-  for (int q = 0; q < nwg; ++q) norm = F_ADD(norm, part[m * nwg + q]);
+#pragma unroll 16
+  for (int q = 0; q < nwg; ++q) norm = F_ADD(norm, sd[q]);
   scale[m] = make_float2(norm, norm > 0.0f ? F_SQRT(F_DIV(tgt[m], norm)) : 1.0f);
 }
 
@@ -325,8 +327,8 @@ struct rq_rb {
   double h = 0;
   RbParams p{};
   float *U = nullptr, *W = nullptr, *P = nullptr, *K = nullptr, *part = nullptr, *tgt_d = nullptr, *slice = nullptr;
-  float4* top = nullptr;
   float2* scale = nullptr;
+  unsigned* done = nullptr;
   unsigned char* mask = nullptr;
   double* acc = nullptr;
   long long t_step = 0, launches = 0;
@@ -352,26 +354,23 @@ dim3 rb_cells_grid(int NN, int planes) {
   return dim3((NM + 31) / 32, (NM + 7) / 8, planes);
 }
 
-dim3 rb_color_grid(int NN) {  // 32 threads cover 64 consecutive k
-  const int NM = NN - 1;
-  return dim3((NM + 2 * kRbTK - 1) / (2 * kRbTK), (NM + kRbTJ - 1) / kRbTJ, NM);
+dim3 rb_color_grid(int NN, int n) {  // 32 threads cover 64 consecutive k
+  const int NM = NN - 1, rows = rb_rows(n);
+  return dim3((NM + 2 * kRbTK - 1) / (2 * kRbTK), (NM + rows - 1) / rows, NM);
 }
 
-// doSteps(n) (realqm_rb.js:891-965): per step rho/competitor, the red pass, the black pass, and
-// the normalisation of every electron when the frame-local step index is a multiple of 5
+// doSteps(n) (realqm_rb.js:891-965): per step the red pass, the black pass, and the
+// normalisation of every electron when the frame-local step index is a multiple of 5
 int rb_frame(rq_rb* s, int n) {
   const int NN = s->cfg.NN;
   for (int q = 0; q < n; ++q) {
-    k_rb_rho_top2<<<rb_cells_grid(NN, NN - 1), dim3(32, 8), 0, s->st>>>(s->p, s->U, s->top);
-    BLAUNCH();
     for (int color = 0; color < 2; ++color) {
-      k_rb_color<<<rb_color_grid(NN), dim3(kRbTK, kRbTJ), 0, s->st>>>(s->p, color, s->U, s->W, s->P, s->K, s->top, s->mask);
+      k_rb_color<<<rb_color_grid(NN, s->n), dim3(kRbTK, rb_rows(s->n), s->n), 0, s->st>>>(s->p, color, s->U, s->W, s->P,
+                                                                                       s->K, s->mask);
       BLAUNCH();
     }
     if (q % 5 == 0) {
-      k_rb_norm_partial<<<dim3(s->nwg, s->n), 128, 0, s->st>>>(s->p, s->U, s->part);
-      BLAUNCH();
-      k_rb_norm_scale<<<1, 32, 0, s->st>>>(s->p, s->part, s->nwg, s->tgt_d, s->scale);
+      k_rb_norm<<<dim3(s->nwg, s->n), 128, 0, s->st>>>(s->p, s->U, s->part, s->tgt_d, s->done, s->scale);
       BLAUNCH();
       k_rb_normalize<<<rb_cells_grid(NN, NN - 1), dim3(32, 8), 0, s->st>>>(s->p, s->U, s->scale);
       BLAUNCH();
@@ -407,7 +406,7 @@ extern "C" int rq_rb_create(const rq_rb_config* cfg, const rq_rb_nucleus* nuclei
   s->S3 = (long long)S * S * S;
   s->h = cfg->screen / NN;
   const long long NM = NN - 1, tot = NM * NM * NM;
-  s->nwg = (int)std::min<long long>(256, (tot + 127) / 128);
+  s->nwg = (int)std::min<long long>(kRbNormWG, (tot + 127) / 128);
   RbParams& p = s->p;
   const double h = s->h, h2 = h * h, h3 = h * h * h, dv = 0.1;
   p.NN = NN; p.S = S; p.N2 = (int)std::floor(NN / 2.0); p.n = nel;
@@ -431,8 +430,8 @@ extern "C" int rq_rb_create(const rq_rb_config* cfg, const rq_rb_nucleus* nuclei
   const size_t fld = sizeof(float) * (size_t)s->S3 * nel;
   int rc;
   if ((rc = alloc((void**)&s->U, fld)) || (rc = alloc((void**)&s->W, fld)) || (rc = alloc((void**)&s->P, fld)) ||
-      (rc = alloc((void**)&s->K, sizeof(float) * s->S3)) || (rc = alloc((void**)&s->top, sizeof(float4) * s->S3)) ||
-      (rc = alloc((void**)&s->part, sizeof(float) * 256 * nel)) || (rc = alloc((void**)&s->tgt_d, sizeof(float) * nel)) ||
+      (rc = alloc((void**)&s->K, sizeof(float) * s->S3)) || (rc = alloc((void**)&s->done, sizeof(unsigned) * nel)) ||
+      (rc = alloc((void**)&s->part, sizeof(float) * kRbNormWG * nel)) || (rc = alloc((void**)&s->tgt_d, sizeof(float) * nel)) ||
       (rc = alloc((void**)&s->scale, sizeof(float2) * nel)) || (rc = alloc((void**)&s->acc, sizeof(double) * 3)) ||
       (rc = alloc((void**)&s->mask, (size_t)s->S3 * nel)) ||
       (rc = alloc((void**)&s->slice, sizeof(float) * (size_t)S * S * (3 * nel + 1))))
@@ -495,7 +494,7 @@ extern "C" void rq_rb_destroy(rq_rb* s) {
   if (!s) return;
   if (s->st) cudaStreamSynchronize(s->st);
   for (auto& kv : s->graphs) cudaGraphExecDestroy(kv.second.first);
-  for (void* q : {(void*)s->U, (void*)s->W, (void*)s->P, (void*)s->K, (void*)s->top, (void*)s->part, (void*)s->tgt_d,
+  for (void* q : {(void*)s->U, (void*)s->W, (void*)s->P, (void*)s->K, (void*)s->done, (void*)s->part, (void*)s->tgt_d,
                   (void*)s->scale, (void*)s->acc, (void*)s->mask, (void*)s->slice})
     if (q) cudaFree(q);
   if (s->st) cudaStreamDestroy(s->st);

@@ -88,3 +88,23 @@ def test_page_frames_and_errors():
     g.close()
     with pytest.raises(ValueError):
         RealqmRb(H2["nuclei"], NN=32, screen=8.0, nelec=3)
+
+
+# Edges of the blocks: a grid smaller than a block, one cell past 64 along k, and 5, 8, 9 and 16 electrons (the
+# electrons of a cell share a block, with fewer rows as they grow).
+@pytest.mark.parametrize("NN,ne", [(8, 2), (9, 16), (66, 2), (65, 5), (20, 8), (21, 9)])
+def test_color_block_edges(NN, ne):
+    c = NN // 2
+    nuc = [{"i": c + (q % 3) - 1, "j": c + (q // 3) % 3 - 1, "k": c + q // 9 - 1, "Z": 1 + q % 2, "rc": 0, "ne": 1,
+            "rc_excl": 0.4 if q % 4 == 3 else 0} for q in range(ne)]
+    ref, gpu = pair(dict(nuclei=nuc, NN=NN, screen=0.25 * NN))
+    for m in range(gpu.nelec):
+        f = ref.fields(m)
+        gpu.set_fields(m, f["U"], f["W"], f["P"])
+    ref.do_steps(6)
+    gpu.doSteps(6)
+    for m in range(gpu.nelec):
+        g, r = gpu.fields(m), ref.fields(m)
+        for key in ("U", "W", "P"):
+            assert same(g[key], r[key]), (m, key)
+    gpu.close()
