@@ -21,10 +21,14 @@
 
 #include "../../include/rq.h"
 #include "rq_internal.cuh"
+#include "vec_stencil.cuh"
 
 namespace rq {
 
 constexpr int kMfMax = 16;
+
+// elements between two electrons' fields: S^3 rounded up to 16-byte vectors
+__host__ __device__ inline long long mf_slot(long long S3) { return (S3 + 3) & ~3LL; }
 
 struct MfParams {  // writeParams (mol_fast.js:838-874) plus the constants templated into the shaders
   int NN, S, N2, n, shell_mode, any_rc;
@@ -40,6 +44,7 @@ struct MfParams {  // writeParams (mol_fast.js:838-874) plus the constants templ
   // upd = (fm, half_d * k_mult, 1 if the Thomas-Fermi term is on, tilt_x) of updateWGSL,
   // red = (fm without USER_FULL_SELF, k_mult * KINETIC_COEFF, same flag, tilt_y) of reduceWGSL
   float4 upd[kMfMax], red[kMfMax];
+  float rc_d2[kMfMax];  // no cell further from the nucleus than sqrt(rc_d2) cells is inside its rc; < 0 without one
   unsigned gmask[kMfMax];  // bit q set: electron q is in this electron's split group
 };
 
@@ -117,121 +122,180 @@ __device__ bool mf_in_sector(const MfParams* __restrict__ p, int m, float x, flo
 constexpr int kMfTK = 32, kMfTJ = 8;
 
 
-// updateWGSL (mol_fast.js:134-351) for every electron of one interior cell.  One thread owns a
-// cell: the cross-electron terms (sum_q P_q, the competitor max) come from one read of each
-// electron's U and P at the cell.  The competitor max over the other electrons is the largest U
-// of the cell unless this electron holds it (then the second largest): both are exact
-// selections, equal to the shader's sequential scan.  The register cap (4 blocks of 256 per SM)
-// lets the per-electron stencil loads of enough warps overlap; the kernel is bound by the
-// instruction issue of the unfused f32 arithmetic, not by DRAM.
-template <int NMAX, bool SHELL>
-__global__ void __launch_bounds__(256, 4) k_mf_update(const MfParams* __restrict__ p, const float* __restrict__ Ui,
-                                                      const float* __restrict__ Wi, const float* __restrict__ Pi,
-                                                      const float* __restrict__ K, float* __restrict__ Uo,
-                                                      float* __restrict__ Wo, float* __restrict__ Po) {
-  const int NN = p->NN;
-  const int k = blockIdx.x * kMfTK + threadIdx.x + 1;
-  const int j = blockIdx.y * kMfTJ + threadIdx.y + 1;
-  const int i = blockIdx.z + 1;
-  if (k >= NN || j >= NN) return;
-  const long long S = p->S, S2 = S * S, S3 = S2 * S;
-  const long long id = (long long)i * S2 + (long long)j * S + k;
+// updateWGSL (mol_fast.js:134-351).  A thread owns a 16-byte vector of four cells (vec_stencil.cuh) and walks
+// the electrons: the cross-electron terms (sum_q P_q, the competitor max) come from one read of each
+// electron's U and P at the cells.  The competitor max over the other electrons is the largest U of
+// the cell unless this electron holds it (then the second largest): both are exact selections, equal to
+// the shader's sequential scan.  The unfused f32 arithmetic (about 120 operations per cell and electron) issues
+// beside 15 vector loads per four cells; with a cell per thread its 21 scalar loads and their addresses took the
+// issue slots twice over.  CH4 at 200^3: 600 us before, XX us now (24 B per cell and electron: 140 us).
+__device__ __noinline__ float mf_shell_front(const MfParams* __restrict__ p, int m, int i, int j, int k, float nw) {
+  const float h = p->h;
+  const float4 at = p->atoms[m];
+  const float rc_m = p->rcs[m].x;
+  const float ro_m = F_MUL(p->r_out[m], p->R_out);
+  const float dxm = F_SUB((float)i, at.x), dym = F_SUB((float)j, at.y), dzm = F_SUB((float)k, at.z);
+  const float r_m = F_MUL(F_SQRT(F_ADD(F_ADD(F_MUL(dxm, dxm), F_MUL(dym, dym)), F_MUL(dzm, dzm))), h);
+  if (rc_m > 0.0f && r_m < rc_m) nw = fminf(nw, mf_cusp(r_m, rc_m, h));
+  if (ro_m > 0.0f && r_m > ro_m) nw = (r_m <= F_ADD(ro_m, h)) ? nw : 0.0f;
+  if (p->split_type[m] != 0 && p->split_fix[m] == 1 && !mf_in_sector(p, m, dxm, dym, dzm, r_m)) nw = 0.0f;
+  return nw;
+}
+
+template <int ROW, bool SHELL>
+__global__ void __launch_bounds__(256, 2) k_mf_update(const MfParams* __restrict__ p, Geo g,
+                                                      const float* __restrict__ Ui, const float* __restrict__ Wi,
+                                                      const float* __restrict__ Pi, const float* __restrict__ K,
+                                                      float* __restrict__ Uo, float* __restrict__ Wo,
+                                                      float* __restrict__ Po) {
+  const int i = 1 + blockIdx.y;
+  const VGroup r = vgroup<float>(g, i, blockIdx.x);
+  const VRow row = vrow(g, r, i);
+  const long long slot = mf_slot(g.S3);
   const int n = p->n;
-  float Ptot = 0.0f, max1 = 0.0f, max2 = 0.0f;
-  int arg1 = -1;
+  int jj[4], kk[4];
+  unsigned in = 0u;
 #pragma unroll
-  for (int q = 0; q < NMAX; ++q)
-    if (q < n) {
-      Ptot = F_ADD(Ptot, __ldg(Pi + q * S3 + id));
-      const float u = __ldg(Ui + q * S3 + id);
-      if (u > max1) { max2 = max1; max1 = u; arg1 = q; }
-      else if (u > max2) max2 = u;
-    }
-  const float h = p->h, dt = p->dt, inv_h = p->inv_h, inv_h2 = p->inv_h2;
-  // frozen-core mode: the rc cusps of all nuclei act on every electron's front; min is exact,
-  // so the cap over the nuclei is taken once per cell (mol_fast.js:249-262)
-  float cap = 2.0f;
-  if (!SHELL && p->any_rc) {
-    for (int a = 0; a < n; ++a) {
-      const float4 at = p->atoms[a];
-      const float rc_a = p->rcs[a].x;
-      const float dx = F_SUB((float)i, at.x), dy = F_SUB((float)j, at.y), dz = F_SUB((float)k, at.z);
-      const float r = F_MUL(F_SQRT(F_ADD(F_ADD(F_MUL(dx, dx), F_MUL(dy, dy)), F_MUL(dz, dz))), h);
-      if (rc_a > 0.0f && r < rc_a) cap = fminf(cap, mf_cusp(r, rc_a, h));
+  for (int e = 0; e < 4; ++e) {
+    jj[e] = row.j;
+    kk[e] = row.k + e;
+    if (kk[e] >= g.S) { kk[e] -= g.S; ++jj[e]; }
+    in |= r.own && vinterior(g, row, e) ? 1u << e : 0u;
+  }
+  // the plane above is new to L2 for every electron; the other rows were met by the blocks of the planes below
+  for (int q = 0; q < n; ++q) {
+    const long long up = q * slot + r.a + g.S2;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(Wi + up));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(Ui + up));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(Pi + up));
+  }
+  float Ptot[4] = {0.0f, 0.0f, 0.0f, 0.0f}, max1[4] = {0.0f, 0.0f, 0.0f, 0.0f}, max2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  int arg1[4] = {-1, -1, -1, -1};
+#pragma unroll 4
+  for (int q = 0; q < n; ++q) {
+    const Quad<float> pq = ldq(Pi + q * slot + r.a), uq = ldq(Ui + q * slot + r.a);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      Ptot[e] = F_ADD(Ptot[e], pq.v[e]);
+      const float u = uq.v[e];
+      if (u > max1[e]) { max2[e] = max1[e]; max1[e] = u; arg1[e] = q; }
+      else if (u > max2[e]) max2[e] = u;
     }
   }
-  const float Kc = __ldg(K + id);
-  const float x_au = F_MUL(F_SUB((float)i, (float)p->N2), h);
-  const float y_au = F_MUL(F_SUB((float)j, (float)p->N2), h);
-  const float beta = p->beta, two_pi_dt = F_MUL(p->two_pi, dt), fxx = F_MUL(p->field_x, x_au);
+  const float h = p->h, dt = p->dt, inv_h = p->inv_h, inv_h2 = p->inv_h2;
+  // frozen-core mode: the rc cusps of all nuclei act on every electron's front; min is exact,
+  // so the cap over the nuclei is taken once per cell (mol_fast.js:249-262), and only nuclei whose sphere
+  // reaches the cell's plane and row are looked at
+  float cap[4] = {2.0f, 2.0f, 2.0f, 2.0f};
+  if (!SHELL && p->any_rc) {
+    for (int a = 0; a < n; ++a) {
+      const float lim = p->rc_d2[a];
+      const float4 at = p->atoms[a];
+      const float dx = F_SUB((float)i, at.x), dx2 = F_MUL(dx, dx);
+      if (!(dx2 <= lim)) continue;
+      const float rc_a = p->rcs[a].x;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float dy = F_SUB((float)jj[e], at.y), dz = F_SUB((float)kk[e], at.z);
+        const float d2 = F_ADD(F_ADD(dx2, F_MUL(dy, dy)), F_MUL(dz, dz));
+        if (!(d2 <= lim)) continue;
+        const float rr = F_MUL(F_SQRT(d2), h);
+        if (rr < rc_a) cap[e] = fminf(cap[e], mf_cusp(rr, rc_a, h));
+      }
+    }
+  }
+  const Quad<float> K4 = ldq(K + r.a);
+  const float beta = p->beta, two_pi_dt = F_MUL(p->two_pi, dt);
   const float dt005 = F_MUL(0.05f, dt), dt1 = F_MUL(1.0f, dt);
-  const int s1 = (int)S, s2 = (int)S2;  // stencil offsets within one field (S^3 < 2^31)
+  const bool field = beta != 0.0f || p->field_x != 0.0f;
 #pragma unroll 1
   for (int m = 0; m < n; ++m) {
-    const long long o = m * S3 + id;
-    const float* __restrict__ u = Ui + o;
-    const float* __restrict__ w = Wi + o;
-    const float* __restrict__ pp = Pi + o;
-    const float uc = __ldg(u), wc = __ldg(w), Pc = __ldg(pp);
-    const float wip = __ldg(w + s2), wim = __ldg(w - s2), wjp = __ldg(w + s1), wjm = __ldg(w - s1);
-    const float wkp = __ldg(w + 1), wkm = __ldg(w - 1);
-    const float uip = __ldg(u + s2), uim = __ldg(u - s2), ujp = __ldg(u + s1), ujm = __ldg(u - s1);
-    const float ukp = __ldg(u + 1), ukm = __ldg(u - 1);
-    const float pip = __ldg(pp + s2), pim = __ldg(pp - s2), pjp = __ldg(pp + s1), pjm = __ldg(pp - s1);
-    const float pkp = __ldg(pp + 1), pkm = __ldg(pp - 1);
+    const long long off = m * slot;
+    const VLoad<float, ROW> lw(Wi + off, r, g), lu(Ui + off, r, g), lp(Pi + off, r, g);
     const float4 cu = p->upd[m];
     const float tilt_y = p->rcs[m].w;
     const unsigned gm = p->gmask[m];
-    const float umax = m == arg1 ? max2 : max1;
-    float Pgrp, rho_other = 0.0f;
-    if (gm == (1u << m)) {  // no split siblings: the group sum is this electron's own P
-      Pgrp = F_ADD(0.0f, Pc);
-    } else {
-      Pgrp = 0.0f;
+    float pot[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) pot[e] = lp.c.v[e];  // the group sum: without split siblings this electron's own P
+    if (gm != (1u << m)) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) pot[e] = 0.0f;
       for (int q = 0; q < n; ++q)
-        if ((gm >> q) & 1u) Pgrp = F_ADD(Pgrp, __ldg(Pi + q * S3 + id));
-    }
-    if (beta != 0.0f) {  // V_Pauli; with beta = 0 it is 0 * (a finite sum of squares) = 0
-      for (int q = 0; q < n; ++q)
-        if (q != m) {
-          const float un = __ldg(Ui + q * S3 + id);
-          rho_other = F_ADD(rho_other, F_MUL(un, un));
+        if ((gm >> q) & 1u) {
+          const Quad<float> pq = ldq(Pi + q * slot + r.a);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) pot[e] = F_ADD(pot[e], pq.v[e]);
         }
     }
-    const float cm = F_SUB(uc, umax);
-    const float lw =
-        F_MUL(F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(wip, wim), wjp), wjm), wkp), wkm), F_MUL(6.0f, wc)), inv_h2);
-    const float gx = F_MUL(F_SUB(wip, wim), inv_h), gy = F_MUL(F_SUB(wjp, wjm), inv_h),
-                gz = F_MUL(F_SUB(wkp, wkm), inv_h);
-    float nw = F_ADD(F_ADD(wc, F_MUL(F_MUL(dt005, fabsf(cm)), lw)),
-                     F_MUL(F_MUL(dt1, cm), F_SQRT(F_ADD(F_ADD(F_MUL(gx, gx), F_MUL(gy, gy)), F_MUL(gz, gz)))));
-    nw = fminf(fmaxf(nw, 0.0f), 1.0f);
-    if (SHELL) {
-      const float4 at = p->atoms[m];
-      const float rc_m = p->rcs[m].x;
-      const float ro_m = F_MUL(p->r_out[m], p->R_out);
-      const float dxm = F_SUB((float)i, at.x), dym = F_SUB((float)j, at.y), dzm = F_SUB((float)k, at.z);
-      const float r_m = F_MUL(F_SQRT(F_ADD(F_ADD(F_MUL(dxm, dxm), F_MUL(dym, dym)), F_MUL(dzm, dzm))), h);
-      if (rc_m > 0.0f && r_m < rc_m) nw = fminf(nw, mf_cusp(r_m, rc_m, h));
-      if (ro_m > 0.0f && r_m > ro_m) nw = (r_m <= F_ADD(ro_m, h)) ? nw : 0.0f;
-      if (p->split_type[m] != 0 && p->split_fix[m] == 1 && !mf_in_sector(p, m, dxm, dym, dzm, r_m)) nw = 0.0f;
-    } else if (cap <= 1.0f) {
-      nw = fminf(nw, cap);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) pot[e] = F_SUB(K4.v[e], F_MUL(2.0f, F_SUB(Ptot[e], F_MUL(cu.x, pot[e]))));
+    // The shader subtracts every further term; one whose coefficient is 0 is +-0 and changes nothing, since the
+    // difference so far is never -0 (K is a sum that starts at +0).
+    if (cu.z != 0.0f) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        pot[e] = F_SUB(pot[e], F_MUL(p->alpha_tf, mf_pow(fmaxf(F_MUL(lu.c.v[e], lu.c.v[e]), 1e-20f), 0.6666667f)));
     }
-    Wo[o] = nw;
-    const float Vother = F_MUL(2.0f, F_SUB(Ptot, F_MUL(cu.x, Pgrp)));
-    const float V_TF = cu.z != 0.0f ? F_MUL(p->alpha_tf, mf_pow(fmaxf(F_MUL(uc, uc), 1e-20f), 0.6666667f)) : 0.0f;
-    const float V_tilt = F_SUB(F_MUL(-cu.w, x_au), F_MUL(tilt_y, y_au));
-    const float V_Pauli = F_MUL(beta, rho_other);
+    if (field || cu.w != 0.0f || tilt_y != 0.0f) {
+      float rho_other[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      for (int q = 0; beta != 0.0f && q < n; ++q)
+        if (q != m) {
+          const Quad<float> uq = ldq(Ui + q * slot + r.a);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) rho_other[e] = F_ADD(rho_other[e], F_MUL(uq.v[e], uq.v[e]));
+        }
+      const float x_au = F_MUL(F_SUB((float)i, (float)p->N2), h);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float y_au = F_MUL(F_SUB((float)jj[e], (float)p->N2), h);
+        const float V_tilt = F_SUB(F_MUL(-cu.w, x_au), F_MUL(tilt_y, y_au));
+        pot[e] = F_SUB(F_SUB(F_SUB(pot[e], V_tilt), beta != 0.0f ? F_MUL(beta, rho_other[e]) : 0.0f),
+                       F_MUL(p->field_x, x_au));
+      }
+    }
+    const Star<float> w = vstar(lw), u = vstar(lu), q = vstar(lp);
+    Quad<float> ow, ou, op;
     const float hd = cu.y;
-    const float fx = F_SUB(F_MUL(F_MUL(F_SUB(uip, uc), F_ADD(wip, nw)), 0.5f), F_MUL(F_MUL(F_SUB(uc, uim), F_ADD(nw, wim)), 0.5f));
-    const float fy = F_SUB(F_MUL(F_MUL(F_SUB(ujp, uc), F_ADD(wjp, nw)), 0.5f), F_MUL(F_MUL(F_SUB(uc, ujm), F_ADD(nw, wjm)), 0.5f));
-    const float fz = F_SUB(F_MUL(F_MUL(F_SUB(ukp, uc), F_ADD(wkp, nw)), 0.5f), F_MUL(F_MUL(F_SUB(uc, ukm), F_ADD(nw, wkm)), 0.5f));
-    const float pot = F_SUB(F_SUB(F_SUB(F_SUB(F_SUB(Kc, Vother), V_TF), V_tilt), V_Pauli), fxx);
-    Uo[o] = F_ADD(F_ADD(F_ADD(F_ADD(uc, F_MUL(hd, fx)), F_MUL(hd, fy)), F_MUL(hd, fz)),
-                  F_MUL(F_MUL(F_MUL(dt, pot), uc), wc));
-    const float lap = F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(pip, pim), pjp), pjm), pkp), pkm), F_MUL(6.0f, Pc));
-    Po[o] = F_ADD(F_ADD(Pc, F_MUL(F_MUL(dt, lap), inv_h2)), F_MUL(F_MUL(two_pi_dt, uc), uc));
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float uc = u.c.v[e], wc = w.c.v[e], Pc = q.c.v[e];
+      const float wip = w.ip.v[e], wim = w.im.v[e], wjp = w.jp.v[e], wjm = w.jm.v[e], wkp = w.kp.v[e], wkm = w.km.v[e];
+      const float cm = F_SUB(uc, m == arg1[e] ? max2[e] : max1[e]);
+      const float lap_w =
+          F_MUL(F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(wip, wim), wjp), wjm), wkp), wkm), F_MUL(6.0f, wc)), inv_h2);
+      const float gx = F_MUL(F_SUB(wip, wim), inv_h), gy = F_MUL(F_SUB(wjp, wjm), inv_h),
+                  gz = F_MUL(F_SUB(wkp, wkm), inv_h);
+      float nw = F_ADD(F_ADD(wc, F_MUL(F_MUL(dt005, fabsf(cm)), lap_w)),
+                       F_MUL(F_MUL(dt1, cm), sqrt0(F_ADD(F_ADD(F_MUL(gx, gx), F_MUL(gy, gy)), F_MUL(gz, gz)))));
+      nw = fminf(fmaxf(nw, 0.0f), 1.0f);
+      if (SHELL)
+        nw = mf_shell_front(p, m, i, jj[e], kk[e], nw);
+      else
+        nw = fminf(nw, cap[e]);  // the shader takes a cap of at most 1 only; nw is at most 1
+      ow.v[e] = nw;
+      const float fx = F_SUB(F_MUL(F_MUL(F_SUB(u.ip.v[e], uc), F_ADD(wip, nw)), 0.5f),
+                             F_MUL(F_MUL(F_SUB(uc, u.im.v[e]), F_ADD(nw, wim)), 0.5f));
+      const float fy = F_SUB(F_MUL(F_MUL(F_SUB(u.jp.v[e], uc), F_ADD(wjp, nw)), 0.5f),
+                             F_MUL(F_MUL(F_SUB(uc, u.jm.v[e]), F_ADD(nw, wjm)), 0.5f));
+      const float fz = F_SUB(F_MUL(F_MUL(F_SUB(u.kp.v[e], uc), F_ADD(wkp, nw)), 0.5f),
+                             F_MUL(F_MUL(F_SUB(uc, u.km.v[e]), F_ADD(nw, wkm)), 0.5f));
+      ou.v[e] = F_ADD(F_ADD(F_ADD(F_ADD(uc, F_MUL(hd, fx)), F_MUL(hd, fy)), F_MUL(hd, fz)),
+                      F_MUL(F_MUL(F_MUL(dt, pot[e]), uc), wc));
+      const float lap = F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(q.ip.v[e], q.im.v[e]), q.jp.v[e]), q.jm.v[e]), q.kp.v[e]),
+                                    q.km.v[e]),
+                              F_MUL(6.0f, Pc));
+      op.v[e] = F_ADD(F_ADD(Pc, F_MUL(F_MUL(dt, lap), inv_h2)), F_MUL(F_MUL(two_pi_dt, uc), uc));
+    }
+    if (in == 15u) {
+      stq(Wo + off + r.a, ow);
+      stq(Uo + off + r.a, ou);
+      stq(Po + off + r.a, op);
+    } else if (in != 0u) {
+      vstore(Wo + off, r, in, ow);
+      vstore(Uo + off, r, in, ou);
+      vstore(Po + off, r, in, op);
+    }
   }
 }
 
@@ -247,7 +311,7 @@ __global__ void __launch_bounds__(128) k_mf_reduce(const MfParams* __restrict__ 
   const long long cell = (long long)blockIdx.x * 128 + lid;
   if (cell < tot) {
     const int k = (int)(cell % NM) + 1, j = (int)((cell / NM) % NM) + 1, i = (int)(cell / (NM * NM)) + 1;
-    const long long S = p->S, S2 = S * S, S3 = S2 * S;
+    const long long S = p->S, S2 = S * S, S3 = mf_slot(S2 * S);
     const long long id = (long long)i * S2 + (long long)j * S + k;
     const float h = p->h, h3 = p->h3;
     float T = 0.0f, VeK = 0.0f, Vee = 0.0f, dx = 0.0f, dy = 0.0f, dz = 0.0f;
@@ -320,7 +384,7 @@ __global__ void __launch_bounds__(256) k_mf_normalize(const MfParams* __restrict
   const int j = blockIdx.y * kMfTJ + threadIdx.y + 1;
   const int i = blockIdx.z + 1;
   if (k >= NN || j >= NN) return;
-  const long long S = p->S, S2 = S * S, S3 = S2 * S;
+  const long long S = p->S, S2 = S * S, S3 = mf_slot(S2 * S);
   const long long id = (long long)i * S2 + (long long)j * S + k;
   for (int m = 0; m < p->n; ++m) {
     const float nrm = sums[m], tgt = p->rcs[m].y;
@@ -336,7 +400,7 @@ __global__ void __launch_bounds__(256) k_mf_residual(const MfParams* __restrict_
   const int j = blockIdx.y * kMfTJ + threadIdx.y + 1;
   const int i = blockIdx.z % NM + 1, m = blockIdx.z / NM;
   if (k >= NN || j >= NN) return;
-  const long long S = p->S, S2 = S * S, S3 = S2 * S;
+  const long long S = p->S, S2 = S * S, S3 = mf_slot(S2 * S);
   const long long o = m * S3 + (long long)i * S2 + (long long)j * S + k;
   const float Pc = __ldg(P + o);
   const float lap = F_MUL(F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(__ldg(P + o + S2), __ldg(P + o - S2)), __ldg(P + o + S)),
@@ -357,7 +421,7 @@ __global__ void __launch_bounds__(256) k_mf_restrict(const MfParams* __restrict_
   const int J = blockIdx.y * kMfTJ + threadIdx.y + 1;
   const int I = blockIdx.z % NCM + 1, m = blockIdx.z / NCM;
   if (K2 >= NC || J >= NC) return;
-  const long long S = p->S, S2 = S * S, S3 = S2 * S;
+  const long long S = p->S, S2 = S * S, S3 = mf_slot(S2 * S);
   const long long SC = NC + 1, SC2 = SC * SC, SC3 = SC2 * SC;
   const float* f = fine + m * S3;
   const long long c = (2LL * I) * S2 + (2LL * J) * S + 2LL * K2;
@@ -399,7 +463,7 @@ __global__ void __launch_bounds__(256) k_mf_prolong(const MfParams* __restrict__
   const int j = blockIdx.y * kMfTJ + threadIdx.y + 1;
   const int i = blockIdx.z % NM + 1, m = blockIdx.z / NM;
   if (k >= NN || j >= NN) return;
-  const long long S = p->S, S2 = S * S, S3 = S2 * S;
+  const long long S = p->S, S2 = S * S, S3 = mf_slot(S2 * S);
   const long long SC = NC + 1, SC2 = SC * SC, SC3 = SC2 * SC;
   const int ci = i / 2, cj = j / 2, ck = k / 2;
   const int ci1 = min(ci + (i & 1), NC), cj1 = min(cj + (j & 1), NC), ck1 = min(ck + (k & 1), NC);
@@ -433,7 +497,7 @@ __global__ void __launch_bounds__(256) k_mf_force(const MfParams* __restrict__ p
     return;
   }
   const int S = p->S, n = p->n;
-  const long long S2 = (long long)S * S, S3 = S2 * S;
+  const long long S2 = (long long)S * S, S3 = mf_slot(S2 * S);
   const int ci = (int)at.x, cj = (int)at.y, ck = (int)at.z;
   const float inv2h = F_MUL(0.5f, p->inv_h);
   for (int t = threadIdx.x; t < 729; t += blockDim.x) {
@@ -497,7 +561,7 @@ __global__ void __launch_bounds__(256) k_mf_extract(const MfParams* __restrict__
   const int i = blockIdx.x * 16 + threadIdx.x, j = blockIdx.y * 16 + threadIdx.y;
   const int NN = p->NN, n = p->n, N2 = p->N2;
   if (i > NN || j > NN) return;
-  const long long SS = NN + 1, S2 = SS * SS, S3 = S2 * SS;
+  const long long SS = NN + 1, S2 = SS * SS, S3 = mf_slot(S2 * SS);
   for (int m = 0; m < n; ++m) {
     const long long idx2 = m * S3 + (long long)i * S2 + (long long)j * SS + N2;
     out[m * SS * SS + i * SS + j] = W[idx2] > 0.1f ? U[idx2] : 0.0f;
@@ -572,6 +636,7 @@ __global__ void __launch_bounds__(256) k_mf_init(const double* __restrict__ nuc,
                                                  float* __restrict__ K, float* __restrict__ U, float* __restrict__ W,
                                                  float* __restrict__ P) {
   const long long S = NN + 1, S2 = S * S, S3 = S2 * S;
+  const long long slot = mf_slot(S3);
   const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= S3) return;
   const int k = (int)(id % S), j = (int)((id / S) % S), i = (int)(id / S2);
@@ -609,9 +674,9 @@ __global__ void __launch_bounds__(256) k_mf_init(const double* __restrict__ nuc,
       const double t = fmax(0.0, fmin(1.0, __ddiv_rn(__dsub_rn(rl[m], edge), __dsub_rn(rc, edge))));
       u = __dmul_rn(u, __dmul_rn(__dmul_rn(t, t), __dsub_rn(3.0, __dmul_rn(2.0, t))));
     }
-    U[m * S3 + id] = (float)u;
-    W[m * S3 + id] = 0.0f;
-    P[m * S3 + id] = (float)__ddiv_rn(__dmul_rn(0.5, nuc[kMfNucLen * m + 3]), __dadd_rn(rl[m], h2v));
+    U[m * slot + id] = (float)u;
+    W[m * slot + id] = 0.0f;
+    P[m * slot + id] = (float)__ddiv_rn(__dmul_rn(0.5, nuc[kMfNucLen * m + 3]), __dadd_rn(rl[m], h2v));
   }
   if (bestM >= 0 && rl[bestM] < R_init) {
     const double rc = nuc[kMfNucLen * bestM + 4], ro = nuc[kMfNucLen * bestM + 5];
@@ -622,7 +687,7 @@ __global__ void __launch_bounds__(256) k_mf_init(const double* __restrict__ nuc,
       w = __dmul_rn(__dmul_rn(t, t), __dsub_rn(3.0, __dmul_rn(2.0, t)));
     }
     if (ro > 0 && rl[bestM] > __dadd_rn(ro, hv)) w = 0;
-    W[bestM * S3 + id] = (float)w;
+    W[bestM * slot + id] = (float)w;
   }
 }
 
@@ -630,7 +695,7 @@ __global__ void __launch_bounds__(256) k_mf_init(const double* __restrict__ nuc,
 // uploadInitialData, mol_fast.js:1024-1037)
 __global__ void __launch_bounds__(256) k_mf_init_norm(const float* __restrict__ U, long long S3, double* __restrict__ acc) {
   __shared__ double red[256];
-  const float* Um = U + blockIdx.y * S3;
+  const float* Um = U + blockIdx.y * mf_slot(S3);
   double s = 0;
   for (long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x; id < S3; id += (long long)gridDim.x * blockDim.x) {
     const double u = Um[id];
@@ -651,7 +716,7 @@ __global__ void __launch_bounds__(256) k_mf_init_scale(float* __restrict__ U, lo
   const double nrm = __dmul_rn(acc[m], h3v), tg = nuc[kMfNucLen * m + 8];
   if (!(nrm > 0 && tg > 0)) return;
   const double sc = __dsqrt_rn(__ddiv_rn(tg, nrm));
-  float* Um = U + m * S3;
+  float* Um = U + m * mf_slot(S3);
   for (long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x; id < S3; id += (long long)gridDim.x * blockDim.x)
     Um[id] = (float)__dmul_rn((double)Um[id], sc);
 }
@@ -743,6 +808,8 @@ void mf_fill_params(rq_mf* s) {
     for (int b = 0; b < s->n; ++b)
       if (p.split_group[b] == p.split_group[a]) gmask |= 1u << b;
     p.gmask[a] = gmask;
+    const double cells = (double)p.rcs[a].x / p.h;  // 1 % of slack over the roundings of the distance
+    p.rc_d2[a] = p.rcs[a].x > 0.0f ? (float)(1.01 * cells * cells) : -1.0f;
   }
 }
 
@@ -758,13 +825,13 @@ dim3 mf_grid(int NN, int planes) {
 
 int mf_launch_update(rq_mf* s, int c) {
   const int nx = 1 - c;
-  const dim3 g = mf_grid(s->NN, s->NN - 1), b(kMfTK, kMfTJ);
+  const Geo g = make_geo(s->S);
   const bool sh = s->cfg.shell_mode != 0;
-#define MF_UPD(NM_, SH_) \
-  k_mf_update<NM_, SH_><<<g, b, 0, s->st>>>(s->dp, s->U[c], s->W[c], s->P[c], s->K, s->U[nx], s->W[nx], s->P[nx])
-  if (s->n <= 4) { if (sh) MF_UPD(4, true); else MF_UPD(4, false); }
-  else if (s->n <= 8) { if (sh) MF_UPD(8, true); else MF_UPD(8, false); }
-  else { if (sh) MF_UPD(16, true); else MF_UPD(16, false); }
+#define MF_UPD(ROW_, SH_)                                                                                        \
+  k_mf_update<ROW_, SH_><<<vgrid<float>(g, 1), 256, 0, s->st>>>(s->dp, g, s->U[c], s->W[c], s->P[c], s->K, s->U[nx], \
+                                                                s->W[nx], s->P[nx])
+  if (s->S % 4 == 1) { if (sh) MF_UPD(kRowP, true); else MF_UPD(kRowP, false); }
+  else { if (sh) MF_UPD(kRowM, true); else MF_UPD(kRowM, false); }
 #undef MF_UPD
   MLAUNCH();
   return RQ_OK;
@@ -846,7 +913,7 @@ extern "C" int rq_mf_create(const rq_mf_config* cfg, const rq_mf_nucleus* nuclei
     if (cudaMemset(*p, 0, bytes) != cudaSuccess) { s->last_error = "cudaMemset"; return RQ_ECUDA; }
     return RQ_OK;
   };
-  const size_t F = sizeof(float), fld = F * (size_t)s->S3 * n, cfld = F * (size_t)s->SC3 * n;
+  const size_t F = sizeof(float), fld = F * (size_t)mf_slot(s->S3) * n, cfld = F * (size_t)s->SC3 * n;
   int rc = RQ_OK;
   for (int b = 0; b < 2 && rc == RQ_OK; ++b)
     if ((rc = alloc((void**)&s->U[b], fld)) || (rc = alloc((void**)&s->W[b], fld)) || (rc = alloc((void**)&s->P[b], fld)) ||
@@ -996,7 +1063,7 @@ extern "C" int rq_mf_extract(rq_mf* s, float* out) {
 
 extern "C" int rq_mf_download(rq_mf* s, int32_t m, float* U, float* W, float* P) {
   if (!s || m < 0 || m >= s->n) return RQ_EINVAL;
-  const size_t S3 = (size_t)s->S3, off = (size_t)m * S3;
+  const size_t S3 = (size_t)s->S3, off = (size_t)m * mf_slot(s->S3);
   const int c = s->cur;
   if (U) MCK(cudaMemcpyAsync(U, s->U[c] + off, sizeof(float) * S3, cudaMemcpyDeviceToHost, s->st));
   if (W) MCK(cudaMemcpyAsync(W, s->W[c] + off, sizeof(float) * S3, cudaMemcpyDeviceToHost, s->st));
@@ -1007,7 +1074,7 @@ extern "C" int rq_mf_download(rq_mf* s, int32_t m, float* U, float* W, float* P)
 
 extern "C" int rq_mf_upload(rq_mf* s, int32_t m, const float* U, const float* W, const float* P) {
   if (!s || m < 0 || m >= s->n) return RQ_EINVAL;
-  const size_t S3 = (size_t)s->S3, off = (size_t)m * S3;
+  const size_t S3 = (size_t)s->S3, off = (size_t)m * mf_slot(s->S3);
   for (int c = 0; c < 2; ++c) {  // both buffer sets, as uploadInitialData writes them
     if (U) MCK(cudaMemcpyAsync(s->U[c] + off, U, sizeof(float) * S3, cudaMemcpyHostToDevice, s->st));
     if (W) MCK(cudaMemcpyAsync(s->W[c] + off, W, sizeof(float) * S3, cudaMemcpyHostToDevice, s->st));

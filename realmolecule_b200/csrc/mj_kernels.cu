@@ -175,22 +175,12 @@ __device__ __forceinline__ unsigned mj_inside(const Geo& g, const VGroup& r, int
   for (int e = 0; e < 4; ++e) m |= vinterior(g, w, e) ? 1u << e : 0u;
   return m;
 }
-__device__ __forceinline__ void mj_store(float* p, const VGroup& r, unsigned in, const Quad<float>& q) {
-  if (in == 15u) {
-    stq(p + r.a, q);
-  } else {
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (in >> e & 1u) p[r.a + e] = q.v[e];
-  }
-}
-
 // x / 9 correctly rounded by the two-constant product of sixth() (checked for every mantissa at |x| >= 2^-119)
 __device__ __forceinline__ float ninth(float x) {
   constexpr float zh = 0x1.c71c72p-4f, zl = -0x1.c71c72p-31f;
   const float a = fabsf(x);
   if (a >= 0x1p-100f && a <= 0x1p126f) return __fmaf_rn(x, zh, __fmul_rn(x, zl));
-  return F_DIV(x, 9.0f);
+  return x == 0.0f ? x : F_DIV(x, 9.0f);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -264,7 +254,7 @@ __global__ void __launch_bounds__(256) k_mj_update(const float* __restrict__ U, 
         }
       }
     }
-    mj_store(Uo, r, in, o);
+    vstore(Uo, r, in, o);
   }
   if (ACC) {
     int same;
@@ -305,7 +295,7 @@ __global__ void __launch_bounds__(256) k_mj_apply_scale(float* __restrict__ U, c
       }
       u.v[e] = F_MUL(u.v[e], scale);
     }
-    mj_store(U, r, in, u);
+    vstore(U, r, in, u);
   }
 }
 
@@ -356,7 +346,7 @@ __global__ void __launch_bounds__(256) k_mj_jacobi(const float* __restrict__ Pin
       o.v[e] = F_ADD(F_MUL(0.3333f, p.c.v[e]), ninth(F_ADD(sn, F_MUL(c0, rho))));
       if (LAST && (in >> e & 1u) && (l.v[e] & kMjMask) == m) Pother[r.a + e] = o.v[e];
     }
-    mj_store(Pout, r, in, o);
+    vstore(Pout, r, in, o);
   }
 }
 
@@ -995,7 +985,7 @@ __global__ void __launch_bounds__(256) k_lob_apply_h(const float* __restrict__ U
           F_ADD(F_MUL(F_MUL(-0.5f, lap), inv_h2), F_MUL(F_ADD(-k4.v[e], F_MUL(2.0f, p4.v[e])), uc));
       o.v[e] = excl ? 0.0f : out;
     }
-    mj_store(HU, r, in, o);
+    vstore(HU, r, in, o);
   }
 }
 
@@ -1277,7 +1267,7 @@ __global__ void __launch_bounds__(256) k_lob_residual(const float* __restrict__ 
       const float diagH = F_ADD(F_ADD(F_MUL(3.0f, inv_h2), vEff), 0.1f);
       o.v[e] = F_DIV(res, diagH);
     }
-    mj_store(W, r, in, o);
+    vstore(W, r, in, o);
   }
 }
 
@@ -1306,8 +1296,8 @@ __global__ void __launch_bounds__(256) k_lob_update(float* __restrict__ X, const
       x.v[e] = F_ADD(F_ADD(F_MUL(c0, x.v[e]), F_MUL(c1, w.v[e])), F_MUL(c2, pv));
       p.v[e] = F_ADD(F_MUL(c1, w.v[e]), F_MUL(c2, pv));
     }
-    mj_store(X, r, in, x);
-    mj_store(Pv, r, in, p);
+    vstore(X, r, in, x);
+    vstore(Pv, r, in, p);
   }
 }
 

@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(512) k_rb_color(const RbParams p, int color, f
   const float lap_w = F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(wxp, wxm), wyp), wym), wzp), wzm), F_MUL(6.0f, wc));
   const float gwx = F_MUL(F_SUB(wxp, wxm), inv_h), gwy = F_MUL(F_SUB(wyp, wym), inv_h),
               gwz = F_MUL(F_SUB(wzp, wzm), inv_h);
-  const float grad_w = F_SQRT(F_ADD(F_ADD(F_MUL(gwx, gwx), F_MUL(gwy, gwy)), F_MUL(gwz, gwz)));
+  const float grad_w = sqrt0(F_ADD(F_ADD(F_MUL(gwx, gwx), F_MUL(gwy, gwy)), F_MUL(gwz, gwz)));
   const float wc2 =
       F_ADD(F_ADD(wc, F_MUL(F_MUL(F_MUL(dt05, fabsf(cc)), lap_w), inv_h2)), F_MUL(F_MUL(dt10, cc), grad_w));
   const float fxp = F_MUL(F_MUL(F_SUB(uxp, uc), F_ADD(wxp, wc2)), 0.5f);

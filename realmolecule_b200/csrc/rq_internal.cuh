@@ -18,6 +18,13 @@
 #define F_DIV(a, b) __fdiv_rn((a), (b))
 #define F_SQRT(a) __fsqrt_rn((a))
 
+// F_SQRT where 0 is a usual argument (the gradient of a front is 0 in most of a box): 0 takes the square
+// root's slow path, a call of its own per element
+__device__ __forceinline__ float sqrt0(float a) {
+  const float r = __fsqrt_rn(a == 0.0f ? 1.0f : a);
+  return a == 0.0f ? a : r;
+}
+
 namespace rq {
 
 constexpr int kThreadsK = 32;  // threads along k (contiguous) per block

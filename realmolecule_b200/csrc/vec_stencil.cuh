@@ -100,6 +100,17 @@ __device__ __forceinline__ bool vinterior(const Geo& g, const VRow& r, int e) {
   return k >= 1 && k < g.NN && j >= 1 && j < g.NN;
 }
 
+// The group's elements with their bit in `in`, the others as the array holds them
+__device__ __forceinline__ void vstore(float* p, const VGroup& r, unsigned in, const Quad<float>& q) {
+  if (in == 15u) {
+    stq(p + r.a, q);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (in >> e & 1u) p[r.a + e] = q.v[e];
+  }
+}
+
 // A field on the group and its six neighbours.  A shift by d = 1 mod W is the aligned group at a + d - 1 and
 // the next lane's first element; d = -1 mod W the aligned group at a + d + 1 and the previous lane's last.
 // Every load is issued by the constructor of VLoad (the shuffles of vstar would otherwise order them), so
@@ -118,7 +129,7 @@ template <typename T, int ROW, bool LDG = true> struct VLoad {
   __device__ __forceinline__ VLoad(const T* p, const VGroup& r, const Geo& g) {
     const T* x = p + r.a;
     up = ROW == kRowAny ? (g.S & 3) == 1 : ROW == kRowP;
-    const long long S = up ? (long long)g.S : -(long long)g.S, S2 = g.S2;
+    const int S = up ? (int)g.S : -(int)g.S, S2 = (int)g.S2;  // 32 bits: one multiply-add per address
     c = q(x);
     ip = q(x + S2 - 1);
     im = q(x - S2 + 1);
@@ -191,7 +202,7 @@ __device__ __forceinline__ float sixth(float x) {
   constexpr float zh = 0x1.555556p-3f, zl = -0x1.555556p-28f;
   const float a = fabsf(x);
   if (a >= 0x1p-100f && a <= 0x1p126f) return __fmaf_rn(x, zh, __fmul_rn(x, zl));
-  return F_DIV(x, 6.0f);
+  return x == 0.0f ? x : F_DIV(x, 6.0f);
 }
 __device__ __forceinline__ double sixth(double x) {
   constexpr double zh = 0x1.5555555555555p-3, zl = 0x1.5555555555555p-57;

@@ -122,3 +122,25 @@ def test_invalid_configs_are_errors():
         MolFast(H2["nuclei"], NN=33)
     with pytest.raises(L.RqError):
         MolFast(H2["nuclei"], NN=32, vcycle_interval=0)
+
+
+# Edges of the 16-byte vectors: both pitches modulo 4, planes of less than a warp's vectors, one electron (no
+# competitor), as many as the solver takes, fields whose size is no multiple of a vector.
+@pytest.mark.parametrize("NN,n,shell", [(8, 1, False), (8, 16, False), (10, 3, True), (34, 5, False), (62, 2, True)])
+def test_vector_edges(NN, n, shell):
+    c = NN / 2
+    nuc = [{"i": c + (q % 3) - 1, "j": c + (q // 3) % 3 - 1.25, "k": c + q // 9, "Z": 1 + q % 2,
+            "rc": 0.6 if q % 3 == 0 else 0} for q in range(n)]
+    if shell:
+        nuc[1].update(split="hemi", split_idx=1, split_axis=[1, 0, 1], r_out=1.5)
+    ref, gpu = pair(dict(nuclei=nuc, NN=NN, screen=0.25 * NN, shell_mode=shell), 4)
+    for m in range(gpu.n):
+        f = ref.fields(m)
+        gpu.set_fields(m, f["U"], f["W"], f["P"])
+    ref.do_steps(6)
+    gpu.doSteps(6)
+    for m in range(gpu.n):
+        g, r = gpu.fields(m), ref.fields(m)
+        for key in ("U", "W", "P"):
+            assert same(g[key], r[key]), (m, key)
+    gpu.close()
