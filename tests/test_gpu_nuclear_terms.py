@@ -164,3 +164,28 @@ def test_force_gather_edges(NN, sigma_h, nuclear_sum, precision):
         w[:, :, 0] = w[:, :, -1] = 0
         ref[a] = [(w * t).sum() for t in d]
     assert np.abs(F - ref).max() <= 1e-11 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("n_nuc,n_seed", [(1, 1), (2, 6), (33, 0), (31, 70), (70, 31)])
+def test_nuclear_repulsion_sums(n_nuc, n_seed):
+    """Energy and forces between point nuclei, entries without nuclear charge in between, against the pair sums in
+    FP64.  A force adds at most 70 terms, each with about 8 roundings: 1e-13 of the largest term's sum holds."""
+    rng = np.random.default_rng(n_nuc)
+    NN, h = 16, 0.5
+    pos = rng.uniform(2.0, 14.0, (n_nuc + n_seed, 3))
+    zn = np.zeros(n_nuc + n_seed)
+    zn[rng.permutation(n_nuc + n_seed)[:n_nuc]] = rng.integers(1, 8, n_nuc)
+    rows = [dict(i=p[0], j=p[1], k=p[2], Z=0.0 if z else 1.0, Z_nuc=z) for p, z in zip(pos, zn)]
+    ctx = ctx_for(NN, NN * h, rows, "fp64")
+    E, F = ctx.nuclear_terms()
+    x, d = pos * h, zn > 0
+    Er, Fr, mag = 0.0, np.zeros_like(pos), 0.0
+    for a in np.flatnonzero(d):
+        for b in np.flatnonzero(d):
+            if a != b:
+                r = x[a] - x[b]
+                Er += 0.5 * zn[a] * zn[b] / np.linalg.norm(r)
+                Fr[a] += zn[a] * zn[b] * r / np.linalg.norm(r) ** 3
+        mag = max(mag, sum(zn[a] * zn[b] / np.sum((x[a] - x[b]) ** 2) for b in np.flatnonzero(d) if b != a))
+    np.testing.assert_allclose(E, Er, rtol=1e-13, atol=0)
+    assert np.abs(F - Fr).max() <= 1e-13 * mag
