@@ -26,7 +26,7 @@ import numpy as np
 import torch
 
 from . import _lib as L
-from .context import Context
+from .context import ATOM_FIELDS, Context
 
 
 class EnergyModel:
@@ -60,11 +60,16 @@ class EnergyModel:
         self.last = None
 
     def _rows(self, pos: np.ndarray):
-        rows = [{"i": p[0] / self.h, "j": p[1] / self.h, "k": p[2] / self.h, "Z": 0.0, "Z_nuc": float(z)}
-                for p, z in zip(pos, self.charges)]
-        rows += [{"i": s[0] / self.h, "j": s[1] / self.h, "k": s[2] / self.h, "Z": 1.0, "Z_nuc": 0.0}
-                 for s in self.seeds]
-        return rows
+        """Atom table: the nuclei (Z 0), then the one-electron domains at their seeds (Z_nuc 0)."""
+        n = min(len(pos), self.n_nuc)
+        tab = np.zeros((n + len(self.seeds), len(ATOM_FIELDS)))
+        if n:
+            tab[:n, :3] = pos[:n, :3] / self.h
+            tab[:n, ATOM_FIELDS.index("Z_nuc")] = self.charges[:n]
+        if len(self.seeds):
+            tab[n:, :3] = self.seeds[:, :3] / self.h
+            tab[n:, ATOM_FIELDS.index("Z")] = 1.0
+        return tab
 
     def evaluate(self, positions: np.ndarray, v=None, dE_dv=None):
         """Energy and total forces on the nuclei (n_nuc x 3) for positions R and external potential v

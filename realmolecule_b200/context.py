@@ -19,8 +19,17 @@ FLAVORS = {"molecule.js": L.FLAVOR_MOLECULE_JS, "molecule": L.FLAVOR_MOLECULE_JS
 PRECISIONS = {"mixed": L.PREC_MIXED, "fp32": L.PREC_MIXED, "fp64": L.PREC_FP64}
 
 
+ATOM_FIELDS = tuple(f for f, _ in L.Atom._fields_)  # the columns of an atom table
+
+
 def make_atoms(rows: Iterable[dict], default_k: Optional[float] = None):
-    """Reference atom dicts ({i, j, k, Z, rc, Z_nuc, initZeff, initRcut}) -> ctypes array."""
+    """Reference atom dicts ({i, j, k, Z, rc, Z_nuc, initZeff, initRcut}) -> ctypes array.  A float64 array with
+    the columns ATOM_FIELDS is taken as it is (copied): dicts of 13000 entries take 25 ms to build and read."""
+    if isinstance(rows, np.ndarray) and rows.dtype == np.float64:
+        tab = np.ascontiguousarray(rows)
+        if tab.ndim != 2 or tab.shape[1] != len(ATOM_FIELDS):
+            raise ValueError(f"an atom table has the columns {ATOM_FIELDS}")
+        return (L.Atom * len(tab)).from_buffer_copy(tab)
     rows = list(rows)
     arr = (L.Atom * len(rows))()
     for n, a in enumerate(rows):

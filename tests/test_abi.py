@@ -81,3 +81,26 @@ def test_no_device_is_an_error_not_a_fallback():
     with pytest.raises(_lib.RqError) as e:
         Context(16, 4.0, [{"i": 8, "j": 8, "k": 8, "Z": 1}])
     assert e.value.status == _lib.RQ_ENODEV
+
+
+def test_atom_table_equals_dict_rows():
+    import numpy as np
+    from realmolecule_b200.autograd import EnergyModel
+    from realmolecule_b200.context import ATOM_FIELDS, make_atoms
+    rng = np.random.default_rng(4)
+    model = EnergyModel.__new__(EnergyModel)
+    for n_nuc, n_seed in ((1, 0), (3, 7), (0, 2)):
+        model.h, model.n_nuc = 0.2, n_nuc
+        model.charges, model.seeds = rng.integers(1, 9, n_nuc).astype(np.float64), rng.uniform(0, 30, (n_seed, 3))
+        pos = rng.uniform(0, 30, (n_nuc, 3))
+        rows = [{"i": p[0] / 0.2, "j": p[1] / 0.2, "k": p[2] / 0.2, "Z": 0.0, "Z_nuc": float(z)}
+                for p, z in zip(pos, model.charges)]
+        rows += [{"i": s[0] / 0.2, "j": s[1] / 0.2, "k": s[2] / 0.2, "Z": 1.0, "Z_nuc": 0.0} for s in model.seeds]
+        assert bytes(make_atoms(model._rows(pos))) == bytes(make_atoms(rows))
+    assert len(make_atoms(np.array([{"i": 1, "j": 2, "k": 3, "Z": 1}], dtype=object))) == 1  # dicts in an array
+    try:
+        make_atoms(np.zeros((2, len(ATOM_FIELDS) - 1)))
+    except ValueError:
+        pass
+    else:
+        raise AssertionError("a table without all columns was taken")
