@@ -24,7 +24,7 @@ ATOM_FIELDS = tuple(f for f, _ in L.Atom._fields_)  # the columns of an atom tab
 
 def make_atoms(rows: Iterable[dict], default_k: Optional[float] = None):
     """Reference atom dicts ({i, j, k, Z, rc, Z_nuc, initZeff, initRcut}) -> ctypes array.  A float64 array with
-    the columns ATOM_FIELDS is taken as it is (copied): dicts of 13000 entries take 25 ms to build and read."""
+    the columns ATOM_FIELDS is taken as it is (copied): dicts of 13000 entries take 32 ms to read, the table 0.8 ms."""
     if isinstance(rows, np.ndarray) and rows.dtype == np.float64:
         tab = np.ascontiguousarray(rows)
         if tab.ndim != 2 or tab.shape[1] != len(ATOM_FIELDS):
