@@ -151,16 +151,39 @@ __global__ void k_adj_norm_coef(const double* __restrict__ scale, const double* 
   coef[2 * d + 1] = Z > 0.0 ? c * h3 * dots[d] / Z : 0.0;
 }
 
-// update^T on 16-byte groups: out = A(K, P) in.  With NORM the input is first normalised (transposed):
-// in <- c in - beta psi_s with the domain's (c, beta), rounded to T; the same-label neighbours share the
-// centre's, so the pass needs psi_s where it needs `in`, and the normalised input goes to `inn` for the
-// accumulation below.
-template <typename T, bool NORM, int ROW>
-__global__ void __launch_bounds__(256) k_adj_update(const T* __restrict__ in, T* __restrict__ inn, T* __restrict__ out,
+// the transposed normalisation lam <- c lam - beta psi_s with the domain's (c, beta), rounded to T, in place.  A
+// pass of its own: folded into the update below it was redone for six neighbours per point and doubled the
+// update's vectors (114 us on 192^3 for 24 + 30 us).
+template <typename T>
+__global__ void __launch_bounds__(256) k_adj_apply(T* __restrict__ lam, const T* __restrict__ psi_s,
+                                                   const int* __restrict__ label, const double* __restrict__ coef,
+                                                   long long S3, int nDom) {
+  constexpr int W = Vec<T>::W;
+  const long long a = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * W;
+  auto value = [&](T x, T p, int l) {
+    return l >= 0 && l < nDom ? (T)(coef[2 * l] * (double)x - coef[2 * l + 1] * (double)p) : x;
+  };
+  if (a + W <= S3) {
+    Quad<T> x = *reinterpret_cast<const Quad<T>*>(lam + a);
+    const Quad<T> p = ldq<T>(psi_s + a);
+    int l[W];
+    VGroup r;
+    r.a = a;
+    vlabels<T>(label, r, l);
+#pragma unroll
+    for (int e = 0; e < W; ++e) x.v[e] = value(x.v[e], p.v[e], l[e]);
+    stq(lam + a, x);
+  } else {
+    for (long long id = a; id < S3; ++id) lam[id] = value(lam[id], psi_s[id], label[id]);
+  }
+}
+
+// update^T on 16-byte groups: out = A(K, P) in
+template <typename T, int ROW>
+__global__ void __launch_bounds__(256) k_adj_update(const T* __restrict__ in, T* __restrict__ out,
                                                     const T* __restrict__ K, const T* __restrict__ P,
-                                                    const unsigned char* __restrict__ mask, const int* __restrict__ label,
-                                                    const T* __restrict__ psi_s, const double* __restrict__ coef, Geo g,
-                                                    double half_dv, double dt, int nDom, int planes) {
+                                                    const unsigned char* __restrict__ mask, Geo g, double half_dv,
+                                                    double dt, int planes) {
   constexpr int W = Vec<T>::W;
   const int i0 = 1 + (int)blockIdx.y * planes, iend = min(i0 + planes, g.NN);
   for (int i = i0; i < iend; ++i) {
@@ -168,37 +191,20 @@ __global__ void __launch_bounds__(256) k_adj_update(const T* __restrict__ in, T*
     const VLoad<T, ROW> l(in, r, g);
     const Quad<T> kq = ldq<T>(K + r.a), pq = ldq<T>(P + r.a);
     const unsigned mw = vbytes<T>(mask, r);
-    Quad<T> o, n;
-    auto point = [&](int e, const Star<T>& u, auto val) {  // val(neighbour element) -> its (normalised) value
+    const Star<T> u = vstar(l);
+    Quad<T> o;
+#pragma unroll
+    for (int e = 0; e < W; ++e) {
       const unsigned m = mw >> (8 * e);
-      const double lc = val(u.c.v[e], 0);
+      const double lc = (double)u.c.v[e];
       double lap = 0.0;
-      if (m & kNmIp) lap += val(u.ip.v[e], 1) - lc;
-      if (m & kNmIm) lap += val(u.im.v[e], 2) - lc;
-      if (m & kNmJp) lap += val(u.jp.v[e], 3) - lc;
-      if (m & kNmJm) lap += val(u.jm.v[e], 4) - lc;
-      if (m & kNmKp) lap += val(u.kp.v[e], 5) - lc;
-      if (m & kNmKm) lap += val(u.km.v[e], 6) - lc;
+      if (m & kNmIp) lap += (double)u.ip.v[e] - lc;
+      if (m & kNmIm) lap += (double)u.im.v[e] - lc;
+      if (m & kNmJp) lap += (double)u.jp.v[e] - lc;
+      if (m & kNmJm) lap += (double)u.jm.v[e] - lc;
+      if (m & kNmKp) lap += (double)u.kp.v[e] - lc;
+      if (m & kNmKm) lap += (double)u.km.v[e] - lc;
       o.v[e] = (m & kNmIn) ? (T)(lc + half_dv * lap + dt * ((double)kq.v[e] - 2.0 * (double)pq.v[e]) * lc) : T(0);
-      n.v[e] = (T)lc;
-    };
-    if constexpr (NORM) {
-      const VLoad<T, ROW> lp(psi_s, r, g);
-      int lab[W];
-      vlabels<T>(label, r, lab);
-      const Star<T> u = vstar(l), s = vstar(lp);
-#pragma unroll
-      for (int e = 0; e < W; ++e) {
-        const bool ok = lab[e] >= 0 && lab[e] < nDom;
-        const double c = ok ? coef[2 * lab[e]] : 1.0, b = ok ? coef[2 * lab[e] + 1] : 0.0;
-        const T sv[7] = {s.c.v[e], s.ip.v[e], s.im.v[e], s.jp.v[e], s.jm.v[e], s.kp.v[e], s.km.v[e]};
-        point(e, u, [&](T x, int q) { return ok ? (double)(T)(c * (double)x - b * (double)sv[q]) : (double)x; });
-      }
-      if (r.own) stq(inn + r.a, n);
-    } else {
-      const Star<T> u = vstar(l);
-#pragma unroll
-      for (int e = 0; e < W; ++e) point(e, u, [](T x, int) { return (double)x; });
     }
     if (r.own) stq(out + r.a, o);
   }
@@ -666,7 +672,7 @@ void nm_adj_record_label(rq_ctx* c) {
 namespace {
 
 // the per-domain coefficients of a transposed normalisation of lam, with the forward scales `scale` at the
-// normalised state psi (applied by the next k_adj_update)
+// normalised state psi (applied by k_adj_apply)
 template <typename T>
 int adj_norm(rq_ctx* c, const T* psi, const T* lam, const double* scale) {
   rq_adj& A = c->adj;
@@ -846,14 +852,14 @@ int adjoint_t(rq_ctx* c, double* F, double* dEdv) {
   T* muP[2] = {(T*)A.muP[0], (T*)A.muP[1]};
   T* lam = (T*)A.lam[0];
   AdjPend pend{};
-  // a lambda buffer that neither the sweep nor a pending sum holds, other than `also`
-  auto spare = [&](const T* also) -> T* {
+  // a lambda buffer that neither the sweep nor a pending sum holds
+  auto spare = [&]() -> T* {
     for (void* p : A.lam) {
-      bool held = p == lam || p == also;
+      bool held = p == lam;
       for (int q = 0; q < pend.n; ++q) held = held || p == pend.lam[q];
       if (!held) return (T*)p;
     }
-    return nullptr;  // not reached: kAdjPend pending, the input and two outputs are A.lam's size
+    return nullptr;  // not reached: fewer than kAdjPend are pending, and A.lam holds one more
   };
   auto accumulate = [&]() -> int {
     if (!pend.n) return RQ_OK;
@@ -871,26 +877,20 @@ int adjoint_t(rq_ctx* c, double* F, double* dEdv) {
     const rq_adj::Rec& R = A.rec[r];
     const T* psi_prev = slot<T>(A.psi, R.psi_slot, S3);
     const T* P_s = slot<T>(A.psum, R.p_slot, S3);
-    T* out = spare(nullptr);
+    T* out = spare();
     if (R.norm) {
       const T* psi_s = r + 1 < (int)A.rec.size() ? slot<T>(A.psi, A.rec[r + 1].psi_slot, S3) : psi;
       if ((rc = adj_norm<T>(c, psi_s, lam, A.scales + (size_t)R.psi_slot * n)) != RQ_OK) return rc;
-      T* inn = spare(out);
-      LAUNCH(RQ_KC_FORCES, (6.0 * sizeof(T) + 5.0) * ni,
-             (with_row(g, [&](auto row) {
-        k_adj_update<T, true, decltype(row)::value><<<vgrid<T>(g, planes), 256, 0, c->st>>>(
-            lam, inn, out, K, P_s, c->nbm, lab, psi_s, A.coef, g, c->half_dv, c->dt, n, planes);
-              }),
-              cudaGetLastError()));
-      lam = inn;
-    } else {
-      LAUNCH(RQ_KC_FORCES, (4.0 * sizeof(T) + 1.0) * ni,
-             (with_row(g, [&](auto row) {
-        k_adj_update<T, false, decltype(row)::value><<<vgrid<T>(g, planes), 256, 0, c->st>>>(
-            lam, nullptr, out, K, P_s, c->nbm, lab, nullptr, nullptr, g, c->half_dv, c->dt, n, planes);
-              }),
+      LAUNCH(RQ_KC_FORCES, (3.0 * sizeof(T) + 4.0) * S3,
+             (k_adj_apply<T><<<nblk(S3, 256 * Vec<T>::W), 256, 0, c->st>>>(lam, psi_s, lab, A.coef, S3, n),
               cudaGetLastError()));
     }
+    LAUNCH(RQ_KC_FORCES, (4.0 * sizeof(T) + 1.0) * ni,
+           (with_row(g, [&](auto row) {
+      k_adj_update<T, decltype(row)::value><<<vgrid<T>(g, planes), 256, 0, c->st>>>(lam, out, K, P_s, c->nbm, g, c->half_dv,
+                                                                                    c->dt, planes);
+            }),
+            cudaGetLastError()));
     pend.lam[pend.n] = lam;
     pend.psi[pend.n++] = psi_prev;
     lam = out;

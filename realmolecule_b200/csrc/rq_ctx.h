@@ -34,7 +34,7 @@ struct rq_adj {
   int next_p = 0, cur_p = -1;
   // reverse-sweep buffers (allocated with the window)
   // adjoint of psi (T, S^3): the sweep's, and those of up to four steps whose sums into dE/dK are pending
-  void* lam[6] = {};
+  void* lam[5] = {};
   void* muP[2] = {nullptr, nullptr};  // adjoint of the fine P (T, S^3; ping-pong through smoothing)
   void* muf = nullptr;                // adjoint of the fine right-hand side (T, S^3)
   double* gK = nullptr;               // dE/dK accumulated (S^3 doubles); dE/dv for the external potential
