@@ -20,7 +20,7 @@ period with the flush before EVERY solver step (every kernel reads HBM cold).
            from pinned host memory, run one period (CUDA-graph replay), read the energies
            back -- copies inside the timed region;
 ``roofline`` the dominant kernel (k_step_sp: the ITP update and one Jacobi sweep in one pass,
-           24 algorithmic B per interior point) against the measured HBM copy bandwidth;
+           21 algorithmic B per interior point) against the measured HBM copy bandwidth;
 ``cpu_baseline`` the reference's own cloud/solver.py kernels compiled for the host
            (oracle/_ref, OpenMP over all host cores) on a bounded sample of the same workload.
 
