@@ -128,7 +128,7 @@ constexpr int kMfTK = 32, kMfTJ = 8;
 // the cell unless this electron holds it (then the second largest): both are exact selections, equal to
 // the shader's sequential scan.  The unfused f32 arithmetic (about 120 operations per cell and electron) issues
 // beside 15 vector loads per four cells; with a cell per thread its 21 scalar loads and their addresses took the
-// issue slots twice over.  CH4 at 200^3: 600 us before, XX us now (24 B per cell and electron: 140 us).
+// issue slots twice over.  CH4 at 200^3: 600 us before, 357 us now (24 B per cell and electron: 150 us).
 __device__ __noinline__ float mf_shell_front(const MfParams* __restrict__ p, int m, int i, int j, int k, float nw) {
   const float h = p->h;
   const float4 at = p->atoms[m];

@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(256) k_mj_apply_scale(float* __restrict__ U, c
 // (they do not depend on one another): slot d % nd of Pin / Pout holds domain doms.m[d].  Blocks of the same
 // cells are neighbours in the grid, so psi and the labels come from memory once for all domains.  LAST:
 // copyPotherForLabel (:651-671) on the way out.  10 sweeps of water's 3 domains at 64^3, with the density and
-// the copy: 387 us as 36 launches of 64 to 1073 blocks, 41 us as 10.
+// the copy: 387 us as 36 launches of 64 to 1073 blocks, 64 us as 10 (each timed alone).
 constexpr int kMjRhoPsi = 0, kMjRhoBuf = 1, kMjRhoOther = 2;
 constexpr int kMjDoms = 8;  // domains of a launch
 struct MjDoms {
