@@ -120,15 +120,9 @@ __device__ bool mf_in_sector(const MfParams* __restrict__ p, int m, float x, flo
 }
 
 constexpr int kMfTK = 32, kMfTJ = 8;
+constexpr int kMfVecBlocks = 400;  // see mf_launch_update
 
 
-// updateWGSL (mol_fast.js:134-351).  A thread owns a 16-byte vector of four cells (vec_stencil.cuh) and walks
-// the electrons: the cross-electron terms (sum_q P_q, the competitor max) come from one read of each
-// electron's U and P at the cells.  The competitor max over the other electrons is the largest U of
-// the cell unless this electron holds it (then the second largest): both are exact selections, equal to
-// the shader's sequential scan.  The unfused f32 arithmetic (about 120 operations per cell and electron) issues
-// beside 15 vector loads per four cells; with a cell per thread its 21 scalar loads and their addresses took the
-// issue slots twice over.  CH4 at 200^3: 600 us before, 357 us now (24 B per cell and electron: 150 us).
 __device__ __noinline__ float mf_shell_front(const MfParams* __restrict__ p, int m, int i, int j, int k, float nw) {
   const float h = p->h;
   const float4 at = p->atoms[m];
@@ -142,6 +136,108 @@ __device__ __noinline__ float mf_shell_front(const MfParams* __restrict__ p, int
   return nw;
 }
 
+// the rc cusp cap of a nucleus on a cell's front (mol_fast.js:249-262); dx2 = (i - at.x)^2
+__device__ __forceinline__ float mf_cap(float cap, float4 at, float rc_a, float lim, float dx2, int j, int k, float h) {
+  const float dy = F_SUB((float)j, at.y), dz = F_SUB((float)k, at.z);
+  const float d2 = F_ADD(F_ADD(dx2, F_MUL(dy, dy)), F_MUL(dz, dz));
+  if (!(d2 <= lim)) return cap;
+  const float r = F_MUL(F_SQRT(d2), h);
+  return r < rc_a ? fminf(cap, mf_cusp(r, rc_a, h)) : cap;
+}
+
+// updateWGSL (mol_fast.js:134-351) of electron m on one cell: w, u and P at the cell and its neighbours, the competitor
+// umax, the potential pot, the cap of the front.  New front, amplitude and P.
+struct MfStar {
+  float c, ip, im, jp, jm, kp, km;
+};
+template <bool SHELL>
+__device__ __forceinline__ void mf_update_cell(const MfParams* __restrict__ p, int m, int i, int j, int k, const MfStar& w,
+                                               const MfStar& u, const MfStar& q, float umax, float pot, float cap,
+                                               float hd, float& ow, float& ou, float& op) {
+  const float dt = p->dt, inv_h = p->inv_h, inv_h2 = p->inv_h2;
+  const float dt005 = F_MUL(0.05f, dt), dt1 = F_MUL(1.0f, dt), two_pi_dt = F_MUL(p->two_pi, dt);
+  const float uc = u.c, wc = w.c, Pc = q.c;
+  const float cm = F_SUB(uc, umax);
+  const float lap_w =
+      F_MUL(F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(w.ip, w.im), w.jp), w.jm), w.kp), w.km), F_MUL(6.0f, wc)), inv_h2);
+  const float gx = F_MUL(F_SUB(w.ip, w.im), inv_h), gy = F_MUL(F_SUB(w.jp, w.jm), inv_h),
+              gz = F_MUL(F_SUB(w.kp, w.km), inv_h);
+  float nw = F_ADD(F_ADD(wc, F_MUL(F_MUL(dt005, fabsf(cm)), lap_w)),
+                   F_MUL(F_MUL(dt1, cm), sqrt0(F_ADD(F_ADD(F_MUL(gx, gx), F_MUL(gy, gy)), F_MUL(gz, gz)))));
+  nw = fminf(fmaxf(nw, 0.0f), 1.0f);
+  if (SHELL)
+    nw = mf_shell_front(p, m, i, j, k, nw);
+  else
+    nw = fminf(nw, cap);  // the shader takes a cap of at most 1 only; nw is at most 1
+  ow = nw;
+  const float fx = F_SUB(F_MUL(F_MUL(F_SUB(u.ip, uc), F_ADD(w.ip, nw)), 0.5f),
+                         F_MUL(F_MUL(F_SUB(uc, u.im), F_ADD(nw, w.im)), 0.5f));
+  const float fy = F_SUB(F_MUL(F_MUL(F_SUB(u.jp, uc), F_ADD(w.jp, nw)), 0.5f),
+                         F_MUL(F_MUL(F_SUB(uc, u.jm), F_ADD(nw, w.jm)), 0.5f));
+  const float fz = F_SUB(F_MUL(F_MUL(F_SUB(u.kp, uc), F_ADD(w.kp, nw)), 0.5f),
+                         F_MUL(F_MUL(F_SUB(uc, u.km), F_ADD(nw, w.km)), 0.5f));
+  ou = F_ADD(F_ADD(F_ADD(F_ADD(uc, F_MUL(hd, fx)), F_MUL(hd, fy)), F_MUL(hd, fz)),
+             F_MUL(F_MUL(F_MUL(dt, pot), uc), wc));
+  const float lap = F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(q.ip, q.im), q.jp), q.jm), q.kp), q.km), F_MUL(6.0f, Pc));
+  op = F_ADD(F_ADD(Pc, F_MUL(F_MUL(dt, lap), inv_h2)), F_MUL(F_MUL(two_pi_dt, uc), uc));
+}
+
+// The potential of W cells: K - Vother, then the terms whose coefficients are not 0.  The shader subtracts every
+// term; one whose coefficient is 0 is +-0 and changes nothing, since the difference so far is never -0 (K is a
+// sum that starts at +0).  pot holds the group sum of P on entry (without split siblings the electron's own P).
+template <int W, class Pq, class Uq>
+__device__ __forceinline__ void mf_potential(const MfParams* __restrict__ p, int m, int i, const int (&jj)[W],
+                                             const float (&K)[W], const float (&Ptot)[W], const float (&uc)[W],
+                                             float (&pot)[W], Pq load_P, Uq load_U) {
+  const int n = p->n;
+  const float4 cu = p->upd[m];
+  const float tilt_y = p->rcs[m].w, beta = p->beta;
+  const unsigned gm = p->gmask[m];
+  if (gm != (1u << m)) {
+#pragma unroll
+    for (int e = 0; e < W; ++e) pot[e] = 0.0f;
+    for (int q = 0; q < n; ++q)
+      if ((gm >> q) & 1u) {
+        float x[W];
+        load_P(q, x);
+#pragma unroll
+        for (int e = 0; e < W; ++e) pot[e] = F_ADD(pot[e], x[e]);
+      }
+  }
+#pragma unroll
+  for (int e = 0; e < W; ++e) pot[e] = F_SUB(K[e], F_MUL(2.0f, F_SUB(Ptot[e], F_MUL(cu.x, pot[e]))));
+  if (cu.z != 0.0f) {
+#pragma unroll
+    for (int e = 0; e < W; ++e)
+      pot[e] = F_SUB(pot[e], F_MUL(p->alpha_tf, mf_pow(fmaxf(F_MUL(uc[e], uc[e]), 1e-20f), 0.6666667f)));
+  }
+  if (beta != 0.0f || p->field_x != 0.0f || cu.w != 0.0f || tilt_y != 0.0f) {
+    float rho_other[W] = {};
+    for (int q = 0; beta != 0.0f && q < n; ++q)
+      if (q != m) {
+        float x[W];
+        load_U(q, x);
+#pragma unroll
+        for (int e = 0; e < W; ++e) rho_other[e] = F_ADD(rho_other[e], F_MUL(x[e], x[e]));
+      }
+    const float x_au = F_MUL(F_SUB((float)i, (float)p->N2), p->h);
+#pragma unroll
+    for (int e = 0; e < W; ++e) {
+      const float y_au = F_MUL(F_SUB((float)jj[e], (float)p->N2), p->h);
+      const float V_tilt = F_SUB(F_MUL(-cu.w, x_au), F_MUL(tilt_y, y_au));
+      pot[e] = F_SUB(F_SUB(F_SUB(pot[e], V_tilt), beta != 0.0f ? F_MUL(beta, rho_other[e]) : 0.0f),
+                     F_MUL(p->field_x, x_au));
+    }
+  }
+}
+
+// The update on 16-byte vectors of four cells (vec_stencil.cuh), walking the electrons: the cross-electron terms
+// (sum_q P_q, the competitor max) come from one read of each electron's U and P at the cells.  The competitor
+// max over the other electrons is the largest U of the cell unless this electron holds it (then the second
+// largest): both are exact selections, equal to the shader's sequential scan.  The unfused f32 arithmetic (about 120
+// operations per cell and electron) issues beside 15 vector loads per four cells; with a cell per thread and a
+// walk its 21 scalar loads and their addresses took the issue slots twice over.  CH4 at 200^3: 600 us before,
+// 357 us now (24 B per cell and electron: 150 us).
 template <int ROW, bool SHELL>
 __global__ void __launch_bounds__(256, 2) k_mf_update(const MfParams* __restrict__ p, Geo g,
                                                       const float* __restrict__ Ui, const float* __restrict__ Wi,
@@ -182,10 +278,8 @@ __global__ void __launch_bounds__(256, 2) k_mf_update(const MfParams* __restrict
       else if (u > max2[e]) max2[e] = u;
     }
   }
-  const float h = p->h, dt = p->dt, inv_h = p->inv_h, inv_h2 = p->inv_h2;
-  // frozen-core mode: the rc cusps of all nuclei act on every electron's front; min is exact,
-  // so the cap over the nuclei is taken once per cell (mol_fast.js:249-262), and only nuclei whose sphere
-  // reaches the cell's plane and row are looked at
+  // frozen-core mode: the rc cusps of all nuclei act on every electron's front; min is exact, so the cap over the nuclei
+  // is taken once per cell, and only nuclei whose sphere reaches the plane are looked at
   float cap[4] = {2.0f, 2.0f, 2.0f, 2.0f};
   if (!SHELL && p->any_rc) {
     for (int a = 0; a < n; ++a) {
@@ -193,100 +287,36 @@ __global__ void __launch_bounds__(256, 2) k_mf_update(const MfParams* __restrict
       const float4 at = p->atoms[a];
       const float dx = F_SUB((float)i, at.x), dx2 = F_MUL(dx, dx);
       if (!(dx2 <= lim)) continue;
-      const float rc_a = p->rcs[a].x;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float dy = F_SUB((float)jj[e], at.y), dz = F_SUB((float)kk[e], at.z);
-        const float d2 = F_ADD(F_ADD(dx2, F_MUL(dy, dy)), F_MUL(dz, dz));
-        if (!(d2 <= lim)) continue;
-        const float rr = F_MUL(F_SQRT(d2), h);
-        if (rr < rc_a) cap[e] = fminf(cap[e], mf_cusp(rr, rc_a, h));
-      }
+      for (int e = 0; e < 4; ++e) cap[e] = mf_cap(cap[e], at, p->rcs[a].x, lim, dx2, jj[e], kk[e], p->h);
     }
   }
   const Quad<float> K4 = ldq(K + r.a);
-  const float beta = p->beta, two_pi_dt = F_MUL(p->two_pi, dt);
-  const float dt005 = F_MUL(0.05f, dt), dt1 = F_MUL(1.0f, dt);
-  const bool field = beta != 0.0f || p->field_x != 0.0f;
 #pragma unroll 1
   for (int m = 0; m < n; ++m) {
     const long long off = m * slot;
     const VLoad<float, ROW> lw(Wi + off, r, g), lu(Ui + off, r, g), lp(Pi + off, r, g);
-    const float4 cu = p->upd[m];
-    const float tilt_y = p->rcs[m].w;
-    const unsigned gm = p->gmask[m];
     float pot[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) pot[e] = lp.c.v[e];  // the group sum: without split siblings this electron's own P
-    if (gm != (1u << m)) {
+    for (int e = 0; e < 4; ++e) pot[e] = lp.c.v[e];
+    auto quad = [&](const float* f, float (&x)[4]) {
+      const Quad<float> v = ldq(f + r.a);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) pot[e] = 0.0f;
-      for (int q = 0; q < n; ++q)
-        if ((gm >> q) & 1u) {
-          const Quad<float> pq = ldq(Pi + q * slot + r.a);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) pot[e] = F_ADD(pot[e], pq.v[e]);
-        }
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) pot[e] = F_SUB(K4.v[e], F_MUL(2.0f, F_SUB(Ptot[e], F_MUL(cu.x, pot[e]))));
-    // The shader subtracts every further term; one whose coefficient is 0 is +-0 and changes nothing, since the
-    // difference so far is never -0 (K is a sum that starts at +0).
-    if (cu.z != 0.0f) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        pot[e] = F_SUB(pot[e], F_MUL(p->alpha_tf, mf_pow(fmaxf(F_MUL(lu.c.v[e], lu.c.v[e]), 1e-20f), 0.6666667f)));
-    }
-    if (field || cu.w != 0.0f || tilt_y != 0.0f) {
-      float rho_other[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      for (int q = 0; beta != 0.0f && q < n; ++q)
-        if (q != m) {
-          const Quad<float> uq = ldq(Ui + q * slot + r.a);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) rho_other[e] = F_ADD(rho_other[e], F_MUL(uq.v[e], uq.v[e]));
-        }
-      const float x_au = F_MUL(F_SUB((float)i, (float)p->N2), h);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float y_au = F_MUL(F_SUB((float)jj[e], (float)p->N2), h);
-        const float V_tilt = F_SUB(F_MUL(-cu.w, x_au), F_MUL(tilt_y, y_au));
-        pot[e] = F_SUB(F_SUB(F_SUB(pot[e], V_tilt), beta != 0.0f ? F_MUL(beta, rho_other[e]) : 0.0f),
-                       F_MUL(p->field_x, x_au));
-      }
-    }
+      for (int e = 0; e < 4; ++e) x[e] = v.v[e];
+    };
+    mf_potential<4>(p, m, i, jj, K4.v, Ptot, lu.c.v, pot, [&](int q, float (&x)[4]) { quad(Pi + q * slot, x); },
+                    [&](int q, float (&x)[4]) { quad(Ui + q * slot, x); });
     const Star<float> w = vstar(lw), u = vstar(lu), q = vstar(lp);
     Quad<float> ow, ou, op;
-    const float hd = cu.y;
+    const float hd = p->upd[m].y;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float uc = u.c.v[e], wc = w.c.v[e], Pc = q.c.v[e];
-      const float wip = w.ip.v[e], wim = w.im.v[e], wjp = w.jp.v[e], wjm = w.jm.v[e], wkp = w.kp.v[e], wkm = w.km.v[e];
-      const float cm = F_SUB(uc, m == arg1[e] ? max2[e] : max1[e]);
-      const float lap_w =
-          F_MUL(F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(wip, wim), wjp), wjm), wkp), wkm), F_MUL(6.0f, wc)), inv_h2);
-      const float gx = F_MUL(F_SUB(wip, wim), inv_h), gy = F_MUL(F_SUB(wjp, wjm), inv_h),
-                  gz = F_MUL(F_SUB(wkp, wkm), inv_h);
-      float nw = F_ADD(F_ADD(wc, F_MUL(F_MUL(dt005, fabsf(cm)), lap_w)),
-                       F_MUL(F_MUL(dt1, cm), sqrt0(F_ADD(F_ADD(F_MUL(gx, gx), F_MUL(gy, gy)), F_MUL(gz, gz)))));
-      nw = fminf(fmaxf(nw, 0.0f), 1.0f);
-      if (SHELL)
-        nw = mf_shell_front(p, m, i, jj[e], kk[e], nw);
-      else
-        nw = fminf(nw, cap[e]);  // the shader takes a cap of at most 1 only; nw is at most 1
-      ow.v[e] = nw;
-      const float fx = F_SUB(F_MUL(F_MUL(F_SUB(u.ip.v[e], uc), F_ADD(wip, nw)), 0.5f),
-                             F_MUL(F_MUL(F_SUB(uc, u.im.v[e]), F_ADD(nw, wim)), 0.5f));
-      const float fy = F_SUB(F_MUL(F_MUL(F_SUB(u.jp.v[e], uc), F_ADD(wjp, nw)), 0.5f),
-                             F_MUL(F_MUL(F_SUB(uc, u.jm.v[e]), F_ADD(nw, wjm)), 0.5f));
-      const float fz = F_SUB(F_MUL(F_MUL(F_SUB(u.kp.v[e], uc), F_ADD(wkp, nw)), 0.5f),
-                             F_MUL(F_MUL(F_SUB(uc, u.km.v[e]), F_ADD(nw, wkm)), 0.5f));
-      ou.v[e] = F_ADD(F_ADD(F_ADD(F_ADD(uc, F_MUL(hd, fx)), F_MUL(hd, fy)), F_MUL(hd, fz)),
-                      F_MUL(F_MUL(F_MUL(dt, pot[e]), uc), wc));
-      const float lap = F_SUB(F_ADD(F_ADD(F_ADD(F_ADD(F_ADD(q.ip.v[e], q.im.v[e]), q.jp.v[e]), q.jm.v[e]), q.kp.v[e]),
-                                    q.km.v[e]),
-                              F_MUL(6.0f, Pc));
-      op.v[e] = F_ADD(F_ADD(Pc, F_MUL(F_MUL(dt, lap), inv_h2)), F_MUL(F_MUL(two_pi_dt, uc), uc));
-    }
+    for (int e = 0; e < 4; ++e)
+      mf_update_cell<SHELL>(
+          p, m, i, jj[e], kk[e],
+          MfStar{w.c.v[e], w.ip.v[e], w.im.v[e], w.jp.v[e], w.jm.v[e], w.kp.v[e], w.km.v[e]},
+          MfStar{u.c.v[e], u.ip.v[e], u.im.v[e], u.jp.v[e], u.jm.v[e], u.kp.v[e], u.km.v[e]},
+          MfStar{q.c.v[e], q.ip.v[e], q.im.v[e], q.jp.v[e], q.jm.v[e], q.kp.v[e], q.km.v[e]},
+          m == arg1[e] ? max2[e] : max1[e], pot[e], cap[e], hd, ow.v[e], ou.v[e], op.v[e]);
     if (in == 15u) {
       stq(Wo + off + r.a, ow);
       stq(Uo + off + r.a, ou);
@@ -296,6 +326,54 @@ __global__ void __launch_bounds__(256, 2) k_mf_update(const MfParams* __restrict
       vstore(Uo + off, r, in, ou);
       vstore(Po + off, r, in, op);
     }
+  }
+}
+
+// The update with a cell per thread, on small grids, where the vectors' four cells are a chain with too little
+// beside it.
+template <bool SHELL>
+__global__ void __launch_bounds__(256, 4) k_mf_update_cell(const MfParams* __restrict__ p, const float* __restrict__ Ui,
+                                                           const float* __restrict__ Wi, const float* __restrict__ Pi,
+                                                           const float* __restrict__ K, float* __restrict__ Uo,
+                                                           float* __restrict__ Wo, float* __restrict__ Po) {
+  const int NN = p->NN, n = p->n, S = p->S, S2 = S * S;
+  const int i = blockIdx.z + 1;
+  const int k = blockIdx.x * kMfTK + threadIdx.x + 1, j = blockIdx.y * kMfTJ + threadIdx.y + 1;
+  if (k >= NN || j >= NN) return;
+  const int id = i * S2 + j * S + k;
+  const long long slot = mf_slot((long long)S2 * S);
+  const float Kc[1] = {__ldg(K + id)};
+  float Ptot[1] = {0.0f}, max1 = 0.0f, max2 = 0.0f;
+  int arg1 = -1;
+#pragma unroll 4
+  for (int e = 0; e < n; ++e) {
+    Ptot[0] = F_ADD(Ptot[0], __ldg(Pi + e * slot + id));
+    const float v = __ldg(Ui + e * slot + id);
+    if (v > max1) { max2 = max1; max1 = v; arg1 = e; }
+    else if (v > max2) max2 = v;
+  }
+  float cap = 2.0f;
+  if (!SHELL && p->any_rc)
+    for (int a = 0; a < n; ++a) {
+      const float lim = p->rc_d2[a];
+      const float4 at = p->atoms[a];
+      const float dx = F_SUB((float)i, at.x), dx2 = F_MUL(dx, dx);
+      if (dx2 <= lim) cap = mf_cap(cap, at, p->rcs[a].x, lim, dx2, j, k, p->h);
+    }
+  const int jj[1] = {j};
+#pragma unroll 1
+  for (int m = 0; m < n; ++m) {
+    const long long off = m * slot + id;
+    auto star = [&](const float* f) {
+      return MfStar{__ldg(f), __ldg(f + S2), __ldg(f - S2), __ldg(f + S), __ldg(f - S), __ldg(f + 1), __ldg(f - 1)};
+    };
+    const MfStar w = star(Wi + off), u = star(Ui + off), q = star(Pi + off);
+    const float uc[1] = {u.c};
+    float pot[1] = {q.c};
+    mf_potential<1>(p, m, i, jj, Kc, Ptot, uc, pot, [&](int e, float (&x)[1]) { x[0] = __ldg(Pi + e * slot + id); },
+                    [&](int e, float (&x)[1]) { x[0] = __ldg(Ui + e * slot + id); });
+    mf_update_cell<SHELL>(p, m, i, j, k, w, u, q, m == arg1 ? max2 : max1, pot[0], cap, p->upd[m].y, Wo[off], Uo[off],
+                          Po[off]);
   }
 }
 
@@ -827,12 +905,23 @@ int mf_launch_update(rq_mf* s, int c) {
   const int nx = 1 - c;
   const Geo g = make_geo(s->S);
   const bool sh = s->cfg.shell_mode != 0;
-#define MF_UPD(ROW_, SH_)                                                                                        \
-  k_mf_update<ROW_, SH_><<<vgrid<float>(g, 1), 256, 0, s->st>>>(s->dp, g, s->U[c], s->W[c], s->P[c], s->K, s->U[nx], \
-                                                                s->W[nx], s->P[nx])
-  if (s->S % 4 == 1) { if (sh) MF_UPD(kRowP, true); else MF_UPD(kRowP, false); }
-  else { if (sh) MF_UPD(kRowM, true); else MF_UPD(kRowM, false); }
+  const dim3 grid = vgrid<float>(g, 1);
+  // Vectors from 400 blocks on, 72^3: there 50 steps with 2 / 5 electrons take 1084 / 2180 us on vectors and 1190 /
+  // 2309 with a cell per thread, at 64^3 (315 blocks, a wave and a bit) 919 / 1813 and 811 / 1535, at 32^3
+  // 523 / 921 and 430 / 712.  An electron per block instead of the walk was slower in both forms above 32^3.
+  if ((long long)grid.x * grid.y >= kMfVecBlocks) {
+#define MF_UPD(ROW_, SH_)                                                                                          \
+  k_mf_update<ROW_, SH_><<<grid, 256, 0, s->st>>>(s->dp, g, s->U[c], s->W[c], s->P[c], s->K, s->U[nx], s->W[nx], s->P[nx])
+    if (s->S % 4 == 1) { if (sh) MF_UPD(kRowP, true); else MF_UPD(kRowP, false); }
+    else { if (sh) MF_UPD(kRowM, true); else MF_UPD(kRowM, false); }
 #undef MF_UPD
+  } else {
+    const dim3 gc = mf_grid(s->NN, s->NN - 1), b(kMfTK, kMfTJ);
+    if (sh)
+      k_mf_update_cell<true><<<gc, b, 0, s->st>>>(s->dp, s->U[c], s->W[c], s->P[c], s->K, s->U[nx], s->W[nx], s->P[nx]);
+    else
+      k_mf_update_cell<false><<<gc, b, 0, s->st>>>(s->dp, s->U[c], s->W[c], s->P[c], s->K, s->U[nx], s->W[nx], s->P[nx]);
+  }
   MLAUNCH();
   return RQ_OK;
 }

@@ -124,9 +124,11 @@ def test_invalid_configs_are_errors():
         MolFast(H2["nuclei"], NN=32, vcycle_interval=0)
 
 
-# Edges of the 16-byte vectors: both pitches modulo 4, planes of less than a warp's vectors, one electron (no
-# competitor), as many as the solver takes, fields whose size is no multiple of a vector.
-@pytest.mark.parametrize("NN,n,shell", [(8, 1, False), (8, 16, False), (10, 3, True), (34, 5, False), (62, 2, True)])
+# Edges of the update's two forms, a cell per thread on small grids and 16-byte vectors from 72^3 on: both pitches modulo
+# 4, planes of less than a warp, one electron (no competitor), as many as the solver takes, fields whose
+# size is no multiple of a vector.
+@pytest.mark.parametrize("NN,n,shell", [(8, 1, False), (8, 16, False), (10, 3, True), (34, 5, False), (62, 2, True),
+                                        (70, 2, False), (72, 2, False), (74, 3, True), (76, 16, False)])
 def test_vector_edges(NN, n, shell):
     c = NN / 2
     nuc = [{"i": c + (q % 3) - 1, "j": c + (q // 3) % 3 - 1.25, "k": c + q // 9, "Z": 1 + q % 2,
