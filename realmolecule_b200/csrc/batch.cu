@@ -93,17 +93,17 @@ __global__ void __launch_bounds__(256) kb_apply_scale(const BInst* __restrict__ 
 template <typename T>
 __global__ void __launch_bounds__(256) kb_norms(const BInst* __restrict__ ins, const BItem* __restrict__ items, int cu,
                                                 int cl, double* __restrict__ norms) {
-  __shared__ NormSmem sm;
+  __shared__ NormSmem<DomTable<1, 128>> sm;
   const BItem it = items[blockIdx.x];
   const BInst& I = ins[it.inst];
-  dom_table_init(sm.tab);
+  dom_table_init(sm.sums);
   __syncthreads();
   const Geo g = I.g;
   const int i0 = 1 + it.bz * kNmNormPlanes;
-  nm_norms_body<T>((const T*)I.U[cu], I.lab[cl], g, I.h * I.h * I.h, I.nDom, norms + I.dom0, sm, it.bx, it.by, i0,
-                   min(i0 + kNmNormPlanes, g.NN));
+  nm_norms_body<T>((const T*)I.U[cu], I.lab[cl], g, I.h * I.h * I.h, I.nDom, TableSums<1>{sm.sums, norms + I.dom0},
+                   sm.list, it.bx, it.by, i0, min(i0 + kNmNormPlanes, g.NN));
   __syncthreads();
-  dom_table_flush(sm.tab, norms + I.dom0);
+  dom_table_flush(sm.sums, norms + I.dom0);
 }
 
 template <typename T, bool FINE, int COLOR>
@@ -164,16 +164,17 @@ __global__ void __launch_bounds__(1024) kb_coarsest(const BInst* __restrict__ in
 template <typename T>
 __global__ void __launch_bounds__(256) kb_energy(const BInst* __restrict__ ins, const BItem* __restrict__ items, int cu,
                                                  int cp, int cl, double* __restrict__ pd, NmTile tile) {
-  __shared__ EnergySmem sm;
+  __shared__ EnergySmem<DomTable<kNmPD, 128>> sm;
   const BItem it = items[blockIdx.x];
   const BInst& I = ins[it.inst];
-  dom_table_init(sm.tab);
+  dom_table_init(sm.sums);
   __syncthreads();
   const Geo g = I.g;
   nm_energy_body<T>((const T*)I.U[cu], (const T*)I.K, (const T*)I.P[cp], I.lab[cl], g, I.h, I.nDom,
-                    pd + kNmPD * I.dom0, sm, it.bx, it.by, it.bz, sizeof(T) == sizeof(float) ? I.K64 : nullptr, tile);
+                    TableSums<kNmPD>{sm.sums, pd + kNmPD * I.dom0}, sm.list, it.bx, it.by, it.bz,
+                    sizeof(T) == sizeof(float) ? I.K64 : nullptr, tile);
   __syncthreads();
-  dom_table_flush(sm.tab, pd + kNmPD * I.dom0);
+  dom_table_flush(sm.sums, pd + kNmPD * I.dom0);
 }
 
 template <typename T>
@@ -923,7 +924,7 @@ static int b_normalize(rq_batch* b) {
     BL("norms");
     return RQ_OK;
   }));
-  BCK(nm_norm_scale<double>(b->dnorm, b->Zdom, b->D, b->scale, b->err, b->st));
+  BCK(nm_norm_scale(b->dnorm, b->Zdom, b->D, b->scale, b->err, b->st));
   b->launches++;
   BRC(each_set([&](auto tag, int p) { return b_apply<decltype(tag)>(b, p); }));
   b->pending = false;
@@ -1010,7 +1011,7 @@ static int b_step(rq_batch* b, int s) {
     if (b->rec) {
       for (int p = 0; p < 2; ++p) b_record(b, kPhScale, p, &b->pl[p].one);
     } else {
-      BCK(nm_norm_scale<double>(b->dnorm, b->Zdom, b->D, b->scale, b->err, b->st));
+      BCK(nm_norm_scale(b->dnorm, b->Zdom, b->D, b->scale, b->err, b->st));
       b->launches++;
     }
     b->pending = true;

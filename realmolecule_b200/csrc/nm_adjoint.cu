@@ -108,10 +108,9 @@ __global__ void __launch_bounds__(256) k_adj_seed(const T* __restrict__ U, const
 template <typename T>
 __global__ void __launch_bounds__(256) k_adj_dot(const T* __restrict__ psi, const T* __restrict__ lam,
                                                  const int* __restrict__ label, Geo g, int nDom,
-                                                 double* __restrict__ dots) {
-  __shared__ NormSmem sm;
-  dom_table_init(sm.tab);
-  __syncthreads();
+                                                 long long* __restrict__ dots) {
+  __shared__ NormSmem<BlockSums<1>> sm;
+  const ExactSums<1> sums{sm.sums, dots};
   RunSumL<1, kNmNormCap> rs;
   rs.reset();
   const int tid = (int)threadIdx.x, k = 1 + (int)blockIdx.x * 32 + (tid & 31), j = 1 + (int)blockIdx.y * 8 + (tid >> 5);
@@ -133,22 +132,24 @@ __global__ void __launch_bounds__(256) k_adj_dot(const T* __restrict__ psi, cons
     for (int t = 0; t < AH; ++t) {
       const bool on = in && i + t < iend && l[t] >= 0 && l[t] < nDom;
       const double v = on ? (double)p[t] * (double)q[t] : 0.0;
-      rs.add(on ? l[t] : -1, &v, sm.list, tid, sm.tab, dots);
+      rs.add(on ? l[t] : -1, &v, sm.list, tid, sums);
     }
   }
-  rs.finish(sm.list, tid, sm.tab, dots);
-  __syncthreads();
-  dom_table_flush(sm.tab, dots);
+  rs.finish(sm.list, tid, sums);
 }
 
-// per-domain (c, beta) of a transposed normalisation: c = the forward scale, beta = c h^3 <psi, lam> / Z
-__global__ void k_adj_norm_coef(const double* __restrict__ scale, const double* __restrict__ Zdom,
-                                const double* __restrict__ dots, int nDom, double h3, double* __restrict__ coef) {
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
+// per-domain (c, beta) of a transposed normalisation: c = the forward scale, beta = c h^3 <psi, lam> / Z; a warp
+// per domain
+__global__ void __launch_bounds__(128) k_adj_norm_coef(const double* __restrict__ scale, const double* __restrict__ Zdom,
+                                                       const long long* __restrict__ dots, int nDom, double h3,
+                                                       double* __restrict__ coef) {
+  const int d = blockIdx.x * 4 + (threadIdx.x >> 5);
   if (d >= nDom) return;
+  const double dot = exact_value_warp(dots + (long long)d * kExWords);
+  if (threadIdx.x % 32 != 0) return;
   const double c = scale[d], Z = Zdom[d];
   coef[2 * d] = c;
-  coef[2 * d + 1] = Z > 0.0 ? c * h3 * dots[d] / Z : 0.0;
+  coef[2 * d + 1] = Z > 0.0 ? c * h3 * dot / Z : 0.0;
 }
 
 // the transposed normalisation lam <- c lam - beta psi_s with the domain's (c, beta), rounded to T, in place.  A
@@ -571,7 +572,7 @@ void nm_adj_free(rq_ctx* c) {
   rq_adj& A = c->adj;
   for (void* q : A.lam)
     if (q) cudaFree(q);
-  void* p[] = {A.psi, A.psum, A.scales, A.muP[0], A.muP[1], A.muf, A.gK, A.dots, A.coef, A.wq};
+  void* p[] = {A.psi, A.psum, A.scales, A.muP[0], A.muP[1], A.muf, A.gK, A.coef, A.wq};
   for (void* q : p)
     if (q) cudaFree(q);
   for (auto& L : A.lv)
@@ -603,7 +604,7 @@ int nm_adj_set_window(rq_ctx* c, int steps) {
             alloc((void**)&A.scales, sizeof(double) * (size_t)steps * n) && alloc(&A.muP[0], S3 * es) &&
             alloc(&A.muP[1], S3 * es) &&
             alloc(&A.muf, S3 * es) && alloc((void**)&A.gK, S3 * sizeof(double)) &&
-            alloc((void**)&A.dots, sizeof(double) * n) && alloc((void**)&A.coef, sizeof(double) * 2 * n) &&
+            alloc((void**)&A.coef, sizeof(double) * 2 * n) &&
             alloc((void**)&A.wq, sizeof(double) * 2 * n);
   const int levels = (int)c->mg.size();
   A.lv.assign(levels, rq_adj::Level());
@@ -677,11 +678,11 @@ template <typename T>
 int adj_norm(rq_ctx* c, const T* psi, const T* lam, const double* scale) {
   rq_adj& A = c->adj;
   const int n = c->n_atoms;
-  CK(cudaMemsetAsync(A.dots, 0, sizeof(double) * n, c->st));
+  CK(cudaMemsetAsync(c->acc, 0, sizeof(long long) * kExWords * n, c->st));
   LAUNCH(RQ_KC_FORCES, (2.0 * sizeof(T) + 4.0) * c->g.S3,
-         (k_adj_dot<T><<<nm_norms_grid(c->g), 256, 0, c->st>>>(psi, lam, c->lab[c->cl], c->g, n, A.dots), cudaGetLastError()));
-  LAUNCH(RQ_KC_FORCES, 32.0 * n,
-         (k_adj_norm_coef<<<nblk(n, 128), 128, 0, c->st>>>(scale, c->Zdom64, A.dots, n, c->h3, A.coef),
+         (k_adj_dot<T><<<nm_norms_grid(c->g), 256, 0, c->st>>>(psi, lam, c->lab[c->cl], c->g, n, c->acc), cudaGetLastError()));
+  LAUNCH(RQ_KC_FORCES, (8.0 * kExWords + 32.0) * n,
+         (k_adj_norm_coef<<<nblk(n, 4), 128, 0, c->st>>>(scale, c->Zdom64, c->acc, n, c->h3, A.coef),
           cudaGetLastError()));
   return RQ_OK;
 }
@@ -836,9 +837,8 @@ int adjoint_t(rq_ctx* c, double* F, double* dEdv) {
   const T* K = (const T*)c->K;
   const int* lab = c->lab[c->cl];
   // the readout's per-domain partials -> (Z/N, Q/N)
-  CK(cudaMemsetAsync(c->dpd, 0, sizeof(double) * kNmPD * n, c->st));
   LAUNCH(RQ_KC_ENERGY, (4.0 * sizeof(T) + 4.0) * ni,
-         nm_energy<T>(psi, K, (const T*)c->P[c->cp], lab, g, c->h, n, c->dpd, c->st, c->K64));
+         nm_energy<T>(psi, K, (const T*)c->P[c->cp], lab, g, c->h, n, c->acc, c->dpd, c->st, c->K64));
   std::vector<double> pd((size_t)kNmPD * n), wq((size_t)2 * n);
   CK(cudaMemcpyAsync(pd.data(), c->dpd, sizeof(double) * pd.size(), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));

@@ -366,17 +366,18 @@ __device__ __forceinline__ void nm_apply_scale_body(T* __restrict__ U, const int
 }
 
 constexpr int kNmNormAhead = 8, kNmNormCap = 4;
+template <class Sm>
 struct NormSmem {
-  DomTable<1, 128> tab;
+  Sm sums;  // DomTable<1, 128> or BlockSums<1>
   RunList<1, kNmNormCap> list;
 };
 // FP64 per-label psi^2 h^3 over the interior (label clipped to [0, nDom); psi is 0 on the faces): a thread
 // walks the planes [i0, iend) of one column of the 32 x 8 tile (bx, by), so it touches the block table about
 // once per domain it crosses.  A flat walk, whose points are 256 apart, touched it at every point: 2.14 ms
 // against 0.40 ms for the 96 clusters.
-template <typename T>
+template <typename T, class Sums>
 __device__ __forceinline__ void nm_norms_body(const T* __restrict__ U, const int* __restrict__ label, const Geo& g,
-                                              double h3, int nDom, double* __restrict__ norms, NormSmem& sm, int bx,
+                                              double h3, int nDom, const Sums& sums, RunList<1, kNmNormCap>& list, int bx,
                                               int by, int i0, int iend) {
   RunSumL<1, kNmNormCap> rs;
   rs.reset();
@@ -397,10 +398,10 @@ __device__ __forceinline__ void nm_norms_body(const T* __restrict__ U, const int
     for (int q = 0; q < kNmNormAhead; ++q) {
       const bool on = in && i + q < iend;
       const double r = on ? (double)u[q] * (double)u[q] * h3 : 0.0;
-      rs.add(on ? min(max(l[q], 0), nDom - 1) : -1, &r, sm.list, tid, sm.tab, norms);
+      rs.add(on ? min(max(l[q], 0), nDom - 1) : -1, &r, list, tid, sums);
     }
   }
-  rs.finish(sm.list, tid, sm.tab, norms);
+  rs.finish(list, tid, sums);
 }
 constexpr int kNmNormPlanes = 16;
 inline dim3 nm_norms_grid(const Geo& g) {
@@ -744,8 +745,9 @@ __device__ __forceinline__ void nm_coarsest_body(T* __restrict__ P, const T* __r
 }
 
 constexpr int kNmEnergyCap = 2;
+template <class Sm>
 struct EnergySmem {
-  DomTable<kNmPD, 128> tab;
+  Sm sums;  // DomTable<kNmPD, 128> or BlockSums<kNmPD>
   RunList<kNmPD, kNmEnergyCap> list;
 };
 // Per-domain readout sums, kNmPD per domain: (norm, T, V_eK, h^3 sum P rho, h^3 sum P (A P)) on the
@@ -757,10 +759,10 @@ struct EnergySmem {
 // With K64 (fp32 fields) the nuclear term reads the FP64 potential: the fields evolve with the f32
 // rounding of K, and reading the energy with the unrounded K removes that rounding from it at first
 // order (the state is stationary, so what is left is second order).
-template <typename T>
+template <typename T, class Sums>
 __device__ __forceinline__ void nm_energy_body(const T* __restrict__ U, const T* __restrict__ K, const T* __restrict__ P,
                                                const int* __restrict__ label, const Geo& g, double h, int nDom,
-                                               double* __restrict__ pd, EnergySmem& sm, int bx, int by, int bz,
+                                               const Sums& sums, RunList<kNmPD, kNmEnergyCap>& list, int bx, int by, int bz,
                                                const double* __restrict__ K64 = nullptr, const NmTile t = kNmTile) {
   RunSumL<kNmPD, kNmEnergyCap> rs;
   rs.reset();
@@ -795,9 +797,9 @@ __device__ __forceinline__ void nm_energy_body(const T* __restrict__ U, const T*
         v[0] = rho * h3; v[1] = 0.5 * tt * h; v[2] = -kv * rho * h3; v[3] = pc * rho * h3; v[4] = pc * ap * h3;
       }
     }
-    rs.add(L, v, sm.list, tid, sm.tab, pd);
+    rs.add(L, v, list, tid, sums);
   }
-  rs.finish(sm.list, tid, sm.tab, pd);
+  rs.finish(list, tid, sums);
 }
 
 // level-set label update (molecule.js:426-540 rule) on psi of type T, march tile

@@ -30,6 +30,9 @@ double interior(const Geo& g) {
   return n * n * n;
 }
 size_t esize(const rq_ctx* c) { return c->fp64 ? sizeof(double) : sizeof(float); }
+cudaError_t clear_norms(rq_ctx* c) {
+  return cudaMemsetAsync(c->acc, 0, sizeof(long long) * kExWords * (size_t)c->n_atoms, c->st);
+}
 }  // namespace
 
 // the same-label neighbour mask of the current labels (read by the update)
@@ -73,6 +76,7 @@ int nm_alloc_levels(rq_ctx* c) {
       cudaMalloc(&c->scale64, sizeof(double) * c->n_atoms) != cudaSuccess ||
       cudaMalloc((void**)&c->rseed, sizeof(unsigned) * 2) != cudaSuccess ||
       cudaMalloc((void**)&c->nbm, (size_t)c->g.S3) != cudaSuccess ||
+      cudaMalloc((void**)&c->acc, sizeof(long long) * kExWords * kNmPD * (size_t)c->n_atoms) != cudaSuccess ||
       cudaMalloc(&c->mg_res, (size_t)c->g.S3 * es) != cudaSuccess)
     return rq_cuda(c, cudaErrorMemoryAllocation, "seed table");
   cudaMemsetAsync(c->rseed, 0, sizeof(unsigned) * 2, c->st);
@@ -134,11 +138,11 @@ template <typename T>
 static int nm_normalize_t(rq_ctx* c, bool accumulate) {
   T* U = (T*)c->U[c->cu];
   if (accumulate) {
-    CK(cudaMemsetAsync(c->dnorm, 0, sizeof(double) * c->n_atoms, c->st));
-    LAUNCH(RQ_KC_NORMALIZE, (sizeof(T) + 4.0) * c->g.S3, nm_norms<T>(U, c->lab[c->cl], c->g, c->h3, c->n_atoms, c->dnorm, c->st));
+    CK(clear_norms(c));
+    LAUNCH(RQ_KC_NORMALIZE, (sizeof(T) + 4.0) * c->g.S3, nm_norms<T>(U, c->lab[c->cl], c->g, c->h3, c->n_atoms, c->acc, c->st));
   }
   LAUNCH(RQ_KC_NORMALIZE, (2.0 * sizeof(T) + 4.0) * c->g.S3,
-         nm_normalize<T>(U, c->lab[c->cl], c->dnorm, c->Zdom64, c->n_atoms, (double*)c->scale64, c->err, c->g, c->st));
+         nm_normalize<T>(U, c->lab[c->cl], c->acc, c->Zdom64, c->n_atoms, (double*)c->scale64, c->err, c->g, c->st));
   c->nm_pending = false;
   c->nm_age = 0;
   return RQ_OK;
@@ -190,20 +194,20 @@ static int nm_step_t(rq_ctx* c, int s) {
   const bool label_step = s % f.label_interval == 0 && (f.label_until <= 0 || s <= f.label_until);
   const bool norm = (s + 1) % f.norm_interval == 0 || (s + 1) % f.poisson_interval == 0 || label_step;
   if (c->adj.cap > 0 && (rc = nm_adj_record_step(c, s % f.poisson_interval == 0, norm)) != RQ_OK) return rc;
-  if (norm) CK(cudaMemsetAsync(c->dnorm, 0, sizeof(double) * c->n_atoms, c->st));
+  if (norm) CK(clear_norms(c));
   const bool sr = !c->fp64 && f.fp32_rounding == 1;
   // bytes: psi, K, P read, psi' written, the neighbour mask; the centre label under a pending scale; the norms'
   // second read of psi and the labels
   LAUNCH(RQ_KC_UPDATE, (4.0 * sizeof(T) + 1.0 + (c->nm_pending ? 4.0 : 0.0) + (norm ? sizeof(T) + 4.0 : 0.0)) * interior(c->g),
          nm_update<T>((const T*)c->U[c->cu], (T*)c->U[1 - c->cu], (const T*)c->K, (const T*)c->P[c->cp], c->lab[c->cl],
-                      c->g, (T)c->half_dv, (T)c->dt, c->h3, c->n_atoms, norm ? c->dnorm : nullptr, c->st,
+                      c->g, (T)c->half_dv, (T)c->dt, c->h3, c->n_atoms, norm ? c->acc : nullptr, c->st,
                       c->nm_pending ? (const double*)c->scale64 : nullptr, sr ? c->rseed + c->cu : nullptr,
                       sr ? c->rseed + (1 - c->cu) : nullptr, c->nbm));
   c->cu ^= 1;
   c->nm_pending = false;  // the update consumed the pending scale
   if (norm) {  // the scale of this step is applied by the next update (or a flush)
-    LAUNCH(RQ_KC_NORMALIZE, 12.0 * c->n_atoms,
-           nm_norm_scale<T>(c->dnorm, c->Zdom64, c->n_atoms, (double*)c->scale64, c->err, c->st));
+    LAUNCH(RQ_KC_NORMALIZE, (8.0 * kExWords + 16.0) * c->n_atoms,
+           nm_norm_scale(c->acc, c->Zdom64, c->n_atoms, (double*)c->scale64, c->err, c->st));
     c->nm_pending = true;
     if (c->adj.cap > 0 && (rc = nm_adj_record_scale(c)) != RQ_OK) return rc;
   }
@@ -466,15 +470,14 @@ int nm_energy(rq_ctx* c, double* out, double* per_domain) {
   const int n = c->n_atoms;
   int frc = nm_ready(c);
   if (frc != RQ_OK) return frc;
-  CK(cudaMemsetAsync(c->dpd, 0, sizeof(double) * kNmPD * n, c->st));
   if (c->fp64)
     LAUNCH(RQ_KC_ENERGY, 36 * interior(c->g),
            nm_energy<double>((const double*)c->U[c->cu], (const double*)c->K, (const double*)c->P[c->cp], c->lab[c->cl],
-                             c->g, c->h, n, c->dpd, c->st));
+                             c->g, c->h, n, c->acc, c->dpd, c->st));
   else
     LAUNCH(RQ_KC_ENERGY, 16 * interior(c->g),
            nm_energy<float>((const float*)c->U[c->cu], (const float*)c->K, (const float*)c->P[c->cp], c->lab[c->cl],
-                            c->g, c->h, n, c->dpd, c->st, c->K64));
+                            c->g, c->h, n, c->acc, c->dpd, c->st, c->K64));
   std::vector<double> pd((size_t)kNmPD * n);
   CK(cudaMemcpyAsync(pd.data(), c->dpd, sizeof(double) * kNmPD * n, cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));

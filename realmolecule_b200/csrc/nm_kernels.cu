@@ -43,13 +43,28 @@ __global__ void __launch_bounds__(256) k_nm_update(const T* U, T* Unew, const T*
                               scale, seed);
 }
 
-// scale[l] = sqrt(Zdom_l / n_l) (FP64) for every domain of the (concatenated) arrays; a norm
-// that is NaN or Inf sets bit 0 of *err and leaves its domain unscaled
-template <typename T>
+// scale[l] = sqrt(Zdom_l / n_l) (FP64) for every domain; a norm that is NaN or Inf sets bit 0 of *err
+// and leaves its domain unscaled.  The norms of a batch's concatenated domains are plain sums, those of a single
+// grid accumulators (exact_sum.h), a warp each.
 __global__ void k_nm_norm_scale(const double* __restrict__ norms, const double* __restrict__ Zdom, int nDom,
                                 double* __restrict__ scale, int* __restrict__ err) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l < nDom) scale[l] = nm_domain_scale(norms[l], Zdom[l], err);
+}
+__global__ void __launch_bounds__(128) k_nm_norm_scale_acc(const long long* __restrict__ acc, const double* __restrict__ Zdom,
+                                                           int nDom, double* __restrict__ scale, int* __restrict__ err) {
+  const int l = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (l >= nDom) return;
+  const double n = exact_value_warp(acc + (long long)l * kExWords);
+  if (threadIdx.x % 32 == 0) scale[l] = nm_domain_scale(n, Zdom[l], err);
+}
+
+// out[q] = the double next to accumulator q
+__global__ void __launch_bounds__(256) k_nm_acc_value(const long long* __restrict__ acc, int n, double* __restrict__ out) {
+  const int q = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (q >= n) return;
+  const double v = exact_value_warp(acc + (long long)q * kExWords);
+  if (threadIdx.x % 32 == 0) out[q] = v;
 }
 
 template <typename T>
@@ -58,14 +73,11 @@ __global__ void __launch_bounds__(256) k_nm_apply_scale(T* U, const int* label, 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_nm_norms(const T* U, const int* label, Geo g, double h3, int nDom, double* norms) {
-  __shared__ NormSmem sm;
-  dom_table_init(sm.tab);
-  __syncthreads();
+__global__ void __launch_bounds__(256) k_nm_norms(const T* U, const int* label, Geo g, double h3, int nDom, long long* acc) {
+  __shared__ NormSmem<BlockSums<1>> sm;
   const int i0 = 1 + (int)blockIdx.z * kNmNormPlanes;
-  nm_norms_body<T>(U, label, g, h3, nDom, norms, sm, blockIdx.x, blockIdx.y, i0, min(i0 + kNmNormPlanes, g.NN));
-  __syncthreads();
-  dom_table_flush(sm.tab, norms);
+  nm_norms_body<T>(U, label, g, h3, nDom, ExactSums<1>{sm.sums, acc}, sm.list, blockIdx.x, blockIdx.y, i0,
+                   min(i0 + kNmNormPlanes, g.NN));
 }
 
 template <typename T, bool FINE, int ROW, int COLOR>
@@ -98,13 +110,10 @@ __global__ void __launch_bounds__(1024) k_nm_coarsest(T* P, const T* f, Geo g, d
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_nm_energy(const T* U, const T* K, const T* P, const int* label, Geo g, double h,
-                                                   int nDom, double* pd, const double* K64) {
-  __shared__ EnergySmem sm;
-  dom_table_init(sm.tab);
-  __syncthreads();
-  nm_energy_body<T>(U, K, P, label, g, h, nDom, pd, sm, blockIdx.x, blockIdx.y, blockIdx.z, K64);
-  __syncthreads();
-  dom_table_flush(sm.tab, pd);
+                                                   int nDom, long long* acc, const double* K64) {
+  __shared__ EnergySmem<BlockSums<kNmPD>> sm;
+  nm_energy_body<T>(U, K, P, label, g, h, nDom, ExactSums<kNmPD>{sm.sums, acc}, sm.list, blockIdx.x, blockIdx.y, blockIdx.z,
+                    K64);
 }
 
 template <typename T>
@@ -152,7 +161,7 @@ cudaError_t nm_init(T* U, int* label, const float4* seeds, int nSeed, const Geo&
 }
 template <typename T>
 cudaError_t nm_update(const T* U, T* Unew, const T* K, const T* P, const int* label, const Geo& g, T half_dv, T dt,
-                      double h3, int nDom, double* norms, cudaStream_t st, const double* scale, const unsigned* seed,
+                      double h3, int nDom, long long* norms, cudaStream_t st, const double* scale, const unsigned* seed,
                       unsigned* seed_next, const unsigned char* mask) {
   if (g.NN < 2) return cudaSuccess;
   const int planes = vplanes<T>(g, false);
@@ -180,19 +189,22 @@ cudaError_t nm_apply(T* U, const int* label, const double* scale, int nDom, cons
   return cudaGetLastError();
 }
 template <typename T>
-cudaError_t nm_normalize(T* U, const int* label, const double* norms, const double* Zdom, int nDom, double* scale, int* err,
-                         const Geo& g, cudaStream_t st) {
-  k_nm_norm_scale<T><<<nblk(nDom, 128), 128, 0, st>>>(norms, Zdom, nDom, scale, err);
+cudaError_t nm_normalize(T* U, const int* label, const long long* norms, const double* Zdom, int nDom, double* scale,
+                         int* err, const Geo& g, cudaStream_t st) {
+  k_nm_norm_scale_acc<<<nblk(nDom, 4), 128, 0, st>>>(norms, Zdom, nDom, scale, err);
   k_nm_apply_scale<T><<<nblk(g.S3, 256 * kNmFlatChunk), 256, 0, st>>>(U, label, scale, g.S3, nDom);
   return cudaGetLastError();
 }
-template <typename T>
 cudaError_t nm_norm_scale(const double* norms, const double* Zdom, int nDom, double* scale, int* err, cudaStream_t st) {
-  k_nm_norm_scale<T><<<nblk(nDom, 128), 128, 0, st>>>(norms, Zdom, nDom, scale, err);
+  k_nm_norm_scale<<<nblk(nDom, 128), 128, 0, st>>>(norms, Zdom, nDom, scale, err);
+  return cudaGetLastError();
+}
+cudaError_t nm_norm_scale(const long long* norms, const double* Zdom, int nDom, double* scale, int* err, cudaStream_t st) {
+  k_nm_norm_scale_acc<<<nblk(nDom, 4), 128, 0, st>>>(norms, Zdom, nDom, scale, err);
   return cudaGetLastError();
 }
 template <typename T>
-cudaError_t nm_norms(const T* U, const int* label, const Geo& g, double h3, int nDom, double* norms, cudaStream_t st) {
+cudaError_t nm_norms(const T* U, const int* label, const Geo& g, double h3, int nDom, long long* norms, cudaStream_t st) {
   k_nm_norms<T><<<nm_norms_grid(g), 256, 0, st>>>(U, label, g, h3, nDom, norms);
   return cudaGetLastError();
 }
@@ -265,10 +277,12 @@ cudaError_t nm_adj_tail(const NmTail& t, size_t smem, const T* mA, T* muf, cudaS
   return cudaGetLastError();
 }
 template <typename T>
-cudaError_t nm_energy(const T* U, const T* K, const T* P, const int* label, const Geo& g, double h, int nDom, double* pd,
-                      cudaStream_t st, const double* K64) {
-  if (g.NN < 2) return cudaSuccess;
-  k_nm_energy<T><<<nm_march_grid(g), nm_march_block(), 0, st>>>(U, K, P, label, g, h, nDom, pd, K64);
+cudaError_t nm_energy(const T* U, const T* K, const T* P, const int* label, const Geo& g, double h, int nDom,
+                      long long* acc, double* pd, cudaStream_t st, const double* K64) {
+  const cudaError_t e = cudaMemsetAsync(acc, 0, sizeof(long long) * kExWords * kNmPD * (size_t)nDom, st);
+  if (e != cudaSuccess) return e;
+  k_nm_energy<T><<<nm_march_grid(g), nm_march_block(), 0, st>>>(U, K, P, label, g, h, nDom, acc, K64);
+  k_nm_acc_value<<<nblk((long long)nDom * kNmPD, 8), 256, 0, st>>>(acc, nDom * kNmPD, pd);
   return cudaGetLastError();
 }
 template <typename T>
@@ -297,13 +311,12 @@ cudaError_t nm_add(T* K, const T* v, long long n, cudaStream_t st) {
   template cudaError_t nm_potential<T>(T*, const double*, int, const Geo&, double, double, cudaStream_t, double*);  \
   template cudaError_t nm_init<T>(T*, int*, const float4*, int, const Geo&, float, cudaStream_t);                   \
   template cudaError_t nm_update<T>(const T*, T*, const T*, const T*, const int*, const Geo&, T, T, double, int,     \
-                                    double*, cudaStream_t, const double*, const unsigned*, unsigned*,                \
+                                    long long*, cudaStream_t, const double*, const unsigned*, unsigned*,             \
                                     const unsigned char*);                                                           \
   template cudaError_t nm_apply<T>(T*, const int*, const double*, int, const Geo&, cudaStream_t);                   \
-  template cudaError_t nm_normalize<T>(T*, const int*, const double*, const double*, int, double*, int*, const Geo&, \
-                                       cudaStream_t);                                                                \
-  template cudaError_t nm_norm_scale<T>(const double*, const double*, int, double*, int*, cudaStream_t);            \
-  template cudaError_t nm_norms<T>(const T*, const int*, const Geo&, double, int, double*, cudaStream_t);           \
+  template cudaError_t nm_normalize<T>(T*, const int*, const long long*, const double*, int, double*, int*,          \
+                                       const Geo&, cudaStream_t);                                                    \
+  template cudaError_t nm_norms<T>(const T*, const int*, const Geo&, double, int, long long*, cudaStream_t);        \
   template cudaError_t nm_rbgs<T>(T*, const T*, bool, const Geo&, double, int, cudaStream_t);                       \
   template cudaError_t nm_residual<T>(const T*, const T*, bool, T*, const Geo&, double, cudaStream_t);               \
   template cudaError_t nm_restrict<T>(const T*, T*, T*, const Geo&, const Geo&, cudaStream_t);                       \
@@ -311,8 +324,8 @@ cudaError_t nm_add(T* K, const T* v, long long n, cudaStream_t st) {
   template cudaError_t nm_coarsest<T>(T*, const T*, const Geo&, double, int, cudaStream_t);                         \
   template cudaError_t nm_tail<T>(const NmTail&, size_t, const T*, T*, cudaStream_t);                                \
   template cudaError_t nm_adj_tail<T>(const NmTail&, size_t, const T*, T*, cudaStream_t);                            \
-  template cudaError_t nm_energy<T>(const T*, const T*, const T*, const int*, const Geo&, double, int, double*,     \
-                                    cudaStream_t, const double*);                                                    \
+  template cudaError_t nm_energy<T>(const T*, const T*, const T*, const int*, const Geo&, double, int, long long*,  \
+                                    double*, cudaStream_t, const double*);                                           \
   template cudaError_t nm_evolve<T>(const int*, int*, const T*, float*, const Geo&, double, double, cudaStream_t);  \
   template cudaError_t nm_force<T>(const T*, const double*, int, const Geo&, double, double, double*, cudaStream_t,  \
                                    const double*);

@@ -40,7 +40,6 @@ struct rq_adj {
   double* gK = nullptr;               // dE/dK accumulated (S^3 doubles); dE/dv for the external potential
   struct Level { void* mu[2] = {nullptr, nullptr}; void* muf = nullptr; void* mur = nullptr; };
   std::vector<Level> lv;              // per multigrid level (level 0: only mur is used)
-  double* dots = nullptr;             // per-domain <psi, lambda>
   double* coef = nullptr;             // per-domain (scale, beta) of a transposed normalisation
   double* wq = nullptr;               // per-domain (Z/N, Q/N) of the energy readout
 };
@@ -94,6 +93,7 @@ struct rq_ctx {
   // new flavour multigrid hierarchy (level 0 = fine)
   std::vector<rq_mg_level> mg;
   void* mg_res = nullptr;  // new flavour: the residual of the level being restricted (T, S^3)
+  long long* acc = nullptr;  // new flavour: the accumulators of the per-domain sums (exact_sum.h), kNmPD per domain
 
   // atoms on the device
   float* atoms5 = nullptr;    // [i,j,k,Z,rc] f32 (cloud/solver.py:378-382)

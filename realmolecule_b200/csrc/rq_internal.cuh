@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "exact_sum.h"
+
 #define F_ADD(a, b) __fadd_rn((a), (b))
 #define F_SUB(a, b) __fsub_rn((a), (b))
 #define F_MUL(a, b) __fmul_rn((a), (b))
@@ -177,10 +179,69 @@ struct RunSum {
   }
 };
 
+// acc += v for an accumulator of exact_sum.h in global memory, from any number of threads
+__device__ __forceinline__ void exact_add(long long* acc, double v) {
+  long long p[3];
+  const int w = exact_split(v, p);
+  auto* a = reinterpret_cast<unsigned long long*>(acc) + w;
+  if (w == kExFlags) {
+    atomicOr(a, (unsigned long long)p[0]);
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+    if (p[q]) atomicAdd(a + q, (unsigned long long)p[q]);
+}
+
+// The double next to an accumulator, by a warp (every lane gets it)
+__device__ __forceinline__ double exact_value_warp(const long long* __restrict__ acc) {
+  const int lane = lane_id();
+  const long long a = acc[lane], b = acc[lane + 32], c = lane < kExWords - 64 ? acc[lane + 64] : 0;
+  const unsigned na = __ballot_sync(0xffffffffu, a != 0), nb = __ballot_sync(0xffffffffu, b != 0),
+                 nc = __ballot_sync(0xffffffffu, c != 0) & ((1u << (kExLimbs - 64)) - 1u);
+  const long long flags = __shfl_sync(0xffffffffu, c, kExFlags - 64);
+  const int first = na ? __ffs(na) - 1 : nb ? 31 + __ffs(nb) : nc ? 63 + __ffs(nc) : 0;
+  const int last = nc ? 95 - __clz(nc) : nb ? 63 - __clz(nb) : na ? 31 - __clz(na) : 0;
+  return exact_round([&](int i) { return __shfl_sync(0xffffffffu, i < 32 ? a : i < 64 ? b : c, i & 31); }, first, last,
+                     flags);
+}
+
+// Where the sums of a walk go (RunSumL).  TableSums: the block table, then the global array, FP64 adds
+// in the order in which the warps come.  ExactSums: one accumulator per domain and quantity, the same whatever the
+// order.  The sums that fp32 fields are scaled by are exact ones: a last bit that depends on the order turns
+// roundings of psi and of the reverse sweep's fields, so two runs of one evaluation differed by 2e-9 in
+// the forces, and by 1e-7 where a value of psi beside a nucleus was turned.
+template <int NQ, int NSLOT = 128>
+struct TableSums {
+  DomTable<NQ, NSLOT>& t;
+  double* global;
+  static constexpr bool kBlock = false;
+  __device__ __forceinline__ void add(int l, const double* v) const { dom_table_add(t, l, v, global); }
+};
+// A warp's first four entries meet those of the other seven in one more butterfly: a big grid of few
+// domains otherwise has 8 x as many additions to the same words (320^3, one domain: 165 us without it, 66 with), and
+// merging all entries, a scan per entry, costs more than the additions (64^3, 13 domains: 21.5 us against 8.2; with
+// block tables of FP64 sums the passes took 66 and 9.4 us).
+template <int NQ>
+struct BlockSums {
+  int label[32];
+  double v[NQ][32];
+};
+template <int NQ>
+struct ExactSums {
+  BlockSums<NQ>& sm;
+  long long* global;  // NQ accumulators per domain
+  static constexpr bool kBlock = true;
+  __device__ __forceinline__ void add(int l, const double* v) const {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) exact_add(global + ((long long)l * NQ + q) * kExWords, v[q]);
+  }
+};
+
 // Running sums of threads that walk columns across many domains.  A thread that meets a new label parks the
 // finished (label, sums) in its own list in shared memory; at the end of the walk the warp goes through the
-// lists together, one entry per lane at a time: a butterfly merges lanes of one label, and the leaders add
-// to the block table.  Adding to the table on the spot cost a compare-and-swap loop per lane (the table's
+// lists together, one entry per lane at a time: a butterfly merges lanes of one label, and the leaders hold
+// what is added.  Adding to the table on the spot cost a compare-and-swap loop per lane (the table's
 // FP64 adds are such loops, and a warp's lanes cross a domain face together), and a butterfly on every
 // plane 130 instructions a point.  A thread that meets more than CAP labels adds the rest on the spot.
 template <int NQ, int CAP>
@@ -200,9 +261,8 @@ struct RunSumL {
     for (int q = 0; q < NQ; ++q) v[q] = 0.0;
   }
   // l = -1: nothing to add
-  template <int NSLOT>
-  __device__ __forceinline__ void add(int l, const double* x, RunList<NQ, CAP>& list, int tid, DomTable<NQ, NSLOT>& t,
-                                      double* global) {
+  template <class Sums>
+  __device__ __forceinline__ void add(int l, const double* x, RunList<NQ, CAP>& list, int tid, const Sums& sums) {
     if (l != label) {
       if (label >= 0) {
         if (n < CAP) {
@@ -211,7 +271,7 @@ struct RunSumL {
           for (int q = 0; q < NQ; ++q) list.v[n][q][tid] = v[q];
           ++n;
         } else {
-          dom_table_add(t, label, v, global);
+          sums.add(label, v);
         }
       }
       label = l;
@@ -222,10 +282,25 @@ struct RunSumL {
       for (int q = 0; q < NQ; ++q) v[q] += x[q];
     }
   }
-  // every lane of the warp together
-  template <int NSLOT>
-  __device__ __forceinline__ void finish(RunList<NQ, CAP>& list, int tid, DomTable<NQ, NSLOT>& t, double* global) {
+  // lanes of one label that a butterfly brings together leave the sum with the lower one; fl = -1: none
+  static __device__ __forceinline__ void merge(int& fl, double (&v)[NQ], int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int ol = __shfl_xor_sync(0xffffffffu, fl, o);
+      const bool same = ol == fl;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        const double y = __shfl_xor_sync(0xffffffffu, v[q], o);
+        if (same && !(lane & o)) v[q] += y;
+      }
+      if (same && (lane & o)) fl = -1;
+    }
+  }
+  // every thread of the block (of 256) together
+  template <class Sums>
+  __device__ __forceinline__ void finish(RunList<NQ, CAP>& list, int tid, const Sums& sums) {
     const int lane = lane_id();
+    int cnt = 0;  // entries that the warp has had
     for (int s = -1; s < CAP; ++s) {  // the running entry, then the parked ones
       int fl = label;
       if (s >= 0) {
@@ -234,18 +309,29 @@ struct RunSumL {
         for (int q = 0; q < NQ; ++q) v[q] = fl >= 0 ? list.v[s][q][tid] : 0.0;
         if (!__any_sync(0xffffffffu, fl >= 0)) break;
       }
+      merge(fl, v, lane);
+      if constexpr (Sums::kBlock) {  // the first four entries of a warp wait for the block's other warps
+        const unsigned bal = __ballot_sync(0xffffffffu, fl >= 0);
+        const int o = cnt + __popc(bal & ((1u << lane) - 1u));
+        cnt += __popc(bal);
+        if (fl >= 0 && o < 4) {
+          sums.sm.label[4 * (tid >> 5) + o] = fl;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int ol = __shfl_xor_sync(0xffffffffu, fl, o);
-        const bool same = ol == fl;
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-          const double y = __shfl_xor_sync(0xffffffffu, v[q], o);
-          if (same && !(lane & o)) v[q] += y;
+          for (int q = 0; q < NQ; ++q) sums.sm.v[q][4 * (tid >> 5) + o] = v[q];
+          fl = -1;
         }
-        if (same && (lane & o)) fl = -1;
       }
-      if (fl >= 0) dom_table_add(t, fl, v, global);
+      if (fl >= 0) sums.add(fl, v);
+    }
+    if constexpr (Sums::kBlock) {
+      if (lane >= cnt && lane < 4) sums.sm.label[4 * (tid >> 5) + lane] = -1;
+      __syncthreads();
+      if (tid >= 32) return;
+      int fl = sums.sm.label[lane];
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) v[q] = fl >= 0 ? sums.sm.v[q][lane] : 0.0;
+      merge(fl, v, lane);
+      if (fl >= 0) sums.add(fl, v);
     }
   }
 };

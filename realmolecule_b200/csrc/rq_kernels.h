@@ -132,20 +132,22 @@ template <typename T>
 cudaError_t nm_init(T* U, int* label, const float4* seeds, int nSeed, const Geo& g, float h, cudaStream_t st);
 template <typename T>
 cudaError_t nm_update(const T* U, T* Unew, const T* K, const T* P, const int* label, const Geo& g, T half_dv, T dt,
-                      double h3, int nDom, double* norms, cudaStream_t st, const double* scale = nullptr,
+                      double h3, int nDom, long long* norms, cudaStream_t st, const double* scale = nullptr,
                       const unsigned* seed = nullptr, unsigned* seed_next = nullptr,
                       const unsigned char* mask = nullptr);
 // the same-label neighbour mask of `label` (S^3 bytes; bit q: neighbour q has the point's label)
 cudaError_t nm_mask(const int* label, unsigned char* mask, const Geo& g, cudaStream_t st);
 template <typename T>
 cudaError_t nm_apply(T* U, const int* label, const double* scale, int nDom, const Geo& g, cudaStream_t st);
+// norms as accumulators (exact_sum.h), one per domain, which the caller clears; those of a batch's concatenated
+// domains as doubles
 template <typename T>
-cudaError_t nm_normalize(T* U, const int* label, const double* norms, const double* Zdom, int nDom, double* scale, int* err,
-                         const Geo& g, cudaStream_t st);
-template <typename T>
+cudaError_t nm_normalize(T* U, const int* label, const long long* norms, const double* Zdom, int nDom, double* scale,
+                         int* err, const Geo& g, cudaStream_t st);
 cudaError_t nm_norm_scale(const double* norms, const double* Zdom, int nDom, double* scale, int* err, cudaStream_t st);
+cudaError_t nm_norm_scale(const long long* norms, const double* Zdom, int nDom, double* scale, int* err, cudaStream_t st);
 template <typename T>
-cudaError_t nm_norms(const T* U, const int* label, const Geo& g, double h3, int nDom, double* norms, cudaStream_t st);
+cudaError_t nm_norms(const T* U, const int* label, const Geo& g, double h3, int nDom, long long* norms, cudaStream_t st);
 template <typename T>
 cudaError_t nm_rbgs(T* P, const T* f, bool fine, const Geo& g, double h2, int color, cudaStream_t st);
 // fc = R (f - A P) (the residual and its full weighting in one pass) and Pc = 0 on the coarse interior
@@ -163,9 +165,10 @@ template <typename T>
 cudaError_t nm_tail(const NmTail& t, size_t smem, const T* f, T* P, cudaStream_t st);
 template <typename T>
 cudaError_t nm_adj_tail(const NmTail& t, size_t smem, const T* mA, T* muf, cudaStream_t st);
+// pd: kNmPD sums per domain; acc: as many accumulators
 template <typename T>
-cudaError_t nm_energy(const T* U, const T* K, const T* P, const int* label, const Geo& g, double h, int nDom, double* pd,
-                      cudaStream_t st, const double* K64 = nullptr);
+cudaError_t nm_energy(const T* U, const T* K, const T* P, const int* label, const Geo& g, double h, int nDom,
+                      long long* acc, double* pd, cudaStream_t st, const double* K64 = nullptr);
 template <typename T>
 cudaError_t nm_evolve(const int* labIn, int* labOut, const T* U, float* W, const Geo& g, double dt_w, double curvReg,
                       cudaStream_t st);
