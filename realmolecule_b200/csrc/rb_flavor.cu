@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "../../include/rq.h"
+#include "rb_index.h"
 #include "rq_internal.cuh"
 
 namespace rq {
@@ -44,6 +45,7 @@ struct RbParams {
 // are issued before the first store, and no thread waits for another electron's arithmetic; what bounds the pass
 // is load latency.  H2 at 100^3 per step: 81 us with a pass for rho_total and the competitor, a thread per cell
 // and a loop over electrons whose stores fenced the next one's loads; 35 us now.
+template <typename I>
 __global__ void __launch_bounds__(512) k_rb_color(const RbParams p, int color, float* __restrict__ U,
                                                   float* __restrict__ W, float* __restrict__ P,
                                                   const float* __restrict__ K, const unsigned char* __restrict__ mask) {
@@ -54,7 +56,7 @@ __global__ void __launch_bounds__(512) k_rb_color(const RbParams p, int color, f
   const int k = k0 + 2 * (blockIdx.x * kRbTK + threadIdx.x);
   const bool in = j < p.NN && k < p.NN;
   const int S = p.S, S2 = S * S;
-  const int id = in ? i * S2 + j * S + k : S2 + S + 1;  // an interior cell whatever the thread
+  const I id = in ? rb_offset<I>(i, j, k, S) : S2 + S + 1;  // an interior cell whatever the thread
   const long long S3 = (long long)S2 * S;
   float* u = U + m * S3 + id;
   float* w = W + m * S3 + id;
@@ -110,6 +112,7 @@ __global__ void __launch_bounds__(512) k_rb_color(const RbParams p, int color, f
 // grid-stride f32 sum over the interior cells in linear order, then the workgroup tree; and normalizeWGSL's sum of
 // the workgroups in order (:398-422) by the electron's last one: norm and scale.  Eight cells are loaded
 // ahead of the chain of additions.  H2 at 100^3: 35 us as two kernels, 13 us.
+template <typename I>
 __global__ void __launch_bounds__(128) k_rb_norm(const RbParams p, const float* __restrict__ U,
                                                  float* __restrict__ part, const float* __restrict__ tgt,
                                                  unsigned* __restrict__ done, float2* __restrict__ scale) {
@@ -117,16 +120,16 @@ __global__ void __launch_bounds__(128) k_rb_norm(const RbParams p, const float* 
   __shared__ bool last;
   constexpr int B = 8;
   const int m = blockIdx.y, lid = threadIdx.x, nwg = gridDim.x;
-  const unsigned NM = (unsigned)(p.NN - 1), tot = NM * NM * NM, stride = (unsigned)nwg * 128u;
-  const int S = p.S, S2 = S * S;
-  const float* u = U + m * ((long long)S2 * S);
+  const int NM = p.NN - 1, S = p.S;
+  const I tot = (I)NM * (I)NM * (I)NM, stride = (I)nwg * 128;
+  const float* u = U + m * ((long long)S * S * S);
   float acc = 0.0f;
-  for (unsigned c0 = blockIdx.x * 128u + lid; c0 < tot; c0 += B * stride) {
+  for (I c0 = (I)blockIdx.x * 128 + lid; c0 < tot; c0 += B * stride) {
     float v[B];
 #pragma unroll
     for (int b = 0; b < B; ++b) {
-      const unsigned cell = c0 + b * stride, y = cell / NM, k = cell - y * NM + 1, i = y / NM, j = y - i * NM + 1;
-      if (cell < tot) v[b] = __ldg(u + (int)((i + 1) * (unsigned)S2 + j * (unsigned)S + k));
+      const I cell = c0 + b * stride;
+      if (cell < tot) v[b] = __ldg(u + rb_interior_offset<I>(cell, NM, S));
     }
 #pragma unroll
     for (int b = 0; b < B; ++b)
@@ -365,12 +368,19 @@ int rb_frame(rq_rb* s, int n) {
   const int NN = s->cfg.NN;
   for (int q = 0; q < n; ++q) {
     for (int color = 0; color < 2; ++color) {
-      k_rb_color<<<rb_color_grid(NN, s->n), dim3(kRbTK, rb_rows(s->n), s->n), 0, s->st>>>(s->p, color, s->U, s->W, s->P,
-                                                                                       s->K, s->mask);
+      const dim3 grd = rb_color_grid(NN, s->n), blk(kRbTK, rb_rows(s->n), s->n);
+      if (rb_offsets_fit_31_bits(NN))
+        k_rb_color<int><<<grd, blk, 0, s->st>>>(s->p, color, s->U, s->W, s->P, s->K, s->mask);
+      else
+        k_rb_color<long long><<<grd, blk, 0, s->st>>>(s->p, color, s->U, s->W, s->P, s->K, s->mask);
       BLAUNCH();
     }
     if (q % 5 == 0) {
-      k_rb_norm<<<dim3(s->nwg, s->n), 128, 0, s->st>>>(s->p, s->U, s->part, s->tgt_d, s->done, s->scale);
+      const dim3 grd(s->nwg, s->n);
+      if (rb_offsets_fit_31_bits(NN))
+        k_rb_norm<unsigned><<<grd, 128, 0, s->st>>>(s->p, s->U, s->part, s->tgt_d, s->done, s->scale);
+      else
+        k_rb_norm<long long><<<grd, 128, 0, s->st>>>(s->p, s->U, s->part, s->tgt_d, s->done, s->scale);
       BLAUNCH();
       k_rb_normalize<<<rb_cells_grid(NN, NN - 1), dim3(32, 8), 0, s->st>>>(s->p, s->U, s->scale);
       BLAUNCH();
