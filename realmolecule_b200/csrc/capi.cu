@@ -256,6 +256,7 @@ extern "C" int rq_create(const rq_config* cfg, const rq_atom* atoms, int32_t n_a
   c->st = c->own_st;
   if (rc == RQ_OK) rc = alloc_all(c);
   if (rc == RQ_OK) rc = upload_atoms(c);
+  if (rc == RQ_OK) rc = nm_label_mask(c);  // of the labels as they are, all 0: a state may come without labels
   if (rc == RQ_OK) rc = rq_cuda(c, cudaStreamSynchronize(c->st), "create sync");
   if (rc != RQ_OK) {
     std::fprintf(stderr, "rq_create: %s\n", c->last_error.c_str());
