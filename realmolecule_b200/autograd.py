@@ -62,6 +62,9 @@ class EnergyModel:
     def _rows(self, pos: np.ndarray):
         """Atom table: the nuclei (Z 0), then the one-electron domains at their seeds (Z_nuc 0)."""
         n = min(len(pos), self.n_nuc)
+        for what, x in (("positions", pos[:n]), ("seeds", self.seeds)):
+            if len(x) and (x.ndim != 2 or x.shape[1] < 3):
+                raise IndexError(f"{what} have three coordinates each")  # one column would broadcast
         tab = np.zeros((n + len(self.seeds), len(ATOM_FIELDS)))
         if n:
             tab[:n, :3] = pos[:n, :3] / self.h
