@@ -19,6 +19,7 @@
 // energy sums were FP64 atomics on one shared word per quantity; a plane inside a block costs a
 // barrier and the f64 chain, ~0.2 us (B200).  A physicsStep of two half-space shells at N = 100 with the
 // multigrid solve: 12.0 ms in 1880 launches before, 1.56 ms in 131.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -322,14 +323,14 @@ __global__ void __launch_bounds__(B * B) k_at_cells(float* __restrict__ U, float
   }
 }
 
-// rhs of every shell's Poisson problem (blockIdx.y = m): 2 pi sum_{n != m} U_n^2 W_n
+// rhs of the Poisson problems of shells m0, m0 + 1, .. (blockIdx.y): 2 pi sum_{n != m} U_n^2 W_n
 // (atom.js:299-308), interior points
-__global__ void k_at_rhs(const float* __restrict__ U, const float* __restrict__ W, float* __restrict__ rhs, int nS,
+__global__ void k_at_rhs(const float* __restrict__ U, const float* __restrict__ W, float* __restrict__ rhs, int nS, int m0,
                          AtGeo g) {
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long n = g.N - 1;
   if (q >= n * n * n) return;
-  const int m = blockIdx.y;
+  const int m = m0 + blockIdx.y;
   const long long id = (1 + q / (n * n)) * g.S2 + (1 + (q / n) % n) * g.S + 1 + q % n;
   double rho = 0.0;
   for (int s = 0; s < nS; ++s)
@@ -337,7 +338,7 @@ __global__ void k_at_rhs(const float* __restrict__ U, const float* __restrict__ 
       const double u = U[s * g.S3 + id];
       rho = __dadd_rn(rho, __dmul_rn(__dmul_rn(u, u), (double)W[s * g.S3 + id]));
     }
-  rhs[m * g.S3 + id] = (float)__dmul_rn(__dmul_rn(2.0, 3.141592653589793), rho);
+  rhs[blockIdx.y * g.S3 + id] = (float)__dmul_rn(__dmul_rn(2.0, 3.141592653589793), rho);
 }
 
 // launch tau of pipelined in-place Gauss-Seidel sweeps (atom.js:127-138): sweep blockIdx.y works on
@@ -451,7 +452,9 @@ struct rq_shells {
   AtGeo g{}, gc{};
   double h = 0;
   float *U = nullptr, *W = nullptr, *P = nullptr, *K = nullptr;
-  float *rhs = nullptr, *cd = nullptr, *Pc = nullptr;  // per shell: right-hand side, coarse residual and correction
+  // of nP shells (1 at least) whose Poisson problems run together: right-hand side, coarse residual and correction
+  int nP = 0;
+  float *rhs = nullptr, *cd = nullptr, *Pc = nullptr;
   double* acc = nullptr;  // 3 + 4 nS energy sums, then nS norms
   AtFixed fixed{};
   cudaStream_t st = nullptr;
@@ -472,24 +475,25 @@ struct rq_shells {
 
 static unsigned blocks_for(long long n) { return (unsigned)((n + 255) / 256); }
 
-// pipelined Gauss-Seidel: `iters` in-place sweeps of every shell's P on grid g in one wavefront of
+// pipelined Gauss-Seidel: `iters` in-place sweeps of the P of n shells on grid g in one wavefront of
 // blocks.  Blocks of 16 as long as a row of blocks is not shorter than the pipeline: with 20 sweeps on a
 // coarse grid the launches are mostly the pipeline's 2 (iters - 1), and blocks of 8 (22 planes a launch
 // instead of 46) are the shorter chain.
 template <int B>
-static int at_smooth_b(rq_shells* s, float* P, const float* rhs, const AtGeo& g, double h2, int iters) {
+static int at_smooth_b(rq_shells* s, float* P, const float* rhs, int n, const AtGeo& g, double h2, int iters) {
   const int nb = (g.N - 1 + B - 1) / B;
   constexpr size_t smem = at_gs_smem<B>();
   SCK(cudaFuncSetAttribute(k_at_gs<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   for (int tau = 0; tau <= 3 * (nb - 1) + 2 * (iters - 1); ++tau) {
-    k_at_gs<B><<<dim3(nb * nb, iters, s->nS), B * B, smem, s->st>>>(P, rhs, g, h2, tau);
+    k_at_gs<B><<<dim3(nb * nb, iters, n), B * B, smem, s->st>>>(P, rhs, g, h2, tau);
     SLAUNCH();
   }
   return RQ_OK;
 }
-static int at_smooth(rq_shells* s, float* P, const float* rhs, const AtGeo& g, double h2, int iters) {
+static int at_smooth(rq_shells* s, float* P, const float* rhs, int n, const AtGeo& g, double h2, int iters) {
   const int nb = (g.N - 1 + kAtB - 1) / kAtB;
-  return 2 * (iters - 1) <= 3 * nb ? at_smooth_b<kAtB>(s, P, rhs, g, h2, iters) : at_smooth_b<8>(s, P, rhs, g, h2, iters);
+  return 2 * (iters - 1) <= 3 * nb ? at_smooth_b<kAtB>(s, P, rhs, n, g, h2, iters)
+                                   : at_smooth_b<8>(s, P, rhs, n, g, h2, iters);
 }
 
 // the cell update of every shell, one launch per block diagonal.  Blocks of 16 where the tiles of two
@@ -533,20 +537,23 @@ static int at_step(rq_shells* s) {
   SCK(cudaMemsetAsync(s->acc, 0, sizeof(double) * (3 + 5 * nS), s->st));
   int rc = at_cells(s);
   if (rc != RQ_OK) return rc;
-  if (!s->cfg.poisson) {  // poissonVcycle per shell (atom.js:186-210, :296-310), all shells together
+  // poissonVcycle per shell (atom.js:186-210, :296-310), as many shells together as there are buffers for
+  for (int m = 0; !s->cfg.poisson && m < s->nS; m += s->nP) {
     const AtGeo& gc = s->gc;
     const long long ncint = (long long)(gc.N - 1) * (gc.N - 1) * (gc.N - 1);
     const double hc = h * 2, hc2 = hc * hc;
-    k_at_rhs<<<dim3(blocks_for(nint), nS), 256, 0, s->st>>>(s->U, s->W, s->rhs, s->nS, g);
+    const int n = std::min(s->nP, s->nS - m);
+    float* P = s->P + m * g.S3;
+    k_at_rhs<<<dim3(blocks_for(nint), n), 256, 0, s->st>>>(s->U, s->W, s->rhs, s->nS, m, g);
     SLAUNCH();
-    if ((rc = at_smooth(s, s->P, s->rhs, g, h2, 4)) != RQ_OK) return rc;
-    k_at_restrict<<<dim3(blocks_for(ncint), nS), 256, 0, s->st>>>(s->P, s->rhs, s->cd, g, gc, h2);
+    if ((rc = at_smooth(s, P, s->rhs, n, g, h2, 4)) != RQ_OK) return rc;
+    k_at_restrict<<<dim3(blocks_for(ncint), n), 256, 0, s->st>>>(P, s->rhs, s->cd, g, gc, h2);
     SLAUNCH();
-    SCK(cudaMemsetAsync(s->Pc, 0, sizeof(float) * gc.S3 * nS, s->st));
-    if ((rc = at_smooth(s, s->Pc, s->cd, gc, hc2, 20)) != RQ_OK) return rc;
-    k_at_prolong<<<dim3(blocks_for(nint), nS), 256, 0, s->st>>>(s->Pc, s->P, g, gc);
+    SCK(cudaMemsetAsync(s->Pc, 0, sizeof(float) * gc.S3 * n, s->st));
+    if ((rc = at_smooth(s, s->Pc, s->cd, n, gc, hc2, 20)) != RQ_OK) return rc;
+    k_at_prolong<<<dim3(blocks_for(nint), n), 256, 0, s->st>>>(s->Pc, P, g, gc);
     SLAUNCH();
-    if ((rc = at_smooth(s, s->P, s->rhs, g, h2, 4)) != RQ_OK) return rc;
+    if ((rc = at_smooth(s, P, s->rhs, n, g, h2, 4)) != RQ_OK) return rc;
   }
   // normalise each shell over the interior
   double* n2 = s->acc + 3 + 4 * nS;
@@ -636,18 +643,30 @@ extern "C" int rq_shells_create(const rq_shells_config* cfg, const rq_shell* she
   };
   int rc = RQ_OK;
   auto alloc = [&](void** p, size_t bytes) -> int {
-    if (cudaMalloc(p, bytes) != cudaSuccess) { s->last_error = "cudaMalloc"; return RQ_ENOMEM; }
+    if (cudaMalloc(p, bytes) != cudaSuccess) { *p = nullptr; s->last_error = "cudaMalloc"; return RQ_ENOMEM; }
     if (cudaMemset(*p, 0, bytes) != cudaSuccess) { s->last_error = "cudaMemset"; return RQ_ECUDA; }
     return RQ_OK;
   };
   const size_t S3 = (size_t)s->g.S3, SC3 = (size_t)s->gc.S3;
   if ((rc = alloc((void**)&s->U, sizeof(float) * S3 * n_shells)) || (rc = alloc((void**)&s->W, sizeof(float) * S3 * n_shells)) ||
       (rc = alloc((void**)&s->P, sizeof(float) * S3 * n_shells)) || (rc = alloc((void**)&s->K, sizeof(float) * S3)) ||
-      (rc = alloc((void**)&s->rhs, sizeof(float) * S3 * n_shells)) ||
-      (rc = alloc((void**)&s->cd, sizeof(float) * SC3 * n_shells)) ||
-      (rc = alloc((void**)&s->Pc, sizeof(float) * SC3 * n_shells)) ||
       (rc = alloc((void**)&s->acc, sizeof(double) * (3 + 5 * n_shells))))
     return fail(rc);
+  // The Poisson buffers: of all shells, or of as many as the memory holds (one shell after the other takes n_shells
+  // chains of launches instead of one).
+  for (s->nP = cfg->poisson ? 0 : n_shells; s->nP > 0; --s->nP) {
+    rc = RQ_OK;
+    if (!(rc = alloc((void**)&s->rhs, sizeof(float) * S3 * s->nP)) && !(rc = alloc((void**)&s->cd, sizeof(float) * SC3 * s->nP)) &&
+        !(rc = alloc((void**)&s->Pc, sizeof(float) * SC3 * s->nP)))
+      break;
+    for (float** p : {&s->rhs, &s->cd, &s->Pc}) {
+      if (*p) cudaFree(*p);
+      *p = nullptr;
+    }
+    cudaGetLastError();  // the allocation that failed
+    if (rc != RQ_ENOMEM) break;
+  }
+  if (rc != RQ_OK) return fail(rc);
   if (cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) != cudaSuccess) {
     s->last_error = "cudaStreamCreate";
     return fail(RQ_ECUDA);

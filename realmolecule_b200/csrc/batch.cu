@@ -699,7 +699,9 @@ static int alloc_fields(rq_batch* b, BInst& I, size_t es) {
       BALLOC(I.lP[l], s3 * es);
       BALLOC(I.lf[l], s3 * es);
     }
-    if (l < I.nlev - 1) BALLOC(I.lr[l], s3 * es);
+    // the finest residual goes to the P buffer that the in-place cycles leave idle
+    if (l == 0) I.lr[0] = I.P[1];
+    else if (l < I.nlev - 1) BALLOC(I.lr[l], s3 * es);
   }
   BALLOC(I.cs, 2 * sizeof(double) * (size_t)I.lg[I.nlev - 1].S3);
   return RQ_OK;
@@ -1690,7 +1692,8 @@ extern "C" int rq_batch_autotune(rq_batch* b, rq_tune_report* out) {
     b_retile(b, keep);
     b->cfg.batch_persistent = keep_persistent;
   }
-  // 2. smoother sweeps: 3 V-cycles from P = 0 on the current psi, P restored after each
+  // 2. smoother sweeps: 3 V-cycles from P = 0 on the current psi, P restored after each from the psi buffer that the
+  // next update writes
   if (rc == RQ_OK && !b->dtune) rc = balloc(b, (void**)&b->dtune, sizeof(double));
   if (rc == RQ_OK) rc = b_flush(b);
   const int cand[7][3] = {{1, 1, 16}, {2, 1, 16}, {1, 2, 16}, {2, 2, 16}, {1, 1, 8}, {1, 1, 32}, {2, 2, 32}};
@@ -1705,7 +1708,7 @@ extern "C" int rq_batch_autotune(rq_batch* b, rq_tune_report* out) {
       if (!b->active[q]) continue;
       const BInst& I = b->hin[q];
       const size_t bytes = (b->f64[q] ? sizeof(double) : sizeof(float)) * (size_t)I.g.S3;
-      if (cudaMemcpyAsync(I.P[1 - b->cp], I.P[b->cp], bytes, cudaMemcpyDeviceToDevice, b->st) != cudaSuccess ||
+      if (cudaMemcpyAsync(I.U[1 - b->cu], I.P[b->cp], bytes, cudaMemcpyDeviceToDevice, b->st) != cudaSuccess ||
           cudaMemsetAsync(I.P[b->cp], 0, bytes, b->st) != cudaSuccess)
         rc = RQ_ECUDA;
     }
@@ -1722,7 +1725,7 @@ extern "C" int rq_batch_autotune(rq_batch* b, rq_tune_report* out) {
       if (!b->active[q]) continue;
       const BInst& I = b->hin[q];
       const size_t bytes = (b->f64[q] ? sizeof(double) : sizeof(float)) * (size_t)I.g.S3;
-      if (cudaMemcpyAsync(I.P[b->cp], I.P[1 - b->cp], bytes, cudaMemcpyDeviceToDevice, b->st) != cudaSuccess) rc = RQ_ECUDA;
+      if (cudaMemcpyAsync(I.P[b->cp], I.U[1 - b->cu], bytes, cudaMemcpyDeviceToDevice, b->st) != cudaSuccess) rc = RQ_ECUDA;
     }
     if (rc != RQ_OK) break;
     const double rho = r0 > 0 ? std::pow(std::sqrt(r3 / r0), 1.0 / 3.0) : 1.0;

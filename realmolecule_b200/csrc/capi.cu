@@ -126,6 +126,7 @@ static int upload_atoms(rq_ctx* c) {
 }
 
 static void free_ctx(rq_ctx* c) {
+  if (c->cfg.flavor == RQ_FLAVOR_SOLVER_PY) c->nbm = nullptr;  // a part of bestU
   nm_adj_free(c);
   nm_ff_free(c);
   for (auto e : c->evpool) cudaEventDestroy(e);
@@ -133,7 +134,7 @@ static void free_ctx(rq_ctx* c) {
     if (gx) cudaGraphExecDestroy(gx);
   void* ptrs[] = {c->U[0], c->U[1], c->P[0], c->P[1], c->K, c->W, c->bestU, c->rho, c->Pother, c->resid, c->lab[0], c->lab[1],
                   c->Ec[0], c->Ec[1], c->fc, c->atoms5, c->scratch_atoms5, c->sic, c->sic2, c->pdirect, c->lob, c->lob_part, c->lob_scal, c->lob_done, c->lock, c->splits, c->bin_start, c->bin_idx, c->bin_far, c->bin_zmax, c->atoms_mj, c->atoms_nm, c->Zdom, c->Zdom64, c->dnorm,
-                  c->dpd, c->dF, c->dsum, c->unorm, c->scale, c->err, c->seeds, c->scale64, c->Kext, c->rseed, c->K64, c->nbm, c->mg_res, c->acc};
+                  c->dpd, c->dF, c->dsum, c->unorm, c->scale, c->err, c->seeds, c->scale64, c->Kext, c->rseed, c->K64, c->nbm, c->acc};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (auto& L : c->mg) {
@@ -166,7 +167,12 @@ static int alloc_all(rq_ctx* c) {
   }
   DALLOC(c->K, S3 * es);
   DALLOC(c->W, S3 * sizeof(float));
-  if (c->cfg.flavor == RQ_FLAVOR_SOLVER_PY || c->cfg.flavor == RQ_FLAVOR_MOLECULE_JS) DALLOC(c->bestU, S3 * sizeof(float));
+  if (c->cfg.flavor == RQ_FLAVOR_MOLECULE_JS) DALLOC(c->bestU, S3 * sizeof(float));
+  if (c->cfg.flavor == RQ_FLAVOR_SOLVER_PY) {
+    // the trial state's scratch; from then on the label step's candidates, and behind them the same-label mask
+    DALLOC(c->bestU, std::max<size_t>(S3 * sizeof(float), sp_list_cells(c->g) * sizeof(float) + S3 + 3));
+    c->nbm = (unsigned char*)(c->bestU + sp_list_cells(c->g));
+  }
   if (c->cfg.flavor == RQ_FLAVOR_MOLECULE_JS) {
     DALLOC(c->rho, S3 * sizeof(float));
     DALLOC(c->Pother, S3 * sizeof(float));
@@ -174,7 +180,7 @@ static int alloc_all(rq_ctx* c) {
     if (c->cfg.sic) {
       DALLOC(c->sic, S3 * sizeof(float));
       DALLOC(c->sic2, S3 * sizeof(float));
-      if (mj_direct(c)) DALLOC(c->pdirect, c->slot() * sizeof(float) * 2 * n);
+      if (mj_direct(c)) DALLOC(c->pdirect, c->slot() * sizeof(float) * n);
     }
     DALLOC(c->lock, sizeof(unsigned long long) * n);
     DALLOC(c->splits, sizeof(MjSplit) * n);
@@ -193,7 +199,6 @@ static int alloc_all(rq_ctx* c) {
   }
   DALLOC(c->atoms5, sizeof(float) * 5 * n);
   DALLOC(c->scratch_atoms5, sizeof(float) * 5 * n);
-  if (c->cfg.flavor == RQ_FLAVOR_SOLVER_PY) DALLOC(c->nbm, S3);
   if (c->cfg.flavor == RQ_FLAVOR_SOLVER_PY) {  // bins of ~1 atom each, at most 64 per axis
     const int S = c->g.S;
     int bin = (int)std::lround(std::cbrt((double)c->g.S3 / std::max(1, n)));
@@ -419,6 +424,7 @@ static int sp_initialize(rq_ctx* c) {
          launch_init_sp((float*)c->U[0], c->lab[0], (float*)c->K, c->bestU, c->atoms5, c->n_atoms, c->g, (float)c->h,
                         (float)c->h2, true, c->st));
   CK(cudaMemcpyAsync(c->lab[1], c->lab[0], sizeof(int) * c->g.S3, cudaMemcpyDeviceToDevice, c->st));
+  CK(cudaMemsetAsync(c->nbm, 0, c->g.S3, c->st));  // the trial state went over the faces' bytes
   int rc = nm_label_mask(c);
   if (rc != RQ_OK) return rc;
   if ((rc = sp_normalize(c, true)) != RQ_OK) return rc;

@@ -198,15 +198,16 @@ static float mj_cheb_omega(rq_ctx* c) {
   return (float)std::min(1.95, std::max(1.0, omega));
 }
 
-// The direct per-electron Poisson solve of every domain with electrons, in shared launches.
+// The direct per-electron Poisson solve of every domain with electrons, in shared launches.  The sweeps'
+// scratch is what the other path and its correction work in, interior cells only.
 static int mj_direct_solve(rq_ctx* c, const MjParams& p) {
   std::vector<int> m;
   for (int q = 0; q < c->n_atoms; ++q)
     if ((float)c->atoms[q].Z != 0.f) m.push_back(q);
-  const size_t slot = c->slot();
+  float* const scratch[kMjDoms] = {c->sic, c->sic2, c->rho, c->resid};
   LAUNCH(RQ_KC_POISSON, 120 * interior(c->g) * (double)m.size(),
          launch_mj_direct((float*)c->U[c->cu], c->lab[c->cl], c->Pother, m.data(), (int)m.size(), c->pdirect,
-                          c->pdirect + (size_t)c->n_atoms * slot, (long long)slot, c->g, p.h2, p.two_pi, c->st));
+                          (long long)c->slot(), scratch, c->g, p.h2, p.two_pi, c->st));
   return RQ_OK;
 }
 

@@ -302,28 +302,29 @@ __global__ void __launch_bounds__(256) k_mj_apply_scale(float* __restrict__ U, c
 // Weighted Jacobi (molecule.js:723-749, :754-774).  RHS: the density from psi, from a buffer (the
 // self-potential solve of the self-interaction correction, :3024-3030), or psi^2 outside the
 // domain (computeRhoOther, :593-612) for the direct path, where one launch sweeps all its domains' P_m
-// (they do not depend on one another): slot d % nd of Pin / Pout holds domain doms.m[d].  Blocks of the same
+// (they do not depend on one another): doms.in / doms.out are those of domain doms.m.  Blocks of the same
 // cells are neighbours in the grid, so psi and the labels come from memory once for all domains.  LAST:
 // copyPotherForLabel (:651-671) on the way out.  10 sweeps of water's 3 domains at 64^3, with the density and
 // the copy: 387 us as 36 launches of 64 to 1073 blocks, 64 us as 10 (each timed alone).
 constexpr int kMjRhoPsi = 0, kMjRhoBuf = 1, kMjRhoOther = 2;
-constexpr int kMjDoms = 8;  // domains of a launch
-struct MjDoms {
+struct MjDoms {  // a __grid_constant__: indexed as it lies, where a plain argument is first copied to local memory
   int n;
   int m[kMjDoms];
-  long long slot;  // elements between two domains' P
+  const float* in[kMjDoms];
+  float* out[kMjDoms];
 };
 template <int RHS, bool LAST>
 __global__ void __launch_bounds__(256) k_mj_jacobi(const float* __restrict__ Pin, float* __restrict__ Pout,
                                                    const float* __restrict__ R, const int* __restrict__ label,
-                                                   float* __restrict__ Pother, MjDoms doms, Geo g, int planes, float h2,
-                                                   float two_pi) {
+                                                   float* __restrict__ Pother, const __grid_constant__ MjDoms doms, Geo g,
+                                                   int planes, float h2, float two_pi) {
   int blk = blockIdx.x, m = 0;
   if (RHS == kMjRhoOther) {
     blk = (int)blockIdx.x / doms.n;
-    m = doms.m[(int)blockIdx.x - blk * doms.n];
-    Pin += m * doms.slot;
-    Pout += m * doms.slot;
+    const int d = (int)blockIdx.x - blk * doms.n;
+    m = doms.m[d];
+    Pin = doms.in[d];
+    Pout = doms.out[d];
   }
   const float c0 = F_MUL(h2, two_pi);
   const int i0 = 1 + blockIdx.y * planes, iend = min(i0 + planes, g.NN);
@@ -772,22 +773,28 @@ cudaError_t launch_mj_direct_init(const MjAtom* atoms, int nAt, int m, float* Pm
   return cudaGetLastError();
 }
 
-cudaError_t launch_mj_direct(const float* U, const int* label, float* Pother, const int* m, int n, float* P, float* P2,
-                             long long slot, const Geo& g, float h2, float two_pi, cudaStream_t st) {
-  // molecule.js:2835-2857 for n domains: 10 Jacobi sweeps of each persistent P_m (P <-> P2, ending
-  // in P) on the density of every other domain, then Pother = P_m on the domain
+cudaError_t launch_mj_direct(const float* U, const int* label, float* Pother, const int* m, int n, float* P,
+                             long long slot, float* const (&scratch)[kMjDoms], const Geo& g, float h2, float two_pi,
+                             cudaStream_t st) {
+  // molecule.js:2835-2857 for n domains: 10 Jacobi sweeps of each persistent P_m (P_m <-> scratch, ending
+  // in P_m) on the density of every other domain, then Pother = P_m on the domain
   const int planes = vplanes<float>(g, false);
   const dim3 grid = vgrid<float>(g, planes);
   for (int d0 = 0; d0 < n; d0 += kMjDoms) {
-    MjDoms doms;
-    doms.n = std::min(n - d0, kMjDoms);
-    doms.slot = slot;
-    for (int d = 0; d < doms.n; ++d) doms.m[d] = m[d0 + d];
-    const dim3 gd(grid.x * doms.n, grid.y);
+    MjDoms there, back;  // P_m -> scratch and the other way
+    there.n = back.n = std::min(n - d0, kMjDoms);
+    for (int d = 0; d < there.n; ++d) {
+      float* p = P + m[d0 + d] * slot;
+      there.m[d] = back.m[d] = m[d0 + d];
+      there.in[d] = back.out[d] = p;
+      there.out[d] = scratch[d];
+      back.in[d] = scratch[d];
+    }
+    const dim3 gd(grid.x * there.n, grid.y);
     for (int js = 0; js < 9; ++js)
-      k_mj_jacobi<kMjRhoOther, false><<<gd, 256, 0, st>>>(js % 2 ? P2 : P, js % 2 ? P : P2, U, label, Pother, doms, g,
+      k_mj_jacobi<kMjRhoOther, false><<<gd, 256, 0, st>>>(nullptr, nullptr, U, label, Pother, js % 2 ? back : there, g,
                                                           planes, h2, two_pi);
-    k_mj_jacobi<kMjRhoOther, true><<<gd, 256, 0, st>>>(P2, P, U, label, Pother, doms, g, planes, h2, two_pi);
+    k_mj_jacobi<kMjRhoOther, true><<<gd, 256, 0, st>>>(nullptr, nullptr, U, label, Pother, back, g, planes, h2, two_pi);
   }
   return cudaGetLastError();
 }

@@ -570,9 +570,7 @@ int snapshot_p(rq_ctx* c) {
 // ----------------------------------------------------------------------------------------
 void nm_adj_free(rq_ctx* c) {
   rq_adj& A = c->adj;
-  for (void* q : A.lam)
-    if (q) cudaFree(q);
-  void* p[] = {A.psi, A.psum, A.scales, A.muP[0], A.muP[1], A.muf, A.gK, A.coef, A.wq};
+  void* p[] = {A.psi, A.psum, A.scales, A.lam[0], A.lam[1], A.muP[0], A.muP[1], A.muf, A.gK, A.coef, A.wq};
   for (void* q : p)
     if (q) cudaFree(q);
   for (auto& L : A.lv)
@@ -601,14 +599,13 @@ int nm_adj_set_window(rq_ctx* c, int steps) {
   };
   const size_t slot_bytes = (size_t)slot_stride((long long)S3) * es;
   bool ok = alloc(&A.psi, steps * slot_bytes) && alloc(&A.psum, np * slot_bytes) &&
-            alloc((void**)&A.scales, sizeof(double) * (size_t)steps * n) && alloc(&A.muP[0], S3 * es) &&
-            alloc(&A.muP[1], S3 * es) &&
+            alloc((void**)&A.scales, sizeof(double) * (size_t)steps * n) && alloc(&A.lam[0], S3 * es) &&
+            alloc(&A.lam[1], S3 * es) && alloc(&A.muP[0], S3 * es) && alloc(&A.muP[1], S3 * es) &&
             alloc(&A.muf, S3 * es) && alloc((void**)&A.gK, S3 * sizeof(double)) &&
             alloc((void**)&A.coef, sizeof(double) * 2 * n) &&
             alloc((void**)&A.wq, sizeof(double) * 2 * n);
   const int levels = (int)c->mg.size();
   A.lv.assign(levels, rq_adj::Level());
-  for (void*& p : A.lam) ok = ok && alloc(&p, S3 * es);
   for (int l = 0; ok && l < levels; ++l) {
     const size_t s3 = (size_t)c->mg[l].g.S3;
     if (l > 0) ok = alloc(&A.lv[l].mu[0], s3 * es) && alloc(&A.lv[l].mu[1], s3 * es) && alloc(&A.lv[l].muf, s3 * es);
@@ -852,14 +849,20 @@ int adjoint_t(rq_ctx* c, double* F, double* dEdv) {
   T* muP[2] = {(T*)A.muP[0], (T*)A.muP[1]};
   T* lam = (T*)A.lam[0];
   AdjPend pend{};
-  // a lambda buffer that neither the sweep nor a pending sum holds
+  // Buffers for lambda: the sweep's and those of the steps whose sums are pending.  Besides the window's two, the
+  // state's idle buffers (the other psi, whose faces are 0 and whose interior the next update writes; the other
+  // P, which holds nothing between V-cycles) and, where dE/df is not kept on the finest level, its buffer.
+  const bool v11 = c->cfg.mg_pre == 1 && c->cfg.mg_post == 1;
+  T* const bufs[kAdjPend + 1] = {(T*)A.lam[0], (T*)A.lam[1], (T*)c->U[1 - c->cu], (T*)c->P[1 - c->cp], (T*)A.muf};
+  const int nbufs = v11 ? kAdjPend + 1 : kAdjPend;
+  CK(launch_zero_faces(bufs[3], g, c->st));
   auto spare = [&]() -> T* {
-    for (void* p : A.lam) {
-      bool held = p == lam;
-      for (int q = 0; q < pend.n; ++q) held = held || p == pend.lam[q];
-      if (!held) return (T*)p;
+    for (int b = 0; b < nbufs; ++b) {
+      bool held = bufs[b] == lam;
+      for (int q = 0; q < pend.n; ++q) held = held || bufs[b] == pend.lam[q];
+      if (!held) return bufs[b];
     }
-    return nullptr;  // not reached: fewer than kAdjPend are pending, and A.lam holds one more
+    return nullptr;  // not reached: at most nbufs - 2 are pending here
   };
   auto accumulate = [&]() -> int {
     if (!pend.n) return RQ_OK;
@@ -894,8 +897,8 @@ int adjoint_t(rq_ctx* c, double* F, double* dEdv) {
     pend.lam[pend.n] = lam;
     pend.psi[pend.n++] = psi_prev;
     lam = out;
-    if ((R.vcycle || pend.n == kAdjPend) && (rc = accumulate()) != RQ_OK) return rc;
-    if (R.vcycle && c->cfg.mg_pre == 1 && c->cfg.mg_post == 1) {
+    if ((R.vcycle || pend.n == nbufs - 1) && (rc = accumulate()) != RQ_OK) return rc;
+    if (R.vcycle && v11) {
       if ((rc = adj_vcycle11<T>(c, 0, muP[mi], muP[1 - mi], psi_prev, lam)) != RQ_OK) return rc;
     } else if (R.vcycle) {
       CK(cudaMemsetAsync(A.muf, 0, sizeof(T) * S3, c->st));

@@ -76,8 +76,7 @@ int nm_alloc_levels(rq_ctx* c) {
       cudaMalloc(&c->scale64, sizeof(double) * c->n_atoms) != cudaSuccess ||
       cudaMalloc((void**)&c->rseed, sizeof(unsigned) * 2) != cudaSuccess ||
       cudaMalloc((void**)&c->nbm, (size_t)c->g.S3) != cudaSuccess ||
-      cudaMalloc((void**)&c->acc, sizeof(long long) * kExWords * kNmPD * (size_t)c->n_atoms) != cudaSuccess ||
-      cudaMalloc(&c->mg_res, (size_t)c->g.S3 * es) != cudaSuccess)
+      cudaMalloc((void**)&c->acc, sizeof(long long) * kExWords * kNmPD * (size_t)c->n_atoms) != cudaSuccess)
     return rq_cuda(c, cudaErrorMemoryAllocation, "seed table");
   cudaMemsetAsync(c->rseed, 0, sizeof(unsigned) * 2, c->st);
   cudaMemsetAsync(c->nbm, 0, (size_t)c->g.S3, c->st);  // the face points' masks stay 0
@@ -112,11 +111,12 @@ static int vcycle_level(rq_ctx* c, int l) {
   for (int s = 0; s < c->cfg.mg_pre; ++s)
     for (int color = 0; color < 2; ++color)
       LAUNCH(kc, sizeof(T) * 2.5 * ip, nm_rbgs<T>(P, f, fine, L.g, h2, color, c->st));
-  // the residual, then its full weighting with the coarse correction cleared (its boundary stays zero from
-  // the allocation)
+  // the residual, into the P buffer that this flavour leaves idle (its cycles are in place), then its full
+  // weighting with the coarse correction cleared (whose boundary stays zero from the allocation)
   rq_mg_level& C = c->mg[l + 1];
-  LAUNCH(kc, sizeof(T) * 3.0 * ip, nm_residual<T>(P, f, fine, (T*)c->mg_res, L.g, 1.0 / h2, c->st));
-  LAUNCH(kc, sizeof(T) * (ip + 2.0 * interior(C.g)), nm_restrict<T>((const T*)c->mg_res, (T*)C.f, (T*)C.P, L.g, C.g, c->st));
+  T* res = (T*)c->P[1 - c->cp];
+  LAUNCH(kc, sizeof(T) * 3.0 * ip, nm_residual<T>(P, f, fine, res, L.g, 1.0 / h2, c->st));
+  LAUNCH(kc, sizeof(T) * (ip + 2.0 * interior(C.g)), nm_restrict<T>(res, (T*)C.f, (T*)C.P, L.g, C.g, c->st));
   NmTail t;
   size_t smem = 0;
   if (l + 1 == tail_of<T>(c, t, smem)) {
@@ -340,8 +340,8 @@ int nm_promote(rq_ctx* c) {
   // Every FP64 buffer (fields and multigrid levels) is allocated before anything is freed or
   // swapped: if one allocation fails the context is left exactly as it was (fp32, its captured
   // graphs still valid).
-  void* nb[7] = {};  // U0, U1, P0, P1, K, Kext, the multigrid residual
-  void* old[7] = {c->U[0], c->U[1], c->P[0], c->P[1], c->K, c->Kext, c->mg_res};
+  void* nb[6] = {};  // U0, U1, P0, P1, K, Kext
+  void* old[6] = {c->U[0], c->U[1], c->P[0], c->P[1], c->K, c->Kext};
   std::vector<void*> lv;  // new multigrid buffers, in the order of the (L.P, L.f) walk below
   auto undo = [&]() {
     for (void* p : nb)
@@ -349,7 +349,7 @@ int nm_promote(rq_ctx* c) {
     for (void* p : lv)
       if (p) cudaFree(p);
   };
-  for (int q = 0; q < 7; ++q)
+  for (int q = 0; q < 6; ++q)
     if (old[q] && cudaMalloc(&nb[q], bytes) != cudaSuccess) {
       undo();
       return rq_cuda(c, cudaErrorMemoryAllocation, "promotion to FP64");
@@ -365,7 +365,7 @@ int nm_promote(rq_ctx* c) {
       lv.push_back(q);
     }
   for (int q = 0; q < 6; ++q)
-    if (old[q] && q != 4) {  // K is recomputed below (and the residual holds nothing between cycles)
+    if (old[q] && q != 4) {  // K is recomputed below
       k_nm_widen<<<148 * 4, 256, 0, c->st>>>((const float*)old[q], (double*)nb[q], n);
       const cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) {
@@ -388,7 +388,6 @@ int nm_promote(rq_ctx* c) {
   for (void* p : old)
     if (p) cudaFree(p);
   c->U[0] = nb[0]; c->U[1] = nb[1]; c->P[0] = nb[2]; c->P[1] = nb[3]; c->K = nb[4]; c->Kext = nb[5];
-  c->mg_res = nb[6];
   li = 0;
   for (rq_mg_level& L : c->mg)
     for (void** p : {&L.P, &L.f})

@@ -33,8 +33,7 @@ struct rq_adj {
   long long next_psi = 0;        // ring positions
   int next_p = 0, cur_p = -1;
   // reverse-sweep buffers (allocated with the window)
-  // adjoint of psi (T, S^3): the sweep's, and those of up to four steps whose sums into dE/dK are pending
-  void* lam[5] = {};
+  void* lam[2] = {nullptr, nullptr};  // adjoint of psi (T, S^3)
   void* muP[2] = {nullptr, nullptr};  // adjoint of the fine P (T, S^3; ping-pong through smoothing)
   void* muf = nullptr;                // adjoint of the fine right-hand side (T, S^3)
   double* gK = nullptr;               // dE/dK accumulated (S^3 doubles); dE/dv for the external potential
@@ -92,16 +91,13 @@ struct rq_ctx {
 
   // new flavour multigrid hierarchy (level 0 = fine)
   std::vector<rq_mg_level> mg;
-  void* mg_res = nullptr;  // new flavour: the residual of the level being restricted (T, S^3)
   long long* acc = nullptr;  // new flavour: the accumulators of the per-domain sums (exact_sum.h), kNmPD per domain
 
   // atoms on the device
   float* atoms5 = nullptr;    // [i,j,k,Z,rc] f32 (cloud/solver.py:378-382)
   float* scratch_atoms5 = nullptr;  // per-call atom table for force variants
   float *sic = nullptr, *sic2 = nullptr;  // molecule.js flavour with SIC: self-potential ping-pong
-  // molecule.js direct path: the persistent P_m of every domain, then as many fields for the sweeps to alternate with
-  // (2 n_atoms x slot())
-  float* pdirect = nullptr;
+  float* pdirect = nullptr;   // molecule.js direct path: the persistent P_m of every domain (n_atoms x slot())
   // molecule.js LOBPCG frames: HX, W, HW, P, HP (5 x slot()) and, per domain, the inner-product partial
   // sums of each workgroup (256 x 12), the count of finished workgroups and the scalars (lambda, Ritz coefficients)
   float* lob = nullptr;

@@ -30,7 +30,14 @@ struct AtomBins {
 // host: fill start/idx/far (sizes nb^3+1, n, n+1) and zmax for atoms5 (n x 5, grid units)
 void build_atom_bins(const float* atoms5, int n, int nb, int bin, std::vector<int>& start, std::vector<int>& idx,
                      std::vector<int>& far, float& zmax);
-// the label step with the argmax over atoms found through the bins (same result as launch_labels_sp)
+// cells that the label step lists at a time: three quarters of the grid's, at most 2^31 (32-bit offsets); a multiple
+// of 4.  Only labels in disorder have more candidates, and take a second pass.
+inline long long sp_list_cells(const Geo& g) {
+  const long long n = (g.S3 / 4 + 1) * 3;
+  return (n < (1LL << 31) ? n + 3 : 1LL << 31) & ~3LL;
+}
+// the label step with the argmax over atoms found through the bins (same result as launch_labels_sp); list:
+// sp_list_cells(g) words
 cudaError_t launch_labels_binned_sp(const int* labIn, int* labOut, const unsigned char* mask, unsigned* list,
                                     unsigned* count, const float* atoms5, int nAtoms, AtomBins bins, const Geo& g,
                                     float h, float h2, cudaStream_t st);
@@ -77,11 +84,14 @@ cudaError_t launch_mj_jacobi(const float* Pin, float* Pout, const float* U, cons
 cudaError_t launch_mj_vcycle(float* P, const float* U, float* rho, float* resid, float* Ec0, float* Ec1, float* fc,
                              const Geo& g, const Geo& gc, float h2, float inv_h2, float two_pi, cudaStream_t st);
 // the direct per-electron Poisson of small systems (molecule.js:2833-2858, :614-671): P_m init and one step's
-// solve for the n domains m (slot m of P persistent, of P2 scratch)
+// solve for the n domains m (slot m of P, persistent), kMjDoms of them per launch with a scratch field each
+// whose faces are 0
+constexpr int kMjDoms = 4;
 cudaError_t launch_mj_direct_init(const MjAtom* atoms, int nAt, int m, float* Pm, float* Pother, const Geo& g, float h,
                                   float h2, cudaStream_t st);
-cudaError_t launch_mj_direct(const float* U, const int* label, float* Pother, const int* m, int n, float* P, float* P2,
-                             long long slot, const Geo& g, float h2, float two_pi, cudaStream_t st);
+cudaError_t launch_mj_direct(const float* U, const int* label, float* Pother, const int* m, int n, float* P,
+                             long long slot, float* const (&scratch)[kMjDoms], const Geo& g, float h2, float two_pi,
+                             cudaStream_t st);
 // the self-interaction correction of one domain m (molecule.js:3018-3075); rho, sic, sic2, resid,
 // Ec0, Ec1 and fc are scratch
 cudaError_t launch_mj_sic_domain(const float* U, const int* label, float* Pother, int m, float frac, float* rho,

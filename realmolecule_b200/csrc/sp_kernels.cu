@@ -352,9 +352,9 @@ cudaError_t launch_labels_binned_sp(const int* labIn, int* labOut, const unsigne
                                     unsigned* count, const float* atoms5, int nAtoms, AtomBins bins, const Geo& g,
                                     float h, float h2, cudaStream_t st) {
   if (g.NN < 2) return cudaSuccess;
-  constexpr long long kChunk = 1LL << 31;  // cells listed at a time (32-bit offsets)
-  for (long long base = 0; base < g.S3; base += kChunk) {
-    const long long end = std::min(g.S3, base + kChunk);
+  const long long chunk = sp_list_cells(g);
+  for (long long base = 0; base < g.S3; base += chunk) {
+    const long long end = std::min(g.S3, base + chunk);
     cudaError_t e = cudaMemsetAsync(count, 0, sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
     k_label_candidates<<<(unsigned)((end - base + 1023) / 1024), 256, 0, st>>>(labIn, labOut, mask, g.S3, base, end, list,
