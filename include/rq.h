@@ -110,9 +110,9 @@ typedef struct rq_config {
                                persistent cooperative launch (blocks take chunks of (instance, tile) items from
                                one queue; an item waits, bounded, only for its instance's previous phase).
                                rq_batch_autotune times both and keeps the faster. */
-  int32_t batch_tile;       /* rq_batch_*: march tile of the update, readout and level-set work lists, as
-                               log2(points along k) | (planes per thread << 8), 256 threads per tile; 0 = 16 x 16
-                               x 16 (4 | 16 << 8).  rq_batch_autotune picks it. */
+  int32_t batch_tile;       /* rq_batch_*: march tile of the readout and level-set work lists, and of the persistent
+                               launch's update, as log2(points along k) | (planes per thread << 8), 256 threads
+                               per tile; 0 = 16 x 16 x 16 (4 | 16 << 8).  rq_batch_autotune picks it. */
 } rq_config;
 
 /* One entry of the reference atom list: a nucleus and/or one electron domain. */
@@ -347,7 +347,9 @@ RQ_API int rq_batch_set_wait(rq_batch* b, int64_t limit_ns, int32_t extra_arriva
  * correction P as it was.
  *   1. March tile x launch form: each candidate (tiles 16 x 16 and 32 x 8 points with 8, 16 or 32
  *      planes per thread; per-kernel graph or persistent launch) runs one schedule period to capture
- *      it and one timed by CUDA events; the fastest per step is kept.
+ *      it and one timed by CUDA events; the fastest per step is kept.  With frozen labels the per-kernel
+ *      steps do not depend on the tile: they are timed once, and where they win a tile of these that the
+ *      batch came with stays.
  *   2. Smoother sweeps (mg_pre, mg_post, mg_coarse_sweeps): from P = 0 each candidate runs 3 V-cycles
  *      on the batch's current psi (rho: fine-grid residual reduction per cycle); the cheapest cycle
  *      whose rho is within 5 % of V(1,1)'s is kept (a warm-started cycle every poisson_interval steps

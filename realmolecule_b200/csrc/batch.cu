@@ -1651,15 +1651,27 @@ extern "C" int rq_batch_autotune(rq_batch* b, rq_tune_report* out) {
   BCK(cudaEventCreate(&e1));
   auto cleanup = [&]() { cudaEventDestroy(e0); cudaEventDestroy(e1); };
   int rc = RQ_OK;
-  // 1. march tile x launch form, timed per step over one captured period
+  // 1. march tile x launch form, timed per step over one captured period.  The per-kernel launches' steps take the
+  // tile in the level-set pass alone: with frozen labels one measurement stands for all tiles, and the tile
+  // that the batch came with is kept (picked from six readings of the same launches it would be chance).
   const NmTile keep = b->tile;
   const int keep_persistent = b->cfg.batch_persistent;
-  double best = 1e300;
+  double best = 1e300, one_ms = -1.0;
   int nt = 0;
   for (int lgk : {4, 5})
     for (int march : {8, 16, 32})
       for (int pers : {0, 1}) {
         if (pers && b->cfg.fp32_rounding == 1) continue;  // that schedule keeps the per-kernel launches
+        const bool tileless = !pers && b->cfg.label_until > 0 && b->steps_done >= b->cfg.label_until;
+        if (tileless && one_ms >= 0.0) {
+          out->tile[nt] = lgk | (march << 8);
+          out->persistent[nt] = 0;
+          out->ms_per_step[nt] = one_ms;
+          if (out->persistent[out->best_tile] == 0 && lgk == keep.lgk && march == keep.march && best == one_ms)
+            out->best_tile = nt;
+          ++nt;
+          continue;
+        }
         if ((rc = b_retile(b, NmTile{lgk, march})) != RQ_OK) break;
         b->cfg.batch_persistent = pers;
         b_drop_graphs(b);
@@ -1679,6 +1691,7 @@ extern "C" int rq_batch_autotune(rq_batch* b, rq_tune_report* out) {
         out->tile[nt] = lgk | (march << 8);
         out->persistent[nt] = pers;
         out->ms_per_step[nt] = ms / period;
+        if (tileless) one_ms = out->ms_per_step[nt];
         if (out->ms_per_step[nt] < best) { best = out->ms_per_step[nt]; out->best_tile = nt; }
         ++nt;
       }
