@@ -693,7 +693,7 @@ static int alloc_fields(rq_batch* b, BInst& I, size_t es) {
   }
   BALLOC(I.K, S3 * es);
   for (int l = 0; l < I.nlev; ++l) {
-    const size_t s3 = (size_t)I.lg[l].S3;
+    const size_t s3 = (size_t)I.lg[l].S3 + kVecPad;
     I.lP[l] = I.lf[l] = I.lr[l] = nullptr;
     if (l > 0) {
       BALLOC(I.lP[l], s3 * es);

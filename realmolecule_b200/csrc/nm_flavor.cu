@@ -62,7 +62,7 @@ int nm_alloc_levels(rq_ctx* c) {
     rq_mg_level& L = c->mg[l];
     L.g = make_geo(nn + 1);
     L.h = h;
-    const size_t n = (size_t)L.g.S3 * es;
+    const size_t n = ((size_t)L.g.S3 + kVecPad) * es;
     if (l > 0) {
       if (cudaMalloc(&L.P, n) != cudaSuccess || cudaMalloc(&L.f, n) != cudaSuccess)
         return rq_cuda(c, cudaErrorMemoryAllocation, "multigrid levels");

@@ -48,6 +48,7 @@ struct VGroup {
   bool own;  // this thread's to store
 };
 constexpr int kVOwn = 240;  // groups owned by a block of 256 threads
+constexpr int kVecPad = 4;  // elements that a field of 3^3 needs behind it (from 5^3 on loads stay inside)
 
 // groups per plane at most (any alignment of the plane)
 template <typename T>
@@ -70,7 +71,7 @@ inline int vplanes(const Geo& g, bool sums) {
 
 // The thread's group of plane i.  The owned groups run from the one that holds (i, 1, 1) to the one that
 // holds (i, NN - 1, NN - 1); with one more on either side their +-S and +-S^2 shifts stay inside the
-// array (S >= 5).
+// array (S >= 5; of 3^3 points they reach one element behind it, kVecPad).
 template <typename T>
 __device__ __forceinline__ VGroup vgroup(const Geo& g, int i, int blk) {
   constexpr int W = Vec<T>::W;
