@@ -27,6 +27,7 @@
 
 #include "../../include/rq.h"
 #include "rq_internal.cuh"
+#include "vec_stencil.cuh"
 
 namespace rq {
 
@@ -55,16 +56,6 @@ template <> struct AtTile<16, float> { static constexpr int R = 19, PS = 342; };
 template <> struct AtTile<8, float> { static constexpr int R = 10, PS = 130; };
 template <> struct AtTile<16, double> { static constexpr int R = 18, PS = 324; };
 template <> struct AtTile<8, double> { static constexpr int R = 10, PS = 105; };
-
-// x / 6 in f64, correctly rounded, by the two-constant product of Brisebarre, Muller and Raina
-// ("Accelerating correctly rounded floating-point division when the divisor is known in advance",
-// 2004): zh + zl is 1/6 to 106 bits and x zh + x zl needs one rounding of a value whose error is far
-// below the distance of x / 6 from any midpoint (at least 1/6 ulp).  It replaces a division in the
-// wavefront's dependent chain.
-__device__ __forceinline__ double at_sixth(double x) {
-  constexpr double zh = 0x1.5555555555555p-3, zl = 0x1.5555555555555p-57;
-  return __fma_rn(x, zh, __dmul_rn(x, zl));
-}
 
 struct AtBlock {
   int i0, j0, k0;  // first interior cell
@@ -370,7 +361,8 @@ __global__ void __launch_bounds__(B * B) k_at_gs(float* __restrict__ P, const fl
       const double f = __dmul_rn(h2, (double)r[lk]);
       const double s6 = __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(sP[id + L::PS], sP[id - L::PS]), sP[id + L::R]),
                                                       sP[id - L::R]), sP[id + 1]), pk);
-      pk = (double)(float)at_sixth(__dadd_rn(s6, f));
+      // f32 values and h^2 times one: 0, or far above 2^-900
+      pk = (double)(float)sixth_in_range(__dadd_rn(s6, f));
       sP[id] = pk;
       ++id;
     }

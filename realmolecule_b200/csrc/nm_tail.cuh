@@ -2,7 +2,7 @@
 //
 // Below ~16 intervals a level is a few thousand points: its six kernels (eight transposed) are launches of
 // 2-5 us whose work is a fraction of that, and the coarsest solve waits for all of them.  One block of 1024
-// threads runs every level from the first that fits through the coarsest and back in shared memory, a
+// threads runs every level of at most 16 intervals through the coarsest and back in shared memory, a
 // barrier where a launch was.  Half a warp takes a row.  Arithmetic and roundings are those of the kernels
 // it stands for (nm_vrbgs_body, nm_vresidual_body, nm_restrict_tile_body, nm_prolong_cells_body, nm_coarsest_body; k_adj_half,
 // k_adj_other, k_adj_prolong, k_adj_restrict, k_adj_res, k_adj_muf, k_adj_coarsest), bit for bit.
@@ -12,7 +12,8 @@
 
 namespace rq {
 
-constexpr int kTailLevels = 6;  // at most
+constexpr int kTailNN = 16;     // intervals of the first level at most
+constexpr int kTailLevels = 5;  // 16, 8, 4, 2, 1
 constexpr int kTailThreads = 1024;
 struct NmTail {
   int n;                   // levels, the coarsest last
@@ -23,21 +24,19 @@ struct NmTail {
 };
 
 // f(id, i, j, k) for every interior point (color < 0) or those with (i + j + k) % 2 == color of a level of at
-// most 17 points a side; half a warp takes a row (or 16 of its points).  Small code throughout: a pass runs
-// only a few iterations and one SM fetches every instruction once (unrolled by three the
-// the two kernels took 28 and 65 us at 16 and 24 intervals).
+// most 16 intervals; half a warp takes a row.  Small code throughout: a pass runs only a few iterations and one
+// SM fetches every instruction once (with the loop unrolled by three the cycle's kernel took 28 us at 16 intervals).
 template <class F>
 __device__ __forceinline__ void tail_map(int NN, int color, F&& f) {
   const int n = NN - 1, S = NN + 1;
   const int hw = (int)threadIdx.x >> 4, lane = (int)threadIdx.x & 15;
-  const int two = color < 0 && n > 16 ? 1 : 0;  // two chunks of 16 points per row
-  const int total = (n * n) << two;
+  const int total = n * n;
   const unsigned inv = 65536u / (unsigned)n + 1u;  // row / n = (row inv) >> 16 for row < 65536 / n
 #pragma unroll 1
-  for (int m = hw; m < total; m += kTailThreads / 16) {
-    const int row = m >> two, i0 = (int)(((unsigned)row * inv) >> 16);
+  for (int row = hw; row < total; row += kTailThreads / 16) {
+    const int i0 = (int)(((unsigned)row * inv) >> 16);
     const int i = 1 + i0, j = 1 + row - i0 * n;
-    const int k = color < 0 ? 1 + lane + 16 * (m & two) : 1 + ((i + j + 1 + color) & 1) + 2 * lane;
+    const int k = color < 0 ? 1 + lane : 1 + ((i + j + 1 + color) & 1) + 2 * lane;
     if (k < NN) f((i * S + j) * S + k, i, j, k);
   }
 }
@@ -56,8 +55,8 @@ __device__ __noinline__ void tail_smooth(T* P, const T* f, int NN, T h2) {
   }
 }
 
-// The coarsest sweeps of a level whose colours hold at most one point per thread: phase(color, id) for each
-// of `phases` half sweeps of alternating colour, first colour `first`.  Only the warps that hold points take
+// The coarsest sweeps (of a level of at most 8 intervals, whose colours hold fewer points than the block has
+// threads): phase(color, id) for each of `phases` half sweeps of alternating colour, first colour `first`.  Only the warps that hold points take
 // part, and a barrier of their own (number 1) separates the phases; the others wait at the block's.
 template <class F>
 __device__ __forceinline__ void tail_phases(int NN, int phases, int first, F&& phase) {
@@ -79,7 +78,7 @@ __device__ __forceinline__ void tail_phases(int NN, int phases, int first, F&& p
   }
   __syncthreads();
 }
-__host__ __device__ inline bool tail_one_each(int NN) { return (NN - 1) * (NN - 1) * (NN / 2) <= kTailThreads; }
+static_assert((kTailNN / 2 - 1) * (kTailNN / 2 - 1) * (kTailNN / 4) <= kTailThreads, "a point per thread and colour");
 
 // src (global) into a, zeros into b and c; four loads at a time
 template <typename T>
@@ -154,13 +153,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_nm_tail(const NmTail t, con
                                                       sP[id - S]), sP[id + 1]), sP[id - 1]);
       return sixth(__dadd_rn(sum, __dmul_rn(h2, sf[id])));
     };
-    if (tail_one_each(NN))
-      tail_phases(NN, 2 * t.sweeps, 0, [&](int, int id) { sP[id] = value(id); });
-    else
-      for (int s = 0; s < 2 * t.sweeps; ++s) {
-        tail_map(NN, s & 1, [&](int id, int, int, int) { sP[id] = value(id); });
-        __syncthreads();
-      }
+    tail_phases(NN, 2 * t.sweeps, 0, [&](int, int id) { sP[id] = value(id); });
   }
   for (int l = last - 1; l >= 0; --l) {
     const int NN = t.NN[l], Sc = t.NN[l + 1] + 1;
@@ -261,13 +254,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_adj_tail(const NmTail t, co
       }
       return own + x;
     };
-    if (tail_one_each(NN))
-      tail_phases(NN, 2 * t.sweeps, 0, [&](int s, int id) { sP[id] = value(s, id); });
-    else
-      for (int s = 0; s < 2 * t.sweeps; ++s) {
-        tail_map(NN, s & 1, [&](int id, int, int, int) { sP[id] = value(s, id); });
-        __syncthreads();
-      }
+    tail_phases(NN, 2 * t.sweeps, 0, [&](int s, int id) { sP[id] = value(s, id); });
     tail_map(NN, 0, [&](int id, int, int, int) { sf[id] = fma(c6, sP[id], sf[id]); });
     __syncthreads();
   }
@@ -307,33 +294,28 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_adj_tail(const NmTail t, co
   }
 }
 
-// The tail of a hierarchy of `levels` levels (NN and spacing of each): the first level, at least 1, from
-// which all arrays fit a block's shared memory; t.n = 0 if fewer than two levels do.  Returns that level.
-// Levels above 16 intervals stay kernels: one SM takes longer over them than the launches cost (at 24 intervals
-// 48 us for the tail against 17 us from 16).
+// The tail of a hierarchy of `levels` levels (NN and spacing of each): from the first level, at least 1, of at
+// most 16 intervals, or none (t.n = 0) if fewer than two levels are that small.  Returns that level, or
+// `levels`.  Levels above 16 intervals stay kernels: one SM takes longer over them than the launches cost (at 24
+// intervals 48 us for the tail against 17 us from 16).
 template <typename T, class GeoAt, class HAt>
 inline int nm_tail_plan(int levels, GeoAt geo, HAt h, int sweeps, NmTail& t, size_t& smem) {
-  constexpr size_t kMax = 220 * 1024;
   t.n = 0;
   t.sweeps = sweeps;
-  for (int first = 1; first + 1 < levels; ++first) {
-    if (levels - first > kTailLevels || geo(first).NN > 16) continue;
-    size_t off = 0;
-    t.n = levels - first;
-    for (int l = first; l < levels; ++l) {
-      const Geo g = geo(l);
-      t.NN[l - first] = g.NN;
-      t.h2[l - first] = h(l) * h(l);
-      t.off[l - first] = (int)off;
-      off += l == levels - 1 ? 2 * sizeof(double) * (size_t)g.S3 : (3 * sizeof(T) * (size_t)g.S3 + 15) / 16 * 16;
-    }
-    if (off <= kMax) {
-      smem = off;
-      return first;
-    }
+  int first = 1;
+  while (first < levels && geo(first).NN > kTailNN) ++first;
+  if (first + 1 >= levels) return levels;
+  size_t off = 0;
+  t.n = levels - first;
+  for (int l = first; l < levels; ++l) {
+    const Geo g = geo(l);
+    t.NN[l - first] = g.NN;
+    t.h2[l - first] = h(l) * h(l);
+    t.off[l - first] = (int)off;
+    off += l == levels - 1 ? 2 * sizeof(double) * (size_t)g.S3 : (3 * sizeof(T) * (size_t)g.S3 + 15) / 16 * 16;
   }
-  t.n = 0;
-  return levels;
+  smem = off;  // at most 3 x 8 (17^3 + 9^3 + 5^3 + 3^3) bytes, 136 KB
+  return first;
 }
 
 }  // namespace rq

@@ -205,11 +205,17 @@ __device__ __forceinline__ float sixth(float x) {
   if (a >= 0x1p-100f && a <= 0x1p126f) return __fmaf_rn(x, zh, __fmul_rn(x, zl));
   return x == 0.0f ? x : F_DIV(x, 6.0f);
 }
-__device__ __forceinline__ double sixth(double x) {
+// For f64: x zh + x zl needs one rounding of a value whose error is far below the distance of x / 6 from any
+// midpoint (at least 1/6 ulp), as long as x zl is a normal number; 0, infinities and NaN come out as the
+// division's.
+__device__ __forceinline__ double sixth_in_range(double x) {
   constexpr double zh = 0x1.5555555555555p-3, zl = 0x1.5555555555555p-57;
+  return __fma_rn(x, zh, __dmul_rn(x, zl));
+}
+__device__ __forceinline__ double sixth(double x) {
   // |x| in [2^-900, 2^1000), by the exponent field: FP64 comparisons are as long a wait as the product
   const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
-  if (ex - (1023u - 900u) < 1900u) return __fma_rn(x, zh, __dmul_rn(x, zl));
+  if (ex - (1023u - 900u) < 1900u) return sixth_in_range(x);
   return __ddiv_rn(x, 6.0);
 }
 
