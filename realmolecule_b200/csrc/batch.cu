@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(256) kb_init(const BInst* __restrict__ ins, co
 
 // force gathers: blocks of points (item: tile bx, by, bz), then one nucleus each (item: entry bx, part by)
 template <typename T>
-__global__ void __launch_bounds__(256) kb_gather(const BInst* __restrict__ ins, const BItem* __restrict__ items, int cu,
+__global__ void __launch_bounds__(256, 3) kb_gather(const BInst* __restrict__ ins, const BItem* __restrict__ items, int cu,
                                                  double sigma, double* __restrict__ F) {
   __shared__ GatherSmem sm;
   const BItem it = items[blockIdx.x];

@@ -972,9 +972,11 @@ __device__ __forceinline__ void nm_gather_core_body(const T* __restrict__ U, con
   double sx = 0, sy = 0, sz = 0;
   if (part == 0 && threadIdx.x == 0) sx = (X - X) + (Y - Y) + (Z - Z);  // NaN for a position that is not finite
   if (n[0] > 0 && n[1] > 0 && n[2] > 0) {
-    const int tot = n[0] * n[1] * n[2];
-    for (int q = part * 256 + (int)threadIdx.x; q < tot; q += 256 * parts) {
-      const int k = lo[2] + q % n[2], j = lo[1] + (q / n[2]) % n[1], i = lo[0] + q / (n[2] * n[1]);
+    // unsigned: a grid of more than 2^32 points does not fit the memory, one of more than 2^31 does
+    const unsigned nk = (unsigned)n[2], nj = (unsigned)n[1], tot = (unsigned)n[0] * nj * nk;
+    for (unsigned q = (unsigned)part * 256 + threadIdx.x; q < tot; q += 256 * parts) {
+      const unsigned row = q / nk;
+      const int k = lo[2] + (int)(q - row * nk), j = lo[1] + (int)(row % nj), i = lo[0] + (int)(row / nj);
       const double dx = __dsub_rn(nm_grid_coord(i, h), X), dy = __dsub_rn(nm_grid_coord(j, h), Y),
                    dz = __dsub_rn(nm_grid_coord(k, h), Z);
       const double r2 = nm_pair_r2(dx, dy, dz);
@@ -1012,12 +1014,23 @@ __device__ __forceinline__ void nm_gather_all_body(const T* __restrict__ U, cons
                                                    GatherSmem& sm) {
   const double scale = gw ? 1.0 : -(h * h * h);
   const int i0 = 1 + bz * kGaI, j0 = 1 + by * kGaJ, k0 = 1 + bx * kGaK;
-  nm_gather_points_body<T>(U, gw, g, h, nm_point_r2(sigma), i0, min(i0 + kGaI, g.NN), j0, min(j0 + kGaJ, g.NN), k0,
-                           min(k0 + kGaK, g.NN), nAt,
+  const int i1 = min(i0 + kGaI, g.NN), j1 = min(j0 + kGaJ, g.NN), k1 = min(k0 + kGaK, g.NN);
+  const double rp2 = nm_point_r2(sigma);
+  nm_gather_points_body<T>(U, gw, g, h, rp2, i0, i1, j0, j1, k0, k1, nAt,
                            [&](int m, double& X, double& Y, double& Z, double& f) -> int {
                              const double q = at[m * 4 + 3];
                              X = at[m * 4]; Y = at[m * 4 + 1]; Z = at[m * 4 + 2];
                              f = scale * q;
+                             // a nucleus whose range holds all points of the block has no pair here (64^3, 400
+                             // nuclei, sigma = 10 h: 1.70 ms with these pairs formed and dropped, 1.19 without);
+                             // no range is that wide unless sigma is
+                             if (rp2 > 0.25 * h * h * (kGaK * kGaK)) {
+                               auto far = [&](double r, int a, int b) {
+                                 const double u = nm_grid_coord(a, h) - r, v = nm_grid_coord(b - 1, h) - r;
+                                 return fmax(u * u, v * v);
+                               };
+                               if (far(X, i0, i1) + far(Y, j0, j1) + far(Z, k0, k1) < rp2 * (1.0 - 1e-12)) return -1;
+                             }
                              return q > 0.0 ? m : -1;
                            },
                            F, sm);

@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(256) k_nm_evolve(const int* labIn, int* labOut
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_nm_gather(const T* U, const double* at, int nAt, Geo g, double h, double sigma,
+__global__ void __launch_bounds__(256, 3) k_nm_gather(const T* U, const double* at, int nAt, Geo g, double h, double sigma,
                                                    double* F, const double* gw) {
   __shared__ GatherSmem sm;
   nm_gather_all_body<T>(U, gw, at, nAt, g, h, sigma, F, blockIdx.x, blockIdx.y, blockIdx.z, sm);
