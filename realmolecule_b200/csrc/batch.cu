@@ -1662,8 +1662,7 @@ extern "C" int rq_batch_autotune(rq_batch* b, rq_tune_report* out) {
     for (int march : {8, 16, 32})
       for (int pers : {0, 1}) {
         if (pers && b->cfg.fp32_rounding == 1) continue;  // that schedule keeps the per-kernel launches
-        const bool tileless = !pers && b->cfg.label_until > 0 && b->steps_done >= b->cfg.label_until;
-        if (tileless && one_ms >= 0.0) {
+        if (!pers && one_ms >= 0.0) {
           out->tile[nt] = lgk | (march << 8);
           out->persistent[nt] = 0;
           out->ms_per_step[nt] = one_ms;
@@ -1681,6 +1680,7 @@ extern "C" int rq_batch_autotune(rq_batch* b, rq_tune_report* out) {
           rc = RQ_OK;
           continue;
         }
+        const bool frozen = b->cfg.label_until > 0 && b->steps_done >= b->cfg.label_until;  // in the timed period
         if (rc == RQ_OK && cudaEventRecord(e0, b->st) != cudaSuccess) rc = RQ_ECUDA;
         if (rc == RQ_OK) rc = rq_batch_step(b, period);
         if (rc == RQ_OK && cudaEventRecord(e1, b->st) != cudaSuccess) rc = RQ_ECUDA;
@@ -1691,7 +1691,7 @@ extern "C" int rq_batch_autotune(rq_batch* b, rq_tune_report* out) {
         out->tile[nt] = lgk | (march << 8);
         out->persistent[nt] = pers;
         out->ms_per_step[nt] = ms / period;
-        if (tileless) one_ms = out->ms_per_step[nt];
+        if (!pers && frozen) one_ms = out->ms_per_step[nt];
         if (out->ms_per_step[nt] < best) { best = out->ms_per_step[nt]; out->best_tile = nt; }
         ++nt;
       }

@@ -7,12 +7,13 @@ from test_gpu_batch import instances
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("steps", [0, 20])  # the labels freeze in the first candidate's untimed period, or before
 @pytest.mark.parametrize("tile", [4 | (32 << 8), 5 | (16 << 8)])
-def test_frozen_labels_keep_the_tile(tile):
+def test_frozen_labels_keep_the_tile(tile, steps):
     from realmolecule_b200.batch import Batch
     b = Batch(instances(), precision="mixed", label_until=1, batch_tile=tile, fp32_rounding=1)  # no persistent form
     b.initialize()
-    b.step(20)
+    b.step(steps)
     rep = b.autotune()
     b.close()
     assert len(rep["tiles"]) == 6 and len({t["ms_per_step"] for t in rep["tiles"]}) == 1
