@@ -30,8 +30,8 @@ struct AtomBins {
 // host: fill start/idx/far (sizes nb^3+1, n, n+1) and zmax for atoms5 (n x 5, grid units)
 void build_atom_bins(const float* atoms5, int n, int nb, int bin, std::vector<int>& start, std::vector<int>& idx,
                      std::vector<int>& far, float& zmax);
-// cells that the label step lists at a time: three quarters of the grid's, at most 2^31 (32-bit offsets); a multiple
-// of 4.  Only labels in disorder have more candidates, and take a second pass.
+// cells that the label step's list holds: three quarters of the grid's, at most 2^31; a multiple of 4.  Only labels
+// in disorder have more candidates.
 inline long long sp_list_cells(const Geo& g) {
   const long long n = (g.S3 / 4 + 1) * 3;
   return (n < (1LL << 31) ? n + 3 : 1LL << 31) & ~3LL;
@@ -160,7 +160,7 @@ template <typename T>
 cudaError_t nm_norms(const T* U, const int* label, const Geo& g, double h3, int nDom, long long* norms, cudaStream_t st);
 template <typename T>
 cudaError_t nm_rbgs(T* P, const T* f, bool fine, const Geo& g, double h2, int color, cudaStream_t st);
-// fc = R (f - A P) (the residual and its full weighting in one pass) and Pc = 0 on the coarse interior
+// r = f - A P on the interior (0 beside it, within a vector); then fc = R r and Pc = 0 on the coarse interior
 template <typename T>
 cudaError_t nm_residual(const T* P, const T* f, bool fine, T* r, const Geo& g, double inv_h2, cudaStream_t st);
 template <typename T>

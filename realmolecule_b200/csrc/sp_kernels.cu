@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(256) k_jacobi_sp(const float* __restrict__ P, 
 // the labels change), the labels themselves are read only where norms accumulate.  The face points of
 // a group are written 0, which is what every buffer holds there.  Traffic: read psi, K, P and the
 // mask byte; write psi', P' = 21 B per point.  Bound: HBM at 300^3 (95 us, 5.9 TB/s, where the scalar
-// march over labels took 165 us), L2 and latency at 128^3 (10.2 us against 14.4 us in the replayed period).
+// march over labels took 165 us), L2 and latency at 128^3 (8.2 us against 12.9 us in the replayed period).
 // ---------------------------------------------------------------------------------------
 template <bool FIRST, bool ACC, int ROW>
 __global__ void __launch_bounds__(256) k_step_sp(const float* __restrict__ U, float* __restrict__ Unew,
@@ -238,21 +238,21 @@ __device__ __forceinline__ float sp_atom_score(const float* __restrict__ atoms5,
 // Two launches: k_label_candidates copies the labels and lists the cells that can flip (read off the
 // same-label mask), k_label_search gives each of them a thread.  In one pass, where a thread marched 16
 // cells and searched where it had to, a warp waited for its slowest lane on every plane: 3.06 ms at 255
-// atoms on 300^3; the period there went from 16.6 to 14.0 ms.
+// atoms on 300^3; the period there went from 16.6 to 14.0 ms.  The list holds `cap` cells.  Labels in disorder
+// can have more candidates: the search then goes through all cells and the mask instead.
+__device__ __forceinline__ bool label_can_flip(unsigned m) { return (m & kNmIn) && __popc(m & 63u) <= 4; }
 __global__ void __launch_bounds__(256) k_label_candidates(const int* __restrict__ labIn, int* __restrict__ labOut,
                                                           const unsigned char* __restrict__ mask, long long S3,
                                                           long long base, long long end, unsigned* __restrict__ list,
-                                                          unsigned* __restrict__ count) {
+                                                          unsigned cap, unsigned* __restrict__ count) {
   const long long a = base + 4 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
   unsigned cand = 0;  // bit e: cell a + e can flip (interior, at most four neighbours of its label)
   if (a + 4 <= S3 && a < end) {
     *reinterpret_cast<int4*>(labOut + a) = __ldg(reinterpret_cast<const int4*>(labIn + a));
     const unsigned m4 = __ldg(reinterpret_cast<const unsigned*>(mask + a));
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const unsigned m = m4 >> (8 * e);
-      if ((m & kNmIn) && __popc(m & 63u) <= 4) cand |= 1u << e;
-    }
+    for (int e = 0; e < 4; ++e)
+      if (label_can_flip(m4 >> (8 * e))) cand |= 1u << e;
   } else if (a < end) {  // the last ids are face points
     for (long long q = a; q < S3; ++q) labOut[q] = labIn[q];
   }
@@ -269,17 +269,24 @@ __global__ void __launch_bounds__(256) k_label_candidates(const int* __restrict_
   at = __shfl_sync(0xffffffffu, at, 31) + pre - n;
 #pragma unroll
   for (int e = 0; e < 4; ++e)
-    if (cand & (1u << e)) list[at++] = (unsigned)(a - base) + e;
+    if (cand & (1u << e)) {
+      if (at < cap) list[at] = (unsigned)(a - base) + e;
+      ++at;
+    }
 }
 
 __global__ void __launch_bounds__(256) k_label_search(const int* __restrict__ labIn, int* __restrict__ labOut,
-                                                      const unsigned* __restrict__ list, const unsigned* __restrict__ count,
-                                                      long long base, const float* __restrict__ atoms5, int nAtoms,
-                                                      AtomBins B, Geo g, float h, float h2) {
+                                                      const unsigned char* __restrict__ mask,
+                                                      const unsigned* __restrict__ list, unsigned cap,
+                                                      const unsigned* __restrict__ count, long long base, long long end,
+                                                      const float* __restrict__ atoms5, int nAtoms, AtomBins B, Geo g,
+                                                      float h, float h2) {
   const double zmax = (double)__ldg(B.zmax);
-  const unsigned n = *count;
+  const bool listed = *count <= cap;
+  const unsigned n = listed ? *count : (unsigned)(end - base);
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    const long long id = base + list[t];
+    const long long id = base + (listed ? list[t] : t);
+    if (!listed && !label_can_flip(mask[id])) continue;
     const int i = (int)(id / g.S2), rem = (int)(id - (long long)i * g.S2), j = rem / g.S, k = rem - j * g.S;
     const int cur = __ldg(labIn + id);
     const float xi = F_MUL((float)i, h), yj = F_MUL((float)j, h), zk = F_MUL((float)k, h);
@@ -352,14 +359,16 @@ cudaError_t launch_labels_binned_sp(const int* labIn, int* labOut, const unsigne
                                     unsigned* count, const float* atoms5, int nAtoms, AtomBins bins, const Geo& g,
                                     float h, float h2, cudaStream_t st) {
   if (g.NN < 2) return cudaSuccess;
-  const long long chunk = sp_list_cells(g);
-  for (long long base = 0; base < g.S3; base += chunk) {
-    const long long end = std::min(g.S3, base + chunk);
+  constexpr long long kChunk = 1LL << 31;  // cells looked at together (32-bit offsets)
+  const unsigned cap = (unsigned)sp_list_cells(g);
+  for (long long base = 0; base < g.S3; base += kChunk) {
+    const long long end = std::min(g.S3, base + kChunk);
     cudaError_t e = cudaMemsetAsync(count, 0, sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
-    k_label_candidates<<<(unsigned)((end - base + 1023) / 1024), 256, 0, st>>>(labIn, labOut, mask, g.S3, base, end, list,
+    k_label_candidates<<<(unsigned)((end - base + 1023) / 1024), 256, 0, st>>>(labIn, labOut, mask, g.S3, base, end, list, cap,
                                                                               count);
-    k_label_search<<<148 * 8, 256, 0, st>>>(labIn, labOut, list, count, base, atoms5, nAtoms, bins, g, h, h2);
+    k_label_search<<<148 * 8, 256, 0, st>>>(labIn, labOut, mask, list, cap, count, base, end, atoms5, nAtoms, bins, g, h,
+                                            h2);
   }
   return cudaGetLastError();
 }
