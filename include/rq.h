@@ -191,8 +191,9 @@ RQ_API void rq_destroy(rq_ctx* ctx);
 /* Binds the context to a CUDA stream (cudaStream_t passed as void*; NULL = the stream the
  * context created for itself).  Pending work on the previous stream is finished first. */
 RQ_API int rq_set_stream(rq_ctx* ctx, void* stream);
-/* Device pointers in info are the live fields; for the new flavour call rq_synchronize first
- * (it materialises a per-domain normalisation that the next update would otherwise apply). */
+/* Device pointers in info are the live fields, to be read (labels are written by rq_upload_state only:
+ * steps keep data derived from them); for the new flavour call rq_synchronize first (it
+ * materialises a per-domain normalisation that the next update would otherwise apply). */
 RQ_API int rq_get_info(const rq_ctx* ctx, rq_info* info);
 RQ_API const char* rq_last_error(const rq_ctx* ctx);
 RQ_API const char* rq_status_string(int status);

@@ -1,6 +1,6 @@
 // vec_stencil.cuh -- 7-point stencil passes on 16-byte vectors of an S^3 field with odd S.
 //
-// The row pitch S = NN + 1 is odd (NN is even in every flavour), so rows start at every alignment and a
+// The row pitch S = NN + 1 is odd (the flavours that come here take even NN), so rows start at every alignment and a
 // scalar pass spends itself on load instructions: 8 per point, each warp load touching 2-4 lines.  Here a
 // thread owns one 16-byte group of consecutive ids (W = 4 floats or 2 doubles) of a plane, whatever rows
 // it straddles, and lane l of a warp owns the l-th of 32 consecutive groups.  A neighbour row or plane
