@@ -129,6 +129,12 @@ def run_reference_arm(a):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import oracle as orc
+    if not os.path.exists(orc.REF_LIB):  # built from the reference's sources, which are not there
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's kernels are not built here (no reference sources)"}),
+              flush=True)
+        return
     # each bench step is one schedule period (100 solver steps) of the same workload
     per = PERIOD
     rate, threads, dt = cpu_reference_rate(cfg, per * a.steps, per * a.warmup)
